@@ -375,8 +375,8 @@ template <int MODE> struct BwdStages { static constexpr int value = MODE == 1 ? 
 struct BwdShared {
   uint64_t bar_x, bar_y[kBwdMaxStages], bar_yfree[kBwdMaxStages], bar_s[2], bar_sfree[2], bar_p[2],
       bar_acc[2], bar_done;
-  alignas(16) float lse[kBwdMaxStages][64];    // MODE 0: per streamed block, bulk-copied by the producer
-  alignas(16) float delta[kBwdMaxStages][64];
+  float lse[kBwdMaxStages][64];    // MODE 0: per streamed block, written by the producer warp
+  float delta[kBwdMaxStages][64];
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -419,7 +419,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
   if (threadIdx.x == 0) {
     mbar_init(&sh->bar_x, 1);
     for (int i = 0; i < kBwdStages; ++i) {
-      mbar_init(&sh->bar_y[i], 1);
+      mbar_init(&sh->bar_y[i], MODE == 0 ? 2 : 1);   // the tiles, and in MODE 0 the statistics
       mbar_init(&sh->bar_yfree[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -446,9 +446,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
   const uint32_t tA1 = tmem + 256, tA2 = tmem + 256 + D;
 
   if (warp == 8) {
-    // producer: one thread issues every bulk copy.  In MODE 0 the streamed queries' lse/delta
-    // (64 contiguous floats each) ride on the same barrier as the tiles.
-    if (elect_one()) {
+    // Producer.  Lane 0 issues every tile copy.  In MODE 0 the whole warp brings the streamed
+    // queries' lse and delta (64 floats each): two of each per lane, loaded a block ahead so that
+    // their latency passes while the ring is full, whatever the block's alignment in the row and
+    // wherever the sequence ends.  (They used to be bulk copies, which need a 16-byte boundary;
+    // blocks without one, or with the sequence's end in them, went through 128 plain loads of a
+    // single thread, and a head's 2048 keys at an odd slice start took 434 us instead of 36.)
+    const int lane = threadIdx.x & 31;
+    const float* lse_row = MODE == 0 ? p.lse2 + static_cast<long long>(bh) * p.lse_stride : nullptr;
+    const float* delta_row = MODE == 0 ? p.delta + static_cast<long long>(bh) * p.lse_stride : nullptr;
+    float nl[2] = {0.0f, 0.0f}, nd[2] = {0.0f, 0.0f};
+    auto fetch_stats = [&](int y0) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int y = y0 + lane + 32 * k;
+        const bool in = y < p.q_end && TP_CHECK(y >= 0 && y < p.lse_stride, p.err, kErrCheckAttn);
+        nl[k] = in ? __ldcg(lse_row + y) : 0.0f;
+        nd[k] = in ? __ldcg(delta_row + y) : 0.0f;
+      }
+    };
+    if (lane == 0) {
       mbar_expect_tx(&sh->bar_x, 2 * DH * kXSub);
       for (int hh = 0; hh < DH; ++hh) {
         if (MODE == 0) {
@@ -459,26 +476,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
           tma_load_3d(sX2 + hh * kXSub, &tmDO128, &sh->bar_x, hi * D + hh * 64, bi, x0);
         }
       }
-      for (int i = 0; i < n_iter; ++i) {
-        const int st = i % kBwdStages;
-        if (!mbar_wait(&sh->bar_yfree[st], ((i / kBwdStages) & 1) ^ 1, wctx, kErrWaitAttn)) break;
-        uint8_t* y1 = sY + st * kStageBytes;
-        uint8_t* y2 = y1 + DH * kYSub;
-        const int y0 = ystart + i * 64;
-        // a block that runs past q_end takes its lse/delta through guarded plain loads instead
-        const bool bulk_stats = MODE == 0 && y0 + 64 <= p.q_end && (y0 & 3) == 0 &&
-                                (p.lse_stride & 3) == 0 &&
-                                TP_CHECK(y0 >= 0 && y0 + 64 <= p.lse_stride, p.err, kErrCheckAttn);
-        if (MODE == 0 && !bulk_stats) {
-          const long long base = static_cast<long long>(bh) * p.lse_stride;
-          for (int k = 0; k < 64; ++k) {
-            const bool in = y0 + k < p.q_end &&
-                            TP_CHECK(y0 + k >= 0 && y0 + k < p.lse_stride, p.err, kErrCheckAttn);
-            sh->lse[st][k] = in ? __ldcg(p.lse2 + base + y0 + k) : 0.0f;
-            sh->delta[st][k] = in ? __ldcg(p.delta + base + y0 + k) : 0.0f;
-          }
-        }
-        mbar_expect_tx(&sh->bar_y[st], kStageBytes + (bulk_stats ? 512 : 0));
+    }
+    if (MODE == 0 && n_iter > 0) fetch_stats(ystart);
+    for (int i = 0; i < n_iter; ++i) {
+      const int st = i % kBwdStages;
+      int ok = 1;
+      if (lane == 0) ok = mbar_wait(&sh->bar_yfree[st], ((i / kBwdStages) & 1) ^ 1, wctx, kErrWaitAttn);
+      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+      uint8_t* y1 = sY + st * kStageBytes;
+      uint8_t* y2 = y1 + DH * kYSub;
+      const int y0 = ystart + i * 64;
+      if (lane == 0) {
+        mbar_expect_tx(&sh->bar_y[st], kStageBytes);
         for (int hh = 0; hh < DH; ++hh) {
           if (MODE == 0) {
             tma_load_3d(y1 + hh * kYSub, &tmQKV64, &sh->bar_y[st], hh * 64, bh, y0);
@@ -488,11 +497,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
             tma_load_3d(y2 + hh * kYSub, &tmQKV64, &sh->bar_y[st], 2 * D + hh * 64, bh, y0);
           }
         }
-        if (bulk_stats) {
-          const long long off = static_cast<long long>(bh) * p.lse_stride + y0;
-          bulk_load_1d(sh->lse[st], p.lse2 + off, 256, &sh->bar_y[st]);
-          bulk_load_1d(sh->delta[st], p.delta + off, 256, &sh->bar_y[st]);
+      }
+      if (MODE == 0) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          sh->lse[st][lane + 32 * k] = nl[k];
+          sh->delta[st][lane + 32 * k] = nd[k];
         }
+        warp_arrive(&sh->bar_y[st]);
+        if (i + 1 < n_iter) fetch_stats(y0 + 64);
       }
     }
   } else if (warp == 9) {
