@@ -1626,6 +1626,8 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
     p.ag_flags = ag->flags; p.ag_epoch_base = ag->epoch_base; p.ag_epoch = ag->epoch;
     p.ag_rows = ag->rows_per_rank; p.ag_rank = ag->rank;
   }
+  if (!ag && pair)
+    apply_tile_order(p, dram_tile_order(p.num_m_tiles, p.num_n_tiles, BM, BN, K, max_pairs()));
   p.out = out; p.ldo = ldo;
   p.bias = bias; p.residual = residual; p.ldr = ldr;
   p.aux_out = aux_out; p.aux_in = aux_in; p.ld_aux = ld_aux;

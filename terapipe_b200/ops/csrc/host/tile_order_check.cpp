@@ -8,7 +8,7 @@
 
 extern "C" {
 
-// kind: 0 plain, 1 all-gather -> GEMM, 2 GEMM -> reduce-scatter.
+// kind: 0 plain, 1 all-gather -> GEMM, 2 GEMM -> reduce-scatter, 3 ordinary product (DRAM traffic).
 // order_out (8 ints, may be null): the TileOrder fields in declaration order.
 // coords_out (2 * num_tiles ints, may be null): (m_idx, n_idx) of tile 0, 1, ...
 // Returns the number of tiles, or -(1 + tile) for the first tile whose coordinates fall outside
@@ -21,6 +21,7 @@ long long tp_tile_order_walk(int kind, int M, int N, long long K, int tile_rows,
   tp::TileOrder o = tp::plain_tile_order(num_m, num_n);
   if (kind == 1) o = tp::ag_tile_order(num_m, num_n, tile_rows, rank, rows_per_rank, pairs);
   if (kind == 2) o = tp::rs_tile_order(M, N, K, num_m, num_n, tile_rows, rank, rows_per_rank, pairs);
+  if (kind == 3) o = tp::dram_tile_order(num_m, num_n, tile_rows, tile_cols, K, pairs);
   if (order_out) {
     const int f[8] = {o.num_m_tiles, o.num_n_tiles, o.m_major, o.m_first,
                       o.order_split, o.order_group, o.order_first_only, o.order_pipelined};
