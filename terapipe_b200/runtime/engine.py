@@ -31,9 +31,9 @@ GEMM + all-reduce kernel over NVLink peer memory (``tp_comm="fused"``).
 """
 from __future__ import annotations
 
-import os
-
+import gc
 import math
+import os
 from typing import Dict, List, Optional, Sequence
 
 import torch
@@ -1119,15 +1119,16 @@ class StageEngine:
         """Copy this replica's ``[L, B, H]`` input into the stage-0 activation buffer.  Rows are
         regrouped per batch slice (each batch slice owns a contiguous ``[L, b, H]`` block)."""
         assert self.is_first
+        if len(self.batch_slices) == 1 and x.dtype == self.dtype:
+            # straight into place: no second copy on the device
+            self.X[0].view(self.L, self.B, self.H).copy_(x, non_blocking=True)
+            return
         x = x.to(self.device, self.dtype, non_blocking=True)
-        if len(self.batch_slices) == 1:
-            self.X[0].view(self.L, self.B, self.H).copy_(x)
-        else:
-            boff = 0
-            for b in self.batch_slices:
-                dst = self.X[0][self.L * boff:self.L * (boff + b)].view(self.L, b, self.H)
-                dst.copy_(x[:, boff:boff + b])
-                boff += b
+        boff = 0
+        for b in self.batch_slices:
+            dst = self.X[0][self.L * boff:self.L * (boff + b)].view(self.L, b, self.H)
+            dst.copy_(x[:, boff:boff + b])
+            boff += b
 
     def output(self) -> torch.Tensor:
         """The stage output as ``[L, B, H]`` (a copy when several batch slices exist)."""
@@ -1175,9 +1176,21 @@ class StageEngine:
     def _capture(self):
         torch.cuda.synchronize()
         graph = torch.cuda.CUDAGraph()
+        if self._cap_stream is None:
+            self._cap_stream = torch.cuda.Stream()
+        # (torch.cuda.graph() would also collect garbage and give torch's cached memory back to
+        # the driver first, which takes far longer than the capture: tens of milliseconds, and
+        # hundreds when another engine has just been released.)  Nothing may be collected while
+        # the capture runs, though: the destructor of an old graph is not a legal call then.
+        collecting = gc.isenabled()
+        gc.disable()
         try:
-            with torch.cuda.graph(graph):
-                self._iteration()
+            with torch.cuda.stream(self._cap_stream):
+                graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    self._iteration()
+                finally:
+                    graph.capture_end()
         except (RuntimeError, KernelError) as e:
             # The whole step could not be captured (seen with a 48-layer stage of GPT3-44B width:
             # a launch inside the capture failed although the same step had just run eagerly).
@@ -1192,6 +1205,9 @@ class StageEngine:
             if self._plan is None and self._seg_graphs is None:
                 self._seg_graphs = {}
             return
+        finally:
+            if collecting:
+                gc.enable()
         self._graph = graph
 
     def check_status(self):
