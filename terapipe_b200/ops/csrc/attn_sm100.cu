@@ -5,9 +5,9 @@
 // from the stage's full-length projection buffer
 //     qkv[L][b][h][3][D]          (position, batch, local head, {q,k,v}, head dim)
 // through 3-D tensor maps, so "appending to the KV cache" is just the QKV GEMM writing its
-// rows; no gather/scatter kernels exist.  Scores never reach memory: S lives in TMEM, P is
-// handed to the second MMA through shared memory, the running output stays in TMEM and is
-// rescaled lazily (only when the row maximum grows by more than 2^8).
+// rows; no gather/scatter kernels exist.  Scores never reach memory: S lives in TMEM, P (and dS)
+// take its place there as 16-bit values and are the next MMA's A operand, the running output
+// stays in TMEM and is rescaled lazily (only when the row maximum grows by more than 2^8).
 //
 // Backward recomputes P from Q, K and the saved log-sum-exp (base 2); see the comment above
 // attn_bwd_kernel.  No gradient accumulator crosses slices: the backward pass walks the
@@ -15,8 +15,8 @@
 // later slices already sit in a full-length buffer, and dK/dV of slice j's keys are computed
 // in one go by streaming over those later queries.
 //
-// Forward CTA = 5 warps: warps 0..3 own one TMEM lane quarter each (one row per thread: softmax
-// needs no shuffles), warp 4 elects one thread that issues all TMA copies and MMAs.
+// Every kernel has two groups of 4 softmax warps (one TMEM lane quarter each, one row per thread,
+// so row reductions need no shuffles), a warp for the TMA copies and one or two for the MMAs.
 #include <math.h>
 #include <string.h>
 
@@ -25,7 +25,7 @@
 
 namespace tp {
 
-constexpr int kAttnThreads = 160;
+constexpr int kAttnThreads = 352;   // forward: 8 softmax warps, TMA, two MMA warps
 
 struct AttnParams {
   int t, c, b, h;
@@ -52,105 +52,127 @@ __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
-// Write one row (64 values) of a [128 x 64] 16-bit operand tile in the 128B-swizzled
-// K-major layout expected by the UMMA descriptors.
-template <typename T>
-__device__ __forceinline__ void store_row64(uint8_t* tile, int row, const float* v) {
-#pragma unroll
-  for (int ch = 0; ch < 8; ++ch) {
-    uint4 u;
-    u.x = Elem<T>::pack2(v[ch * 8 + 0], v[ch * 8 + 1]);
-    u.y = Elem<T>::pack2(v[ch * 8 + 2], v[ch * 8 + 3]);
-    u.z = Elem<T>::pack2(v[ch * 8 + 4], v[ch * 8 + 5]);
-    u.w = Elem<T>::pack2(v[ch * 8 + 6], v[ch * 8 + 7]);
-    *reinterpret_cast<uint4*>(tile + row * 128 + ((ch ^ (row & 7)) << 4)) = u;
-  }
+// A descriptor's low word is the address / 16 and the leading offset / 16; the high word is the same
+// for every tile here (umma_desc_sw128).
+constexpr uint32_t kDescHi = (1024 >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_k(uint32_t addr) { return (addr >> 4) | (1u << 16); }   // K-major
+__device__ __forceinline__ uint32_t desc_n(uint32_t addr, uint32_t chunk) {                       // N-major
+  return (addr >> 4) | ((chunk >> 4) << 16);
+}
+__device__ __forceinline__ uint64_t desc64(uint32_t lo) {
+  return (static_cast<uint64_t>(kDescHi) << 32) | lo;
 }
 
-// D[tmem] (+)= A * B^T with both operands K-major, K = DH*64 split in DH sub-tiles.
+// D[tmem] = A * B^T with both operands K-major, K = DH*64 split in DH sub-tiles.
 template <int DH>
-__device__ __forceinline__ void mma_kk(uint32_t tmem_d, uint32_t a_base, uint32_t a_sub,
-                                       uint32_t b_base, uint32_t b_sub, uint32_t idesc) {
+__device__ __forceinline__ void mma_kk(uint32_t tmem_d, uint32_t a, uint32_t a_sub, uint32_t b,
+                                       uint32_t b_sub, uint32_t idesc) {
 #pragma unroll
   for (int hh = 0; hh < DH; ++hh)
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      umma_f16(tmem_d, umma_desc_sw128(a_base + hh * a_sub + k * 32, 16, 1024),
-               umma_desc_sw128(b_base + hh * b_sub + k * 32, 16, 1024), idesc,
+      umma_f16(tmem_d, desc64(a + hh * (a_sub >> 4) + k * 2), desc64(b + hh * (b_sub >> 4) + k * 2), idesc,
                (hh | k) != 0 ? 1u : 0u);
 }
 
-// D[tmem] (+)= A[128 x 64, K-major] * B[64 (k) x N, N-major tile with 64-wide chunks b_sub apart]
-__device__ __forceinline__ void mma_kn(uint32_t tmem_d, uint32_t a_base, uint32_t b_base,
-                                       uint32_t b_sub, uint32_t idesc, bool accumulate) {
+// D[tmem] (+)= A * B: A = [128 x 64] 16-bit values in TMEM (two per column), B = [64 (k) x N] N-major.
+__device__ __forceinline__ void mma_tn(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, uint32_t idesc,
+                                       bool accumulate) {
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    umma_f16(tmem_d, umma_desc_sw128(a_base + k * 32, 16, 1024),
-             umma_desc_sw128(b_base + k * 2048, b_sub, 1024), idesc,
-             (accumulate || k != 0) ? 1u : 0u);
+    umma_f16_ta(tmem_d, tmem_a + k * 8, desc64(b + k * 128), idesc, (accumulate || k != 0) ? 1u : 0u);
 }
 
-struct AttnShared {
-  uint64_t bars[20];
+// Which tile of which head a CTA takes.  CTAs start in the order of their index.  Heads go in
+// chunks of kHeadChunk whose operands stay in L2 together (2 MB a head at 2048 x 128), and inside a
+// chunk the tiles with the longest streams come first, so that what is left at the end is short.
+constexpr int kHeadChunk = 16;
+__device__ __forceinline__ void tile_of_cta(int idx, int tiles, int heads, int& rank, int& bh) {
+  const int chunk = idx / (tiles * kHeadChunk);
+  const int in = idx - chunk * (tiles * kHeadChunk);
+  const int width = min(kHeadChunk, heads - chunk * kHeadChunk);
+  rank = in / width;                 // 0 = longest stream
+  bh = chunk * kHeadChunk + in % width;
+}
+
+// ============================================================================ forward
+// A CTA owns 256 queries of one head, 128 per softmax group, and streams the keys in blocks of
+// 64: both groups use every K/V tile.  Where only one tile of queries is left (short slices, the
+// end of a long one) the two groups take alternate key blocks of that tile, and their partial
+// outputs are merged at the end.
+//
+// Each group has two S buffers and an MMA warp of its own.  P overwrites the S it came from, and
+// the scores of block k + 2 overwrite that P: they are issued right after P V of block k (MMAs of one
+// thread execute in order, so nobody waits in between), and a group finds the scores of its next
+// block ready when it has handed in P.  With O that is 4 x 64 + 2 x D columns of TMEM, all 512 at
+// D = 128.  One MMA warp for both groups spent 185 cycles on each of six waits and as much on
+// commits per pair of blocks, 2700 cycles at either D.
+//
+// What bounds it: 128 queries x 64 keys take 512 cycles of the exponential unit; S takes 384 cycles
+// (6 KB of operands through shared memory per 32 cycles of tensor work) and P V 256 at D = 128,
+// half of that at D = 64.
+struct FwdShared {
+  uint64_t bar_q[2], bar_k[4], bar_kfree[4], bar_v[4], bar_vfree[4], bar_s[2][2], bar_p[2][2], bar_o[2],
+      bar_fin[2];
+  float m[2][128], l[2][128];   // split mode: row statistics of the two groups
   uint32_t tmem_slot;
   int abort_flag;
 };
 
-// ============================================================================ forward
-// Software pipeline: K/V tiles sit in a 4-stage ring (the prefix is streamed from HBM, so
-// loads must be issued several blocks ahead), the S accumulator and the P tile are double
-// buffered, and the
-// MMA thread issues S(j+1) = Q K(j+1)^T before it waits for the softmax of block j, so the
-// tensor core computes the next scores while the 128 softmax threads work on the current ones.
+constexpr int kFwdStages = 4;   // depth of the K and of the V ring
+
 template <typename T, int D>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
                 const AttnParams p) {
   constexpr int DH = D / 64;
-  constexpr int kQSub = 128 * 128, kKSub = 64 * 128;
-  constexpr uint32_t kTmemCols = 256;
-  constexpr int KS = 4;  // K/V ring depth
+  constexpr int kQSub = 128 * 128, kKSub = 64 * 128;   // [rows][64 columns] 16-bit, 128-byte swizzle
+  constexpr int kQTile = DH * kQSub, kKTile = DH * kKSub;
+  constexpr int KS = kFwdStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + DH * kQSub;          // [KS][DH][kKSub]
-  uint8_t* sV = sK + KS * DH * kKSub;     // [KS][DH][kKSub]
-  uint8_t* sP = sV + KS * DH * kKSub;     // [2][128][128B]
-  AttnShared* sh = reinterpret_cast<AttnShared*>(sP + 2 * 128 * 128);
-  uint64_t* bar_q = &sh->bars[0];
-  uint64_t* bar_k = &sh->bars[1];      // [KS]
-  uint64_t* bar_v = &sh->bars[5];      // [KS]
-  uint64_t* bar_s = &sh->bars[9];      // [2]
-  uint64_t* bar_sfree = &sh->bars[11]; // [2]
-  uint64_t* bar_p = &sh->bars[13];     // [2]
-  uint64_t* bar_pv = &sh->bars[15];    // [2]
+  uint8_t* sQ = smem;                      // [2][kQTile]
+  uint8_t* sK = sQ + 2 * kQTile;           // [KS][kKTile]
+  uint8_t* sV = sK + KS * kKTile;          // [KS][kKTile]
+  FwdShared* sh = reinterpret_cast<FwdShared*>(sV + KS * kKTile);
 
   const int warp = threadIdx.x >> 5;
   const WaitCtx wctx{&sh->abort_flag, p.err};
-  const int q0 = blockIdx.x * 128;
-  const int bh = blockIdx.y;
+  const int tiles = (p.t + 255) / 256;
+  int rank, bh;
+  tile_of_cta(blockIdx.x, tiles, p.b * p.h, rank, bh);
   const int bi = bh / p.h, hi = bh % p.h;
-  const int q_hi = min(p.t, q0 + 128);
-  const int nkb = (p.c + q_hi + 63) / 64;
+  const int q0 = (tiles - 1 - rank) * 256;
+  const bool split = q0 + 128 >= p.t;      // one tile of queries: the groups share its key blocks
+  // key blocks of the first tile and of the last
+  const int nb0 = (p.c + min(p.t, q0 + 128) + 63) / 64;
+  const int n = (p.c + min(p.t, q0 + 256) + 63) / 64;   // = nb0 when split; blocks that are loaded
+  // blocks of the two groups: the k-th block of group w is blk(w, k)
+  const int n_it0 = split ? (nb0 + 1) / 2 : nb0, n_it1 = split ? nb0 / 2 : n;
+  auto blk = [&](int w, int k) { return split ? 2 * k + w : k; };
 
   if (threadIdx.x == 0) {
-    mbar_init(bar_q, 1);
-    for (int i = 0; i < KS; ++i) {
-      mbar_init(&bar_k[i], 1);
-      mbar_init(&bar_v[i], 1);
-    }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bar_s[i], 1);
-      mbar_init(&bar_sfree[i], 4);
-      mbar_init(&bar_p[i], 4);
-      mbar_init(&bar_pv[i], 1);
+      mbar_init(&sh->bar_q[i], 1);
+      mbar_init(&sh->bar_o[i], 1);
+      mbar_init(&sh->bar_fin[i], 1);
+      for (int k = 0; k < 2; ++k) {
+        mbar_init(&sh->bar_s[i][k], 1);
+        mbar_init(&sh->bar_p[i][k], 4);
+      }
+    }
+    for (int i = 0; i < KS; ++i) {
+      mbar_init(&sh->bar_k[i], 1);
+      mbar_init(&sh->bar_kfree[i], split ? 1 : 2);   // users of a block
+      mbar_init(&sh->bar_v[i], 1);
+      mbar_init(&sh->bar_vfree[i], split ? 1 : 2);
     }
     sh->abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 4) {
-    tmem_alloc(&sh->tmem_slot, kTmemCols);
+  if (warp == 9) {
+    tmem_alloc(&sh->tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -158,163 +180,242 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_after();
   pdl_wait();  // set-up done; from here on the predecessor's results are read
   const uint32_t tmem = sh->tmem_slot;
-  const uint32_t tO = tmem + 128;   // S[0] at 0, S[1] at 64, O at 128
+  // columns: S / P of group w at 128 w (+ 64 for the odd blocks), O of group w at 256 + D w
 
-  if (warp == 4) {
+  if (warp == 8) {
     if (elect_one()) {
-      constexpr uint32_t idesc_s = umma_idesc_f16(Elem<T>::fmt, 0, 0, 128, 64);
-      constexpr uint32_t idesc_pv = umma_idesc_f16(Elem<T>::fmt, 0, 1, 128, D);
-      auto load_kv = [&](int j) {
-        const int st = j % KS;
-        mbar_expect_tx(&bar_k[st], DH * kKSub);
+      auto load_q = [&](int w) {
+        mbar_expect_tx(&sh->bar_q[w], kQTile);
         for (int hh = 0; hh < DH; ++hh)
-          tma_load_3d(sK + (st * DH + hh) * kKSub, &tmKV, &bar_k[st], D + hh * 64, bh, j * 64);
-        mbar_expect_tx(&bar_v[st], DH * kKSub);
-        for (int hh = 0; hh < DH; ++hh)
-          tma_load_3d(sV + (st * DH + hh) * kKSub, &tmKV, &bar_v[st], 2 * D + hh * 64, bh, j * 64);
+          tma_load_3d(sQ + w * kQTile + hh * kQSub, &tmQ, &sh->bar_q[w], hh * 64, bh, p.c + q0 + w * 128);
       };
-      auto issue_s = [&](int j) -> bool {
-        const int ks = j % KS, sb = j & 1;
-        if (!mbar_wait(&bar_k[ks], (j / KS) & 1, wctx, kErrWaitAttn)) return false;
-        if (!mbar_wait(&bar_sfree[sb], ((j >> 1) & 1) ^ 1, wctx, kErrWaitAttn)) return false;
-        tc_fence_after();
-        mma_kk<DH>(tmem + sb * 64, smem_u32(sQ), kQSub, smem_u32(sK + ks * DH * kKSub), kKSub, idesc_s);
-        umma_commit(&bar_s[sb]);
+      auto load_kv = [&](uint8_t* ring, uint64_t* full, uint64_t* freed, int col, int j) -> bool {
+        const int st = j % KS;
+        if (!mbar_wait(&freed[st], ((j / KS) & 1) ^ 1, wctx, kErrWaitAttn)) return false;
+        mbar_expect_tx(&full[st], kKTile);
+        for (int hh = 0; hh < DH; ++hh)
+          tma_load_3d(ring + st * kKTile + hh * kKSub, &tmKV, &full[st], col + hh * 64, bh, j * 64);
         return true;
       };
-      mbar_expect_tx(bar_q, DH * kQSub);
-      for (int hh = 0; hh < DH; ++hh)
-        tma_load_3d(sQ + hh * kQSub, &tmQ, bar_q, hh * 64, bh, p.c + q0);
-      for (int j = 0; j < KS && j < nkb; ++j) load_kv(j);
-      bool ok = mbar_wait(bar_q, 0, wctx, kErrWaitAttn);
-      if (ok) ok = issue_s(0);
-      for (int j = 0; j < nkb && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (j + 1 < nkb) ok = issue_s(j + 1);
-        if (!ok) break;
-        ok = mbar_wait(&bar_p[st], ph, wctx, kErrWaitAttn) &&
-             mbar_wait(&bar_v[j % KS], (j / KS) & 1, wctx, kErrWaitAttn);
-        if (!ok) break;
-        tc_fence_after();
-        mma_kn(tO, smem_u32(sP + st * 128 * 128), smem_u32(sV + (j % KS) * DH * kKSub), kKSub, idesc_pv, j > 0);
-        umma_commit(&bar_pv[st]);
-        if (j >= 1 && j - 1 + KS < nkb) {
-          // ring stage (j-1) % KS is reusable once PV(j-1) has finished reading V(j-1); waiting
-          // for the PREVIOUS block keeps this thread off the critical path of the current one
-          ok = mbar_wait(&bar_pv[(j - 1) & 1], ((j - 1) >> 1) & 1, wctx, kErrWaitAttn);
-          if (!ok) break;
-          load_kv(j - 1 + KS);
-        }
+      // in the order of use: each group has the scores of two blocks ahead of P V
+      const int ahead = split ? 4 : 2;
+      load_q(0);
+      bool ok = load_kv(sK, sh->bar_k, sh->bar_kfree, D, 0);
+      if (!split) load_q(1);
+      for (int j = 1; j < ahead && j < n && ok; ++j) ok = load_kv(sK, sh->bar_k, sh->bar_kfree, D, j);
+      for (int j = 0; j < n && ok; ++j) {
+        // (the groups differ by at most two blocks, which are the last ones: their tiles, which
+        // group 1 alone uses, are not waited for)
+        ok = load_kv(sV, sh->bar_v, sh->bar_vfree, 2 * D, j);
+        if (ok && j + ahead < n) ok = load_kv(sK, sh->bar_k, sh->bar_kfree, D, j + ahead);
       }
     }
+  } else if (warp >= 9) {
+    const int w = warp - 9;
+    const int n_it = w == 0 ? n_it0 : n_it1;
+    if (n_it > 0 && elect_one()) {
+      constexpr uint32_t idesc_s = umma_idesc_f16(Elem<T>::fmt, 0, 0, 128, 64);
+      constexpr uint32_t idesc_pv = umma_idesc_f16(Elem<T>::fmt, 0, 1, 128, D);
+      const uint32_t dQ = desc_k(smem_u32(sQ + (split ? 0 : w * kQTile))), dK = desc_k(smem_u32(sK)),
+                     dV = desc_n(smem_u32(sV), kKSub);
+      const uint32_t tSw = tmem + w * 128, tOw = tmem + 256 + w * D;
+      auto issue_s = [&](int k) {
+        const int st = blk(w, k) % KS;
+        mma_kk<DH>(tSw + (k & 1) * 64, dQ, kQSub, dK + st * (kKTile >> 4), kKSub, idesc_s);
+        umma_commit(&sh->bar_s[w][k & 1]);
+        umma_commit(&sh->bar_kfree[st]);
+      };
+      bool ok = mbar_wait(&sh->bar_q[split ? 0 : w], 0, wctx, kErrWaitAttn);
+      for (int k = 0; k < 2 && k < n_it && ok; ++k) {
+        const int j = blk(w, k);
+        ok = mbar_wait(&sh->bar_k[j % KS], (j / KS) & 1, wctx, kErrWaitAttn);
+        tc_fence_after();
+        if (ok) issue_s(k);
+      }
+      for (int k = 0; k < n_it && ok; ++k) {
+        const int j = blk(w, k), j2 = blk(w, k + 2);
+        const bool more = k + 2 < n_it;
+        uint64_t *bp = &sh->bar_p[w][k & 1], *bv = &sh->bar_v[j % KS], *bk = &sh->bar_k[j2 % KS];
+        ok = more ? mbar_wait_all(bp, (k >> 1) & 1, bv, (j / KS) & 1, bk, (j2 / KS) & 1, wctx, kErrWaitAttn)
+                  : mbar_wait_all(bp, (k >> 1) & 1, bv, (j / KS) & 1, wctx, kErrWaitAttn);
+        if (!ok) break;
+        tc_fence_after();
+        mma_tn(tOw, tSw + (k & 1) * 64, dV + (j % KS) * (kKTile >> 4), idesc_pv, k > 0);
+        umma_commit(&sh->bar_o[w]);
+        umma_commit(&sh->bar_vfree[j % KS]);
+        if (more) issue_s(k + 2);
+      }
+      if (ok) umma_commit(&sh->bar_fin[w]);
+    }
   } else {
-    const int r = threadIdx.x;  // row of the tile = TMEM lane
-    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    const int qi = q0 + r;
+    const int w = warp >> 2;               // softmax group
+    const int r = threadIdx.x & 127;       // row of the tile = TMEM lane
+    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t tS = tmem + w * 128 + lane_base, tO = tmem + 256 + w * D + lane_base;
+    const int qt = q0 + (split ? 0 : w * 128);   // first query of the tile
+    const int qi = qt + r;
     const int qpos = p.c + qi;
-    float m = -INFINITY, l = 0.0f;
+    const int n_it = w == 0 ? n_it0 : n_it1;
+    float m = -INFINITY;
+    float2 l2 = make_float2(0.0f, 0.0f);
     bool ok = true;
-    for (int j = 0; j < nkb; ++j) {
-      const int st = j & 1;
-      ok = mbar_wait(&bar_s[st], (j >> 1) & 1, wctx, kErrWaitAttn);
+    for (int k = 0; k < n_it; ++k) {
+      ok = mbar_wait(&sh->bar_s[w][k & 1], (k >> 1) & 1, wctx, kErrWaitAttn);
       if (!ok) break;
       tc_fence_after();
-      float s[64];
-      {
-        uint32_t r0[32], r1[32];
-        __syncwarp();
-        tmem_ld_32x32(tmem + st * 64 + lane_base, r0);
-        tmem_ld_32x32(tmem + st * 64 + lane_base + 32, r1);
-        tmem_ld_wait();
+      const int kbase = blk(w, k) * 64;
+      const uint32_t tSk = tS + (k & 1) * 64;
+      uint32_t s[2][32];
+      __syncwarp();
+      tmem_ld_32x32(tSk, s[0]);
+      tmem_ld_32x32(tSk + 32, s[1]);
+      tmem_ld_wait();
+      if (kbase + 63 > p.c + qt) {         // the causal edge runs through this block
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          s[i] = __uint_as_float(r0[i]);
-          s[32 + i] = __uint_as_float(r1[i]);
-        }
+        for (int g = 0; g < 2; ++g)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (kbase + g * 32 + i > qpos) s[g][i] = 0xff800000u;   // -inf
       }
-      tc_fence_before();
-      warp_arrive(&bar_sfree[st]);
-      float mx = -INFINITY;
-      const int kbase = j * 64;
-      if (kbase + 63 <= p.c + q0) {   // every key of the block is visible to every row
+      float mx4[4];
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          s[i] *= p.scale2;
-          mx = fmaxf(mx, s[i]);
-        }
-      } else {
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t* sg = &s[g >> 1][(g & 1) * 16];
+        mx4[g] = fmaxf(__uint_as_float(sg[0]), __uint_as_float(sg[1]));
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          s[i] = (kbase + i <= qpos) ? s[i] * p.scale2 : -INFINITY;
-          mx = fmaxf(mx, s[i]);
-        }
+        for (int i = 2; i < 16; i += 2) mx4[g] = max3(mx4[g], __uint_as_float(sg[i]), __uint_as_float(sg[i + 1]));
       }
+      const float mx = fmaxf(max3(mx4[0], mx4[1], mx4[2]), mx4[3]) * p.scale2;
       bool need = false;
       float alpha = 1.0f;
-      if (j == 0) {
+      if (k == 0) {
         m = mx;
       } else if (mx > m + 8.0f) {
         need = true;
         alpha = exp2f(m - mx);
         m = mx;
-        l *= alpha;
+        l2 = mul2(l2, dup2(alpha));
       }
       if (__any_sync(0xffffffffu, need)) {
-        // O may only be touched once PV(j-1) has been accumulated
-        ok = mbar_wait(&bar_pv[(j - 1) & 1], ((j - 1) >> 1) & 1, wctx, kErrWaitAttn);
+        // O may only be touched once P V of the group's previous block has been added to it
+        ok = mbar_wait(&sh->bar_o[w], (k - 1) & 1, wctx, kErrWaitAttn);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
         for (int ch = 0; ch < D / 32; ++ch) {
           uint32_t raw[32];
-          tmem_ld_32x32(tO + lane_base + ch * 32, raw);
+          tmem_ld_32x32(tO + ch * 32, raw);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) raw[i] = __float_as_uint(__uint_as_float(raw[i]) * alpha);
-          tmem_st_32x32(tO + lane_base + ch * 32, raw);
+          tmem_st_32x32(tO + ch * 32, raw);
         }
-        tmem_st_wait();
       }
-      float sum = 0.0f;
+      // a row that has seen no key yet (second group, its first block beyond the diagonal) has m = -inf
+      const float2 nm = dup2(m == -INFINITY ? 0.0f : -m), sc = dup2(p.scale2);
 #pragma unroll
-      for (int i = 0; i < 64; ++i) {
-        s[i] = exp2f(s[i] - m);
-        sum += s[i];
+      for (int g = 0; g < 2; ++g) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float2 e = fma2(make_float2(__uint_as_float(s[g][2 * i]), __uint_as_float(s[g][2 * i + 1])), sc, nm);
+          e.x = exp2f(e.x);
+          e.y = exp2f(e.y);
+          l2 = add2(l2, e);
+          pk[i] = Elem<T>::pack2(e.x, e.y);
+        }
+        tmem_st_32x16(tSk + g * 16, pk);
       }
-      l += sum;
-      store_row64<T>(sP + st * 128 * 128, r, s);
-      fence_proxy_async();
+      tmem_st_wait();
       tc_fence_before();
-      warp_arrive(&bar_p[st]);
+      warp_arrive(&sh->bar_p[w][k & 1]);
     }
-    if (ok) ok = mbar_wait(&bar_pv[(nkb - 1) & 1], ((nkb - 1) >> 1) & 1, wctx, kErrWaitAttn);
-    if (ok) {
-      tc_fence_after();
-      const float inv_l = 1.0f / l;
-      // checked build: the row's statistics slot and its columns of the output exist
-      const bool row_ok = qi < p.t && TP_CHECK(qpos >= 0 && qpos < p.lse_stride && (hi + 1) * D <= p.ld_o,
-                                               p.err, kErrCheckAttn);
-      T* orow = static_cast<T*>(p.o) + (static_cast<long long>(qi) * p.b + bi) * p.ld_o + hi * D;
-#pragma unroll 1
-      for (int ch = 0; ch < D / 32; ++ch) {
-        uint32_t raw[32];
-        __syncwarp();
-        tmem_ld_32x32(tO + lane_base + ch * 32, raw);
-        tmem_ld_wait();
-        if (row_ok) {
+    float l = l2.x + l2.y;
+    // checked build: the row's statistics slot and its columns of the output exist
+    const bool row_ok = qi < p.t && TP_CHECK(qpos >= 0 && qpos < p.lse_stride && (hi + 1) * D <= p.ld_o,
+                                             p.err, kErrCheckAttn);
+    T* orow = static_cast<T*>(p.o) + (static_cast<long long>(qi) * p.b + bi) * p.ld_o + hi * D;
+    float* lse_slot = p.lse2 + static_cast<long long>(bh) * p.lse_stride + qpos;
+    auto store32 = [&](int col, const float (&v)[32], float mul) {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 u;
-            u.x = Elem<T>::pack2(__uint_as_float(raw[g * 8 + 0]) * inv_l, __uint_as_float(raw[g * 8 + 1]) * inv_l);
-            u.y = Elem<T>::pack2(__uint_as_float(raw[g * 8 + 2]) * inv_l, __uint_as_float(raw[g * 8 + 3]) * inv_l);
-            u.z = Elem<T>::pack2(__uint_as_float(raw[g * 8 + 4]) * inv_l, __uint_as_float(raw[g * 8 + 5]) * inv_l);
-            u.w = Elem<T>::pack2(__uint_as_float(raw[g * 8 + 6]) * inv_l, __uint_as_float(raw[g * 8 + 7]) * inv_l);
-            *reinterpret_cast<uint4*>(orow + ch * 32 + g * 8) = u;
-          }
+      for (int g = 0; g < 4; ++g) {
+        uint4 u;
+        u.x = Elem<T>::pack2(v[g * 8 + 0] * mul, v[g * 8 + 1] * mul);
+        u.y = Elem<T>::pack2(v[g * 8 + 2] * mul, v[g * 8 + 3] * mul);
+        u.z = Elem<T>::pack2(v[g * 8 + 4] * mul, v[g * 8 + 5] * mul);
+        u.w = Elem<T>::pack2(v[g * 8 + 6] * mul, v[g * 8 + 7] * mul);
+        *reinterpret_cast<uint4*>(orow + col + g * 8) = u;
+      }
+    };
+    auto load32 = [&](int col, float (&v)[32]) {
+      uint32_t raw[32];
+      __syncwarp();
+      tmem_ld_32x32(tO + col, raw);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(raw[i]);
+    };
+    if (!split) {
+      if (ok) ok = mbar_wait(&sh->bar_fin[w], 0, wctx, kErrWaitAttn);
+      if (ok) {
+        tc_fence_after();
+        const float inv_l = 1.0f / l;
+#pragma unroll 1
+        for (int ch = 0; ch < D / 32; ++ch) {
+          float v[32];
+          load32(ch * 32, v);
+          if (row_ok) store32(ch * 32, v, inv_l);
+        }
+        if (row_ok) *lse_slot = m + log2f(l);
+      }
+    } else {
+      // Each group finishes half of the columns and hands the other half over through the K and V
+      // rings (every tile has been used once both groups' last products are done).
+      if (ok) ok = mbar_wait(&sh->bar_fin[0], 0, wctx, kErrWaitAttn);
+      if (ok && n_it1 > 0) ok = mbar_wait(&sh->bar_fin[1], 0, wctx, kErrWaitAttn);
+      tc_fence_after();
+      float* give = reinterpret_cast<float*>(sK) + w * (D / 2) * 128;        // [D / 2][128 rows]
+      const float* take = reinterpret_cast<const float*>(sK) + (w ^ 1) * (D / 2) * 128;
+      sh->m[w][r] = m;
+      sh->l[w][r] = l;
+      if (ok && n_it > 0) {
+#pragma unroll 1
+        for (int ch = 0; ch < D / 64; ++ch) {
+          float v[32];
+          load32((w ^ 1) * (D / 2) + ch * 32, v);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) give[(ch * 32 + i) * 128 + r] = v[i];
         }
       }
-      if (row_ok) p.lse2[static_cast<long long>(bh) * p.lse_stride + qpos] = m + log2f(l);
+      named_bar_sync(1, 256);
+      if (ok) {
+        const float m_o = sh->m[w ^ 1][r], l_o = sh->l[w ^ 1][r];
+        const bool other = w == 1 || n_it1 > 0;    // the other group had blocks
+        const float mm = fmaxf(m, m_o);
+        const float a = m == -INFINITY ? 0.0f : exp2f(m - mm);
+        const float a_o = m_o == -INFINITY ? 0.0f : exp2f(m_o - mm);
+        l = l * a + l_o * a_o;
+        const float inv_l = 1.0f / l;
+#pragma unroll 1
+        for (int ch = 0; ch < D / 64; ++ch) {
+          const int col = w * (D / 2) + ch * 32;
+          float v[32];
+          if (n_it > 0) {
+            load32(col, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] *= a;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+          }
+          if (other) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] += take[(ch * 32 + i) * 128 + r] * a_o;
+          }
+          if (row_ok) store32(col, v, inv_l);
+        }
+        if (row_ok && w == 0) *lse_slot = mm + log2f(l);
+      }
     }
   }
 
@@ -325,32 +426,61 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
   tc_fence_after();
-  if (warp == 4) tmem_dealloc(tmem, kTmemCols);
+  if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
 // ============================================================================ delta = rowsum(dO * O)
-template <typename T>
-__global__ void attn_delta_kernel(const T* __restrict__ o, long long ld_o, const T* __restrict__ d_o,
-                                  long long ld_do, float* __restrict__ delta,
-                                  long long delta_stride, int c, int t, int b, int h, int D) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+// A row (one position of one head) is D / 8 lanes of 16 bytes each, and every lane has four rows in
+// flight: memory bound.  (One warp per row with 4-byte loads kept 256 bytes per warp in flight:
+// 16384 x 2048 took 67 us.)  o_vec = 0: `o` is only 4-byte aligned.
+constexpr int kDeltaThreads = 256, kDeltaUnroll = 4;
+template <int D> struct DeltaRows { static constexpr int value = kDeltaThreads / (D / 8) * kDeltaUnroll; };
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kDeltaThreads)
+attn_delta_kernel(const T* __restrict__ o, long long ld_o, const T* __restrict__ d_o, long long ld_do,
+                  float* __restrict__ delta, long long delta_stride, int c, int t, int b, int h, int o_vec) {
+  constexpr int kLanes = D / 8, kGroups = kDeltaThreads / kLanes;
+  const int lane = threadIdx.x % kLanes;
+  const long long row0 = static_cast<long long>(blockIdx.x) * DeltaRows<D>::value + threadIdx.x / kLanes;
+  const long long rows = static_cast<long long>(t) * b * h;
   pdl_wait();
-  if (warp >= t * b * h) return;
-  const int hi = warp % h;
-  const int bi = (warp / h) % b;
-  const int i = warp / (h * b);
-  const T* po = o + (static_cast<long long>(i) * b + bi) * ld_o + hi * D;
-  const T* pd = d_o + (static_cast<long long>(i) * b + bi) * ld_do + hi * D;
-  float acc = 0.0f;
-  for (int e = lane * 2; e < D; e += 64) {
-    const float2 a = Elem<T>::unpack2(*reinterpret_cast<const uint32_t*>(po + e));
-    const float2 g = Elem<T>::unpack2(*reinterpret_cast<const uint32_t*>(pd + e));
-    acc += a.x * g.x + a.y * g.y;
+  uint4 vo[kDeltaUnroll], vd[kDeltaUnroll];
+#pragma unroll
+  for (int k = 0; k < kDeltaUnroll; ++k) {
+    const long long row = row0 + k * kGroups;
+    vo[k] = vd[k] = make_uint4(0, 0, 0, 0);
+    if (row < rows) {
+      const long long pos = row / h;          // position * b + batch
+      const int col = static_cast<int>(row - pos * h) * D + lane * 8;
+      const T* po = o + pos * ld_o + col;
+      if (o_vec) {
+        vo[k] = *reinterpret_cast<const uint4*>(po);
+      } else {
+        const uint32_t* p4 = reinterpret_cast<const uint32_t*>(po);
+        vo[k] = make_uint4(p4[0], p4[1], p4[2], p4[3]);
+      }
+      vd[k] = *reinterpret_cast<const uint4*>(d_o + pos * ld_do + col);
+    }
   }
 #pragma unroll
-  for (int o2 = 16; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
-  if (lane == 0) delta[static_cast<long long>(bi * h + hi) * delta_stride + c + i] = acc;
+  for (int k = 0; k < kDeltaUnroll; ++k) {
+    const uint32_t wo[4] = {vo[k].x, vo[k].y, vo[k].z, vo[k].w};
+    const uint32_t wd[4] = {vd[k].x, vd[k].y, vd[k].z, vd[k].w};
+    float acc = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 x = Elem<T>::unpack2(wo[q]), g = Elem<T>::unpack2(wd[q]);
+      acc += x.x * g.x + x.y * g.y;
+    }
+#pragma unroll
+    for (int m = kLanes / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    const long long row = row0 + k * kGroups;
+    if (lane == 0 && row < rows) {
+      const int bh = static_cast<int>(row % (static_cast<long long>(b) * h));   // batch * h + head
+      delta[bh * delta_stride + c + row / (static_cast<long long>(b) * h)] = acc;
+    }
+  }
 }
 
 // ============================================================================ backward
@@ -362,21 +492,25 @@ __global__ void attn_delta_kernel(const T* __restrict__ o, long long ld_o, const
 //   MODE 1 (dQ): stationary = 128 queries of the current slice (Q, dO tiles); streams the keys
 //     k <= q (K, V tiles of 64 rows).
 // Per streamed block:  S = X1 Y1^T, dP = X2 Y2^T (TMEM, double buffered);
-//   P = exp2(S*scale2 - lse), dS = P (dP - delta)  -> 16-bit tiles in shared memory;
-//   MODE 0: dV += P^T-tile * dO, dK += dS^T-tile * Q;   MODE 1: dQ += dS * K.
+//   P = exp2(S*scale2 - lse), dS = P (dP - delta)  -> 16-bit, into the columns of S and dP;
+//   MODE 0: dV += P * dO, dK += dS * Q;   MODE 1: dQ += dS * K   (P, dS are A operands from TMEM).
 // 10 warps: two worker groups of 4 warps alternate over the streamed blocks (each owns one
-// S/dP buffer), warp 8 elects the TMA thread, warp 9 the MMA thread.
+// S/dP buffer), warp 8 brings the streamed tiles, warp 9 elects the MMA thread.
+//
+// What bounds it: shared memory.  A 128 x 64 block of S reads 6 KB of operands for 32 cycles of
+// tensor work (48 cycles of shared memory), so at D = 128 a block takes 1280 cycles in MODE 0
+// and 1024 in MODE 1.  P and dS used to go through shared memory as well, single buffered: each
+// block's store waited for the previous block's products and these for the store, and a block took
+// 4000 cycles.  The MMA thread now issues the products of block i and then the scores of block
+// i + 2, which overwrite the same columns: MMAs of one thread execute in order, so only the
+// workers' arrival is waited for.
 constexpr int kBwdThreads = 320;
-constexpr int kBwdMaxStages = 4;
-// Ring depth of the streamed tiles: the dQ mode needs no P tile and spends that shared memory
-// on a fourth stage (the streamed K/V come from HBM, so loads must run well ahead).
-template <int MODE> struct BwdStages { static constexpr int value = MODE == 1 ? 4 : 3; };
+constexpr int kBwdStages = 4;   // ring depth of the streamed tiles
 
 struct BwdShared {
-  uint64_t bar_x, bar_y[kBwdMaxStages], bar_yfree[kBwdMaxStages], bar_s[2], bar_sfree[2], bar_p[2],
-      bar_acc[2], bar_done;
-  float lse[kBwdMaxStages][64];    // MODE 0: per streamed block, written by the producer warp
-  float delta[kBwdMaxStages][64];
+  uint64_t bar_x, bar_y[kBwdStages], bar_yfree[kBwdStages], bar_s[2], bar_p[2], bar_done;
+  alignas(16) float nlse[kBwdStages][64];   // MODE 0: per streamed block, negated, by the producer warp
+  alignas(16) float ndelta[kBwdStages][64];
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -390,7 +524,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
   constexpr int DH = D / 64;
   constexpr int kXSub = 128 * 128, kYSub = 64 * 128;
   constexpr int kStageBytes = 2 * DH * kYSub;
-  constexpr int kBwdStages = BwdStages<MODE>::value;
   constexpr uint32_t kTmemCols = 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -398,22 +531,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
   uint8_t* sX1 = smem;
   uint8_t* sX2 = sX1 + DH * kXSub;
   uint8_t* sY = sX2 + DH * kXSub;                 // [stages][Y1 | Y2][DH][kYSub]
-  uint8_t* sP = sY + kBwdStages * kStageBytes;    // [128][128B], MODE 0 only
-  uint8_t* sdS = MODE == 0 ? sP + 128 * 128 : sP;
-  BwdShared* sh = reinterpret_cast<BwdShared*>(sdS + 128 * 128);
+  BwdShared* sh = reinterpret_cast<BwdShared*>(sY + kBwdStages * kStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const WaitCtx wctx{&sh->abort_flag, p.err};
-  const int bh = blockIdx.y;
+  const int tiles = (p.t + 127) / 128;
+  int rank, bh;
+  tile_of_cta(blockIdx.x, tiles, p.b * p.h, rank, bh);
   const int bi = bh / p.h, hi = bh % p.h;
-  const int x0 = p.c + blockIdx.x * 128;  // first stationary row (absolute position)
+  // dK/dV: the first keys have the most queries; dQ: the last queries have the most keys
+  const int xt = (MODE == 0 ? rank : tiles - 1 - rank) * 128;
+  const int x0 = p.c + xt;                // first stationary row (absolute position)
   int ystart, n_iter;
   if (MODE == 0) {
     ystart = x0;
     n_iter = (p.q_end - x0 + 63) / 64;
   } else {
     ystart = 0;
-    n_iter = (p.c + min(p.t, static_cast<int>(blockIdx.x) * 128 + 128) + 63) / 64;
+    n_iter = (p.c + min(p.t, xt + 128) + 63) / 64;
   }
 
   if (threadIdx.x == 0) {
@@ -424,11 +559,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sh->bar_s[i], 1);
-      mbar_init(&sh->bar_sfree[i], 4);
       mbar_init(&sh->bar_p[i], 4);
     }
-    mbar_init(&sh->bar_acc[0], 1);
-    mbar_init(&sh->bar_acc[1], 1);
     mbar_init(&sh->bar_done, 1);
     sh->abort_flag = 0;
     fence_barrier_init();
@@ -442,7 +574,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
   tc_fence_after();
   pdl_wait();  // set-up done; from here on the predecessor's results are read
   const uint32_t tmem = sh->tmem_slot;
-  // columns: S[0] 0, S[1] 64, dP[0] 128, dP[1] 192, Acc1 256, Acc2 256 + D
+  // columns: S / P of buffer 0 at 0, of 1 at 64, dP / dS at 128 and 192, Acc1 256, Acc2 256 + D
   const uint32_t tA1 = tmem + 256, tA2 = tmem + 256 + D;
 
   if (warp == 8) {
@@ -501,8 +633,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
       if (MODE == 0) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          sh->lse[st][lane + 32 * k] = nl[k];
-          sh->delta[st][lane + 32 * k] = nd[k];
+          sh->nlse[st][lane + 32 * k] = -nl[k];
+          sh->ndelta[st][lane + 32 * k] = -nd[k];
         }
         warp_arrive(&sh->bar_y[st]);
         if (i + 1 < n_iter) fetch_stats(y0 + 64);
@@ -512,33 +644,35 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
     if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_f16(Elem<T>::fmt, 0, 0, 128, 64);
       constexpr uint32_t idesc_g = umma_idesc_f16(Elem<T>::fmt, 0, 1, 128, D);
-      bool ok = mbar_wait(&sh->bar_x, 0, wctx, kErrWaitAttn);
-      auto issue_acc = [&](int j) -> bool {
-        if (!mbar_wait(&sh->bar_p[j & 1], (j >> 1) & 1, wctx, kErrWaitAttn)) return false;
-        tc_fence_after();
-        const int st = j % kBwdStages;
-        const uint32_t y1 = smem_u32(sY + st * kStageBytes);
-        const uint32_t y2 = y1 + DH * kYSub;
-        if (MODE == 0) mma_kn(tA1, smem_u32(sP), y2, kYSub, idesc_g, j > 0);
-        mma_kn(tA2, smem_u32(sdS), y1, kYSub, idesc_g, j > 0);
-        umma_commit(&sh->bar_yfree[st]);
-        umma_commit(&sh->bar_acc[j & 1]);
-        return true;
+      const uint32_t dX1 = desc_k(smem_u32(sX1)), dX2 = desc_k(smem_u32(sX2)), dY = desc_k(smem_u32(sY)),
+                     dYn = desc_n(smem_u32(sY), kYSub);
+      constexpr uint32_t kStage16 = kStageBytes >> 4, kY2 = (DH * kYSub) >> 4;   // descriptor steps
+      auto issue_s = [&](int i) {
+        const uint32_t y = dY + (i % kBwdStages) * kStage16;
+        mma_kk<DH>(tmem + (i & 1) * 64, dX1, kXSub, y, kYSub, idesc_s);
+        mma_kk<DH>(tmem + 128 + (i & 1) * 64, dX2, kXSub, y + kY2, kYSub, idesc_s);
+        umma_commit(&sh->bar_s[i & 1]);
       };
+      bool ok = mbar_wait(&sh->bar_x, 0, wctx, kErrWaitAttn);
+      for (int i = 0; i < 2 && i < n_iter && ok; ++i) {
+        ok = mbar_wait(&sh->bar_y[i], 0, wctx, kErrWaitAttn);
+        tc_fence_after();
+        if (ok) issue_s(i);
+      }
       for (int i = 0; i < n_iter && ok; ++i) {
-        const int st = i % kBwdStages, buf = i & 1;
-        ok = mbar_wait(&sh->bar_y[st], (i / kBwdStages) & 1, wctx, kErrWaitAttn) &&
-             mbar_wait(&sh->bar_sfree[buf], ((i >> 1) & 1) ^ 1, wctx, kErrWaitAttn);
+        const int st = i % kBwdStages;
+        const bool more = i + 2 < n_iter;
+        uint64_t *bp = &sh->bar_p[i & 1], *by = &sh->bar_y[(i + 2) % kBwdStages];
+        ok = more ? mbar_wait_all(bp, (i >> 1) & 1, by, ((i + 2) / kBwdStages) & 1, wctx, kErrWaitAttn)
+                  : mbar_wait(bp, (i >> 1) & 1, wctx, kErrWaitAttn);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t y1 = smem_u32(sY + st * kStageBytes);
-        const uint32_t y2 = y1 + DH * kYSub;
-        mma_kk<DH>(tmem + buf * 64, smem_u32(sX1), kXSub, y1, kYSub, idesc_s);
-        mma_kk<DH>(tmem + 128 + buf * 64, smem_u32(sX2), kXSub, y2, kYSub, idesc_s);
-        umma_commit(&sh->bar_s[buf]);
-        if (i >= 1) ok = issue_acc(i - 1);
+        const uint32_t buf = (i & 1) * 64;
+        if (MODE == 0) mma_tn(tA1, tmem + buf, dYn + st * kStage16 + kY2, idesc_g, i > 0);
+        mma_tn(tA2, tmem + 128 + buf, dYn + st * kStage16, idesc_g, i > 0);
+        umma_commit(&sh->bar_yfree[st]);
+        if (more) issue_s(i + 2);
       }
-      if (ok && n_iter > 0) ok = issue_acc(n_iter - 1);
       if (ok) umma_commit(&sh->bar_done);
     }
   } else {
@@ -550,66 +684,75 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
     const bool x_ok = xabs < p.c + p.t &&
                       TP_CHECK(xabs >= p.c && xabs < p.lse_stride && (hi + 1) * 3 * D <= p.ld_dqkv, p.err,
                                kErrCheckAttn);
-    float lse_r = 0.0f, delta_r = 0.0f;
+    float2 nlse_r = make_float2(0.0f, 0.0f), ndelta_r = make_float2(0.0f, 0.0f);
     if (MODE == 1 && x_ok) {
-      lse_r = p.lse2[static_cast<long long>(bh) * p.lse_stride + xabs];
-      delta_r = p.delta[static_cast<long long>(bh) * p.lse_stride + xabs];
+      nlse_r = dup2(-p.lse2[static_cast<long long>(bh) * p.lse_stride + xabs]);
+      ndelta_r = dup2(-p.delta[static_cast<long long>(bh) * p.lse_stride + xabs]);
     }
+    const uint32_t tS = tmem + grp * 64 + lane_base, tP = tmem + 128 + grp * 64 + lane_base;
+    const float2 sc = dup2(p.scale2);
     bool ok = true;
     for (int i = grp; i < n_iter; i += 2) {
       const int y0 = ystart + i * 64;
       const int st = i % kBwdStages;
-      ok = mbar_wait(&sh->bar_s[grp], (i >> 1) & 1, wctx, kErrWaitAttn);
+      // MODE 0: the statistics came with the tiles; half of them are fetched ahead of the scores
+      float4 nl4[8], nd4[8];
+      auto fetch_stats = [&](int g) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          nl4[k] = *reinterpret_cast<const float4*>(&sh->nlse[st][g * 32 + 4 * k]);
+          nd4[k] = *reinterpret_cast<const float4*>(&sh->ndelta[st][g * 32 + 4 * k]);
+        }
+      };
+      if (MODE == 0) {
+        ok = mbar_wait(&sh->bar_y[st], (i / kBwdStages) & 1, wctx, kErrWaitAttn);
+        if (ok) fetch_stats(0);
+      }
+      if (ok) ok = mbar_wait(&sh->bar_s[grp], (i >> 1) & 1, wctx, kErrWaitAttn);
       if (!ok) break;
       tc_fence_after();
-      float sv[64], dv[64];
-      {
-        uint32_t r0[32], r1[32], r2[32], r3[32];
-        __syncwarp();
-        tmem_ld_32x32(tmem + grp * 64 + lane_base, r0);
-        tmem_ld_32x32(tmem + grp * 64 + lane_base + 32, r1);
-        tmem_ld_32x32(tmem + 128 + grp * 64 + lane_base, r2);
-        tmem_ld_32x32(tmem + 128 + grp * 64 + lane_base + 32, r3);
-        tmem_ld_wait();
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          sv[k] = __uint_as_float(r0[k]);
-          sv[32 + k] = __uint_as_float(r1[k]);
-          dv[k] = __uint_as_float(r2[k]);
-          dv[32 + k] = __uint_as_float(r3[k]);
-        }
-      }
-      tc_fence_before();
-      warp_arrive(&sh->bar_sfree[grp]);
       // blocks strictly inside the causal region need no per-element mask
       const bool full = MODE == 0 ? (y0 >= x0 + 127 && y0 + 64 <= p.q_end) : (y0 + 63 <= x0);
-      if (full) {
+      // P into the columns of S and dS into those of dP, 32 columns at a time.  The first half's
+      // results take 16 columns that were read already; the second half's scores lie beyond them.
 #pragma unroll
-        for (int k = 0; k < 64; ++k) {
-          const float l2 = MODE == 0 ? sh->lse[st][k] : lse_r;
-          const float dl = MODE == 0 ? sh->delta[st][k] : delta_r;
-          const float pr = exp2f(sv[k] * p.scale2 - l2);
-          dv[k] = pr * (dv[k] - dl);
-          sv[k] = pr;
-        }
-      } else {
+      for (int g = 0; g < 2; ++g) {
+        uint32_t s[32], d[32], pk[16], dk[16];
+        __syncwarp();
+        tmem_ld_32x32(tS + g * 32, s);
+        tmem_ld_32x32(tP + g * 32, d);
+        if (MODE == 0 && g > 0) fetch_stats(g);
+        tmem_ld_wait();
 #pragma unroll
-        for (int k = 0; k < 64; ++k) {
-          const int yabs = y0 + k;
-          const float l2 = MODE == 0 ? sh->lse[st][k] : lse_r;
-          const float dl = MODE == 0 ? sh->delta[st][k] : delta_r;
-          const bool valid = MODE == 0 ? ((yabs < p.q_end) && (xabs <= yabs)) : (x_ok && (yabs <= xabs));
-          const float pr = valid ? exp2f(sv[k] * p.scale2 - l2) : 0.0f;
-          dv[k] = pr * (dv[k] - dl);
-          sv[k] = pr;
+        for (int k = 0; k < 16; k += 2) {   // four columns
+          float2 nl[2] = {nlse_r, nlse_r}, nd[2] = {ndelta_r, ndelta_r};
+          if (MODE == 0) {
+            const float4 a = nl4[k / 2], e = nd4[k / 2];
+            nl[0] = make_float2(a.x, a.y); nl[1] = make_float2(a.z, a.w);
+            nd[0] = make_float2(e.x, e.y); nd[1] = make_float2(e.z, e.w);
+          }
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int e = 2 * (k + q);       // column within the half
+            float2 pr = fma2(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc, nl[q]);
+            pr.x = exp2f(pr.x);
+            pr.y = exp2f(pr.y);
+            if (!full) {
+              const int yabs = y0 + g * 32 + e;
+              const bool v0 = MODE == 0 ? (yabs < p.q_end && xabs <= yabs) : (x_ok && yabs <= xabs);
+              const bool v1 = MODE == 0 ? (yabs + 1 < p.q_end && xabs <= yabs + 1) : (x_ok && yabs + 1 <= xabs);
+              pr.x = v0 ? pr.x : 0.0f;
+              pr.y = v1 ? pr.y : 0.0f;
+            }
+            const float2 ds = mul2(pr, add2(make_float2(__uint_as_float(d[e]), __uint_as_float(d[e + 1])), nd[q]));
+            if (MODE == 0) pk[k + q] = Elem<T>::pack2(pr.x, pr.y);
+            dk[k + q] = Elem<T>::pack2(ds.x, ds.y);
+          }
         }
+        if (MODE == 0) tmem_st_32x16(tS + g * 16, pk);
+        tmem_st_32x16(tP + g * 16, dk);
       }
-      // the operand tiles are free once the accumulating MMAs of the previous block are done
-      if (i >= 1) ok = mbar_wait(&sh->bar_acc[(i - 1) & 1], ((i - 1) >> 1) & 1, wctx, kErrWaitAttn);
-      if (!ok) break;
-      if (MODE == 0) store_row64<T>(sP, r, sv);
-      store_row64<T>(sdS, r, dv);
-      fence_proxy_async();
+      tmem_st_wait();
       tc_fence_before();
       warp_arrive(&sh->bar_p[grp]);
     }
@@ -683,11 +826,11 @@ template <typename K> static bool set_smem(K kern, int bytes) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
 }
 
-template <int D> constexpr int fwd_smem() { return (D / 64) * (128 * 128 + 8 * 64 * 128) + 2 * 128 * 128 + 1024 + 512; }
-template <int D, int MODE> constexpr int bwd_smem() {
-  return (D / 64) * (2 * 128 * 128 + BwdStages<MODE>::value * 2 * 64 * 128) +
-         (MODE == 0 ? 2 : 1) * 128 * 128 + 1024 +
-         static_cast<int>(sizeof(BwdShared)) + 64;
+template <int D> constexpr int fwd_smem() {
+  return (D / 64) * (2 * 128 * 128 + 2 * kFwdStages * 64 * 128) + 1024 + static_cast<int>(sizeof(FwdShared)) + 64;
+}
+template <int D> constexpr int bwd_smem() {
+  return (D / 64) * (2 * 128 * 128 + kBwdStages * 2 * 64 * 128) + 1024 + static_cast<int>(sizeof(BwdShared)) + 64;
 }
 
 template <typename T, int D>
@@ -699,8 +842,10 @@ static int attn_fwd_launch(const void* qkv, const AttnParams& p, bool bf16, cuda
   auto kern = attn_fwd_kernel<T, D>;
   static bool cfg = false;
   if (!cfg) { if (!set_smem(kern, fwd_smem<D>())) return kErrLaunch; cfg = true; }
-  dim3 grid((p.t + 127) / 128, p.b * p.h);
-  return launch_pdl(kern, grid, dim3(kAttnThreads), fwd_smem<D>(), s, 1, tmQ, tmKV, p) == cudaSuccess
+  const long long ctas = static_cast<long long>((p.t + 255) / 256) * p.b * p.h;
+  if (ctas > 0x7fffffffLL) return kErrTooLarge;
+  return launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), dim3(kAttnThreads), fwd_smem<D>(), s, 1, tmQ, tmKV,
+                    p) == cudaSuccess
              ? kOk
              : kErrLaunch;
 }
@@ -714,27 +859,30 @@ static int attn_bwd_launch(const void* qkv, const void* o, const void* do_full, 
       !do_tmap(&tmdO64, do_full, ld_do, D, p.b, p.h, p.q_end, 64, bf16) ||
       !do_tmap(&tmdO128, do_full, ld_do, D, p.b, p.h, p.q_end, 128, bf16))
     return kErrDriver;
+  const long long ctas = static_cast<long long>((p.t + 127) / 128) * p.b * p.h;
+  if (ctas > 0x7fffffffLL) return kErrTooLarge;
   {
-    const long long warps = static_cast<long long>(p.t) * p.b * p.h;
-    const int threads = 256;
-    const int blocks = static_cast<int>((warps * 32 + threads - 1) / threads);
+    const long long rows = static_cast<long long>(p.t) * p.b * p.h;
+    const long long blocks = (rows + DeltaRows<D>::value - 1) / DeltaRows<D>::value;
     const T* do_slice = static_cast<const T*>(do_full) + static_cast<long long>(p.c) * p.b * ld_do;
-    if (launch_pdl(attn_delta_kernel<T>, dim3(blocks), dim3(threads), 0, s, 1, static_cast<const T*>(o),
-                   p.ld_o, do_slice, ld_do, p.delta, p.lse_stride, p.c, p.t, p.b, p.h, D) != cudaSuccess)
+    const int o_vec = (reinterpret_cast<uintptr_t>(o) & 15) == 0 ? 1 : 0;
+    if (launch_pdl(attn_delta_kernel<T, D>, dim3(static_cast<unsigned>(blocks)), dim3(kDeltaThreads), 0, s, 1,
+                   static_cast<const T*>(o), p.ld_o, do_slice, ld_do, p.delta, p.lse_stride, p.c, p.t, p.b,
+                   p.h, o_vec) != cudaSuccess)
       return kErrLaunch;
   }
   auto k0 = attn_bwd_kernel<T, D, 0>;
   auto k1 = attn_bwd_kernel<T, D, 1>;
   static bool cfg = false;
   if (!cfg) {
-    if (!set_smem(k0, bwd_smem<D, 0>()) || !set_smem(k1, bwd_smem<D, 1>())) return kErrLaunch;
+    if (!set_smem(k0, bwd_smem<D>()) || !set_smem(k1, bwd_smem<D>())) return kErrLaunch;
     cfg = true;
   }
-  dim3 grid((p.t + 127) / 128, p.b * p.h);
-  if (launch_pdl(k0, grid, dim3(kBwdThreads), bwd_smem<D, 0>(), s, 1, tm128, tm64, tmdO128, tmdO64, p) !=
+  const dim3 grid(static_cast<unsigned>(ctas));
+  if (launch_pdl(k0, grid, dim3(kBwdThreads), bwd_smem<D>(), s, 1, tm128, tm64, tmdO128, tmdO64, p) !=
       cudaSuccess)
     return kErrLaunch;
-  return launch_pdl(k1, grid, dim3(kBwdThreads), bwd_smem<D, 1>(), s, 1, tm128, tm64, tmdO128, tmdO64, p) ==
+  return launch_pdl(k1, grid, dim3(kBwdThreads), bwd_smem<D>(), s, 1, tm128, tm64, tmdO128, tmdO64, p) ==
                  cudaSuccess
              ? kOk
              : kErrLaunch;

@@ -155,13 +155,6 @@ template <int BN, int MT = 1, bool AR = false> struct GemmCfg {
 // of the next tile (K = 2048: 16.7 k cycles for 256 columns per lane).  With two calls of erff per
 // value it did not: 1024 x 8192 x 2048 took 51 us with GeLU and 57 us with its derivative
 // against 31 us without; now 36 us and 42 us.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  union U { float2 f; unsigned long long u; } ua{a}, ub{b}, uc{c}, ud;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(ud.u) : "l"(ua.u), "l"(ub.u), "l"(uc.u));
-  return ud.f;
-}
-__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
-
 __device__ __forceinline__ float min_nan(float a, float b) {   // NaN stays NaN
   float r;
   asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));

@@ -114,6 +114,33 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+__device__ __forceinline__ uint32_t mbar_try(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok;
+}
+// Several phases at once.  A single wait costs 80 to 190 cycles even when the phase is long complete (the
+// latency of the shared-memory unit under load); the first looks at all barriers overlap here.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1,
+                                              const WaitCtx& w, int code) {
+  const uint32_t k0 = mbar_try(b0, p0), k1 = mbar_try(b1, p1);
+  return (k0 || mbar_wait(b0, p0, w, code)) && (k1 || mbar_wait(b1, p1, w, code));
+}
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, uint64_t* b2,
+                                              uint32_t p2, const WaitCtx& w, int code) {
+  const uint32_t k0 = mbar_try(b0, p0), k1 = mbar_try(b1, p1), k2 = mbar_try(b2, p2);
+  return (k0 || mbar_wait(b0, p0, w, code)) && (k1 || mbar_wait(b1, p1, w, code)) &&
+         (k2 || mbar_wait(b2, p2, w, code));
+}
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -206,6 +233,18 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with A in TMEM: 128 lanes x 16 elements of K, two 16-bit elements per column.
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // Arrive on an mbarrier once all MMAs issued so far by this thread have completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -253,6 +292,39 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+        "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+        "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+// ---------------------------------------------------------------- packed fp32 pairs
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  union U { float2 f; unsigned long long u; } ua{a}, ub{b}, uc{c}, ud;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(ud.u) : "l"(ua.u), "l"(ub.u), "l"(uc.u));
+  return ud.f;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  union U { float2 f; unsigned long long u; } ua{a}, ub{b}, ud;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(ud.u) : "l"(ua.u), "l"(ub.u));
+  return ud.f;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  union U { float2 f; unsigned long long u; } ua{a}, ub{b}, ud;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(ud.u) : "l"(ua.u), "l"(ub.u));
+  return ud.f;
+}
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
 // ---------------------------------------------------------------- CTA pairs (cta_group::2)
