@@ -218,10 +218,11 @@ class StageEngine:
         # the slices' results differ only where a sum over rows is split differently.  GPT3-1B
         # width (5 layers), batch 8, 16 slices of 128: a step took 40.5 ms slice by slice, 31.1 merged;
         # the 24-layer test model in 8 slices of 32 rows 17.4 ms against 3.4.
-        # Slices stay where something is made for them: a recorded plan, per-segment graphs that
-        # were asked for, an eager run (use_graph=False), a slice timeline, and tensor-parallel
-        # exchange buffers, whose size is a slice's.
-        self._merged = (self.pp == 1 and self.tp == 1 and (self.use_graph or self.dp > 1)
+        # Slices stay where something is made for them: a recorded plan or per-segment graphs that
+        # the caller decided about, a slice timeline, and tensor-parallel exchange buffers, whose size
+        # is a slice's.  An eager run merges like a captured one, so that both take the same sums in the
+        # same order and agree bit for bit.
+        self._merged = (self.pp == 1 and self.tp == 1
                         and self._plan is None and launch_plan is None and segment_graphs is None)
         self._alloc_activations()
         self.status = F.status_word(dev)

@@ -9,16 +9,17 @@ pytestmark = pytest.mark.gpu
                                                      ([1, 2], [37, 91])])
 def test_merged_pass_equals_slice_by_slice(batch_slices, seq_slices):
     """fp16 rounding of 2 layers' activations apart (rows come from the same kernels; sums over rows
-    are split differently), the merged engine and the eager sliced one agree."""
+    are split differently), the merged engine and one that was told to keep its slices agree."""
     from terapipe_b200.models import TransformerConfig
     from terapipe_b200.runtime.engine import StageEngine
     cfg = TransformerConfig(batch_size=3, seq_len=128, n_layers=2, embedding_dim=256,
                             num_attention_heads=4, n_devices=1)
     x = torch.randn(128, 3, 256, generator=torch.Generator().manual_seed(1))
     got = []
-    for use_graph in (True, False):
-        eng = StageEngine(cfg, batch_slices, seq_slices, use_graph=use_graph, loss_scale=1024.0, lr=1e-4)
-        assert eng._merged == use_graph
+    for merged in (True, False):
+        how = dict(use_graph=True) if merged else dict(use_graph=False, launch_plan=False)
+        eng = StageEngine(cfg, batch_slices, seq_slices, loss_scale=1024.0, lr=1e-4, **how)
+        assert eng._merged == merged
         eng.set_input(x)
         eng.compute_grads()
         grads = eng.named_grads()
