@@ -98,8 +98,8 @@ __device__ __forceinline__ void tile_of_cta(int idx, int tiles, int heads, int& 
 // ============================================================================ forward
 // A CTA owns 256 queries of one head, 128 per softmax group, and streams the keys in blocks of
 // 64: both groups use every K/V tile.  Where only one tile of queries is left (short slices, the
-// end of a long one) the two groups take alternate key blocks of that tile, and their partial
-// outputs are merged at the end.
+// end of a long one) and it has at least kSplitBlocks key blocks, the two groups take alternate
+// blocks of that tile, and their partial outputs are merged at the end.
 //
 // Each group has two S buffers and an MMA warp of its own.  P overwrites the S it came from, and
 // the scores of block k + 2 overwrite that P: they are issued right after P V of block k (MMAs of one
@@ -120,6 +120,9 @@ struct FwdShared {
 };
 
 constexpr int kFwdStages = 4;   // depth of the K and of the V ring
+// The merge costs about a microsecond: 128 queries of 8 heads took 10.8 us split over 2 blocks, 10.2 not
+// split; at 32 blocks (128 queries behind 1920 keys, 8 x 16 heads) the split takes 38.7 us, 47.4 before it.
+constexpr int kSplitBlocks = 8;
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kAttnThreads, 1)
@@ -144,12 +147,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tile_of_cta(blockIdx.x, tiles, p.b * p.h, rank, bh);
   const int bi = bh / p.h, hi = bh % p.h;
   const int q0 = (tiles - 1 - rank) * 256;
-  const bool split = q0 + 128 >= p.t;      // one tile of queries: the groups share its key blocks
   // key blocks of the first tile and of the last
   const int nb0 = (p.c + min(p.t, q0 + 128) + 63) / 64;
-  const int n = (p.c + min(p.t, q0 + 256) + 63) / 64;   // = nb0 when split; blocks that are loaded
+  const int n = (p.c + min(p.t, q0 + 256) + 63) / 64;   // blocks that are loaded
+  const bool single = q0 + 128 >= p.t;                  // one tile of queries (n = nb0)
+  const bool split = single && nb0 >= kSplitBlocks;     // the groups share its key blocks
   // blocks of the two groups: the k-th block of group w is blk(w, k)
-  const int n_it0 = split ? (nb0 + 1) / 2 : nb0, n_it1 = split ? nb0 / 2 : n;
+  const int n_it0 = split ? (nb0 + 1) / 2 : nb0, n_it1 = split ? nb0 / 2 : single ? 0 : n;
   auto blk = [&](int w, int k) { return split ? 2 * k + w : k; };
 
   if (threadIdx.x == 0) {
@@ -164,9 +168,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     for (int i = 0; i < KS; ++i) {
       mbar_init(&sh->bar_k[i], 1);
-      mbar_init(&sh->bar_kfree[i], split ? 1 : 2);   // users of a block
+      mbar_init(&sh->bar_kfree[i], single ? 1 : 2);   // users of a block
       mbar_init(&sh->bar_v[i], 1);
-      mbar_init(&sh->bar_vfree[i], split ? 1 : 2);
+      mbar_init(&sh->bar_vfree[i], single ? 1 : 2);
     }
     sh->abort_flag = 0;
     fence_barrier_init();
@@ -201,7 +205,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int ahead = split ? 4 : 2;
       load_q(0);
       bool ok = load_kv(sK, sh->bar_k, sh->bar_kfree, D, 0);
-      if (!split) load_q(1);
+      if (!single) load_q(1);
       for (int j = 1; j < ahead && j < n && ok; ++j) ok = load_kv(sK, sh->bar_k, sh->bar_kfree, D, j);
       for (int j = 0; j < n && ok; ++j) {
         // (the groups differ by at most two blocks, which are the last ones: their tiles, which
@@ -216,7 +220,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (n_it > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_f16(Elem<T>::fmt, 0, 0, 128, 64);
       constexpr uint32_t idesc_pv = umma_idesc_f16(Elem<T>::fmt, 0, 1, 128, D);
-      const uint32_t dQ = desc_k(smem_u32(sQ + (split ? 0 : w * kQTile))), dK = desc_k(smem_u32(sK)),
+      const uint32_t dQ = desc_k(smem_u32(sQ + (single ? 0 : w * kQTile))), dK = desc_k(smem_u32(sK)),
                      dV = desc_n(smem_u32(sV), kKSub);
       const uint32_t tSw = tmem + w * 128, tOw = tmem + 256 + w * D;
       auto issue_s = [&](int k) {
@@ -225,7 +229,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         umma_commit(&sh->bar_s[w][k & 1]);
         umma_commit(&sh->bar_kfree[st]);
       };
-      bool ok = mbar_wait(&sh->bar_q[split ? 0 : w], 0, wctx, kErrWaitAttn);
+      bool ok = mbar_wait(&sh->bar_q[single ? 0 : w], 0, wctx, kErrWaitAttn);
       for (int k = 0; k < 2 && k < n_it && ok; ++k) {
         const int j = blk(w, k);
         ok = mbar_wait(&sh->bar_k[j % KS], (j / KS) & 1, wctx, kErrWaitAttn);
@@ -252,7 +256,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int r = threadIdx.x & 127;       // row of the tile = TMEM lane
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS = tmem + w * 128 + lane_base, tO = tmem + 256 + w * D + lane_base;
-    const int qt = q0 + (split ? 0 : w * 128);   // first query of the tile
+    const int qt = q0 + (single ? 0 : w * 128);   // first query of the tile
     const int qi = qt + r;
     const int qpos = p.c + qi;
     const int n_it = w == 0 ? n_it0 : n_it1;
@@ -356,6 +360,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(raw[i]);
     };
     if (!split) {
+      ok = ok && n_it > 0;     // (the second group of a short single tile has nothing)
       if (ok) ok = mbar_wait(&sh->bar_fin[w], 0, wctx, kErrWaitAttn);
       if (ok) {
         tc_fence_after();
