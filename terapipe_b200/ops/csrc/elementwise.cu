@@ -293,74 +293,135 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
   push_signal(pd);
 }
 
-// dgamma[c] += sum_p scratch[p][0][c]; dbeta[c] += sum_p scratch[p][1][c]; optionally clears the
-// slots afterwards.  blockDim = (32, 8): 32 columns per CTA, 8 lanes over the slots (4 loads in
-// flight per thread), fixed-order tree in shared memory.
+// ------------------------------------------------------------------ bias and LayerNorm gradients
+// All column sums of a layer in one launch: db[n] += sum_rows dy[row][n] for up to kMaxColsums
+// matrices of the same number of rows, and the fold of up to kMaxFolds sets of LayerNorm partial
+// slots (as layernorm_bwd_reduce_kernel, clearing the slots).  Each is a handful of CTAs or a few
+// microseconds long, so separate launches cost more than the sums.  A CTA of 32 x 8 threads
+// takes 256 columns of a chunk of rows, 8 rows of 16 bytes per thread in flight.  The (at most 8) chunks
+// of a column block form a cluster whose first CTA adds them up in order through distributed shared
+// memory, so the sums do not depend on timing; 8 chunks give a 2048-wide layer 576 CTAs.  (One launch per
+// matrix with one load in flight per thread ran on 64 of 148 SMs: 16384 x 2048 took 63 us, 1.1 TB/s.)
+constexpr int kMaxColsums = 4, kMaxFolds = 2;
+struct SumJobs {
+  const void* dy[kMaxColsums];
+  float* db[kMaxColsums];
+  long long ld[kMaxColsums];
+  int N[kMaxColsums];
+  int cta_end[kMaxColsums];      // CTAs [cta_end[i - 1], cta_end[i]) work on matrix i
+  int n, rows, chunks, rows_per_chunk;   // chunks = cluster size
+  float* slots[kMaxFolds];
+  float* dgamma[kMaxFolds];
+  float* dbeta[kMaxFolds];
+  int folds, parts, H;           // the CTAs behind the matrices' fold 32 columns each
+};
+
+// Fold 32 columns, from column c0 on, of slots [parts][2][H]; thread (tx, ty) of (32, 8), 4 loads in
+// flight each, fixed-order tree in shared memory.
 // clear bit 0: zero the slots afterwards; bit 1: overwrite dgamma/dbeta instead of adding.
+__device__ __forceinline__ void fold_slots(float* __restrict__ slots, int parts, int H, int c0,
+                                           float* __restrict__ dgamma, float* __restrict__ dbeta,
+                                           int tx, int ty, int clear, float (&sm)[8][33]) {
+  const int c = c0 + tx;
+  const long long stride = 2ll * H;
+  float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+  if (c < 2 * H) {
+    int p = ty;
+    for (; p + 24 < parts; p += 32) {
+      s0 += __ldcg(slots + p * stride + c);
+      s1 += __ldcg(slots + (p + 8) * stride + c);
+      s2 += __ldcg(slots + (p + 16) * stride + c);
+      s3 += __ldcg(slots + (p + 24) * stride + c);
+    }
+    for (; p < parts; p += 8) s0 += __ldcg(slots + p * stride + c);
+    if (clear & 1)
+      for (int q = ty; q < parts; q += 8) slots[q * stride + c] = 0.0f;
+  }
+  sm[ty][tx] = (s0 + s1) + (s2 + s3);
+  __syncthreads();
+  if (ty == 0 && c < 2 * H) {
+    float t = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += sm[i][tx];
+    float* dst = c < H ? dgamma + c : dbeta + (c - H);
+    *dst = (clear & 2) ? t : *dst + t;
+  }
+}
+
+// dgamma[c] += sum_p scratch[p][0][c]; dbeta[c] += sum_p scratch[p][1][c]; blockDim = (32, 8), 32
+// columns per CTA; `clear` as in fold_slots.
 __global__ void layernorm_bwd_reduce_kernel(float* __restrict__ scratch, int parts, int H,
                                             float* __restrict__ dgamma, float* __restrict__ dbeta,
                                             int clear) {
   __shared__ float sm[8][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  const long long stride = 2ll * H;
-  float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-  if (c < 2 * H) {
-    int p = threadIdx.y;
-    for (; p + 24 < parts; p += 32) {
-      s0 += __ldcg(scratch + p * stride + c);
-      s1 += __ldcg(scratch + (p + 8) * stride + c);
-      s2 += __ldcg(scratch + (p + 16) * stride + c);
-      s3 += __ldcg(scratch + (p + 24) * stride + c);
-    }
-    for (; p < parts; p += 8) s0 += __ldcg(scratch + p * stride + c);
-    if (clear & 1)
-      for (int q = threadIdx.y; q < parts; q += 8) scratch[q * stride + c] = 0.0f;
-  }
-  sm[threadIdx.y][threadIdx.x] = (s0 + s1) + (s2 + s3);
-  __syncthreads();
-  if (threadIdx.y == 0 && c < 2 * H) {
-    float t = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t += sm[i][threadIdx.x];
-    if (clear & 2) {
-      if (c < H) dgamma[c] = t;
-      else dbeta[c - H] = t;
-    } else {
-      if (c < H) dgamma[c] += t;
-      else dbeta[c - H] += t;
-    }
-  }
+  pdl_wait();
+  fold_slots(scratch, parts, H, blockIdx.x * 32, dgamma, dbeta, threadIdx.x, threadIdx.y, clear, sm);
 }
 
-// ------------------------------------------------------------------ bias gradient
-// db[n] += sum_rows dy[row][n]; blockDim = (32, 16): 32 vectors of 8 columns, 16 row lanes.
 template <typename T>
-__global__ void colsum_kernel(const T* __restrict__ dy, long long ld, int rows, int N,
-                              float* __restrict__ db) {
-  __shared__ float sm[16][32][8 + 1];
-  const int col = (blockIdx.x * 32 + threadIdx.x) * 8;
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (col < N) {
-    for (int r = blockIdx.y * 16 + threadIdx.y; r < rows; r += 16 * gridDim.y) {
-      float v[8];
-      load8(dy + static_cast<long long>(r) * ld + col, v);
+__global__ void __launch_bounds__(256)
+layer_sums_kernel(const SumJobs j) {
+  __shared__ union { float col[8][32][8 + 1]; float fold[8][33]; } sm;
+  __shared__ float chunk_sum[256];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int cta = blockIdx.x;
+  pdl_wait();
+  int first = 0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += v[j];
+  for (int i = 0; i < kMaxColsums; ++i) {
+    if (i >= j.n) break;
+    if (cta < j.cta_end[i]) {
+      const int chunk = (cta - first) % j.chunks;
+      const int col = ((cta - first) / j.chunks * 32 + tx) * 8;
+      const int r_end = min(j.rows, (chunk + 1) * j.rows_per_chunk);
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (col < j.N[i]) {
+        const T* src = static_cast<const T*>(j.dy[i]) + col;
+        for (int r = chunk * j.rows_per_chunk + ty; r < r_end; r += 64) {
+          uint4 v[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            v[k] = r + 8 * k < r_end ? *reinterpret_cast<const uint4*>(src + (r + 8 * k) * j.ld[i])
+                                     : make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            float f[8];
+            unpack8<T>(v[k], f);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q] += f[q];
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) sm.col[ty][tx][q] = acc[q];
+      __syncthreads();
+      // thread (tx, ty) finishes column ty of vector tx
+      float s = 0.0f;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) s += sm.col[r][tx][ty];
+      if (j.chunks > 1) {   // (the CTAs of a cluster are the chunks of one column block)
+        chunk_sum[ty * 32 + tx] = s;
+        cluster_sync_all();
+        if (chunk == 0) {
+          for (int q = 1; q < j.chunks; ++q) {
+            float v;
+            asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                         : "=f"(v) : "r"(mapa_u32(smem_u32(&chunk_sum[ty * 32 + tx]), q)) : "memory");
+            s += v;
+          }
+        }
+        cluster_sync_all();   // nobody leaves while its sums may be read
+        if (chunk != 0) return;
+      }
+      if (col < j.N[i]) j.db[i][col + ty] += s;
+      return;
     }
+    first = j.cta_end[i];
   }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) sm[threadIdx.y][threadIdx.x][j] = acc[j];
-  __syncthreads();
-  if (threadIdx.y < 8) {
-    // thread (x, y<8) finishes column col + y
-    float s = 0.0f;
-#pragma unroll
-    for (int r = 0; r < 16; ++r) s += sm[r][threadIdx.x][threadIdx.y];
-    if (col + threadIdx.y < N) {
-      if (gridDim.y == 1) db[col + threadIdx.y] += s;
-      else atomicAdd(&db[col + threadIdx.y], s);
-    }
-  }
+  const int per_fold = (2 * j.H + 31) / 32;
+  const int f = (cta - first) / per_fold;
+  if (f >= j.folds) return;        // (the grid is a whole number of clusters)
+  fold_slots(j.slots[f], j.parts, j.H, (cta - first) % per_fold * 32, j.dgamma[f], j.dbeta[f], tx, ty, 1, sm.fold);
 }
 
 // ------------------------------------------------------------------ fused Adam
@@ -565,8 +626,8 @@ static int layernorm_bwd_launch(int dtype, const void* dy, const void* x, const 
   else { TP_LN_DISPATCH(__half, LN_BWD) }
 #undef LN_BWD
   if (mode == 0)
-    layernorm_bwd_reduce_kernel<<<(2 * H + 31) / 32, dim3(32, 8), 0, s>>>(scratch, parts, H, dgamma,
-                                                                          dbeta, 0);
+    launch_pdl(layernorm_bwd_reduce_kernel, dim3((2 * H + 31) / 32), dim3(32, 8), 0, s, 1, scratch, parts, H,
+               dgamma, dbeta, 0);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 }  // namespace tp
@@ -604,8 +665,8 @@ extern "C" int tp_layernorm_bwd_accum_push(int dtype, const void* dy, const void
 // Fold `parts` slots into dgamma/dbeta (+=) and clear them for the next backward pass.
 extern "C" int tp_layernorm_bwd_finish(float* slots, int parts, int H, float* dgamma, float* dbeta,
                                        void* stream) {
-  layernorm_bwd_reduce_kernel<<<(2 * H + 31) / 32, dim3(32, 8), 0, static_cast<cudaStream_t>(stream)>>>(
-      slots, parts, H, dgamma, dbeta, 1);
+  launch_pdl(layernorm_bwd_reduce_kernel, dim3((2 * H + 31) / 32), dim3(32, 8), 0,
+             static_cast<cudaStream_t>(stream), 1, slots, parts, H, dgamma, dbeta, 1);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
@@ -613,25 +674,60 @@ extern "C" int tp_layernorm_bwd_finish(float* slots, int parts, int H, float* dg
 // sums of several ranks are added up afterwards, see tp_peer_sum).
 extern "C" int tp_layernorm_bwd_finish_assign(float* slots, int parts, int H, float* dgamma,
                                               float* dbeta, void* stream) {
-  layernorm_bwd_reduce_kernel<<<(2 * H + 31) / 32, dim3(32, 8), 0, static_cast<cudaStream_t>(stream)>>>(
-      slots, parts, H, dgamma, dbeta, 3);
+  launch_pdl(layernorm_bwd_reduce_kernel, dim3((2 * H + 31) / 32), dim3(32, 8), 0,
+             static_cast<cudaStream_t>(stream), 1, slots, parts, H, dgamma, dbeta, 3);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
+
+namespace tp {
+static int layer_sums_launch(int dtype, SumJobs& j, cudaStream_t s) {
+  // chunks of at least 64 rows (one round of loads), a portable cluster of them at most
+  j.chunks = 1;
+  while (j.n > 0 && j.chunks < 8 && j.rows >= 128 * j.chunks) j.chunks *= 2;
+  j.rows_per_chunk = (j.rows + j.chunks - 1) / j.chunks;
+  long long ctas = 0;
+  for (int i = 0; i < j.n; ++i) {
+    ctas += (j.N[i] / 8 + 31) / 32 * static_cast<long long>(j.chunks);
+    j.cta_end[i] = static_cast<int>(ctas);
+  }
+  ctas += static_cast<long long>(j.folds) * ((2 * j.H + 31) / 32);
+  if (ctas == 0) return kOk;
+  ctas = (ctas + j.chunks - 1) / j.chunks * j.chunks;
+  if (ctas > 0x7fffffffLL) return kErrTooLarge;
+  const dim3 grid(static_cast<unsigned>(ctas)), block(32, 8);
+  const cudaError_t e = dtype == 1 ? launch_pdl(layer_sums_kernel<__nv_bfloat16>, grid, block, 0, s, j.chunks, j)
+                                   : launch_pdl(layer_sums_kernel<__half>, grid, block, 0, s, j.chunks, j);
+  return e == cudaSuccess ? kOk : kErrLaunch;
+}
+}  // namespace tp
 
 extern "C" int tp_colsum(int dtype, const void* dy, long long ld, int rows, int N, float* db,
                          void* stream) {
   if (rows <= 0) return kOk;
-  if (N % 8 || ld % 8) return kErrBadArgument;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  dim3 block(32, 16);
-  int gy = rows / 256;
-  gy = gy < 1 ? 1 : (gy > 8 ? 8 : gy);
-  dim3 grid((N / 8 + 31) / 32, gy);
-  if (dtype == 1)
-    colsum_kernel<__nv_bfloat16><<<grid, block, 0, s>>>(static_cast<const __nv_bfloat16*>(dy), ld, rows, N, db);
-  else
-    colsum_kernel<__half><<<grid, block, 0, s>>>(static_cast<const __half*>(dy), ld, rows, N, db);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+  if (N <= 0 || N % 8 || ld % 8) return kErrBadArgument;
+  SumJobs j = {};
+  j.dy[0] = dy; j.ld[0] = ld; j.N[0] = N; j.db[0] = db;
+  j.n = 1; j.rows = rows;
+  return layer_sums_launch(dtype, j, static_cast<cudaStream_t>(stream));
+}
+
+// The bias gradients (`n` <= 4 matrices dy[i] [rows][N[i]], added to db[i]) and LayerNorm parameter
+// gradients (`folds` <= 2 sets of slots as for tp_layernorm_bwd_finish) of one layer in one launch.
+extern "C" int tp_layer_sums(int dtype, int n, const void* const* dy, const long long* ld, const int* N,
+                             float* const* db, int rows, int folds, float* const* slots, int parts, int H,
+                             float* const* dgamma, float* const* dbeta, void* stream) {
+  if (n < 0 || n > kMaxColsums || folds < 0 || folds > kMaxFolds || rows < 0 ||
+      (folds > 0 && (H <= 0 || parts <= 0)))
+    return kErrBadArgument;
+  SumJobs j = {};
+  j.n = n; j.rows = rows;
+  for (int i = 0; i < n; ++i) {
+    if (N[i] <= 0 || N[i] % 8 || ld[i] % 8) return kErrBadArgument;
+    j.dy[i] = dy[i]; j.ld[i] = ld[i]; j.N[i] = N[i]; j.db[i] = db[i];
+  }
+  j.folds = folds; j.parts = parts; j.H = H;
+  for (int f = 0; f < folds; ++f) { j.slots[f] = slots[f]; j.dgamma[f] = dgamma[f]; j.dbeta[f] = dbeta[f]; }
+  return layer_sums_launch(dtype, j, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tp_adam_tick(float* state, float beta1, float beta2, void* stream) {

@@ -88,6 +88,7 @@ SIGNATURES = {
     "tp_layernorm_bwd_accum": [I, P, P, P, P, P, P, P, P, I, I, P],
     "tp_layernorm_bwd_finish": [P, I, I, P, P, P],
     "tp_colsum": [I, P, L, I, I, P, P],
+    "tp_layer_sums": [I, I, P, P, P, P, I, I, P, I, I, P, P, P],
     "tp_adam_tick": [P, F, F, P],
     "tp_fused_adam": [I, P, P, P, P, P, L, P, F, F, F, F, F, F, P],
     "tp_fill": [I, P, L, F, P],

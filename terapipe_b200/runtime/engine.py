@@ -31,6 +31,7 @@ GEMM + all-reduce kernel over NVLink peer memory (``tp_comm="fused"``).
 """
 from __future__ import annotations
 
+import ctypes
 import gc
 import math
 import os
@@ -234,11 +235,11 @@ class StageEngine:
         self._streams_ready = False
         # launches of this library's own kernels (NCCL and torch kernels are not counted):
         # per layer and slice 7 forward (2 LN, 4 GEMM, attention) and 9 backward (4 GEMM,
-        # 2 LN, 3 attention); per layer 10 after the last slice (4 weight-gradient GEMMs, 4 bias
-        # column sums, 2 LayerNorm-gradient reductions); plus 2 for the optimizer
+        # 2 LN, 3 attention); per layer 5 after the last slice (4 weight-gradient GEMMs, the bias
+        # and LayerNorm gradients in one); plus 2 for the optimizer
         n_slices = len(self.batch_slices) * len(self.seq_slices)
         per_layer = 12 + 4 * len(self.batch_slices) if self._merged else 16 * n_slices
-        self.launches_per_step = self.n_layers * (per_layer + 10) + 2
+        self.launches_per_step = self.n_layers * (per_layer + 5 + (2 if self.sp else 0)) + 2
         self.launch_count = 0
         self._ar_calls_per_step = n_slices * self.n_layers * 4 + 1
         # sequence parallel: all-gather pushes per step (2 per layer and slice forward; backward one
@@ -833,17 +834,18 @@ class StageEngine:
             dfc, dqkv = self.dFc[l].data_ptr(), self.dQKV[l].data_ptr()
             self._gemm(dxo, H, self.fa[l].data_ptr(), Fl, self._p(l, "fc2.weight", g), Fl, H, Fl, R,
                        a_mn=1, b_mn=1, out_f32=1, accumulate=1)
-            self._ln("tp_colsum", dt, dxo, H, R, H, self._p(l, "fc2.bias", g), s)
             self._gemm(dfc, Fl, self.ln2[l].data_ptr(), H, self._p(l, "fc1.weight", g), H, Fl, H, R,
                        a_mn=1, b_mn=1, out_f32=1, accumulate=1)
-            self._ln("tp_colsum", dt, dfc, Fl, R, Fl, self._p(l, "fc1.bias", g), s)
             self._gemm(dmid, H, self.ao[l].data_ptr(), Hl, self._p(l, "attn.out_proj.weight", g), Hl,
                        H, Hl, R, a_mn=1, b_mn=1, out_f32=1, accumulate=1)
-            self._ln("tp_colsum", dt, dmid, H, R, H, self._p(l, "attn.out_proj.bias", g), s)
             self._gemm(dqkv, 3 * Hl, self.ln1[l].data_ptr(), H, self._p(l, "attn.in_proj.weight", g),
                        H, 3 * Hl, H, R, a_mn=1, b_mn=1, out_f32=1, accumulate=1)
-            self._ln("tp_colsum", dt, dqkv, 3 * Hl, R, 3 * Hl, self._p(l, "attn.in_proj.bias", g), s)
             slots = self.ln_slots[l].data_ptr()
+            # all bias gradients (column sums of the same dY) and, unless the ranks' sums have to be
+            # added up first, the LayerNorm gradients: one launch
+            self._layer_sums(l, ((dxo, H, "fc2.bias"), (dfc, Fl, "fc1.bias"), (dmid, H, "attn.out_proj.bias"),
+                                 (dqkv, 3 * Hl, "attn.in_proj.bias")),
+                             () if self.sp else ((slots, "attn_ln"), (slots + self.ln_parts * 2 * H * 4, "fc_ln")))
             if self.sp:
                 # this rank's slots hold the sums over its token shards only: fold them into a
                 # peer-visible pack; the sums of all ranks are added after the barrier below
@@ -851,11 +853,6 @@ class StageEngine:
                 self._ln("tp_layernorm_bwd_finish_assign", slots, self.ln_parts, H, pack, pack + H * 4, s)
                 self._ln("tp_layernorm_bwd_finish_assign", slots + self.ln_parts * 2 * H * 4, self.ln_parts, H,
                                                    pack + 2 * H * 4, pack + 3 * H * 4, s)
-                continue
-            self._ln("tp_layernorm_bwd_finish", slots, self.ln_parts, H, self._p(l, "attn_ln.weight", g),
-                                        self._p(l, "attn_ln.bias", g), s)
-            self._ln("tp_layernorm_bwd_finish", slots + self.ln_parts * 2 * H * 4, self.ln_parts, H,
-                                        self._p(l, "fc_ln.weight", g), self._p(l, "fc_ln.bias", g), s)
         if overlap and self.n_layers:
             self._dp_layer_done(0, works)
             if self.dp_sym is not None:
@@ -870,6 +867,17 @@ class StageEngine:
                                 self.tp_idx, s)
                 self._ln("tp_peer_sum", self._p(l, "fc_ln.weight", g), 2 * H, self.ar.out_ptrs(off + 2 * H * 4),
                                 self.tp, self.tp_idx, s)
+
+    def _layer_sums(self, l, mats, folds) -> None:
+        """``mats``: (address of ``[rows, width]``, width, bias name) whose column sums are added to the
+        bias gradient; ``folds``: (address of the partial slots, LayerNorm name)."""
+        n, m, g = len(mats), len(folds), self.grad
+        P, LL, I = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
+        self._ln("tp_layer_sums", self.dt, n, (P * n)(*[a for a, _, _ in mats]), (LL * n)(*[w for _, w, _ in mats]),
+                 (I * n)(*[w for _, w, _ in mats]), (P * n)(*[self._p(l, name, g) for _, _, name in mats]), self.rows,
+                 m, (P * m)(*[a for a, _ in folds]), self.ln_parts, self.H,
+                 (P * m)(*[self._p(l, name + ".weight", g) for _, name in folds]),
+                 (P * m)(*[self._p(l, name + ".bias", g) for _, name in folds]), self._stream)
 
     def _group_barrier(self, index: int) -> None:
         """Device-side barrier of the tensor-parallel group (``index`` 1 or 2 within a step)."""
