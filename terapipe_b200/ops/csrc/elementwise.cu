@@ -107,8 +107,11 @@ __device__ __forceinline__ float group_sum_named(float v, float* red, int slot, 
   return t;
 }
 
+// Forward.  Memory bound: what counts is how many rows an SM has in flight.  The row stays in its 16-bit
+// form (NV registers of 16 bytes; unpacked again for each of the three passes over it), which lets four
+// CTAs of 8 warps share an SM; with the row in fp32 only two fitted and 16384 x 2048 took 52 us.
 template <typename T, int NV, int WPR>
-__global__ void __launch_bounds__(LnGeom<WPR>::kThreads)
+__global__ void __launch_bounds__(LnGeom<WPR>::kThreads, 1024 / LnGeom<WPR>::kThreads)
 layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
                      const T* __restrict__ beta, const PushDst pd, float* __restrict__ mean_out,
                      float* __restrict__ rstd_out, int rows, int H, float eps) {
@@ -119,23 +122,19 @@ layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   pdl_wait();
   const long long row = static_cast<long long>(blockIdx.x) * G::kRowsPerCta + grp;
   const bool row_ok = row < rows;
-  float v[NV][8];
-  uint4 gq[NV], bq[NV];   // gamma / beta of this lane's columns, fetched with the row (16-bit, packed)
-  float s = 0.0f;
+  uint4 xq[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int col = ((i * WPR + wr) * 32 + lane) * 8;
+    xq[i] = row_ok && col < H ? *reinterpret_cast<const uint4*>(x + row * H + col) : make_uint4(0, 0, 0, 0);
+  }
+  float s = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[i][j] = 0.0f;
-    gq[i] = make_uint4(0, 0, 0, 0);
-    bq[i] = make_uint4(0, 0, 0, 0);
-    if (row_ok && col < H) {
-      load8(x + row * H + col, v[i]);
-      gq[i] = *reinterpret_cast<const uint4*>(gamma + col);
-      bq[i] = *reinterpret_cast<const uint4*>(beta + col);
+  for (int i = 0; i < NV; ++i) {
+    float v[8];
+    unpack8<T>(xq[i], v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += v[i][j];
-    }
+    for (int j = 0; j < 8; ++j) s += v[j];
   }
   const float mean = group_sum_named<WPR, G::kRowsPerCta>(s, red, 0, grp, wr, lane) / H;
   float q = 0.0f;
@@ -143,9 +142,11 @@ layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   for (int i = 0; i < NV; ++i) {
     const int col = ((i * WPR + wr) * 32 + lane) * 8;
     if (col < H) {
+      float v[8];
+      unpack8<T>(xq[i], v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float d = v[i][j] - mean;
+        const float d = v[j] - mean;
         q += d * d;
       }
     }
@@ -160,11 +161,12 @@ layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
     for (int i = 0; i < NV; ++i) {
       const int col = ((i * WPR + wr) * 32 + lane) * 8;
       if (col < H) {
-        float g[8], b[8], o[8];
-        unpack8<T>(gq[i], g);
-        unpack8<T>(bq[i], b);
+        float v[8], g[8], b[8], o[8];
+        unpack8<T>(xq[i], v);
+        load8(gamma + col, g);
+        load8(beta + col, b);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = (v[i][j] - mean) * rstd * g[j] + b[j];
+        for (int j = 0; j < 8; ++j) o[j] = (v[j] - mean) * rstd * g[j] + b[j];
         for (int d = 0; d < pd.n; ++d) store8(static_cast<T*>(pd.dst[d]) + row * H + col, o);
       }
     }
@@ -172,10 +174,10 @@ layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   push_signal(pd);
 }
 
-// Backward geometry: 16 warps per CTA, so a CTA holds 16 / WPR rows at a time (8 rows of 2048
-// columns; one CTA per SM then covers 1184 rows, a whole 1024-row token slice, in one pass).
+// Backward geometry: one CTA per SM of 24 warps (16 where a row takes 16), so an SM holds 24 / WPR
+// rows at a time, each with its three inputs in flight.
 template <int WPR> struct LnBwdGeom {
-  static constexpr int kWarps = 16;
+  static constexpr int kWarps = WPR == 16 ? 16 : 24;
   static constexpr int kRowsPerCta = kWarps / WPR;
   static constexpr int kThreads = kWarps * 32;
 };
@@ -183,10 +185,13 @@ template <int WPR> struct LnBwdGeom {
 // dx = rstd * (g - mean(g) - xhat * mean(g * xhat)) (+ dres), g = dy * gamma.
 // Persistent CTAs stride over rows.  The partial sums of dgamma = sum dy*xhat and dbeta = sum dy
 // live in shared memory, one [2][H] region per row group, each lane adding to its own columns
-// (no synchronisation inside the loop, and no accumulator registers: 512 threads fit).  Inside a
-// region the two 16-byte halves of a lane's 8 columns lie in two planes, [array][half][H / 8][4],
-// so that neighbouring lanes touch neighbouring 16 bytes (no bank conflicts).  At the end the regions are added in a fixed order and the CTA writes (or adds to) one
-// slot of scratch[gridDim.x][2][H]; a second kernel adds the slots into the fp32 gradients.
+// (no synchronisation inside the loop).  Inside a region the two 16-byte halves of a lane's 8
+// columns lie in two planes, [array][half][H / 8][4], so that neighbouring lanes touch neighbouring
+// 16 bytes (no bank conflicts).  At the end the regions are added in a fixed order and the CTA
+// writes (or adds to) one slot of scratch[gridDim.x][2][H]; a second kernel adds the slots into
+// the fp32 gradients.  x, dy and dres of a row are loaded together and stay in their 16-bit form (xhat
+// and g are computed twice), which fits 24 warps; 16 warps that fetched dres after the row's
+// reductions took 98 us for 16384 x 2048.
 template <typename T, int NV, int WPR>
 __global__ void __launch_bounds__(LnBwdGeom<WPR>::kThreads, 1)
 layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
@@ -199,51 +204,51 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = warp / WPR, wr = warp % WPR;
   float* my_part = part_smem + static_cast<long long>(grp) * 2 * H;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int col = ((i * WPR + wr) * 32 + lane) * 8;
-    if (col < H) {
-      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      float4* sgam = reinterpret_cast<float4*>(my_part + (col >> 1));
-      float4* sbet = reinterpret_cast<float4*>(my_part + H + (col >> 1));
-      sgam[0] = z; sgam[H >> 3] = z; sbet[0] = z; sbet[H >> 3] = z;
-    }
-  }
   pdl_wait();
   int parity = 0;
+  bool fresh = true;      // the group's region holds nothing yet
+  const uint4 zero4 = make_uint4(0, 0, 0, 0);
   for (long long base = static_cast<long long>(blockIdx.x) * G::kRowsPerCta; base < rows;
-       base += static_cast<long long>(gridDim.x) * G::kRowsPerCta, parity ^= 1) {
+       base += static_cast<long long>(gridDim.x) * G::kRowsPerCta, parity ^= 1, fresh = false) {
     const long long row = base + grp;
     const bool row_ok = row < rows;
+    uint4 xq[NV], dq[NV], rq[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int col = ((i * WPR + wr) * 32 + lane) * 8;
+      const bool in = row_ok && col < H;
+      xq[i] = in ? *reinterpret_cast<const uint4*>(x + row * H + col) : zero4;
+      dq[i] = in ? *reinterpret_cast<const uint4*>(dy + row * H + col) : zero4;
+      rq[i] = in && dres ? *reinterpret_cast<const uint4*>(dres + row * H + col) : zero4;
+    }
     const float mu = row_ok ? mean[row] : 0.0f, rs = row_ok ? rstd[row] : 0.0f;
-    float xh[NV][8], g[NV][8];
     float s1 = 0.0f, s2 = 0.0f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int col = ((i * WPR + wr) * 32 + lane) * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { xh[i][j] = 0.0f; g[i][j] = 0.0f; }
-      if (row_ok && col < H) {
-        float xv[8], dyv[8], gam[8];
-        load8(x + row * H + col, xv);
-        load8(dy + row * H + col, dyv);
+      if (col < H) {
+        float xv[8], dyv[8], gam[8], pg[8];
+        unpack8<T>(xq[i], xv);
+        unpack8<T>(dq[i], dyv);
         load8(gamma + col, gam);
-        float4* sgam = reinterpret_cast<float4*>(my_part + (col >> 1));      // half 0; half 1 is
-        float4* sbet = reinterpret_cast<float4*>(my_part + H + (col >> 1));  // H / 2 floats further
-        float pg[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] = (xv[j] - mu) * rs;
-          g[i][j] = dyv[j] * gam[j];
-          s1 += g[i][j];
-          s2 += g[i][j] * xh[i][j];
-          pg[j] = dyv[j] * xh[i][j];
+          const float xh = (xv[j] - mu) * rs, g = dyv[j] * gam[j];
+          s1 += g;
+          s2 += g * xh;
+          pg[j] = dyv[j] * xh;
         }
+        float4* sgam = reinterpret_cast<float4*>(my_part + (col >> 1));      // half 0; half 1 is
+        float4* sbet = reinterpret_cast<float4*>(my_part + H + (col >> 1));  // H / 2 floats further
 #pragma unroll
         for (int hlf = 0; hlf < 2; ++hlf) {
-          float4 a = sgam[hlf * (H >> 3)], c = sbet[hlf * (H >> 3)];
-          a.x += pg[4 * hlf]; a.y += pg[4 * hlf + 1]; a.z += pg[4 * hlf + 2]; a.w += pg[4 * hlf + 3];
-          c.x += dyv[4 * hlf]; c.y += dyv[4 * hlf + 1]; c.z += dyv[4 * hlf + 2]; c.w += dyv[4 * hlf + 3];
+          float4 a = make_float4(pg[4 * hlf], pg[4 * hlf + 1], pg[4 * hlf + 2], pg[4 * hlf + 3]);
+          float4 c = make_float4(dyv[4 * hlf], dyv[4 * hlf + 1], dyv[4 * hlf + 2], dyv[4 * hlf + 3]);
+          if (!fresh) {
+            const float4 a0 = sgam[hlf * (H >> 3)], c0 = sbet[hlf * (H >> 3)];
+            a.x += a0.x; a.y += a0.y; a.z += a0.z; a.w += a0.w;
+            c.x += c0.x; c.y += c0.y; c.z += c0.z; c.w += c0.w;
+          }
           sgam[hlf * (H >> 3)] = a;
           sbet[hlf * (H >> 3)] = c;
         }
@@ -256,15 +261,14 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
       for (int i = 0; i < NV; ++i) {
         const int col = ((i * WPR + wr) * 32 + lane) * 8;
         if (col < H) {
-          float o[8];
+          float xv[8], dyv[8], gam[8], r[8], o[8];
+          unpack8<T>(xq[i], xv);
+          unpack8<T>(dq[i], dyv);
+          unpack8<T>(rq[i], r);
+          load8(gamma + col, gam);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = rs * (g[i][j] - m1 - xh[i][j] * m2);
-          if (dres) {
-            float r[8];
-            load8(dres + row * H + col, r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += r[j];
-          }
+          for (int j = 0; j < 8; ++j)
+            o[j] = rs * (dyv[j] * gam[j] - m1 - (xv[j] - mu) * rs * m2) + r[j];
           for (int d = 0; d < pd.n; ++d) store8(static_cast<T*>(pd.dst[d]) + row * H + col, o);
         }
       }
@@ -589,12 +593,12 @@ template <typename K> static void ln_allow_smem(K kern) {
   const void* key = reinterpret_cast<const void*>(kern);
   for (int i = 0; i < n_seen; ++i)
     if (seen[i] == key) return;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
   if (n_seen < 64) seen[n_seen++] = key;
 }
 
 static int ln_parts(int rows, int wpr) {
-  const int rpc = 16 / wpr;   // LnBwdGeom<WPR>::kRowsPerCta
+  const int rpc = wpr == 16 ? 1 : 24 / wpr;   // LnBwdGeom<WPR>::kRowsPerCta
   int parts = (rows + rpc - 1) / rpc;
   const int cap = tp_layernorm_bwd_parts(rows);
   return parts > cap ? cap : parts;
@@ -611,8 +615,8 @@ static int layernorm_bwd_launch(int dtype, const void* dy, const void* x, const 
   int nv, wpr;
   if (!ln_geometry(H, &nv, &wpr)) return kErrBadArgument;
   const int parts = ln_parts(rows, wpr);
-  // one [2][H] fp32 region per row group of the CTA: at most 128 KB (H <= 1024 * WPR)
-  const size_t smem = static_cast<size_t>(16 / wpr) * 2 * H * sizeof(float);
+  // one [2][H] fp32 region per row group of the CTA: at most 192 KB (H <= 1024 * WPR)
+  const size_t smem = static_cast<size_t>(wpr == 16 ? 1 : 24 / wpr) * 2 * H * sizeof(float);
 #define LN_BWD(T, NV, WPR)                                                                      \
   {                                                                                             \
     auto kern = layernorm_bwd_kernel<T, NV, WPR>;                                               \

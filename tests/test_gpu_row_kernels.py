@@ -1,4 +1,5 @@
-"""The batched column sums and folds of a layer against fp64."""
+"""LayerNorm at every geometry of its kernels (warps per row, vectors per lane, rows that leave row
+groups empty) and the batched column sums, against fp64."""
 import ctypes
 
 import pytest
@@ -9,6 +10,32 @@ pytestmark = pytest.mark.gpu
 
 def _rel(a, ref):
     return ((a.double() - ref).norm() / ref.norm()).item()
+
+
+# H: 1, 2, 4, 8 and 16 warps a row, columns that end inside a vector round; rows: one, fewer than
+# and just more than a CTA holds, more than one round of all CTAs
+@pytest.mark.parametrize("H,rows", [(8, 5), (264, 25), (1024, 3700), (1600, 13), (2048, 1800), (2560, 7),
+                                    (4096, 900), (5120, 500), (8200, 3), (12288, 160)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_layernorm_geometries(H, rows, dtype):
+    from terapipe_b200.ops import functional as F
+    g = torch.Generator(device="cuda").manual_seed(H + rows)
+    x, dy, dres = (torch.randn(rows, H, device="cuda", generator=g).to(dtype) for _ in range(3))
+    gamma = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).to(dtype)
+    beta = (0.1 * torch.randn(H, device="cuda", generator=g)).to(dtype)
+    y, dx = torch.empty_like(x), torch.empty_like(x)
+    mean, rstd = torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda")
+    F.layernorm_fwd(x, gamma, beta, y, mean, rstd)
+    dgamma, dbeta = torch.ones(H, device="cuda"), torch.full((H,), 2.0, device="cuda")
+    scratch = torch.full((F.layernorm_bwd_scratch_floats(rows, H),), float("nan"), device="cuda")
+    F.layernorm_bwd(dy, x, mean, rstd, gamma, dx, dgamma, dbeta, scratch, dres=dres)
+    x64, ga, be = (t.double().requires_grad_() for t in (x, gamma, beta))
+    ref = torch.nn.functional.layer_norm(x64, (H,), ga, be)
+    ref.backward(dy.double())
+    eps = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8    # rounding of the 16-bit results
+    assert _rel(y, ref.detach()) < eps and _rel(dx, x64.grad + dres.double()) < eps
+    # fp32 sums over the rows of values computed in fp32
+    assert _rel(dgamma, ga.grad + 1) < 2e-5 and _rel(dbeta, be.grad + 2) < 2e-5
 
 
 @pytest.mark.parametrize("rows,widths", [(1, (8,)), (63, (264, 8)), (127, (256, 72)), (128, (512, 8, 1032, 256)),
