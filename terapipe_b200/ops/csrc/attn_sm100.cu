@@ -20,6 +20,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -700,62 +702,93 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
     for (int i = grp; i < n_iter; i += 2) {
       const int y0 = ystart + i * 64;
       const int st = i % kBwdStages;
-      // MODE 0: the statistics came with the tiles; half of them are fetched ahead of the scores
-      float4 nl4[8], nd4[8];
-      auto fetch_stats = [&](int g) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          nl4[k] = *reinterpret_cast<const float4*>(&sh->nlse[st][g * 32 + 4 * k]);
-          nd4[k] = *reinterpret_cast<const float4*>(&sh->ndelta[st][g * 32 + 4 * k]);
-        }
-      };
-      if (MODE == 0) {
-        ok = mbar_wait(&sh->bar_y[st], (i / kBwdStages) & 1, wctx, kErrWaitAttn);
-        if (ok) fetch_stats(0);
-      }
-      if (ok) ok = mbar_wait(&sh->bar_s[grp], (i >> 1) & 1, wctx, kErrWaitAttn);
-      if (!ok) break;
-      tc_fence_after();
       // blocks strictly inside the causal region need no per-element mask
       const bool full = MODE == 0 ? (y0 >= x0 + 127 && y0 + 64 <= p.q_end) : (y0 + 63 <= x0);
-      // P into the columns of S and dS into those of dP, 32 columns at a time.  The first half's
-      // results take 16 columns that were read already; the second half's scores lie beyond them.
+      if (MODE == 0) {
+        // The statistics belong to columns here.  With a row per thread each thread read all 64 of
+        // both (32 16-byte loads a warp and block, under the MMAs' operand traffic: half of the
+        // block's time).  As MMA fragments, 16 lanes at a time, a thread has 16 columns of four rows.
+        const int lane = threadIdx.x & 31;
+        ok = mbar_wait(&sh->bar_y[st], (i / kBwdStages) & 1, wctx, kErrWaitAttn);
+        if (!ok) break;
+        float2 nl[8], nd[8];     // columns 8 k + 2 (lane % 4) and the next
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t s[32], d[32], pk[16], dk[16];
-        __syncwarp();
-        tmem_ld_32x32(tS + g * 32, s);
-        tmem_ld_32x32(tP + g * 32, d);
-        if (MODE == 0 && g > 0) fetch_stats(g);
-        tmem_ld_wait();
-#pragma unroll
-        for (int k = 0; k < 16; k += 2) {   // four columns
-          float2 nl[2] = {nlse_r, nlse_r}, nd[2] = {ndelta_r, ndelta_r};
-          if (MODE == 0) {
-            const float4 a = nl4[k / 2], e = nd4[k / 2];
-            nl[0] = make_float2(a.x, a.y); nl[1] = make_float2(a.z, a.w);
-            nd[0] = make_float2(e.x, e.y); nd[1] = make_float2(e.z, e.w);
-          }
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int e = 2 * (k + q);       // column within the half
-            float2 pr = fma2(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc, nl[q]);
-            pr.x = exp2f(pr.x);
-            pr.y = exp2f(pr.y);
-            if (!full) {
-              const int yabs = y0 + g * 32 + e;
-              const bool v0 = MODE == 0 ? (yabs < p.q_end && xabs <= yabs) : (x_ok && yabs <= xabs);
-              const bool v1 = MODE == 0 ? (yabs + 1 < p.q_end && xabs <= yabs + 1) : (x_ok && yabs + 1 <= xabs);
-              pr.x = v0 ? pr.x : 0.0f;
-              pr.y = v1 ? pr.y : 0.0f;
-            }
-            const float2 ds = mul2(pr, add2(make_float2(__uint_as_float(d[e]), __uint_as_float(d[e + 1])), nd[q]));
-            if (MODE == 0) pk[k + q] = Elem<T>::pack2(pr.x, pr.y);
-            dk[k + q] = Elem<T>::pack2(ds.x, ds.y);
-          }
+        for (int k = 0; k < 8; ++k) {
+          nl[k] = *reinterpret_cast<const float2*>(&sh->nlse[st][8 * k + 2 * (lane & 3)]);
+          nd[k] = *reinterpret_cast<const float2*>(&sh->ndelta[st][8 * k + 2 * (lane & 3)]);
         }
-        if (MODE == 0) tmem_st_32x16(tS + g * 16, pk);
-        tmem_st_32x16(tP + g * 16, dk);
+        ok = mbar_wait(&sh->bar_s[grp], (i >> 1) & 1, wctx, kErrWaitAttn);
+        if (!ok) break;
+        tc_fence_after();
+        // (one copy of the loop per case: with the mask inside, its tests cost as much as the rest)
+        auto halves = [&](auto masked) {
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {     // lanes 0-15, 16-31 of the warp's quarter
+            const uint32_t half = static_cast<uint32_t>(hf * 16) << 16;
+            uint32_t s[32], d[32], pk[16], dk[16];
+            __syncwarp();
+            tmem_ld_16x64(tS + half, s);
+            tmem_ld_16x64(tP + half, d);
+            tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                const int e = 4 * k + 2 * q;
+                float2 pr = fma2(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc, nl[k]);
+                pr.x = exp2f(pr.x);
+                pr.y = exp2f(pr.y);
+                if (decltype(masked)::value) {
+                  const int row = x0 + (warp & 3) * 32 + hf * 16 + q * 8 + (lane >> 2);
+                  const int yabs = y0 + 8 * k + 2 * (lane & 3);
+                  pr.x = yabs < p.q_end && row <= yabs ? pr.x : 0.0f;
+                  pr.y = yabs + 1 < p.q_end && row <= yabs + 1 ? pr.y : 0.0f;
+                }
+                const float2 ds = mul2(pr, add2(make_float2(__uint_as_float(d[e]), __uint_as_float(d[e + 1])), nd[k]));
+                pk[2 * k + q] = Elem<T>::pack2(pr.x, pr.y);
+                dk[2 * k + q] = Elem<T>::pack2(ds.x, ds.y);
+              }
+            }
+            // (these lanes' scores have all been read)
+            tmem_st_16x32(tS + half, pk);
+            tmem_st_16x32(tP + half, dk);
+          }
+        };
+        if (full) halves(std::false_type());
+        else halves(std::true_type());
+      } else {
+        ok = mbar_wait(&sh->bar_s[grp], (i >> 1) & 1, wctx, kErrWaitAttn);
+        if (!ok) break;
+        tc_fence_after();
+        // dS into the columns of dP, 32 columns at a time.  The first half's results take 16 columns that
+        // were read already; the second half's values lie beyond them.
+        auto halves = [&](auto masked) {
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            uint32_t s[32], d[32], dk[16];
+            __syncwarp();
+            tmem_ld_32x32(tS + g * 32, s);
+            tmem_ld_32x32(tP + g * 32, d);
+            tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+              const int e = 2 * k;             // column within the half
+              float2 pr = fma2(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), sc, nlse_r);
+              pr.x = exp2f(pr.x);
+              pr.y = exp2f(pr.y);
+              if (decltype(masked)::value) {
+                const int yabs = y0 + g * 32 + e;
+                pr.x = x_ok && yabs <= xabs ? pr.x : 0.0f;
+                pr.y = x_ok && yabs + 1 <= xabs ? pr.y : 0.0f;
+              }
+              const float2 ds = mul2(pr, add2(make_float2(__uint_as_float(d[e]), __uint_as_float(d[e + 1])), ndelta_r));
+              dk[k] = Elem<T>::pack2(ds.x, ds.y);
+            }
+            tmem_st_32x16(tP + g * 16, dk);
+          }
+        };
+        if (full) halves(std::false_type());
+        else halves(std::true_type());
       }
       tmem_st_wait();
       tc_fence_before();
