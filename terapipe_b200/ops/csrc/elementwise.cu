@@ -301,11 +301,14 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
 // All column sums of a layer in one launch: db[n] += sum_rows dy[row][n] for up to kMaxColsums
 // matrices of the same number of rows, and the fold of up to kMaxFolds sets of LayerNorm partial
 // slots (as layernorm_bwd_reduce_kernel, clearing the slots).  Each is a handful of CTAs or a few
-// microseconds long, so separate launches cost more than the sums.  A CTA of 32 x 8 threads
-// takes 256 columns of a chunk of rows, 8 rows of 16 bytes per thread in flight.  The (at most 8) chunks
-// of a column block form a cluster whose first CTA adds them up in order through distributed shared
-// memory, so the sums do not depend on timing; 8 chunks give a 2048-wide layer 576 CTAs.  (One launch per
-// matrix with one load in flight per thread ran on 64 of 148 SMs: 16384 x 2048 took 63 us, 1.1 TB/s.)
+// microseconds long, so separate launches cost more than the sums.  A CTA of 256 threads takes 8 V
+// columns of a chunk of rows, 8 rows of 16 bytes per thread in flight.  The (at most 8) chunks of a
+// column block form a cluster whose first CTA adds them up in order through distributed shared
+// memory, so the sums do not depend on timing.  V = 32 reads longer pieces of a row (4096 rows of a
+// 12288-wide layer: 191 us against 239 for V = 8), but gives a 2048-wide layer 72 clusters, a few more
+// than the GPCs hold at once: 156 us for 16384 rows (604 MB) against 114.  So V = 32 from 128 blocks of
+// 256 columns on.  (One launch per matrix with one load in flight per thread ran on 64 of 148 SMs:
+// 16384 x 2048 alone took 63 us.)
 constexpr int kMaxColsums = 4, kMaxFolds = 2;
 struct SumJobs {
   const void* dy[kMaxColsums];
@@ -362,12 +365,13 @@ __global__ void layernorm_bwd_reduce_kernel(float* __restrict__ scratch, int par
   fold_slots(scratch, parts, H, blockIdx.x * 32, dgamma, dbeta, threadIdx.x, threadIdx.y, clear, sm);
 }
 
-template <typename T>
+template <typename T, int V>
 __global__ void __launch_bounds__(256)
 layer_sums_kernel(const SumJobs j) {
-  __shared__ union { float col[8][32][8 + 1]; float fold[8][33]; } sm;
-  __shared__ float chunk_sum[256];
-  const int tx = threadIdx.x, ty = threadIdx.y;
+  constexpr int kCols = 8 * V, kRows = 256 / V;   // columns of a CTA, rows of one load
+  __shared__ union { float col[kRows][kCols + 1]; float fold[8][33]; } sm;
+  __shared__ float chunk_sum[kCols];
+  const int tid = threadIdx.x, vec = tid % V, lane_row = tid / V;
   const int cta = blockIdx.x;
   pdl_wait();
   int first = 0;
@@ -376,17 +380,17 @@ layer_sums_kernel(const SumJobs j) {
     if (i >= j.n) break;
     if (cta < j.cta_end[i]) {
       const int chunk = (cta - first) % j.chunks;
-      const int col = ((cta - first) / j.chunks * 32 + tx) * 8;
+      const int col0 = (cta - first) / j.chunks * kCols, col = col0 + vec * 8;
       const int r_end = min(j.rows, (chunk + 1) * j.rows_per_chunk);
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       if (col < j.N[i]) {
         const T* src = static_cast<const T*>(j.dy[i]) + col;
-        for (int r = chunk * j.rows_per_chunk + ty; r < r_end; r += 64) {
+        for (int r = chunk * j.rows_per_chunk + lane_row; r < r_end; r += 8 * kRows) {
           uint4 v[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k)
-            v[k] = r + 8 * k < r_end ? *reinterpret_cast<const uint4*>(src + (r + 8 * k) * j.ld[i])
-                                     : make_uint4(0, 0, 0, 0);
+            v[k] = r + kRows * k < r_end ? *reinterpret_cast<const uint4*>(src + (r + kRows * k) * j.ld[i])
+                                         : make_uint4(0, 0, 0, 0);
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             float f[8];
@@ -397,27 +401,28 @@ layer_sums_kernel(const SumJobs j) {
         }
       }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) sm.col[ty][tx][q] = acc[q];
+      for (int q = 0; q < 8; ++q) sm.col[lane_row][vec * 8 + q] = acc[q];
       __syncthreads();
-      // thread (tx, ty) finishes column ty of vector tx
       float s = 0.0f;
+      if (tid < kCols) {
 #pragma unroll
-      for (int r = 0; r < 8; ++r) s += sm.col[r][tx][ty];
+        for (int r = 0; r < kRows; ++r) s += sm.col[r][tid];
+      }
       if (j.chunks > 1) {   // (the CTAs of a cluster are the chunks of one column block)
-        chunk_sum[ty * 32 + tx] = s;
+        if (tid < kCols) chunk_sum[tid] = s;
         cluster_sync_all();
-        if (chunk == 0) {
+        if (chunk == 0 && tid < kCols) {
           for (int q = 1; q < j.chunks; ++q) {
             float v;
             asm volatile("ld.shared::cluster.f32 %0, [%1];"
-                         : "=f"(v) : "r"(mapa_u32(smem_u32(&chunk_sum[ty * 32 + tx]), q)) : "memory");
+                         : "=f"(v) : "r"(mapa_u32(smem_u32(&chunk_sum[tid]), q)) : "memory");
             s += v;
           }
         }
         cluster_sync_all();   // nobody leaves while its sums may be read
         if (chunk != 0) return;
       }
-      if (col < j.N[i]) j.db[i][col + ty] += s;
+      if (tid < kCols && col0 + tid < j.N[i]) j.db[i][col0 + tid] += s;
       return;
     }
     first = j.cta_end[i];
@@ -425,7 +430,8 @@ layer_sums_kernel(const SumJobs j) {
   const int per_fold = (2 * j.H + 31) / 32;
   const int f = (cta - first) / per_fold;
   if (f >= j.folds) return;        // (the grid is a whole number of clusters)
-  fold_slots(j.slots[f], j.parts, j.H, (cta - first) % per_fold * 32, j.dgamma[f], j.dbeta[f], tx, ty, 1, sm.fold);
+  fold_slots(j.slots[f], j.parts, j.H, (cta - first) % per_fold * 32, j.dgamma[f], j.dbeta[f],
+             tid & 31, tid >> 5, 1, sm.fold);
 }
 
 // ------------------------------------------------------------------ fused Adam
@@ -488,14 +494,14 @@ __global__ void fill_kernel(T* p, long long n, float value) {
 
 using namespace tp;
 
-// Geometry: the smallest power-of-two warps-per-row (<= 16) that keeps at most 4 vectors of 8
+// Geometry: the smallest power-of-two warps-per-row (<= 16) that keeps at most `most` vectors of 8
 // elements per lane.
-static inline bool ln_geometry(int H, int* nv, int* wpr) {
+static inline bool ln_geometry(int H, int* nv, int* wpr, int most = 4) {
   if (H % 8 || H <= 0) return false;
   const int vecs = H / 8;
   for (int w = 1; w <= 16; w *= 2) {
     const int n = (vecs + 32 * w - 1) / (32 * w);
-    if (n <= 4) { *nv = n; *wpr = w; return true; }
+    if (n <= most) { *nv = n; *wpr = w; return true; }
   }
   return false;
 }
@@ -612,8 +618,11 @@ static int layernorm_bwd_launch(int dtype, const void* dy, const void* x, const 
                                 const PushDst& pd, float* dgamma, float* dbeta, float* scratch,
                                 int rows, int H, int mode, cudaStream_t s) {
   if (rows <= 0) return kOk;
+  // at most three vectors per lane where that is possible: a fourth one of each input leaves too few
+  // of the 80 registers to keep all loads in flight (16384 x 2048: 85 us with four, 75 with two;
+  // 4096 x 1024: 28 and 14)
   int nv, wpr;
-  if (!ln_geometry(H, &nv, &wpr)) return kErrBadArgument;
+  if (!ln_geometry(H, &nv, &wpr, 3) && !ln_geometry(H, &nv, &wpr, 4)) return kErrBadArgument;
   const int parts = ln_parts(rows, wpr);
   // one [2][H] fp32 region per row group of the CTA: at most 192 KB (H <= 1024 * WPR)
   const size_t smem = static_cast<size_t>(wpr == 16 ? 1 : 24 / wpr) * 2 * H * sizeof(float);
@@ -685,22 +694,31 @@ extern "C" int tp_layernorm_bwd_finish_assign(float* slots, int parts, int H, fl
 
 namespace tp {
 static int layer_sums_launch(int dtype, SumJobs& j, cudaStream_t s) {
-  // chunks of at least 64 rows (one round of loads), a portable cluster of them at most
+  long long blocks = 0;           // of 256 columns
+  for (int i = 0; i < j.n; ++i) blocks += (j.N[i] + 255) / 256;
+  const bool wide = blocks >= 128;
+  const int cols = wide ? 256 : 64, round = 8 * 256 / (cols / 8);   // rows of one round of loads
+  // chunks of at least one round, a portable cluster of them at most
   j.chunks = 1;
-  while (j.n > 0 && j.chunks < 8 && j.rows >= 128 * j.chunks) j.chunks *= 2;
+  while (j.n > 0 && j.chunks < 8 && j.rows >= 2 * round * j.chunks) j.chunks *= 2;
   j.rows_per_chunk = (j.rows + j.chunks - 1) / j.chunks;
   long long ctas = 0;
   for (int i = 0; i < j.n; ++i) {
-    ctas += (j.N[i] / 8 + 31) / 32 * static_cast<long long>(j.chunks);
+    ctas += (j.N[i] + cols - 1) / cols * static_cast<long long>(j.chunks);
     j.cta_end[i] = static_cast<int>(ctas);
   }
   ctas += static_cast<long long>(j.folds) * ((2 * j.H + 31) / 32);
   if (ctas == 0) return kOk;
   ctas = (ctas + j.chunks - 1) / j.chunks * j.chunks;
   if (ctas > 0x7fffffffLL) return kErrTooLarge;
-  const dim3 grid(static_cast<unsigned>(ctas)), block(32, 8);
-  const cudaError_t e = dtype == 1 ? launch_pdl(layer_sums_kernel<__nv_bfloat16>, grid, block, 0, s, j.chunks, j)
-                                   : launch_pdl(layer_sums_kernel<__half>, grid, block, 0, s, j.chunks, j);
+  const dim3 grid(static_cast<unsigned>(ctas)), block(256);
+  cudaError_t e;
+  if (dtype == 1)
+    e = wide ? launch_pdl(layer_sums_kernel<__nv_bfloat16, 32>, grid, block, 0, s, j.chunks, j)
+             : launch_pdl(layer_sums_kernel<__nv_bfloat16, 8>, grid, block, 0, s, j.chunks, j);
+  else
+    e = wide ? launch_pdl(layer_sums_kernel<__half, 32>, grid, block, 0, s, j.chunks, j)
+             : launch_pdl(layer_sums_kernel<__half, 8>, grid, block, 0, s, j.chunks, j);
   return e == cudaSuccess ? kOk : kErrLaunch;
 }
 }  // namespace tp
