@@ -124,16 +124,29 @@ inline bool make_tmap_out(CUtensorMap* out, const void* base, uint64_t cols, uin
   return true;
 }
 
+inline int num_sms() {
+  static int n = 0;
+  if (!n) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (n <= 0) n = 148;
+  }
+  return n;
+}
+
 // Launch with programmatic stream serialization (see pdl_wait in ptx.cuh).  The kernel must call
-// pdl_wait() in every thread before its first access to global data.  The attribute is off
-// unless tp_set_pdl(1) was called or the environment variable TERAPIPE_PDL=1 is set at first use
-// (it measured no gain on a step that runs at the power cap: time saved in gaps came back as a
-// lower clock).
+// pdl_wait() in every thread before its first access to global data.  On unless tp_set_pdl(0) was
+// called or the environment variable TERAPIPE_PDL=0 is set at first use: the set-up of a kernel
+// (barriers, TMEM, tensor maps) under the end of its predecessor saves 1 to 2 us a launch, 9 % of a
+// step of the 24-layer test model, 6 % of a 1024-row slice of a 2048-wide layer.  Launches of more
+// than two CTAs per SM go without: with them included, 8192 rows of a 768-wide model (attention,
+// row kernels and sums of 400 to 1000 CTAs) took 1.7 % longer instead of 0.3 % less.
 inline int& pdl_enabled() {
   static int enabled = -1;
   if (enabled < 0) {
     const char* e = getenv("TERAPIPE_PDL");
-    enabled = (e && e[0] == '1') ? 1 : 0;
+    enabled = (e && e[0] == '0') ? 0 : 1;
   }
   return enabled;
 }
@@ -155,7 +168,7 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     attr[n].val.clusterDim.z = 1;
     ++n;
   }
-  if (pdl_enabled()) {
+  if (pdl_enabled() && static_cast<long long>(grid.x) * grid.y * grid.z <= 2ll * num_sms()) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n].val.programmaticStreamSerializationAllowed = 1;
     ++n;
@@ -163,17 +176,6 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   cfg.attrs = attr;
   cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
-inline int num_sms() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
 }
 
 }  // namespace tp

@@ -119,7 +119,7 @@ layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   __shared__ float red[2 * G::kRowsPerCta * WPR + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = warp / WPR, wr = warp % WPR;
-  pdl_wait();
+  pdl_wait(pd.n <= 1);
   const long long row = static_cast<long long>(blockIdx.x) * G::kRowsPerCta + grp;
   const bool row_ok = row < rows;
   uint4 xq[NV];
@@ -204,7 +204,7 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = warp / WPR, wr = warp % WPR;
   float* my_part = part_smem + static_cast<long long>(grp) * 2 * H;
-  pdl_wait();
+  pdl_wait(pd.n <= 1);
   int parity = 0;
   bool fresh = true;      // the group's region holds nothing yet
   const uint4 zero4 = make_uint4(0, 0, 0, 0);
@@ -830,8 +830,8 @@ extern "C" int tp_layernorm_bwd_noalloc(int dtype, const void* dy, const void* x
                               scratch_of_device[dev], rows, H, 0, static_cast<cudaStream_t>(stream));
 }
 
-// Programmatic dependent launch of the GEMM, attention and LayerNorm kernels (off by default;
-// TERAPIPE_PDL=1 in the environment or tp_set_pdl(1) turns it on).
+// Programmatic dependent launch of the GEMM, attention and LayerNorm kernels (on by default;
+// TERAPIPE_PDL=0 in the environment or tp_set_pdl(0) turns it off).
 extern "C" int tp_set_pdl(int enabled) {
   tp::pdl_enabled() = enabled ? 1 : 0;
   return kOk;

@@ -491,7 +491,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();  // set-up done; from here on the predecessor's results are read
+  pdl_wait(!AR);  // set-up done; from here on the predecessor's results are read
 
   const int num_kb = (p.K + kBK - 1) / kBK;
   const int ar_epoch = AR ? (ar.epoch + (ar.epoch_base ? *ar.epoch_base : 0)) : 0;
@@ -975,7 +975,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote arrival
-  pdl_wait();          // set-up done; from here on the predecessor's results are read
+  pdl_wait(!AR && !RS && p.ag_flags == nullptr);          // set-up done; from here on the predecessor's results are read
   // The producer warp starts loading at once; the other five warps meet again after the TMEM
   // allocation (named barrier 1, 288 threads).
   uint32_t tmem_base = 0;

@@ -38,9 +38,11 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // and its memory operations are visible; every thread calls it before it touches global data.
 // The trigger directly after it lets the successor do the same with this kernel, and no
 // earlier, so at most two kernels overlap.  Without the attribute both are no-ops.
-__device__ __forceinline__ void pdl_wait() {
+// trigger = false: a kernel that waits for other ranks keeps the SMs to itself and to the small
+// kernels of other streams that its peers wait for; its successor starts when it has ended.
+__device__ __forceinline__ void pdl_wait(bool trigger = true) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 __device__ __forceinline__ bool elect_one() {
