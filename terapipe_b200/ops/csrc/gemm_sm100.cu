@@ -792,10 +792,13 @@ constexpr int kPairEpiWarps = 8;
 
 template <int BN> struct PairCfg {
   static constexpr int kABytes = kBM * kBK * 2;
-  static constexpr int kBBytes = (BN / 2) * kBK * 2;
+  // a CTA's half of B comes in 64-column chunks where N is contiguous, so its last one may be cut
+  static constexpr int kBChunks = (BN / 2 + 63) / 64;
+  static constexpr int kBBytes = kBChunks * 64 * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = BN == 256 ? 5 : 6;
-  static constexpr int kTmemCols = 2 * BN;
+  static constexpr int kStages = BN > 128 ? 5 : 6;
+  static constexpr int kAccCols = BN > 128 ? 256 : 128;   // TMEM columns of one accumulator
+  static constexpr int kTmemCols = 2 * kAccCols;
   static constexpr int kEpiStageBytes = kPairEpiWarps * kEpiBytesPerWarp;
   static constexpr int kSmemBytes = kStages * kStageBytes + kEpiStageBytes + 1024 /*align*/ + 256 /*barriers*/;
 };
@@ -1034,7 +1037,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (TRACE) stall += clock64() - t_w;
           uint8_t* sA = smem + stage * Cfg::kStageBytes;
           uint8_t* sB = sA + Cfg::kABytes;
-          if (cta == 0) mbar_expect_tx(&full[stage], 2 * Cfg::kStageBytes);
+          if (cta == 0) mbar_expect_tx(&full[stage], 2 * (Cfg::kABytes + (B_MN ? Cfg::kBBytes : HB * kBK * 2)));
           if (p.prefetch > 0 && kb + p.prefetch < num_kb) {
             // operands that come from DRAM (weights of a step are cold in L2) have a latency
             // the ring alone cannot cover; an L2 prefetch further ahead does
@@ -1049,7 +1052,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               tma_prefetch_2d(&tmB, kp, n0);
             } else {
 #pragma unroll
-              for (int c = 0; c < HB / 64; ++c) tma_prefetch_2d(&tmB, n0 + c * 64, kp);
+              for (int c = 0; c < Cfg::kBChunks; ++c) tma_prefetch_2d(&tmB, n0 + c * 64, kp);
             }
           }
           const uint32_t bar = mapa_u32(smem_u32(&full[stage]), 0);
@@ -1064,7 +1067,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tma_load_2d_pair(sB, &tmB, bar, kb * kBK, n0);
           } else {
 #pragma unroll
-            for (int c = 0; c < HB / 64; ++c)
+            for (int c = 0; c < Cfg::kBChunks; ++c)
               tma_load_2d_pair(sB + c * (kBK * 128), &tmB, bar, n0 + c * 64, kb * kBK);
           }
           if (++stage == S) { stage = 0; phase ^= 1; }
@@ -1088,7 +1091,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!ok) break;
         if (TRACE) stall_acc += clock64() - t_a;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * Cfg::kAccCols;
         for (int kb = 0; kb < num_kb; ++kb) {
           const long long t_w = TRACE ? clock64() : 0;
           ok = mbar_wait(&full[stage], phase, wctx, kErrWaitMma);
@@ -1155,7 +1158,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (RS) {
         const int unit = m0 / kBM + n_idx * num_m128;   // 128-row block x column tile
         const int owner = min(row0 / ar.rows_per_rank, ar.tp - 1);
-        const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+        const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kAccCols;
         const long long tile_elems = kBM * BN;
         const bool mine = row0 < p.M && owner == ar.rank;
         // checked build: the block's slot in the staging and flag arrays, and the owner's rank
@@ -1250,7 +1253,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                               TP_CHECK(ar_tile >= 0 && ar_tile < ar.max_tiles && ar.tp <= kMaxTp, p.err,
                                        kErrCheckStaging);
         const int owner = ar_tile % ar.tp;
-        const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+        const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kAccCols;
         T* tile_dst = static_cast<T*>(ar.stage[owner]) +
                       (static_cast<long long>(ar.rank) * ar.max_tiles + ar_tile) * (kBM * BN);
 #pragma unroll 1
@@ -1351,7 +1354,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int nc = (min(BN, p.N - n0) + 31) / 32;
         const long long t_l = TRACE ? clock64() : 0;
         epilogue_rows<T, OUT_F32, TRACE>(
-            p, &tmO, es, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN, nc, row0,
+            p, &tmO, es, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kAccCols, nc, row0,
             n0, lane, half, 2, cyc3);
         if (TRACE) cyc_rest += clock64() - t_l;
       }
@@ -1513,7 +1516,7 @@ static int dispatch_layout_pair(int a_mn, int b_mn, int out_f32, const CUtensorM
 }
 
 // Tile choice.  Codes: 64 / 128 / 256 = one CTA, 128 x BN tile; 512 = one CTA, 256 x 256;
-// 1128 / 1256 = CTA pair, 256 x 128 / 256 x 256.  Relative time of one tile =
+// 1000 + BN = CTA pair, 256 x BN (BN = 128, 192, 224, 256).  Relative time of one tile =
 // (tile FLOPs per SM) / (fraction of the MMA rate the shared-memory feed sustains for that
 // shape); total = waves x that.  Wave quantisation matters because M is only ~1024 rows per
 // token slice.
@@ -1530,8 +1533,13 @@ struct TileCand {
   bool pair;
   float loop, epi_each, tail;
 };
-static const TileCand kTileCands[6] = {
+// 192 and 224 columns are for products of a few waves, whose last one is nearly empty with 256: 2048 x
+// 5120 is 160 tiles of 256 columns on 74 pairs (3 waves of 16.7) or 216 of 192 (3 waves of 13.2).
+// 2048 x 5120 x 10240 took 201 us with 256 columns and takes 163 with 192, 2048 x 7680 x 5120 121 and
+// 110 with 224.
+static const TileCand kTileCands[8] = {
     {1256, 256, 256, true, 16.7f, 0.0f, 8.5f}, {1128, 256, 128, true, 10.0f, 0.0f, 5.5f},
+    {1224, 256, 224, true, 15.0f, 0.0f, 7.8f}, {1192, 256, 192, true, 13.2f, 0.0f, 7.0f},
     {512, 256, 256, false, 36.0f, 18.0f, 0.0f}, {256, 128, 256, false, 24.7f, 0.0f, 10.0f},
     {128, 128, 128, false, 16.4f, 0.0f, 5.4f}, {64, 128, 64, false, 9.5f, 0.0f, 3.0f}};
 
@@ -1539,6 +1547,7 @@ static int pick_tile(int M, int N, int K, int forced, bool allow_256x256, bool a
   if (forced == 64 || forced == 128 || forced == 256) return forced;
   if (forced == 512) return allow_256x256 ? 512 : 256;
   if (forced == 1128 || forced == 1256) return allow_pair ? forced : forced - 1000;
+  if (forced == 1192 || forced == 1224) return allow_pair ? forced : 256;
   const int sms = num_sms();
   int best = 128;
   float best_t = 1e30f;
@@ -1549,7 +1558,9 @@ static int pick_tile(int M, int N, int K, int forced, bool allow_256x256, bool a
     const int slots = c.pair ? sms / 2 : sms;
     const float waves = static_cast<float>((tiles + slots - 1) / slots);
     const float t = waves * (c.loop * static_cast<float>(K) / 2048.0f + c.epi_each) + c.tail;
-    if (t < best_t) { best_t = t; best = c.code; }
+    // (near ties go to the full widths)
+    const bool cut = c.bn == 192 || c.bn == 224;
+    if (t < (cut ? 0.97f : 1.0f) * best_t) { best_t = t; best = c.code; }
   }
   return best;
 }
@@ -1631,6 +1642,8 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define TP_DISPATCH(T)                                                                   \
   (pair ? (BN == 256 ? dispatch_layout_pair<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)  \
+           : BN == 224 ? dispatch_layout_pair<T, 224>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s) \
+           : BN == 192 ? dispatch_layout_pair<T, 192>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s) \
                      : dispatch_layout_pair<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)) \
    : tile_code == 512 ? dispatch_layout<T, 256, 2>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)  \
    : BN == 256 ? dispatch_layout<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)            \
