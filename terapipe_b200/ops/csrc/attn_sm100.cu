@@ -112,7 +112,8 @@ __device__ __forceinline__ void tile_of_cta(int idx, int tiles, int heads, int& 
 //
 // What bounds it: 128 queries x 64 keys take 512 cycles of the exponential unit; S takes 384 cycles
 // (6 KB of operands through shared memory per 32 cycles of tensor work) and P V 256 at D = 128,
-// half of that at D = 64.
+// half of that at D = 64.  With P through shared memory and one group of 128 queries per CTA, 8 x 16 heads
+// of 2048 x 128 took 302 us, now 161; 48 heads of 2048 x 64 113 and 67.
 struct FwdShared {
   uint64_t bar_q[2], bar_k[4], bar_kfree[4], bar_v[4], bar_vfree[4], bar_s[2][2], bar_p[2][2], bar_o[2],
       bar_fin[2];
@@ -510,7 +511,7 @@ attn_delta_kernel(const T* __restrict__ o, long long ld_o, const T* __restrict__
 // block's store waited for the previous block's products and these for the store, and a block took
 // 4000 cycles.  The MMA thread now issues the products of block i and then the scores of block
 // i + 2, which overwrite the same columns: MMAs of one thread execute in order, so only the
-// workers' arrival is waited for.
+// workers' arrival is waited for.  8 x 16 heads of 2048 x 128, both modes and delta: 858 us before, 566 now.
 constexpr int kBwdThreads = 320;
 constexpr int kBwdStages = 4;   // ring depth of the streamed tiles
 
