@@ -320,6 +320,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       // a row that has seen no key yet (second group, its first block beyond the diagonal) has m = -inf
       const float2 nm = dup2(m == -INFINITY ? 0.0f : -m), sc = dup2(p.scale2);
+      float2 sum = make_float2(0.0f, 0.0f);   // of this block first: shorter chains of additions
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         uint32_t pk[16];
@@ -328,11 +329,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           float2 e = fma2(make_float2(__uint_as_float(s[g][2 * i]), __uint_as_float(s[g][2 * i + 1])), sc, nm);
           e.x = exp2f(e.x);
           e.y = exp2f(e.y);
-          l2 = add2(l2, e);
+          sum = add2(sum, e);
           pk[i] = Elem<T>::pack2(e.x, e.y);
         }
         tmem_st_32x16(tSk + g * 16, pk);
       }
+      l2 = add2(l2, sum);
       tmem_st_wait();
       tc_fence_before();
       warp_arrive(&sh->bar_p[w][k & 1]);
