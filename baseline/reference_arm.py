@@ -177,7 +177,7 @@ class ReferenceArm:
                 parallelism=f"pp{pp}xtp{tp}xdp{dp}", batch_slices=batch_slices, seq_slices=seq_slices,
                 activation="relu", mixed_precision="fp32 master weights, loss scale 128",
                 optimizer="torch.optim.Adam(fused=True) standing in for apex FusedAdam",
-                attention_recompute=recompute, cuda_graph=False, launch_plan=False,
+                attention_recompute=recompute, cuda_graph=False, launch_plan=False, merged_slices=False,
                 tp_comm="nccl" if tp > 1 else "none", dp_comm="nccl" if dp > 1 else "none",
                 l2=self.l2_note),
             "gpu_launches": None, "clocks": clocks,

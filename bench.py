@@ -204,7 +204,7 @@ def config_dict(**kw):
     """The `config` object of a block; both arms fill the same keys."""
     keys = ("model", "n_layers", "hidden", "heads", "global_batch", "seq_len", "parallelism",
             "batch_slices", "seq_slices", "activation", "mixed_precision", "optimizer",
-            "attention_recompute", "cuda_graph", "launch_plan", "tp_comm", "dp_comm", "l2")
+            "attention_recompute", "cuda_graph", "launch_plan", "merged_slices", "tp_comm", "dp_comm", "l2")
     return {k: kw.get(k) for k in keys}
 
 
@@ -371,7 +371,8 @@ class OursArm:
                 optimizer="fused mixed-precision Adam (this library)",
                 attention_recompute=True, cuda_graph=("step" if eng.use_graph else
                                                       ("segments" if eng._seg_graphs is not None else False)),
-                launch_plan=eng._plan is not None, tp_comm=eng.tp_comm, dp_comm=eng.dp_comm, l2=L2_NOTE),
+                launch_plan=eng._plan is not None, merged_slices=eng.merges_slices, tp_comm=eng.tp_comm,
+                dp_comm=eng.dp_comm, l2=L2_NOTE),
             "gpu_launches": launches, "clocks": clocks, "e2e": e2e,
             "peak_memory_gb_torch_allocator": round(peak_gb, 2),
         }

@@ -18,9 +18,11 @@ What one rank owns
   read-modify-write GEMM per slice); in a pipeline this also takes the weight-gradient work
   off the inter-stage critical path.
 
-Schedule (same as the reference, test_transformer_terapipe.py:107-175,270-287): for each
-batch slice all token slices forward in order; backward visits batch slices and token
-slices in reverse; data-parallel gradient reduction; optimizer.  There is no autograd graph:
+Schedule of a stage with pipeline neighbours or tensor parallelism (same as the reference,
+test_transformer_terapipe.py:107-175,270-287): for each batch slice all token slices forward in
+order; backward visits batch slices and token slices in reverse; data-parallel gradient
+reduction; optimizer.  A stage with neither has nobody to hand a slice to and walks every layer
+once over all rows instead (``merge_slices``).  There is no autograd graph:
 every kernel of the forward and backward pass is launched explicitly, which lets the whole
 iteration be captured in one CUDA graph when the stage does not communicate.
 
@@ -56,6 +58,17 @@ PARAM_ORDER = ("attn_ln.weight", "attn_ln.bias", "attn.in_proj.weight", "attn.in
 
 def _align(n: int, a: int = 8) -> int:
     return (n + a - 1) // a * a
+
+
+def wants_merged_slices(merge_slices: Optional[bool], pp: int, tp: int, per_slice: bool) -> bool:
+    """Does a stage walk all rows at once?  ``merge_slices`` is the caller's wish.  ``None``: wherever
+    nothing depends on the slices, that is without pipeline neighbours (they work on one slice while
+    this stage works on the next), without tensor parallelism (its exchange buffers hold one slice)
+    and unless the launches are recorded or captured slice by slice (``per_slice``)."""
+    alone = pp == 1 and tp == 1
+    if merge_slices and not alone:
+        raise ValueError("merge_slices needs a stage without pipeline neighbours and tensor parallelism")
+    return alone and not per_slice if merge_slices is None else bool(merge_slices)
 
 
 class _Layout:
@@ -95,7 +108,7 @@ class StageEngine:
                  seq_slices: Sequence[int], dtype=torch.float16, loss_scale=LOSS_SCALE_FACTOR,
                  lr=1e-10, seed=0, init="device", use_graph: Optional[bool] = None,
                  tp_comm="nccl", dp_comm="nccl", device=None, launch_plan: Optional[bool] = None,
-                 segment_graphs: Optional[bool] = None):
+                 segment_graphs: Optional[bool] = None, merge_slices: Optional[bool] = None):
         assert torch.cuda.is_available(), "StageEngine needs a CUDA device (sm_100a)"
         self.cfg = config
         self.batch_slices, self.seq_slices = list(batch_slices), list(seq_slices)
@@ -219,12 +232,10 @@ class StageEngine:
         # the slices' results differ only where a sum over rows is split differently.  GPT3-1B
         # width (5 layers), batch 8, 16 slices of 128: a step took 40.5 ms slice by slice, 31.1 merged;
         # the 24-layer test model in 8 slices of 32 rows 17.4 ms against 3.4.
-        # Slices stay where something is made for them: a recorded plan or per-segment graphs that
-        # the caller decided about, a slice timeline, and tensor-parallel exchange buffers, whose size
-        # is a slice's.  An eager run merges like a captured one, so that both take the same sums in the
-        # same order and agree bit for bit.
-        self._merged = (self.pp == 1 and self.tp == 1
-                        and self._plan is None and launch_plan is None and segment_graphs is None)
+        # An eager run merges like a captured one, so that both take the same sums in the same order
+        # and agree bit for bit.
+        self._merged = wants_merged_slices(merge_slices, self.pp, self.tp,
+                                           per_slice=self._plan is not None or bool(segment_graphs))
         self._alloc_activations()
         self.status = F.status_word(dev)
         self.loss_buf = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -232,14 +243,16 @@ class StageEngine:
         self._cap_stream = None
         self.timeline = None   # set to a utils.trace.SliceTimeline to record per-slice device times
         self.step_count = 0
+        self._walked_merged = self._merged
         self._streams_ready = False
         # launches of this library's own kernels (NCCL and torch kernels are not counted):
         # per layer and slice 7 forward (2 LN, 4 GEMM, attention) and 9 backward (4 GEMM,
         # 2 LN, 3 attention); per layer 5 after the last slice (4 weight-gradient GEMMs, the bias
         # and LayerNorm gradients in one); plus 2 for the optimizer
         n_slices = len(self.batch_slices) * len(self.seq_slices)
-        per_layer = 12 + 4 * len(self.batch_slices) if self._merged else 16 * n_slices
-        self.launches_per_step = self.n_layers * (per_layer + 5 + (2 if self.sp else 0)) + 2
+        self._launches = {merged: self.n_layers * (per_layer + 5 + (2 if self.sp else 0)) + 2
+                          for merged, per_layer in ((True, 12 + 4 * len(self.batch_slices)),
+                                                    (False, 16 * n_slices))}
         self.launch_count = 0
         self._ar_calls_per_step = n_slices * self.n_layers * 4 + 1
         # sequence parallel: all-gather pushes per step (2 per layer and slice forward; backward one
@@ -250,12 +263,22 @@ class StageEngine:
         if self.sp:
             # one flag kernel per all-gather, two group barriers, the sums of the LayerNorm
             # gradients over the group and the three counter updates of a step
-            self.launches_per_step += (self._ag_calls_per_step - 1) + 2 + 2 * self.n_layers + 3
+            self._launches[False] += (self._ag_calls_per_step - 1) + 2 + 2 * self.n_layers + 3
         elif self.tp_comm == "fused":
-            self.launches_per_step += 1      # the epoch counter update
+            self._launches[False] += 1       # the epoch counter update
         self._ag_stream, self._ag_pending = None, False
         self._first_step_synced = False
         self._ag_in_kernel = os.environ.get("TERAPIPE_AG_PUSH", "0") == "1"
+
+    @property
+    def merges_slices(self) -> bool:
+        """Whether the next iteration walks all rows at once (a slice timeline needs the slices)."""
+        return self._merged and self.timeline is None
+
+    @property
+    def launches_per_step(self) -> int:
+        """Launches of this library's kernels that the next iteration makes."""
+        return self._launches[self.merges_slices]
 
     # ------------------------------------------------------------------ parameters
     def param(self, layer: int, name: str, buf: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -984,7 +1007,7 @@ class StageEngine:
         nb, ns = len(self.batch_slices), len(self.seq_slices)
         if self.timeline is not None:
             self.timeline.begin_iteration()
-        merged = self._merged and self.timeline is None
+        merged = self._walked_merged = self.merges_slices
         sends = []
         recvs = self._post_recvs(True) if (pipelined and not self.is_first) else None
         if merged:
@@ -1180,7 +1203,7 @@ class StageEngine:
             if self.use_graph:
                 self._capture()
         self.step_count += 1
-        self.launch_count += self.launches_per_step
+        self.launch_count += self._launches[self._walked_merged]   # of the iteration that ran, or was captured
 
     def _capture(self):
         torch.cuda.synchronize()

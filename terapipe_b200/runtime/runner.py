@@ -42,7 +42,7 @@ class NCCLTransformerRunner:
                  rank: int, local_rank: int, mixed_precision: bool = False, use_mpi: bool = False,
                  init_process_group: bool = False, checkpoint_gradients: bool = False,
                  engine: str = "auto", dtype=torch.float16, tp_comm: str = "fused",
-                 use_graph=None, init: str = "device"):
+                 use_graph=None, init: str = "device", merge_slices: Optional[bool] = None):
         self.config = config
         self.batch_slices, self.seq_slices = list(batch_slices), list(seq_slices)
         self.rank, self.local_rank, self.world_size = rank, local_rank, world_size
@@ -70,7 +70,7 @@ class NCCLTransformerRunner:
             from .engine import StageEngine
             self.impl = StageEngine(config, self.batch_slices, self.seq_slices, dtype=dtype,
                                     loss_scale=LOSS_SCALE_FACTOR, init=init, use_graph=use_graph,
-                                    tp_comm=tp_comm)
+                                    tp_comm=tp_comm, merge_slices=merge_slices)
         else:
             from .portable import PortablePipeline
             self.impl = PortablePipeline(config, self.batch_slices, self.seq_slices,
@@ -85,6 +85,11 @@ class NCCLTransformerRunner:
     @property
     def n_input_slices(self):
         return len(self.seq_slices)
+
+    @property
+    def merges_slices(self) -> bool:
+        """Whether a step walks all rows at once instead of slice by slice (one stage on one GPU)."""
+        return self.engine_kind == "b200" and self.impl.merges_slices
 
     def _input(self):
         impl = self.impl
@@ -159,8 +164,9 @@ class NCCLTransformerRunner:
     def _grads_for(self, batch_slices, seq_slices, x):
         if self.engine_kind == "b200":
             from .engine import StageEngine
+            # the schedule is what is compared: the slices must run as given on one stage, too
             eng = StageEngine(self.config, batch_slices, seq_slices, dtype=self.impl.dtype,
-                              init="device", use_graph=False, tp_comm="nccl")
+                              init="device", use_graph=False, tp_comm="nccl", merge_slices=False)
             eng.load_state_dict(self.impl.state_dict())
             if eng.is_first:
                 eng.set_input(x)

@@ -8,7 +8,8 @@
 model.  ``batch_size`` is the batch of ONE data-parallel replica; the data-parallel size is
 ``world_size // (tp * pp)``.  Inputs are hidden states ``[seq, batch, hidden]`` (the
 benchmark harness has no embedding, as in the reference, terapipe.py:48-49); the loss is
-the mean of the final output.
+the mean of the final output.  With ``pp = tp = 1`` the stage has no use for token slices and
+walks all rows at once; ``merge_slices=False`` makes it run the slices all the same.
 """
 from __future__ import annotations
 
@@ -31,7 +32,7 @@ class Trainer:
                  seq_slices: Optional[Sequence[int]] = None, dtype="fp16",
                  n_layers: Optional[int] = None, activation: str = "gelu", use_graph=None,
                  tp_comm: str = "nccl", dp_comm: str = "nccl", lr: float = 1e-10, seed: int = 0, init: str = "device",
-                 loss_scale: float = 128.0):
+                 loss_scale: float = 128.0, merge_slices: Optional[bool] = None):
         if dist.is_initialized():
             if not mpu.model_parallel_is_initialized():
                 mpu.initialize_model_parallel(tp, pp, verbose=False)
@@ -54,7 +55,8 @@ class Trainer:
         self.seed = seed
         self.engine = StageEngine(self.config, batch_slices, seq_slices, dtype=self.dtype,
                                   loss_scale=loss_scale, lr=lr, seed=seed, init=init,
-                                  use_graph=use_graph, tp_comm=tp_comm, dp_comm=dp_comm)
+                                  use_graph=use_graph, tp_comm=tp_comm, dp_comm=dp_comm,
+                                  merge_slices=merge_slices)
         self._staging = None
         # host mirror of the device status word (bounded device waits report through it)
         self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory()

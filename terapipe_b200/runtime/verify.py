@@ -36,8 +36,9 @@ except Exception:  # pragma: no cover - filelock is an optional dependency
 def _build(engine: str, cfg, batch_slices, seq_slices, device, dtype):
     if engine == "b200":
         from .engine import StageEngine
+        # the slices are part of what is checked: they run as given, on one stage, too
         return StageEngine(cfg, batch_slices, seq_slices, dtype=dtype or torch.float16,
-                           init="reference", use_graph=False)
+                           init="reference", use_graph=False, merge_slices=False)
     from .portable import PortablePipeline
     return PortablePipeline(cfg, batch_slices, seq_slices, device=device,
                             mixed_precision=dtype is not None, dtype=dtype or torch.float16)

@@ -47,7 +47,7 @@ class TerapipeLatencyModel:
         cfg.seq_len = ctx + seqlen
         slices = ([ctx] if ctx else []) + [seqlen]
         self.engine = StageEngine(cfg, [batch_size], slices, init="device", use_graph=False,
-                                  tp_comm=tp_comm, segment_graphs=False)
+                                  tp_comm=tp_comm, segment_graphs=False, merge_slices=False)
         self.engine.set_input(torch.randn(cfg.seq_len, batch_size, cfg.embedding_dim))
         self.target = self.engine.slices[0][-1]
 

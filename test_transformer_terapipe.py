@@ -81,8 +81,10 @@ def main():
             else:
                 mean_time, std_time = runner.run(args.n_steps, verbose=args.verbose)
                 result["mean_time"], result["std_time"] = mean_time, std_time
-                # beyond the reference's schema: job throughput, device-timed step of the slowest
-                # rank, this rank's peak memory
+                # beyond the reference's schema: whether one stage walked all rows at once (the slices
+                # then do not run), job throughput, device-timed step of the slowest rank, this
+                # rank's peak memory
+                result["merged_slices"] = runner.merges_slices
                 result["tokens_per_s"] = batch * dp * config.seq_len / mean_time
                 result["max_over_ranks_device_ms"] = runner.max_over_ranks_device_ms()
                 result["peak_memory_gb"] = runner.last_peak_memory_gb

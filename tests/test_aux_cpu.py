@@ -3,6 +3,7 @@ import os
 import sys
 import time
 
+import pytest
 import torch
 
 from terapipe_b200.utils import launcher
@@ -162,3 +163,15 @@ def test_launch_plan_records_once_and_replays():
     assert ("fwd", 0) not in cache.segments
     cache.run(("fwd", 0), segment, 1)
     assert ("fwd", 0) in cache.segments
+
+
+def test_a_stage_merges_its_slices_only_where_nothing_depends_on_them():
+    from terapipe_b200.runtime.engine import wants_merged_slices as wants
+    assert wants(None, 1, 1, per_slice=False)
+    assert not wants(None, 1, 1, per_slice=True)       # recorded or captured slice by slice
+    assert not wants(None, 2, 1, per_slice=False) and not wants(None, 1, 2, per_slice=False)
+    assert wants(True, 1, 1, per_slice=True) and not wants(False, 1, 1, per_slice=False)
+    for pp, tp in ((2, 1), (1, 2)):
+        assert not wants(False, pp, tp, per_slice=False)
+        with pytest.raises(ValueError):
+            wants(True, pp, tp, per_slice=False)

@@ -62,10 +62,11 @@ def test_selftest_check_fires_in_the_checked_build_only():
     assert "build 0" in _run(body, checked=False)
 
 
-def test_engine_steps_are_identical_and_clean_under_the_checked_build():
-    """Training steps (GEMM, attention, LayerNorm, Adam; sliced, two batch slices) under the
-    checked library: no check fires and the parameters equal those of the regular library bit
-    for bit."""
+@pytest.mark.parametrize("merge", [True, False])
+def test_engine_steps_are_identical_and_clean_under_the_checked_build(merge):
+    """Training steps (GEMM, attention, LayerNorm, Adam; two batch slices, all rows at once and
+    sliced) under the checked library: no check fires and the parameters equal those of the
+    regular library bit for bit."""
     body = """
         import torch
         from terapipe_b200.models import TransformerConfig
@@ -73,14 +74,16 @@ def test_engine_steps_are_identical_and_clean_under_the_checked_build():
         cfg = TransformerConfig(batch_size=2, seq_len=256, n_layers=2, embedding_dim=256,
                                 num_attention_heads=4, n_devices=1)
         g = torch.Generator().manual_seed(5)
-        eng = StageEngine(cfg, [1, 1], [96, 32, 128], init="device", use_graph=False, lr=1e-3)
+        eng = StageEngine(cfg, [1, 1], [96, 32, 128], init="device", use_graph=False, lr=1e-3,
+                          merge_slices=MERGE)
+        assert eng._merged == MERGE
         for _ in range(3):
             eng.set_input(torch.randn(cfg.seq_len, cfg.batch_size, cfg.embedding_dim, generator=g))
             eng.step()
         torch.cuda.synchronize()
         eng.check_status()
         print("sum", eng.master.double().sum().item().hex(), eng.exp_avg_sq.double().sum().item().hex())
-    """
+    """.replace("MERGE", str(merge))
     a = [ln for ln in _run(body, checked=True).splitlines() if ln.startswith("sum")]
     b = [ln for ln in _run(body, checked=False).splitlines() if ln.startswith("sum")]
     assert a and a == b

@@ -20,7 +20,8 @@ def _oracle(cfg, x):
 @pytest.mark.parametrize("activation", ["gelu", "relu"])
 @pytest.mark.parametrize("batch_slices,seq_slices", [([2], [128]), ([2], [16] * 8),
                                                      ([1, 1], [40, 8, 16, 64])])
-def test_engine_matches_portable_oracle(dtype, activation, batch_slices, seq_slices):
+@pytest.mark.parametrize("merge", [True, False])
+def test_engine_matches_portable_oracle(dtype, activation, batch_slices, seq_slices, merge):
     from terapipe_b200.models import TransformerConfig
     from terapipe_b200.runtime.engine import StageEngine
     cfg = TransformerConfig(batch_size=2, seq_len=128, n_layers=2, embedding_dim=256,
@@ -28,7 +29,9 @@ def test_engine_matches_portable_oracle(dtype, activation, batch_slices, seq_sli
     g = torch.Generator().manual_seed(123)
     x = torch.randn(cfg.seq_len, cfg.batch_size, cfg.embedding_dim, generator=g).cuda()
     oracle = _oracle(cfg, x)
-    eng = StageEngine(cfg, batch_slices, seq_slices, dtype=dtype, init="reference", use_graph=False)
+    eng = StageEngine(cfg, batch_slices, seq_slices, dtype=dtype, init="reference", use_graph=False,
+                      merge_slices=merge)
+    assert eng._merged == merge
     # same weights (the oracle draws from the same seeded CPU generator)
     for (name, a), b in zip(eng.state_dict().items(), oracle.layers.state_dict().values()):
         assert _rel(a, b) < 5e-3, name
@@ -104,8 +107,9 @@ def test_trainer_step_and_checkpoint_roundtrip(tmp_path):
     assert a == b
 
 
+@pytest.mark.parametrize("merge", [True, False])
 @pytest.mark.parametrize("heads,hidden", [(4, 320), (4, 384)])
-def test_engine_with_head_dim_80_and_96_matches_portable_oracle(heads, hidden, tmp_path):
+def test_engine_with_head_dim_80_and_96_matches_portable_oracle(heads, hidden, merge, tmp_path):
     """Heads of 80 (gpt3-2b) and 96 columns (megatron-*, gpt3-7hm) run on the 128-wide attention
     kernels with zero-padded projections: outputs, gradients (in the model's own shapes), an
     optimizer step and a checkpoint must match what the unpadded model gives, and the padding
@@ -118,7 +122,9 @@ def test_engine_with_head_dim_80_and_96_matches_portable_oracle(heads, hidden, t
     g = torch.Generator().manual_seed(7)
     x = torch.randn(cfg.seq_len, cfg.batch_size, cfg.embedding_dim, generator=g).cuda()
     oracle = _oracle(cfg, x)
-    eng = StageEngine(cfg, [1, 1], [40, 24, 64], init="reference", use_graph=False, lr=1e-3)
+    eng = StageEngine(cfg, [1, 1], [40, 24, 64], init="reference", use_graph=False, lr=1e-3,
+                      merge_slices=merge)
+    assert eng._merged == merge
     assert eng.Dk == 128 and eng.D == hidden // heads
     sd = eng.state_dict()
     for (name, a), b in zip(sd.items(), oracle.layers.state_dict().values()):

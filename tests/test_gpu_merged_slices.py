@@ -17,8 +17,8 @@ def test_merged_pass_equals_slice_by_slice(batch_slices, seq_slices):
     x = torch.randn(128, 3, 256, generator=torch.Generator().manual_seed(1))
     got = []
     for merged in (True, False):
-        how = dict(use_graph=True) if merged else dict(use_graph=False, launch_plan=False)
-        eng = StageEngine(cfg, batch_slices, seq_slices, loss_scale=1024.0, lr=1e-4, **how)
+        eng = StageEngine(cfg, batch_slices, seq_slices, loss_scale=1024.0, lr=1e-4, use_graph=merged,
+                          merge_slices=merged)
         assert eng._merged == merged
         eng.set_input(x)
         eng.compute_grads()
@@ -34,3 +34,81 @@ def test_merged_pass_equals_slice_by_slice(batch_slices, seq_slices):
     for a, b in zip(got[0][1:3], got[1][1:3]):
         assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 2e-3
     assert got[0][3] <= got[1][3]
+
+
+def _engine(**kw):
+    from terapipe_b200.models import TransformerConfig
+    from terapipe_b200.runtime.engine import StageEngine
+    cfg = TransformerConfig(batch_size=2, seq_len=64, n_layers=1, embedding_dim=256,
+                            num_attention_heads=4, n_devices=1)
+    return StageEngine(cfg, [2], [24, 40], use_graph=False, **kw)
+
+
+def test_refusing_plans_and_segment_graphs_leaves_the_schedule_alone():
+    assert _engine()._merged
+    assert _engine(launch_plan=False)._merged and _engine(segment_graphs=False)._merged
+    assert not _engine(launch_plan=True)._merged and not _engine(segment_graphs=True)._merged
+    assert not _engine(merge_slices=False)._merged
+
+
+def test_trainer_takes_the_schedule():
+    from terapipe_b200.runtime.trainer import Trainer
+    for merge in (None, True, False):
+        tr = Trainer("test", batch_size=2, n_layers=1, batch_slices=[2], seq_slices=[64, 64], merge_slices=merge)
+        assert tr.engine._merged == (merge is not False)
+
+
+def test_launches_are_those_of_the_pass_that_ran():
+    """Counted by the calls into the library: one layer, two token slices."""
+    from terapipe_b200.utils.trace import SliceTimeline
+    eng = _engine(segment_graphs=False)
+    lib, calls = eng.lib, []
+
+    class Counting:
+        def __getattr__(self, name):
+            fn = getattr(lib, name)
+
+            def call(*args):
+                # attention's backward is three kernels in one call
+                calls.append(3 if name.startswith("tp_attn_bwd") else 1)
+                return fn(*args)
+            return call
+
+    eng.lib = Counting()
+    for timeline in (None, SliceTimeline(stage=0), None):
+        eng.timeline = timeline
+        eng.set_input(torch.randn(64, 2, 256))
+        before = eng.launch_count
+        calls.clear()
+        eng.step()
+        # (the optimizer's two launches do not go through eng.lib)
+        assert eng.launch_count - before == sum(calls) + 2
+        assert sum(calls) == (12 + 4 + 5 if timeline is None else 2 * 16 + 5)
+
+
+def _count_slices(monkeypatch):
+    from terapipe_b200.runtime.engine import StageEngine
+    seen, real = [], StageEngine._forward_slice
+    monkeypatch.setattr(StageEngine, "_forward_slice", lambda self, sl: (seen.append(sl[3]), real(self, sl))[1])
+    return seen
+
+
+def test_runner_verify_runs_the_slices(monkeypatch):
+    from terapipe_b200.models import TransformerConfig
+    from terapipe_b200.runtime.runner import NCCLTransformerRunner
+    cfg = TransformerConfig(batch_size=2, seq_len=64, n_layers=1, embedding_dim=256,
+                            num_attention_heads=4, n_devices=1)
+    runner = NCCLTransformerRunner(cfg, [2], [24, 40], "env://", 1, 1, 1, 1, 0, 0, mixed_precision=True)
+    assert runner.merges_slices
+    seen = _count_slices(monkeypatch)
+    runner.verify()
+    assert seen == [24, 40, 64]        # the sliced engine, then the whole sequence
+
+
+def test_golden_check_runs_the_slices(monkeypatch, tmp_path):
+    from terapipe_b200.runtime import verify
+    kw = dict(model="test", n_layers=1, batch_size=2, device="cuda", engine="b200", dtype=torch.float16)
+    verify.verify_one_step(str(tmp_path), "save", **kw)
+    seen = _count_slices(monkeypatch)
+    verify.verify_one_step(str(tmp_path), "load", n_input_slices=4, **kw)
+    assert seen == [32] * 4

@@ -75,8 +75,9 @@ def test_trainer_raises_when_the_status_word_is_set():
     assert isinstance(tr.train_step(x), float)
 
 
+@pytest.mark.parametrize("merge", [True, False])
 @pytest.mark.parametrize("use_graph", [False, True])
-def test_repeated_runs_are_bit_identical(use_graph):
+def test_repeated_runs_are_bit_identical(use_graph, merge):
     """No kernel accumulates through atomics in an order that varies: two engines built and
     stepped the same way end with identical parameters, moments and loss."""
     from terapipe_b200.models import TransformerConfig
@@ -87,7 +88,9 @@ def test_repeated_runs_are_bit_identical(use_graph):
     xs = [torch.randn(cfg.seq_len, cfg.batch_size, cfg.embedding_dim, generator=g) for _ in range(3)]
     runs = []
     for _ in range(2):
-        eng = StageEngine(cfg, [1, 1], [96, 32, 128], init="device", use_graph=use_graph, lr=1e-3)
+        eng = StageEngine(cfg, [1, 1], [96, 32, 128], init="device", use_graph=use_graph, lr=1e-3,
+                          merge_slices=merge)
+        assert eng._merged == merge
         for x in xs:
             eng.set_input(x)
             eng.step()
@@ -99,11 +102,13 @@ def test_repeated_runs_are_bit_identical(use_graph):
     assert runs[0][2] == runs[1][2]
 
 
+@pytest.mark.parametrize("merge", [True, False])
 @pytest.mark.parametrize("use_graph", [False, True])
-def test_engine_at_gpt3_1b_width_matches_fp32_oracle(use_graph):
-    """Two layers of GPT3-1B width (hidden 2048, head dim 128, FFN 8192) with 1024-row slices, the
-    shapes of the headline run (CTA-pair 256-wide tiles, several waves per product), against the
-    fp32 autograd pipeline on the same weights."""
+def test_engine_at_gpt3_1b_width_matches_fp32_oracle(use_graph, merge):
+    """Two layers of GPT3-1B width (hidden 2048, head dim 128, FFN 8192), all 4096 rows at once and
+    in 1024-row slices, the shapes of the headline run on one stage and on several (CTA-pair
+    256-wide tiles, several waves per product), against the fp32 autograd pipeline on the same
+    weights."""
     from terapipe_b200.models import TransformerConfig
     from terapipe_b200.runtime.engine import StageEngine
     from terapipe_b200.runtime.portable import PortablePipeline
@@ -113,7 +118,8 @@ def test_engine_at_gpt3_1b_width_matches_fp32_oracle(use_graph):
     x = torch.randn(cfg.seq_len, cfg.batch_size, cfg.embedding_dim, generator=g).cuda()
     oracle = PortablePipeline(cfg, [cfg.batch_size], [cfg.seq_len], device="cuda")
     oracle.compute_grads(x.float())
-    eng = StageEngine(cfg, [8], [128] * 4, init="reference", use_graph=use_graph, lr=0.0)
+    eng = StageEngine(cfg, [8], [128] * 4, init="reference", use_graph=use_graph, lr=0.0, merge_slices=merge)
+    assert eng._merged == merge
     eng.set_input(x)
     if use_graph:
         # a graph replays whole steps: with lr = 0 the parameters stay put, and the gradients are

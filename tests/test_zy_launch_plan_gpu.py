@@ -16,7 +16,7 @@ def test_replayed_steps_match_derived_steps():
     models = []
     for plan in (False, True):
         eng = StageEngine(cfg, [1, 1], [32, 96], init="device", use_graph=False, lr=1e-3,
-                          launch_plan=plan)
+                          launch_plan=plan, merge_slices=False)
         assert (eng._plan is not None) == plan
         for x in xs:
             eng.set_input(x)
@@ -42,7 +42,7 @@ def test_segment_graph_steps_match_eager_steps():
     models = []
     for seg in (False, True):
         eng = StageEngine(cfg, [1, 1], [32, 96], init="device", use_graph=False, lr=1e-3,
-                          launch_plan=False, segment_graphs=seg)
+                          launch_plan=False, segment_graphs=seg, merge_slices=False)
         assert (eng._seg_graphs is not None) == seg
         for x in xs:
             eng.set_input(x)
