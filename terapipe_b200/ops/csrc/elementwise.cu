@@ -836,3 +836,5 @@ extern "C" int tp_set_pdl(int enabled) {
   tp::pdl_enabled() = enabled ? 1 : 0;
   return kOk;
 }
+// 1 or 0, so that a caller who changes it can put it back.
+extern "C" int tp_pdl_enabled(void) { return tp::pdl_enabled(); }

@@ -172,7 +172,8 @@ def test_attention_long_context_8192():
         assert _rel(got[:, :, :, i], want[:, :, :, i]) < 1.2e-2, name
 
 
-def test_programmatic_dependent_launch_gives_identical_steps():
+@pytest.mark.parametrize("merge", [True, False])
+def test_programmatic_dependent_launch_gives_identical_steps(merge):
     """The GEMM, attention and LayerNorm kernels launched with the programmatic-serialization
     attribute (every kernel waits for its predecessor after its own set-up) produce the same
     parameters as ordinary launches, eagerly and from a captured graph."""
@@ -180,6 +181,7 @@ def test_programmatic_dependent_launch_gives_identical_steps():
     from terapipe_b200.ops.lib import cuda_lib
     from terapipe_b200.runtime.engine import StageEngine
     lib = cuda_lib()
+    before = lib.tp_pdl_enabled()
     cfg = TransformerConfig(batch_size=2, seq_len=256, n_layers=2, embedding_dim=256,
                             num_attention_heads=4, n_devices=1)
     g = torch.Generator().manual_seed(17)
@@ -188,7 +190,8 @@ def test_programmatic_dependent_launch_gives_identical_steps():
     try:
         for pdl, use_graph in ((0, False), (1, False), (1, True)):
             lib.tp_set_pdl(pdl)
-            eng = StageEngine(cfg, [2], [64, 64, 128], init="device", use_graph=use_graph, lr=1e-3)
+            eng = StageEngine(cfg, [2], [64, 64, 128], init="device", use_graph=use_graph, lr=1e-3,
+                              merge_slices=merge)
             for x in xs:
                 eng.set_input(x)
                 eng.step()
@@ -196,5 +199,5 @@ def test_programmatic_dependent_launch_gives_identical_steps():
             eng.check_status()
             results.append(eng.master.clone())
     finally:
-        lib.tp_set_pdl(0)
+        lib.tp_set_pdl(before)
     assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])

@@ -1,9 +1,26 @@
 """Recorded launch plans on the real engine: replayed steps must equal derived ones bit for bit.
 (The recorder itself is covered on CPU in tests/test_aux_cpu.py.)"""
+import os
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def set_pdl():
+    from terapipe_b200.ops.lib import cuda_lib
+    before = cuda_lib().tp_pdl_enabled()
+    yield cuda_lib().tp_set_pdl
+    cuda_lib().tp_set_pdl(before)
+
+
+def test_kernels_are_launched_as_shipped():
+    """Programmatic dependent launch is on unless the environment says otherwise; a test of an
+    earlier file that switched it has to have put it back."""
+    from terapipe_b200.ops.lib import cuda_lib
+    assert cuda_lib().tp_pdl_enabled() == (0 if os.environ.get("TERAPIPE_PDL", "1")[:1] == "0" else 1)
 
 
 def test_replayed_steps_match_derived_steps():
@@ -30,9 +47,12 @@ def test_replayed_steps_match_derived_steps():
     assert models[0][1] == models[1][1]
 
 
-def test_segment_graph_steps_match_eager_steps():
+@pytest.mark.parametrize("pdl", [1, 0])
+def test_segment_graph_steps_match_eager_steps(pdl, set_pdl):
     """Per-segment CUDA graphs (the default for stages that cannot capture the whole step):
-    steps replayed from the segment graphs equal eagerly launched steps bit for bit."""
+    steps replayed from the segment graphs equal eagerly launched steps bit for bit, with and
+    without programmatic dependent launch."""
+    set_pdl(pdl)
     from terapipe_b200.models import TransformerConfig
     from terapipe_b200.runtime.engine import StageEngine
     cfg = TransformerConfig(batch_size=2, seq_len=128, n_layers=2, embedding_dim=256,
