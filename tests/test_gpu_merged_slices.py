@@ -112,3 +112,23 @@ def test_golden_check_runs_the_slices(monkeypatch, tmp_path):
     seen = _count_slices(monkeypatch)
     verify.verify_one_step(str(tmp_path), "load", n_input_slices=4, **kw)
     assert seen == [32] * 4
+
+
+def test_a_turned_round_host_input_is_not_rearranged_on_the_host():
+    """[B, L, H] in pinned memory, handed over as an [L, B, H] view."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    eng = _engine()
+    x = torch.randn(2, 64, 256).half().pin_memory().transpose(0, 1)
+    assert not x.is_contiguous()
+    uploads = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if func is torch.ops.aten.copy_.default and not args[1].is_cuda and args[0].is_cuda:
+                uploads.append(args[1].stride() == args[0].stride())
+            return func(*args, **(kwargs or {}))
+
+    with Watch():
+        eng.set_input(x)
+    assert all(uploads)
+    assert torch.equal(eng.X[0].view(64, 2, 256).cpu(), x)
