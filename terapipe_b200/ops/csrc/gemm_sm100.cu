@@ -34,6 +34,7 @@
 // allocations mapped through CUDA IPC; only ordinary loads and stores touch peer memory.
 #include "common.cuh"
 #include "ptx.cuh"
+#include "tile_choice.h"
 #include "tile_order.h"
 
 namespace tp {
@@ -1515,54 +1516,17 @@ static int dispatch_layout_pair(int a_mn, int b_mn, int out_f32, const CUtensorM
   return kErrBadArgument;
 }
 
-// Tile choice.  Codes: 64 / 128 / 256 = one CTA, 128 x BN tile; 512 = one CTA, 256 x 256;
-// 1000 + BN = CTA pair, 256 x BN (BN = 128, 192, 224, 256).  Relative time of one tile =
-// (tile FLOPs per SM) / (fraction of the MMA rate the shared-memory feed sustains for that
-// shape); total = waves x that.  Wave quantisation matters because M is only ~1024 rows per
-// token slice.
 static bool g_pair_default = true;
 static int g_prefetch = 0;             // L2 prefetch distance of the CTA-pair kernel, in k-steps
 static bool g_ar_exchange = false;     // one-hop exchange instead of reduce-scatter + all-gather
 
-// Measured model of one launch, in kilo-cycles: waves x (main loop of one tile, proportional to
-// K, + epilogue where it does not overlap the next tile) + exposed epilogue of the last tile.
-// `loop` is per 2048 of K: the CTA-pair tiles run at 80-98 % of the MMA rate, the one-CTA tiles
-// at 50-67 % (L2 -> shared-memory feed of one SM).
-struct TileCand {
-  int code, bm, bn;
-  bool pair;
-  float loop, epi_each, tail;
-};
-// 192 and 224 columns are for products of a few waves, whose last one is nearly empty with 256: 2048 x
-// 5120 is 160 tiles of 256 columns on 74 pairs (3 waves of 16.7) or 216 of 192 (3 waves of 13.2).
-// 2048 x 5120 x 10240 took 201 us with 256 columns and takes 163 with 192, 2048 x 7680 x 5120 121 and
-// 110 with 224.
-static const TileCand kTileCands[8] = {
-    {1256, 256, 256, true, 16.7f, 0.0f, 8.5f}, {1128, 256, 128, true, 10.0f, 0.0f, 5.5f},
-    {1224, 256, 224, true, 15.0f, 0.0f, 7.8f}, {1192, 256, 192, true, 13.2f, 0.0f, 7.0f},
-    {512, 256, 256, false, 36.0f, 18.0f, 0.0f}, {256, 128, 256, false, 24.7f, 0.0f, 10.0f},
-    {128, 128, 128, false, 16.4f, 0.0f, 5.4f}, {64, 128, 64, false, 9.5f, 0.0f, 3.0f}};
-
-static int pick_tile(int M, int N, int K, int forced, bool allow_256x256, bool allow_pair) {
+// `forced` is a tile code (tile_choice.h), 0: by the model.
+static int pick_tile(int M, int N, int K, bool b_mn, int forced, bool allow_256x256, bool allow_pair) {
   if (forced == 64 || forced == 128 || forced == 256) return forced;
   if (forced == 512) return allow_256x256 ? 512 : 256;
   if (forced == 1128 || forced == 1256) return allow_pair ? forced : forced - 1000;
   if (forced == 1192 || forced == 1224) return allow_pair ? forced : 256;
-  const int sms = num_sms();
-  int best = 128;
-  float best_t = 1e30f;
-  for (const TileCand& c : kTileCands) {
-    if (c.code == 512 && !allow_256x256) continue;
-    if (c.pair && !(allow_pair && g_pair_default)) continue;
-    const int tiles = ((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
-    const int slots = c.pair ? sms / 2 : sms;
-    const float waves = static_cast<float>((tiles + slots - 1) / slots);
-    const float t = waves * (c.loop * static_cast<float>(K) / 2048.0f + c.epi_each) + c.tail;
-    // (near ties go to the full widths)
-    const bool cut = c.bn == 192 || c.bn == 224;
-    if (t < (cut ? 0.97f : 1.0f) * best_t) { best_t = t; best = c.code; }
-  }
-  return best;
+  return choose_tile(M, N, K, b_mn, allow_256x256, allow_pair && g_pair_default, num_sms());
 }
 
 }  // namespace tp
@@ -1594,7 +1558,7 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   const bool common_layout = (!a_mn && !out_f32) || (a_mn && b_mn && out_f32);
   // only the three layouts of a Linear layer's forward / dgrad / wgrad products have the
   // 256-row tiles instantiated
-  int tile_code = pick_tile(M, N, K, force_bn, common_layout, common_layout);
+  int tile_code = pick_tile(M, N, K, b_mn != 0, force_bn, common_layout, common_layout);
   if (ag) {
     // the wait lives in the CTA-pair kernel's producer
     if (a_mn || !common_layout || ag->rows_per_rank <= 0) return kErrBadArgument;

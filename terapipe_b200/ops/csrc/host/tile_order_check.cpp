@@ -4,6 +4,7 @@
 // CPU tests; no CUDA involved.
 #include <vector>
 
+#include "../tile_choice.h"
 #include "../tile_order.h"
 
 extern "C" {
@@ -39,6 +40,11 @@ long long tp_tile_order_walk(int kind, int M, int N, long long K, int tile_rows,
     s = 1;
   }
   return total;
+}
+
+// The tile code of an ordinary product (all tiles allowed).
+int tp_choose_tile(int M, int N, int K, int b_mn, int sms) {
+  return tp::choose_tile(M, N, K, b_mn != 0, true, true, sms);
 }
 
 }  // extern "C"

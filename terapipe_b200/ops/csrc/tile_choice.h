@@ -1,0 +1,62 @@
+// Which output tile an ordinary product runs on: plain C++, shared by the launch code and the host
+// harness of the CPU tests.
+#pragma once
+
+namespace tp {
+
+// Codes: 64 / 128 / 256 = one CTA, 128 x BN tile; 512 = one CTA, 256 x 256; 1000 + BN = CTA pair,
+// 256 x BN (BN = 128, 192, 224, 256).  Measured model of one launch, in kilo-cycles: waves x (main
+// loop of one tile, proportional to K, + epilogue where it does not overlap the next tile) + exposed
+// epilogue of the last tile.  Wave quantisation matters because M is only ~1024 rows per token slice.
+// `loop` is per 2048 of K: the CTA-pair tiles run at 80-98 % of the MMA rate, the one-CTA tiles
+// at 50-67 % (L2 -> shared-memory feed of one SM).
+struct TileCand {
+  int code, bm, bn;
+  bool pair;
+  float loop, epi_each, tail;
+};
+constexpr TileCand kTileCands[6] = {
+    {1256, 256, 256, true, 16.7f, 0.0f, 8.5f}, {1128, 256, 128, true, 10.0f, 0.0f, 5.5f},
+    {512, 256, 256, false, 36.0f, 18.0f, 0.0f}, {256, 128, 256, false, 24.7f, 0.0f, 10.0f},
+    {128, 128, 128, false, 16.4f, 0.0f, 5.4f}, {64, 128, 64, false, 9.5f, 0.0f, 3.0f}};
+// 192 and 224 columns are for products of a few waves, whose last one is nearly empty with 256: 2048 x
+// 5120 is 160 tiles of 256 columns on 74 pairs (3 waves of 16.7) or 216 of 192 (3 waves of 13.2).
+// 2048 x 5120 x 10240 took 201 us with 256 columns and takes 163 with 192, 2048 x 7680 x 5120 121 and
+// 110 with 224.
+constexpr TileCand kCutCands[2] = {{1224, 256, 224, true, 15.0f, 0.0f, 7.8f},
+                                   {1192, 256, 192, true, 13.2f, 0.0f, 7.0f}};
+
+inline float tile_waves(const TileCand& c, int M, int N, int sms) {
+  const long long tiles = static_cast<long long>((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
+  const int slots = c.pair ? sms / 2 : sms;
+  return static_cast<float>((tiles + slots - 1) / slots);
+}
+
+inline int choose_tile(int M, int N, int K, bool b_mn, bool allow_256x256, bool allow_pair, int sms) {
+  int best = 128;
+  float best_t = 1e30f;
+  for (const TileCand& c : kTileCands) {
+    if ((c.code == 512 && !allow_256x256) || (c.pair && !allow_pair)) continue;
+    const float t = tile_waves(c, M, N, sms) * (c.loop * static_cast<float>(K) / 2048.0f + c.epi_each) + c.tail;
+    if (t < best_t) { best_t = t; best = c.code; }
+  }
+  // A one-CTA tile of 128 or 256 columns wins where the rows are an odd number of 128-row blocks, few
+  // of them: the second CTA of the last pair row has no rows.  The model puts such a tile too slow by
+  // up to a third, so a cut pair tile may not take its place: 77 x 12288 x 4096 takes 21.8 us on
+  // 128 columns and 27.0 on a pair's 192, 300 x 12288 x 3072 26.3 on 256 columns and 34.7; of 47 such
+  // products between 16 and 800 rows, 45 took longer with the cut tile.
+  if (!allow_pair || best == 128 || best == 256) return best;
+  for (const TileCand& c : kCutCands) {
+    const float waves = tile_waves(c, M, N, sms);
+    // Where N is contiguous, B comes in 64-column chunks: a CTA's 96 or 112 columns take the loads of
+    // 128.  In a long row of waves each costs 4 % and 0.3 more than the model says: 10240 x 3840 x
+    // 1280 took 71 us with 256 columns and 79 with 192, 8192 x 3072 x 768 32.7 and 35.4.
+    const bool chunks = b_mn && waves > 4.0f;
+    const float loop = c.loop * (chunks ? 1.04f : 1.0f) * static_cast<float>(K) / 2048.0f;
+    const float t = waves * (loop + c.epi_each + (chunks ? 0.3f : 0.0f)) + c.tail;
+    if (t < 0.97f * best_t) { best_t = t; best = c.code; }   // near ties go to the full widths
+  }
+  return best;
+}
+
+}  // namespace tp

@@ -10,8 +10,8 @@ uniform slices.  Inside a training step the kernels run back to back (CUDA graph
 queue), and their times follow from a handful of measured constants:
 
 * GEMMs: cycles = set-up + waves x main loop of one tile (proportional to K) + exposed epilogue
-  of the last tile, for the tile shapes of ``csrc/gemm_sm100.cu`` (the same table as its
-  ``pick_tile``), at the SM clock seen under load;
+  of the last tile, for the full-width tile shapes of ``csrc/tile_choice.h`` (it was calibrated
+  with these, before the 192- and 224-column tiles), at the SM clock seen under load;
 * attention: a fixed part plus a cost per 128-key (forward, dQ) or 128-query (dK/dV) block and
   wave of CTAs;
 * LayerNorm and the all-reduce: a fixed part plus bytes over an effective bandwidth.
@@ -38,7 +38,7 @@ class B200KernelModel:
     sm_mhz: float = 1792.0          # median SM clock during a step (power capped)
     launch_us: float = 5.0          # kernel-to-kernel gap + prologue not covered by the cycle counts
     n_sms: int = 148
-    # ---- GEMM (kilo-cycles; same candidates as pick_tile in csrc/gemm_sm100.cu)
+    # ---- GEMM (kilo-cycles; the full-width candidates of csrc/tile_choice.h)
     gemm_setup_kc: float = 2.7
     gemm_cold_l2: float = 1.2       # operands of a step are cold in L2: main loop slow-down
     gemm_long_k: float = 1.45       # K >= 8192: DRAM streaming and power cap stretch the main loop

@@ -35,3 +35,22 @@ def test_every_tile_once_and_operands_few_times(M, N, K, cols):
         key = 1 if order[2] == 2 else 0
         seen = [t[key] // order[5] for t in tiles]
         assert seen == sorted(seen)
+
+
+def _tile(M, N, K, b_mn=0):
+    from terapipe_b200.ops.lib import host_lib
+    return host_lib().tp_choose_tile(M, N, K, b_mn, 148)
+
+
+@pytest.mark.parametrize("M,N,K,b_mn,code", [
+    # an odd number of 128-row blocks, few of them: a pair's second CTA would have no rows
+    (16, 15360, 5120, 1, 128), (77, 12288, 4096, 0, 128), (77, 12288, 4096, 1, 128), (128, 10240, 2560, 0, 128),
+    (300, 12288, 3072, 1, 256), (600, 6912, 2304, 0, 256), (800, 2560, 10240, 1, 128),
+    # N contiguous and more than four waves, which cost more than with K contiguous
+    (10240, 3840, 1280, 1, 1256), (8192, 4800, 1600, 1, 1256), (8192, 3072, 768, 1, 1256),
+    # few waves, the last one nearly empty at full width
+    (2048, 5120, 10240, 0, 1192), (2048, 5120, 10240, 1, 1192), (2048, 7680, 5120, 0, 1224),
+    # full widths where they fit, small products on small tiles
+    (1024, 2048, 8192, 0, 1128), (16384, 8192, 2048, 1, 1256), (256, 256, 256, 0, 64)])
+def test_tile_choice(M, N, K, b_mn, code):
+    assert _tile(M, N, K, b_mn) == code
