@@ -42,9 +42,9 @@ long long tp_tile_order_walk(int kind, int M, int N, long long K, int tile_rows,
   return total;
 }
 
-// The tile code of an ordinary product (all tiles allowed).
-int tp_choose_tile(int M, int N, int K, int b_mn, int sms) {
-  return tp::choose_tile(M, N, K, b_mn != 0, true, true, sms);
+// The tile code of an ordinary product, or (cut = 0) of an all-gather -> GEMM product.
+int tp_choose_tile(int M, int N, int K, int b_mn, int cut, int sms) {
+  return tp::choose_tile(M, N, K, b_mn != 0, true, true, cut != 0, sms);
 }
 
 }  // extern "C"

@@ -32,7 +32,10 @@ inline float tile_waves(const TileCand& c, int M, int N, int sms) {
   return static_cast<float>((tiles + slots - 1) / slots);
 }
 
-inline int choose_tile(int M, int N, int K, bool b_mn, bool allow_256x256, bool allow_pair, int sms) {
+// allow_cut: an all-gather -> GEMM product keeps the full widths, with which its order of tiles (this
+// rank's row blocks first) was built and measured on several GPUs.
+inline int choose_tile(int M, int N, int K, bool b_mn, bool allow_256x256, bool allow_pair, bool allow_cut,
+                       int sms) {
   int best = 128;
   float best_t = 1e30f;
   for (const TileCand& c : kTileCands) {
@@ -45,7 +48,7 @@ inline int choose_tile(int M, int N, int K, bool b_mn, bool allow_256x256, bool 
   // up to a third, so a cut pair tile may not take its place: 77 x 12288 x 4096 takes 21.8 us on
   // 128 columns and 27.0 on a pair's 192, 300 x 12288 x 3072 26.3 on 256 columns and 34.7; of 47 such
   // products between 16 and 800 rows, 45 took longer with the cut tile.
-  if (!allow_pair || best == 128 || best == 256) return best;
+  if (!allow_pair || !allow_cut || best == 128 || best == 256) return best;
   for (const TileCand& c : kCutCands) {
     const float waves = tile_waves(c, M, N, sms);
     // Where N is contiguous, B comes in 64-column chunks: a CTA's 96 or 112 columns take the loads of

@@ -144,3 +144,28 @@ def test_colsum_and_fused_adam():
         assert grad.abs().max().item() == 0.0
     assert _rel(p, ref_p.detach()) < 1e-5
     assert _rel(model, p) < 1e-3
+
+
+# products that an ordinary call runs on 192 and 224 columns; rows end inside a block of the last rank
+@pytest.mark.parametrize("M,N,K", [(2048, 5120, 640), (2040, 7680, 320)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_all_gather_product_with_every_rank_arrived(M, N, K, b_mn):
+    """tp_gemm_ag as rank 1 of 4 whose peers' rows are all there (their flags are up before the
+    launch, so nothing waits): the order of tiles, the tile width and the epilogue."""
+    from terapipe_b200.ops import functional as F
+    from terapipe_b200.ops.lib import check, cuda_lib
+    torch.manual_seed(8)
+    a = torch.randn(M, K, device="cuda").half()
+    w = (torch.randn(*((K, N) if b_mn else (N, K)), device="cuda") * 0.05).half()
+    bias = torch.randn(N, device="cuda").half()
+    out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float16)
+    pre = torch.full_like(out, float("nan"))
+    flags = torch.full((16,), 7, device="cuda", dtype=torch.int32)
+    base = torch.zeros(1, device="cuda", dtype=torch.int32)
+    check(cuda_lib().tp_gemm_ag(0, int(b_mn), a.data_ptr(), K, w.data_ptr(), w.stride(0), out.data_ptr(), N, M, N, K,
+                                bias.data_ptr(), 2, pre.data_ptr(), 0, None, N, flags.data_ptr(), base.data_ptr(),
+                                5, 512, 1, F.status_word().data_ptr(), torch.cuda.current_stream().cuda_stream),
+          "tp_gemm_ag")
+    F.check_device_status()
+    z = a.float() @ (w.float() if b_mn else w.float().t()) + bias.float()
+    assert _rel(pre, z) < 2e-3 and _rel(out, torch.nn.functional.gelu(z)) < 3e-3

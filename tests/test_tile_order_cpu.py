@@ -37,9 +37,9 @@ def test_every_tile_once_and_operands_few_times(M, N, K, cols):
         assert seen == sorted(seen)
 
 
-def _tile(M, N, K, b_mn=0):
+def _tile(M, N, K, b_mn=0, cut=1):
     from terapipe_b200.ops.lib import host_lib
-    return host_lib().tp_choose_tile(M, N, K, b_mn, 148)
+    return host_lib().tp_choose_tile(M, N, K, b_mn, cut, 148)
 
 
 @pytest.mark.parametrize("M,N,K,b_mn,code", [
@@ -54,3 +54,10 @@ def _tile(M, N, K, b_mn=0):
     (1024, 2048, 8192, 0, 1128), (16384, 8192, 2048, 1, 1256), (256, 256, 256, 0, 64)])
 def test_tile_choice(M, N, K, b_mn, code):
     assert _tile(M, N, K, b_mn) == code
+
+
+@pytest.mark.parametrize("M,N,K,b_mn", [(2048, 5120, 10240, 0), (2048, 5120, 10240, 1), (2048, 7680, 5120, 0),
+                                        (1024, 6144, 2048, 0)])
+def test_all_gather_products_keep_full_widths(M, N, K, b_mn):
+    assert _tile(M, N, K, b_mn) in (1192, 1224)
+    assert _tile(M, N, K, b_mn, cut=0) in (1128, 1256)
