@@ -123,8 +123,14 @@ struct FwdShared {
 };
 
 constexpr int kFwdStages = 4;   // depth of the K and of the V ring
-// The merge costs about a microsecond: 128 queries of 8 heads took 10.8 us split over 2 blocks, 10.2 not
-// split; at 32 blocks (128 queries behind 1920 keys, 8 x 16 heads) the split takes 38.7 us, 47.4 before it.
+// A split saves a part of every block and pays for the merge, which has more columns to move at D = 128.
+// 128 queries, us split / not split, at 8 heads and at 256:
+//   key blocks         5          8          12         32
+//   D = 64, 8       6.0/6.1    7.5/7.9    9.2/10.3   17.8/22.4
+//   D = 64, 256   12.8/12.7  15.6/16.5   19.4/21.5   38.7/48.0
+//   D = 128, 8      7.8/7.0    9.2/8.9   11.1/11.4   20.0/23.7
+//   D = 128, 256  16.6/15.1  20.4/19.6   27.7/27.5   54.4/55.0
+// 8 lies between the two widths' even points, 5 and 10 to 12.
 constexpr int kSplitBlocks = 8;
 
 template <typename T, int D>
@@ -135,6 +141,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr int kQSub = 128 * 128, kKSub = 64 * 128;   // [rows][64 columns] 16-bit, 128-byte swizzle
   constexpr int kQTile = DH * kQSub, kKTile = DH * kKSub;
   constexpr int KS = kFwdStages;
+  static_assert(kSplitBlocks >= 2, "both groups of a split tile have blocks");
+  static_assert(D * 128 * 4 <= KS * kKTile, "the groups of a split tile exchange their halves through the K ring");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -318,7 +326,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_st_32x32(tO + ch * 32, raw);
         }
       }
-      // a row that has seen no key yet (second group, its first block beyond the diagonal) has m = -inf
+      // m = -inf: every score so far has overflowed (a row sees keys in its group's first block)
       const float2 nm = dup2(m == -INFINITY ? 0.0f : -m), sc = dup2(p.scale2);
       float2 sum = make_float2(0.0f, 0.0f);   // of this block first: shorter chains of additions
 #pragma unroll
@@ -379,16 +387,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (row_ok) *lse_slot = m + log2f(l);
       }
     } else {
-      // Each group finishes half of the columns and hands the other half over through the K and V
-      // rings (every tile has been used once both groups' last products are done).
+      // Each group finishes half of the columns and hands the other half over through the K ring
+      // (every tile has been used once both groups' last products are done).
       if (ok) ok = mbar_wait(&sh->bar_fin[0], 0, wctx, kErrWaitAttn);
-      if (ok && n_it1 > 0) ok = mbar_wait(&sh->bar_fin[1], 0, wctx, kErrWaitAttn);
+      if (ok) ok = mbar_wait(&sh->bar_fin[1], 0, wctx, kErrWaitAttn);
       tc_fence_after();
       float* give = reinterpret_cast<float*>(sK) + w * (D / 2) * 128;        // [D / 2][128 rows]
       const float* take = reinterpret_cast<const float*>(sK) + (w ^ 1) * (D / 2) * 128;
       sh->m[w][r] = m;
       sh->l[w][r] = l;
-      if (ok && n_it > 0) {
+      if (ok) {
 #pragma unroll 1
         for (int ch = 0; ch < D / 64; ++ch) {
           float v[32];
@@ -400,8 +408,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       named_bar_sync(1, 256);
       if (ok) {
         const float m_o = sh->m[w ^ 1][r], l_o = sh->l[w ^ 1][r];
-        const bool other = w == 1 || n_it1 > 0;    // the other group had blocks
         const float mm = fmaxf(m, m_o);
+        // (both groups see keys of every row; m = -inf are scores that overflowed)
         const float a = m == -INFINITY ? 0.0f : exp2f(m - mm);
         const float a_o = m_o == -INFINITY ? 0.0f : exp2f(m_o - mm);
         l = l * a + l_o * a_o;
@@ -410,18 +418,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int ch = 0; ch < D / 64; ++ch) {
           const int col = w * (D / 2) + ch * 32;
           float v[32];
-          if (n_it > 0) {
-            load32(col, v);
+          load32(col, v);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] *= a;
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.0f;
-          }
-          if (other) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] += take[(ch * 32 + i) * 128 + r] * a_o;
-          }
+          for (int i = 0; i < 32; ++i) v[i] = fmaf(take[(ch * 32 + i) * 128 + r], a_o, v[i] * a);
           if (row_ok) store32(col, v, inv_l);
         }
         if (row_ok && w == 0) *lse_slot = mm + log2f(l);
