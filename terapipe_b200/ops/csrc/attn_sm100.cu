@@ -873,6 +873,9 @@ template <int D> constexpr int bwd_smem() {
   return (D / 64) * (2 * 128 * 128 + kBwdStages * 2 * 64 * 128) + 1024 + static_cast<int>(sizeof(BwdShared)) + 64;
 }
 
+static_assert(fwd_smem<64>() >= kTmemKernelMinSmem && bwd_smem<64>() >= kTmemKernelMinSmem,
+              "allocate TMEM before pdl_wait");
+
 template <typename T, int D>
 static int attn_fwd_launch(const void* qkv, const AttnParams& p, bool bf16, cudaStream_t s) {
   CUtensorMap tmQ, tmKV;

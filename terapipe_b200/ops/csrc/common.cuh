@@ -135,6 +135,12 @@ inline int num_sms() {
   return n;
 }
 
+// A kernel may let its successor start before it has allocated its TMEM (the CTA-pair GEMM does).  A
+// successor that allocated all of it first and then waited for that kernel would never end, so the two
+// must not fit on one SM together: every kernel that allocates TMEM before pdl_wait() takes at least
+// kTmemKernelMinSmem of shared memory, and one that allocates it afterwards leaves less than that.
+constexpr int kSmemPerSm = 228 * 1024, kTmemKernelMinSmem = 96 * 1024;
+
 // Launch with programmatic stream serialization (see pdl_wait in ptx.cuh).  The kernel must call
 // pdl_wait() in every thread before its first access to global data.  On unless tp_set_pdl(0) was
 // called or the environment variable TERAPIPE_PDL=0 is set at first use: the set-up of a kernel

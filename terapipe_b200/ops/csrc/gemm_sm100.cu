@@ -736,6 +736,7 @@ template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool AR = fals
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmO,
                        const GemmParams& p, cudaStream_t stream, const ArParams* arp = nullptr) {
   using Cfg = GemmCfg<BN, MT, AR>;
+  static_assert(Cfg::kSmemBytes >= kTmemKernelMinSmem, "allocates TMEM before pdl_wait");
   auto kern = gemm_kernel<T, BN, A_MN, B_MN, OUT_F32, AR, MT>;
   ArParams ar;
   if (arp) ar = *arp;
@@ -1488,6 +1489,7 @@ template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool TRACE = f
 static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmO,
                             const GemmParams& p, cudaStream_t stream, const ArParams* arp = nullptr) {
   using Cfg = PairCfg<BN>;
+  static_assert(Cfg::kSmemBytes + kTmemKernelMinSmem > kSmemPerSm, "allocates TMEM after pdl_wait");
   auto kern = gemm_pair_kernel<T, BN, A_MN, B_MN, OUT_F32, TRACE, AR, RS>;
   static bool configured = false;
   if (!configured) {
