@@ -107,7 +107,7 @@ def build_cuda(force=False, verbose=False, ptxas_info=False, checked=False) -> P
 
 def build_host(force=False, verbose=False) -> Path:
     srcs = sorted((CSRC / "host").glob("*.cpp"))
-    deps = srcs + [CSRC / "tile_order.h", CSRC / "tile_choice.h"]   # shared with the kernels' launch code
+    deps = srcs + sorted(CSRC.glob("*.h"))     # plain C++, shared with the kernels' launch code
     if not force and not _stale(HOST_LIB, deps):
         return HOST_LIB
     tmp = HOST_LIB.with_suffix(".so.tmp")

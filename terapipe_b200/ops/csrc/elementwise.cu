@@ -2,6 +2,7 @@
 // column sums, the fused mixed-precision Adam update and small helpers.  All use 16-byte
 // vector accesses; statistics and reductions are fp32.
 #include "common.cuh"
+#include "ln_geometry.h"
 #include "ptx.cuh"
 
 namespace tp {
@@ -174,11 +175,11 @@ layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   push_signal(pd);
 }
 
-// Backward geometry: one CTA per SM of 24 warps (16 where a row takes 16), so an SM holds 24 / WPR
-// rows at a time, each with its three inputs in flight.
-template <int WPR> struct LnBwdGeom {
-  static constexpr int kWarps = WPR == 16 ? 16 : 24;
-  static constexpr int kRowsPerCta = kWarps / WPR;
+// Backward geometry (ln_geometry.h): one CTA per SM, so an SM holds kRowsPerCta rows at a time, each with
+// its three inputs in flight.
+template <int NV, int WPR> struct LnBwdGeom {
+  static constexpr int kWarps = ln_bwd_warps(NV, WPR);
+  static constexpr int kRowsPerCta = ln_bwd_rows(NV, WPR);
   static constexpr int kThreads = kWarps * 32;
 };
 
@@ -190,15 +191,15 @@ template <int WPR> struct LnBwdGeom {
 // 16 bytes (no bank conflicts).  At the end the regions are added in a fixed order and the CTA
 // writes (or adds to) one slot of scratch[gridDim.x][2][H]; a second kernel adds the slots into
 // the fp32 gradients.  x, dy and dres of a row are loaded together and stay in their 16-bit form (xhat
-// and g are computed twice), which fits 24 warps; 16 warps that fetched dres after the row's
+// and g are computed twice), which fits 16 to 24 warps; 16 that fetched dres after the row's
 // reductions took 98 us for 16384 x 2048.
 template <typename T, int NV, int WPR>
-__global__ void __launch_bounds__(LnBwdGeom<WPR>::kThreads, 1)
+__global__ void __launch_bounds__(LnBwdGeom<NV, WPR>::kThreads, 1)
 layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                      const float* __restrict__ mean, const float* __restrict__ rstd,
                      const T* __restrict__ gamma, const T* __restrict__ dres, const PushDst pd,
                      float* __restrict__ scratch, int rows, int H, int accumulate_slots) {
-  using G = LnBwdGeom<WPR>;
+  using G = LnBwdGeom<NV, WPR>;
   extern __shared__ __align__(16) float part_smem[];  // [kRowsPerCta][2][H]
   __shared__ float red[2 * 2 * G::kRowsPerCta * WPR + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -494,18 +495,6 @@ __global__ void fill_kernel(T* p, long long n, float value) {
 
 using namespace tp;
 
-// Geometry: the smallest power-of-two warps-per-row (<= 16) that keeps at most `most` vectors of 8
-// elements per lane.
-static inline bool ln_geometry(int H, int* nv, int* wpr, int most = 4) {
-  if (H % 8 || H <= 0) return false;
-  const int vecs = H / 8;
-  for (int w = 1; w <= 16; w *= 2) {
-    const int n = (vecs + 32 * w - 1) / (32 * w);
-    if (n <= most) { *nv = n; *wpr = w; return true; }
-  }
-  return false;
-}
-
 #define TP_LN_DISPATCH_WPR(T, NV, CALL)                  \
   switch (wpr) {                                          \
     case 1: CALL(T, NV, 1); break;                        \
@@ -547,7 +536,7 @@ static int layernorm_fwd_launch(int dtype, const void* x, const void* gamma, con
                                 float eps, cudaStream_t s) {
   if (rows <= 0) return kOk;
   int nv, wpr;
-  if (!ln_geometry(H, &nv, &wpr)) return kErrBadArgument;
+  if (!ln_geometry(H, &nv, &wpr, 4)) return kErrBadArgument;
 #define LN_FWD(T, NV, WPR)                                                                       \
   launch_pdl(layernorm_fwd_kernel<T, NV, WPR>,                                                   \
              dim3((rows + LnGeom<WPR>::kRowsPerCta - 1) / LnGeom<WPR>::kRowsPerCta),             \
@@ -603,9 +592,8 @@ template <typename K> static void ln_allow_smem(K kern) {
   if (n_seen < 64) seen[n_seen++] = key;
 }
 
-static int ln_parts(int rows, int wpr) {
-  const int rpc = wpr == 16 ? 1 : 24 / wpr;   // LnBwdGeom<WPR>::kRowsPerCta
-  int parts = (rows + rpc - 1) / rpc;
+static int ln_parts(int rows, int rows_per_cta) {
+  int parts = (rows + rows_per_cta - 1) / rows_per_cta;
   const int cap = tp_layernorm_bwd_parts(rows);
   return parts > cap ? cap : parts;
 }
@@ -618,19 +606,17 @@ static int layernorm_bwd_launch(int dtype, const void* dy, const void* x, const 
                                 const PushDst& pd, float* dgamma, float* dbeta, float* scratch,
                                 int rows, int H, int mode, cudaStream_t s) {
   if (rows <= 0) return kOk;
-  // at most three vectors per lane where that is possible: a fourth one of each input leaves too few
-  // of the 80 registers to keep all loads in flight (16384 x 2048: 85 us with four, 75 with two;
-  // 4096 x 1024: 28 and 14)
   int nv, wpr;
-  if (!ln_geometry(H, &nv, &wpr, 3) && !ln_geometry(H, &nv, &wpr, 4)) return kErrBadArgument;
-  const int parts = ln_parts(rows, wpr);
+  if (!ln_bwd_geometry(H, rows, num_sms(), &nv, &wpr)) return kErrBadArgument;
+  const int rows_per_cta = ln_bwd_rows(nv, wpr);
+  const int parts = ln_parts(rows, rows_per_cta);
   // one [2][H] fp32 region per row group of the CTA: at most 192 KB (H <= 1024 * WPR)
-  const size_t smem = static_cast<size_t>(wpr == 16 ? 1 : 24 / wpr) * 2 * H * sizeof(float);
+  const size_t smem = static_cast<size_t>(rows_per_cta) * 2 * H * sizeof(float);
 #define LN_BWD(T, NV, WPR)                                                                      \
   {                                                                                             \
     auto kern = layernorm_bwd_kernel<T, NV, WPR>;                                               \
     if (smem > 40 * 1024) ln_allow_smem(kern); /* dynamic + static must stay under 48 KB */    \
-    launch_pdl(kern, dim3(parts), dim3(LnBwdGeom<WPR>::kThreads), smem, s, 1,                   \
+    launch_pdl(kern, dim3(parts), dim3(LnBwdGeom<NV, WPR>::kThreads), smem, s, 1,                   \
                static_cast<const T*>(dy), static_cast<const T*>(x), mean, rstd,                 \
                static_cast<const T*>(gamma), static_cast<const T*>(dres), pd, scratch,           \
                rows, H, mode);                                                                  \

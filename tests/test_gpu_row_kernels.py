@@ -12,10 +12,13 @@ def _rel(a, ref):
     return ((a.double() - ref).norm() / ref.norm()).item()
 
 
-# H: 1, 2, 4, 8 and 16 warps a row, columns that end inside a vector round; rows: one, fewer than
+# (csrc/ln_geometry.h) H: 1, 2, 4, 8 and 16 warps a row, columns that end inside a vector round; rows: one, fewer than
 # and just more than a CTA holds, more than one round of all CTAs
 @pytest.mark.parametrize("H,rows", [(8, 5), (264, 25), (1024, 3700), (1600, 13), (2048, 1800), (2560, 7),
-                                    (4096, 900), (5120, 500), (8200, 3), (12288, 160)])
+                                    (4096, 900), (5120, 500), (8200, 3), (12288, 160),
+                                    # one round of one, two and four vectors a lane; 24 warps of four
+                                    (768, 40), (2304, 300), (5120, 64), (1600, 1100), (4096, 590), (8192, 2049),
+                                    (16384, 160)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_layernorm_geometries(H, rows, dtype):
     from terapipe_b200.ops import functional as F
