@@ -305,11 +305,9 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
 // microseconds long, so separate launches cost more than the sums.  A CTA of 256 threads takes 8 V
 // columns of a chunk of rows, 8 rows of 16 bytes per thread in flight.  The (at most 8) chunks of a
 // column block form a cluster whose first CTA adds them up in order through distributed shared
-// memory, so the sums do not depend on timing.  V = 32 reads longer pieces of a row (4096 rows of a
-// 12288-wide layer: 191 us against 239 for V = 8), but gives a 2048-wide layer 72 clusters, a few more
-// than the GPCs hold at once: 156 us for 16384 rows (604 MB) against 114.  So V = 32 from 128 blocks of
-// 256 columns on.  (One launch per matrix with one load in flight per thread ran on 64 of 148 SMs:
-// 16384 x 2048 alone took 63 us.)
+// memory, so the sums do not depend on timing.  V = 32 reads longer pieces of a row and V = 8 makes four
+// times as many CTAs of them; layer_sums_launch has the line between them.  (One launch per matrix with
+// one load in flight per thread ran on 64 of 148 SMs: 16384 x 2048 alone took 63 us.)
 constexpr int kMaxColsums = 4, kMaxFolds = 2;
 struct SumJobs {
   const void* dy[kMaxColsums];
@@ -682,11 +680,23 @@ namespace tp {
 static int layer_sums_launch(int dtype, SumJobs& j, cudaStream_t s) {
   long long blocks = 0;           // of 256 columns
   for (int i = 0; i < j.n; ++i) blocks += (j.N[i] + 255) / 256;
-  const bool wide = blocks >= 128;
+  // V = 32 once its CTAs fill the chip, us V = 8 / V = 32:
+  //   one layer's four matrices of width  768 (27 blocks)   2048 (72)     4096 (144)
+  //     rows    256                         3.8 / 5.0       5.3 / 6.3     7.8 / 10.2
+  //     rows   1024                         6.0 / 6.6      11.0 / 10.4   21.7 / 14.3
+  //     rows  16384                        49.1 / 60.3      108 / 93.6    203 / 182
+  const bool wide = blocks >= 128 || (blocks >= 48 && blocks * j.rows >= 48 * 1024);
   const int cols = wide ? 256 : 64, round = 8 * 256 / (cols / 8);   // rows of one round of loads
-  // chunks of at least one round, a portable cluster of them at most
+  // Chunks of at least one round, a portable cluster of them at most; with V = 32 no more than 4 CTAs per
+  // SM, which run at once (2560-wide layer, 16384 rows: 156 us with 8 chunks a block, 131 with 4;
+  // 5120-wide, 1024 rows: 28.6 with 8, 21.8 with 2), unless even two chunks take several rounds.
+  int most = 8;
+  if (wide) {
+    while (most > 2 && blocks * most > 4 * num_sms()) most /= 2;
+    if (blocks * most > 4 * num_sms()) most = 4;
+  }
   j.chunks = 1;
-  while (j.n > 0 && j.chunks < 8 && j.rows >= 2 * round * j.chunks) j.chunks *= 2;
+  while (j.n > 0 && j.chunks < most && j.rows >= 2 * round * j.chunks) j.chunks *= 2;
   j.rows_per_chunk = (j.rows + j.chunks - 1) / j.chunks;
   long long ctas = 0;
   for (int i = 0; i < j.n; ++i) {

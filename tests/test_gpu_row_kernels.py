@@ -43,7 +43,9 @@ def test_layernorm_geometries(H, rows, dtype):
 
 @pytest.mark.parametrize("rows,widths", [(1, (8,)), (63, (264, 8)), (127, (256, 72)), (128, (512, 8, 1032, 256)),
                                          (1000, (768, 3072)), (4100, (2048, 512, 768, 1536)), (70, (32768,)),
-                                         (1025, (12288, 16384, 4096))])
+                                         (1025, (12288, 16384, 4096)),
+                                         # 256-column blocks: 48 of them in 8 chunks, 200 in 2, 320 in 4
+                                         (2100, (12288,)), (1100, (10240, 40960)), (1030, (81920,))])
 def test_layer_sums_and_folds(rows, widths):
     from terapipe_b200.ops.lib import check, cuda_lib
     g = torch.Generator(device="cuda").manual_seed(rows)
