@@ -34,7 +34,6 @@ GEMM + all-reduce kernel over NVLink peer memory (``tp_comm="fused"``).
 from __future__ import annotations
 
 import ctypes
-import gc
 import math
 import os
 from typing import Dict, List, Optional, Sequence
@@ -46,6 +45,7 @@ from .. import parallel as mpu
 from ..models import TransformerConfig
 from ..ops import functional as F
 from ..ops.lib import KernelError, cuda_lib
+from ..utils.misc import collection_paused
 
 LOSS_SCALE_FACTOR = 128.0
 _ACT = {"none": 0, "relu": 1, "gelu": 2}
@@ -1218,10 +1218,8 @@ class StageEngine:
         # the driver first, which takes far longer than the capture: tens of milliseconds, and
         # hundreds when another engine has just been released.)  Nothing may be collected while
         # the capture runs, though: the destructor of an old graph is not a legal call then.
-        collecting = gc.isenabled()
-        gc.disable()
         try:
-            with torch.cuda.stream(self._cap_stream):
+            with collection_paused(), torch.cuda.stream(self._cap_stream):
                 graph.capture_begin(capture_error_mode="thread_local")
                 try:
                     self._iteration()
@@ -1241,9 +1239,6 @@ class StageEngine:
             if self._plan is None and self._seg_graphs is None:
                 self._seg_graphs = {}
             return
-        finally:
-            if collecting:
-                gc.enable()
         self._graph = graph
 
     def check_status(self):

@@ -5,6 +5,7 @@ Counterparts of the reference's utils.py (:11-111).
 from __future__ import annotations
 
 import builtins
+import contextlib
 import errno
 import functools
 import gc
@@ -20,6 +21,29 @@ import torch
 
 class TimeoutError(Exception):  # noqa: A001 - name kept for callers of the reference API
     pass
+
+
+_gc_lock = threading.Lock()
+_gc_pauses, _gc_was_on = 0, False
+
+
+@contextlib.contextmanager
+def collection_paused():
+    """No garbage collection inside the block.  Blocks of several threads may overlap: the collector
+    comes back, if it was on before the first, when the last of them ends."""
+    global _gc_pauses, _gc_was_on
+    with _gc_lock:
+        if _gc_pauses == 0:
+            _gc_was_on = gc.isenabled()
+            gc.disable()
+        _gc_pauses += 1
+    try:
+        yield
+    finally:
+        with _gc_lock:
+            _gc_pauses -= 1
+            if _gc_pauses == 0 and _gc_was_on:
+                gc.enable()
 
 
 def timeout(seconds: int = 10, error_message: str = os.strerror(errno.ETIME)):

@@ -175,3 +175,42 @@ def test_a_stage_merges_its_slices_only_where_nothing_depends_on_them():
         assert not wants(False, pp, tp, per_slice=False)
         with pytest.raises(ValueError):
             wants(True, pp, tp, per_slice=False)
+
+
+@pytest.mark.parametrize("on", [True, False])
+def test_overlapping_pauses_of_garbage_collection(on):
+    """Two threads whose captures overlap: nothing is collected until both have ended."""
+    import gc
+    import threading
+    from terapipe_b200.utils.misc import collection_paused
+    was = gc.isenabled()
+    first_in, second_in, first_out = (threading.Event() for _ in range(3))
+    seen = []
+
+    def first():
+        with collection_paused():
+            first_in.set()
+            second_in.wait(10)
+        first_out.set()
+
+    def second():
+        first_in.wait(10)
+        with collection_paused():
+            second_in.set()
+            first_out.wait(10)
+            seen.append(gc.isenabled())
+
+    (gc.enable if on else gc.disable)()
+    try:
+        threads = [threading.Thread(target=f) for f in (first, second)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(20)
+        assert seen == [False] and gc.isenabled() == on
+        with pytest.raises(KeyError):
+            with collection_paused():
+                raise KeyError
+        assert gc.isenabled() == on
+    finally:
+        (gc.enable if was else gc.disable)()
