@@ -1211,13 +1211,17 @@ class StageEngine:
 
     def _capture(self):
         torch.cuda.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        if self._cap_stream is None:
-            self._cap_stream = torch.cuda.Stream()
         # (torch.cuda.graph() would also collect garbage and give torch's cached memory back to
         # the driver first, which takes far longer than the capture: tens of milliseconds, and
         # hundreds when another engine has just been released.)  Nothing may be collected while
-        # the capture runs, though: the destructor of an old graph is not a legal call then.
+        # the capture runs, though: the destructor of an old graph is not a legal call then.  And
+        # torch does not give memory back during a capture: where little is left for the stream, the
+        # loss sum (2 and 20 MB segments of a new pool) and the graph itself, it is given back before.
+        if torch.cuda.mem_get_info(self.device)[0] < 256 << 20:
+            torch.cuda.empty_cache()
+        graph = torch.cuda.CUDAGraph()
+        if self._cap_stream is None:
+            self._cap_stream = torch.cuda.Stream()
         try:
             with collection_paused(), torch.cuda.stream(self._cap_stream):
                 graph.capture_begin(capture_error_mode="thread_local")

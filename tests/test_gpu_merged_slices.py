@@ -132,3 +132,21 @@ def test_a_turned_round_host_input_is_not_rearranged_on_the_host():
         eng.set_input(x)
     assert all(uploads)
     assert torch.equal(eng.X[0].view(64, 2, 256).cpu(), x)
+
+
+@pytest.mark.parametrize("free", [1 << 20, 1 << 30])
+def test_capture_makes_room_when_memory_is_short(free, monkeypatch):
+    """Torch cannot give cached memory back while a capture runs."""
+    from terapipe_b200.models import TransformerConfig
+    from terapipe_b200.runtime.engine import StageEngine
+    cfg = TransformerConfig(batch_size=2, seq_len=64, n_layers=1, embedding_dim=256,
+                            num_attention_heads=4, n_devices=1)
+    eng = StageEngine(cfg, [2], [64], use_graph=True)
+    emptied = []
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (free, 180 << 30))
+    monkeypatch.setattr(torch.cuda, "empty_cache",
+                        lambda: emptied.append(torch.cuda.is_current_stream_capturing()))
+    eng.set_input(torch.randn(64, 2, 256))
+    eng.step()
+    assert eng._graph is not None
+    assert emptied == ([False] if free < 256 << 20 else [])
