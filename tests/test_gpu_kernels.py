@@ -57,34 +57,43 @@ def test_gemm_wgrad_layout_accumulates(dtype):
     F.check_device_status()
 
 
+# 0: the tile that the size gets; the CTA-pair widths on a ragged last tile in both directions (456 and 680
+# end inside a 32-column chunk of a 192- and of a 224-column tile)
+@pytest.mark.parametrize("M,N,bn", [(256, 512, 0)] + [(M, N, bn) for M, N in ((1000, 456), (413, 680))
+                                                      for bn in (0, 1128, 1192, 1224, 1256)])
 @pytest.mark.parametrize("act", ["relu", "gelu"])
-def test_gemm_activation_epilogues(act):
+def test_gemm_activation_epilogues(act, M, N, bn):
     from terapipe_b200.ops import functional as F
     torch.manual_seed(3)
     dtype = torch.float16
-    M, N, K = 256, 512, 256
+    K = 256
     x = torch.randn(M, K, device="cuda", dtype=dtype)
     w = torch.randn(N, K, device="cuda", dtype=dtype) * 0.1
     b = torch.randn(N, device="cuda", dtype=dtype)
     res = torch.randn(M, N, device="cuda", dtype=dtype)
-    out = torch.empty(M, N, device="cuda", dtype=dtype)
-    pre = torch.empty(M, N, device="cuda", dtype=dtype)
-    F.gemm(x, w, out, bias=b, act=act, aux_out=pre if act == "gelu" else None)
+    # results are windows of larger matrices, whose rest must stay as it is
+    whole = [torch.full((M + 3, N + 8), float("nan"), device="cuda", dtype=dtype) for _ in range(2)]
+    out, pre = (t[:M, :N] for t in whole)
+    F.gemm(x, w, out, bias=b, act=act, aux_out=pre if act == "gelu" else None, force_bn=bn)
     z = x.float() @ w.float().t() + b.float()
     ref = torch.relu(z) if act == "relu" else torch.nn.functional.gelu(z)
     assert _rel(out, ref) < 3e-3
     if act == "gelu":
         assert _rel(pre, z) < 2e-3
     # residual epilogue
-    F.gemm(x, w, out, bias=b, residual=res)
+    out.fill_(float("nan"))
+    F.gemm(x, w, out, bias=b, residual=res, force_bn=bn)
     assert _rel(out, z + res.float()) < 2e-3
     # derivative epilogue: d/dz act(z) * upstream, upstream = x @ w^T (re-used as a stand-in)
     aux = (ref.to(dtype) if act == "relu" else z.to(dtype))
-    F.gemm(x, w, out, dact=act, aux_in=aux)
+    out.fill_(float("nan"))
+    F.gemm(x, w, out, dact=act, aux_in=aux, force_bn=bn)
     up = x.float() @ w.float().t()
     zz = aux.float().requires_grad_()
     (torch.relu(zz) if act == "relu" else torch.nn.functional.gelu(zz)).backward(up)
     assert _rel(out, zz.grad) < 5e-3
+    for t in whole:
+        assert bool(t[M:].isnan().all()) and bool(t[:, N:].isnan().all())
     F.check_device_status()
 
 

@@ -17,7 +17,7 @@ def _walk(M, N, K, rows=256, cols=256, pairs=74):
 @pytest.mark.parametrize("M,N,K", [(16384, 15360, 5120), (16384, 2048, 8192), (20480, 5120, 16384),
                                    (1024, 6144, 2048), (257, 8200, 128), (12288, 49152, 4096),
                                    (8, 8, 8), (18433, 2305, 768)])
-@pytest.mark.parametrize("cols", [128, 256])
+@pytest.mark.parametrize("cols", [128, 192, 224, 256])
 def test_every_tile_once_and_operands_few_times(M, N, K, cols):
     tiles, order = _walk(M, N, K, cols=cols)
     # distinct row and column blocks of a wave, against a square wave and against walking columns
