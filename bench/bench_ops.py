@@ -143,7 +143,7 @@ def case_gemm_trace(a):
 
 def case_attn(a):
     dt, dev, H = a.dtype, "cuda", a.hidden
-    D, b, L, t = 128, a.batch, a.seq, a.slice
+    D, b, L, t = a.head_dim, a.batch, a.seq, a.slice
     h = H // D
     qkv = torch.randn(L, b, h * 3 * D, device=dev, dtype=dt)
     o = torch.zeros(L * b, h * D, device=dev, dtype=dt)
@@ -211,6 +211,7 @@ def main():
     ap.add_argument("--seq", type=int, default=2048)
     ap.add_argument("--slice", type=int, default=128)
     ap.add_argument("--ctx", type=int, default=None)
+    ap.add_argument("--head-dim", type=int, default=128, choices=[64, 128])
     ap.add_argument("--params", type=int, default=302_000_000)
     ap.add_argument("--dtype", default="fp16", choices=["fp16", "bf16"])
     ap.add_argument("--tile", default="0", help="gemm: comma list of tile codes to force")

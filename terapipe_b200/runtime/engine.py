@@ -1214,21 +1214,17 @@ class StageEngine:
         # (torch.cuda.graph() would also collect garbage and give torch's cached memory back to
         # the driver first, which takes far longer than the capture: tens of milliseconds, and
         # hundreds when another engine has just been released.)  Nothing may be collected while
-        # the capture runs, though: the destructor of an old graph is not a legal call then.  And
-        # torch does not give memory back during a capture: where little is left for the stream, the
-        # loss sum (2 and 20 MB segments of a new pool) and the graph itself, it is given back before.
-        if torch.cuda.mem_get_info(self.device)[0] < 256 << 20:
-            torch.cuda.empty_cache()
-        graph = torch.cuda.CUDAGraph()
-        if self._cap_stream is None:
-            self._cap_stream = torch.cuda.Stream()
+        # the capture runs, though: the destructor of an old graph is not a legal call then.
         try:
-            with collection_paused(), torch.cuda.stream(self._cap_stream):
-                graph.capture_begin(capture_error_mode="thread_local")
-                try:
-                    self._iteration()
-                finally:
-                    graph.capture_end()
+            try:
+                self._graph = self._captured_iteration()
+            except (RuntimeError, KernelError):
+                # Torch does not give memory back during a capture, so one that finds a few MB free
+                # beside a large cache has no room for its stream, the loss sum or the graph.
+                torch.cuda.synchronize()
+                torch.cuda.empty_cache()
+                self._ag_pending = False
+                self._graph = self._captured_iteration()
         except (RuntimeError, KernelError) as e:
             # The whole step could not be captured (seen with a 48-layer stage of GPT3-44B width:
             # a launch inside the capture failed although the same step had just run eagerly).
@@ -1242,8 +1238,18 @@ class StageEngine:
             self._ag_pending = False
             if self._plan is None and self._seg_graphs is None:
                 self._seg_graphs = {}
-            return
-        self._graph = graph
+
+    def _captured_iteration(self):
+        graph = torch.cuda.CUDAGraph()
+        if self._cap_stream is None:
+            self._cap_stream = torch.cuda.Stream()
+        with collection_paused(), torch.cuda.stream(self._cap_stream):
+            graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                self._iteration()
+            finally:
+                graph.capture_end()
+        return graph
 
     def check_status(self):
         F.check_device_status(self.device)

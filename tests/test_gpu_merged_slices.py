@@ -134,19 +134,33 @@ def test_a_turned_round_host_input_is_not_rearranged_on_the_host():
     assert torch.equal(eng.X[0].view(64, 2, 256).cpu(), x)
 
 
-@pytest.mark.parametrize("free", [1 << 20, 1 << 30])
-def test_capture_makes_room_when_memory_is_short(free, monkeypatch):
-    """Torch cannot give cached memory back while a capture runs."""
+@pytest.mark.parametrize("failures", [0, 1, 2])
+def test_capture_makes_room_when_memory_is_short(failures, monkeypatch):
+    """Torch cannot give cached memory back while a capture runs: one that fails is tried again with
+    the cache emptied, and a second failure leaves the step to smaller graphs."""
+    import warnings
     from terapipe_b200.models import TransformerConfig
     from terapipe_b200.runtime.engine import StageEngine
     cfg = TransformerConfig(batch_size=2, seq_len=64, n_layers=1, embedding_dim=256,
                             num_attention_heads=4, n_devices=1)
-    eng = StageEngine(cfg, [2], [64], use_graph=True)
-    emptied = []
-    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (free, 180 << 30))
+    eng = StageEngine(cfg, [2], [64], use_graph=True, lr=1e-3)
+    real, emptied, left = eng._iteration, [], [failures]
+
+    def iteration(*args, **kw):
+        real(*args, **kw)
+        if torch.cuda.is_current_stream_capturing() and left[0]:
+            left[0] -= 1
+            raise torch.OutOfMemoryError("out of memory")
+
+    monkeypatch.setattr(eng, "_iteration", iteration)
     monkeypatch.setattr(torch.cuda, "empty_cache",
                         lambda: emptied.append(torch.cuda.is_current_stream_capturing()))
     eng.set_input(torch.randn(64, 2, 256))
-    eng.step()
-    assert eng._graph is not None
-    assert emptied == ([False] if free < 256 << 20 else [])
+    with warnings.catch_warnings(record=True) as caught:
+        warnings.simplefilter("always")
+        for _ in range(3):
+            eng.step()
+    eng.check_status()
+    assert (eng._graph is not None) == (failures < 2) and len(caught) == (failures == 2)
+    assert emptied == [False] * (failures > 0)
+    assert abs(eng.adam_state[0].item() - 3.0) < 1e-6 and eng.grad.abs().max().item() == 0.0
