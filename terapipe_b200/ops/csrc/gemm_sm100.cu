@@ -1523,13 +1523,13 @@ static int g_prefetch = 0;             // L2 prefetch distance of the CTA-pair k
 static bool g_ar_exchange = false;     // one-hop exchange instead of reduce-scatter + all-gather
 
 // `forced` is a tile code (tile_choice.h), 0: by the model.
-static int pick_tile(int M, int N, int K, bool b_mn, int forced, bool allow_256x256, bool allow_pair,
-                     bool allow_cut) {
+static int pick_tile(int M, int N, int K, bool b_mn, bool second, int forced, bool allow_256x256,
+                     bool allow_pair, bool allow_cut) {
   if (forced == 64 || forced == 128 || forced == 256) return forced;
   if (forced == 512) return allow_256x256 ? 512 : 256;
   if (forced == 1128 || forced == 1256) return allow_pair ? forced : forced - 1000;
   if (forced == 1192 || forced == 1224) return allow_pair ? forced : 256;
-  return choose_tile(M, N, K, b_mn, allow_256x256, allow_pair && g_pair_default, allow_cut, num_sms());
+  return choose_tile(M, N, K, b_mn, second, allow_256x256, allow_pair && g_pair_default, allow_cut, num_sms());
 }
 
 }  // namespace tp
@@ -1561,7 +1561,8 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   const bool common_layout = (!a_mn && !out_f32) || (a_mn && b_mn && out_f32);
   // only the three layouts of a Linear layer's forward / dgrad / wgrad products have the
   // 256-row tiles instantiated
-  int tile_code = pick_tile(M, N, K, b_mn != 0, force_bn, common_layout, common_layout, ag == nullptr);
+  int tile_code = pick_tile(M, N, K, b_mn != 0, residual || aux_in || aux_out, force_bn, common_layout,
+                            common_layout, ag == nullptr);
   if (ag) {
     // the wait lives in the CTA-pair kernel's producer
     if (a_mn || !common_layout || ag->rows_per_rank <= 0) return kErrBadArgument;

@@ -43,8 +43,8 @@ long long tp_tile_order_walk(int kind, int M, int N, long long K, int tile_rows,
 }
 
 // The tile code of an ordinary product, or (cut = 0) of an all-gather -> GEMM product.
-int tp_choose_tile(int M, int N, int K, int b_mn, int cut, int sms) {
-  return tp::choose_tile(M, N, K, b_mn != 0, true, true, cut != 0, sms);
+int tp_choose_tile(int M, int N, int K, int b_mn, int second, int cut, int sms) {
+  return tp::choose_tile(M, N, K, b_mn != 0, second != 0, true, true, cut != 0, sms);
 }
 
 }  // extern "C"

@@ -32,10 +32,11 @@ inline float tile_waves(const TileCand& c, int M, int N, int sms) {
   return static_cast<float>((tiles + slots - 1) / slots);
 }
 
+// second: the epilogue reads or writes a second matrix of the output's size (residual, pre-activation).
 // allow_cut: an all-gather -> GEMM product keeps the full widths, with which its order of tiles (this
 // rank's row blocks first) was built and measured on several GPUs.
-inline int choose_tile(int M, int N, int K, bool b_mn, bool allow_256x256, bool allow_pair, bool allow_cut,
-                       int sms) {
+inline int choose_tile(int M, int N, int K, bool b_mn, bool second, bool allow_256x256, bool allow_pair,
+                       bool allow_cut, int sms) {
   int best = 128;
   float best_t = 1e30f;
   for (const TileCand& c : kTileCands) {
@@ -53,8 +54,11 @@ inline int choose_tile(int M, int N, int K, bool b_mn, bool allow_256x256, bool 
     const float waves = tile_waves(c, M, N, sms);
     // Where N is contiguous, B comes in 64-column chunks: a CTA's 96 or 112 columns take the loads of
     // 128.  In a long row of waves each costs 4 % and 0.3 more than the model says: 10240 x 3840 x
-    // 1280 took 71 us with 256 columns and 79 with 192, 8192 x 3072 x 768 32.7 and 35.4.
-    const bool chunks = b_mn && waves > 4.0f;
+    // 1280 took 71 us with 256 columns and 79 with 192, 8192 x 3072 x 768 32.7 and 35.4.  Not where a
+    // short K and a second matrix leave the epilogue to bound a wave: with an activation's derivative or a
+    // residual the latter product takes 8 % less with 192 columns, 5120 x 4096 x 1024 6 % less;
+    // 5120 x 4096 x 2048 takes 2 to 6 % more.
+    const bool chunks = b_mn && waves > 4.0f && !(second && K <= 1600);
     const float loop = c.loop * (chunks ? 1.04f : 1.0f) * static_cast<float>(K) / 2048.0f;
     const float t = waves * (loop + c.epi_each + (chunks ? 0.3f : 0.0f)) + c.tail;
     if (t < 0.97f * best_t) { best_t = t; best = c.code; }   // near ties go to the full widths

@@ -37,9 +37,9 @@ def test_every_tile_once_and_operands_few_times(M, N, K, cols):
         assert seen == sorted(seen)
 
 
-def _tile(M, N, K, b_mn=0, cut=1):
+def _tile(M, N, K, b_mn=0, cut=1, second=0):
     from terapipe_b200.ops.lib import host_lib
-    return host_lib().tp_choose_tile(M, N, K, b_mn, cut, 148)
+    return host_lib().tp_choose_tile(M, N, K, b_mn, second, cut, 148)
 
 
 @pytest.mark.parametrize("M,N,K,b_mn,code", [
@@ -54,6 +54,11 @@ def _tile(M, N, K, b_mn=0, cut=1):
     (1024, 2048, 8192, 0, 1128), (16384, 8192, 2048, 1, 1256), (256, 256, 256, 0, 64)])
 def test_tile_choice(M, N, K, b_mn, code):
     assert _tile(M, N, K, b_mn) == code
+
+
+@pytest.mark.parametrize("M,N,K,code", [(8192, 3072, 768, 1192), (5120, 4096, 1024, 1192), (5120, 4096, 2048, 1256)])
+def test_a_second_matrix_bounds_the_waves_of_a_short_product(M, N, K, code):
+    assert _tile(M, N, K, b_mn=1, second=1) == code and _tile(M, N, K, b_mn=1) == 1256
 
 
 @pytest.mark.parametrize("M,N,K,b_mn", [(2048, 5120, 10240, 0), (2048, 5120, 10240, 1), (2048, 7680, 5120, 0),
