@@ -230,8 +230,8 @@ class StageEngine:
         # attention still runs batch slice by batch slice, because the row layout of its buffers
         # is per batch slice.  Every row is computed from the same inputs by the same kernels, so
         # the slices' results differ only where a sum over rows is split differently.  GPT3-1B
-        # width (5 layers), batch 8, 16 slices of 128: a step took 40.5 ms slice by slice, 31.1 merged;
-        # the 24-layer test model in 8 slices of 32 rows 17.4 ms against 3.4.
+        # width (5 layers), batch 8, 16 slices of 128: a step takes 36.2 ms slice by slice, 27.7 merged;
+        # the 24-layer test model in 8 slices of 32 rows 12.8 and 2.5.
         # An eager run merges like a captured one, so that both take the same sums in the same order
         # and agree bit for bit.
         self._merged = wants_merged_slices(merge_slices, self.pp, self.tp,
