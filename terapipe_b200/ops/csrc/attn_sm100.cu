@@ -112,8 +112,10 @@ __device__ __forceinline__ void tile_of_cta(int idx, int tiles, int heads, int& 
 //
 // What bounds it: 128 queries x 64 keys take 512 cycles of the exponential unit; S takes 384 cycles
 // (6 KB of operands through shared memory per 32 cycles of tensor work) and P V 256 at D = 128,
-// half of that at D = 64.  With P through shared memory and one group of 128 queries per CTA, 8 x 16 heads
-// of 2048 x 128 took 302 us, now 161; 48 heads of 2048 x 64 113 and 67.
+// half of that at D = 64.  Over a whole kernel the exponential unit is busy half of the time and the tensor
+// pipe 44 % (D = 128) or 25 %: a CTA's start and end overlap nothing, for it holds all of TMEM.  With P
+// through shared memory and one group of 128 queries per CTA, 8 x 16 heads of 2048 x 128 took 302 us, now
+// 161; 48 heads of 2048 x 64 113 and 67.
 struct FwdShared {
   uint64_t bar_q[2], bar_k[4], bar_kfree[4], bar_v[4], bar_vfree[4], bar_s[2][2], bar_p[2][2], bar_o[2],
       bar_fin[2];
