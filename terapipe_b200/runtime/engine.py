@@ -939,8 +939,9 @@ class StageEngine:
                 self._cap_stream = torch.cuda.Stream()
             graph = torch.cuda.CUDAGraph()
             outer = self._stream
-            # thread-local capture mode: NCCL's watchdog thread may query events meanwhile
-            with torch.cuda.stream(self._cap_stream):
+            # thread-local capture mode: NCCL's watchdog thread may query events meanwhile.  Nothing may
+            # be collected while the capture runs: the destructor of an old graph is not a legal call then.
+            with collection_paused(), torch.cuda.stream(self._cap_stream):
                 graph.capture_begin(capture_error_mode="thread_local")
                 try:
                     self._stream = self._cap_stream.cuda_stream
