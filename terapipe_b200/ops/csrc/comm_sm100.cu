@@ -417,12 +417,13 @@ extern "C" int tp_peer_sum(float* out, int n, void* const* src_ptrs, int n_ranks
 TP_DEFINE_WAIT_LIMIT_SETTER(tp_set_wait_limit_ns_comm)
 extern "C" int tp_set_wait_limit_ns_gemm(unsigned long long ns);
 extern "C" int tp_set_wait_limit_ns_attn(unsigned long long ns);
+extern "C" int tp_set_wait_limit_ns_wgrad(unsigned long long ns);
 extern "C" int tp_set_wait_limit_ns(unsigned long long ns) {
   if (ns == 0) return kErrBadArgument;
   if (cudaDeviceSynchronize() != cudaSuccess) return kErrDriver;
   const int a = tp_set_wait_limit_ns_comm(ns), b = tp_set_wait_limit_ns_gemm(ns),
-            c = tp_set_wait_limit_ns_attn(ns);
-  return (a | b | c) ? kErrDriver : kOk;
+            c = tp_set_wait_limit_ns_attn(ns), d = tp_set_wait_limit_ns_wgrad(ns);
+  return (a | b | c | d) ? kErrDriver : kOk;
 }
 
 // Which build this is: 1 when the kernels carry their index checks (-DTP_CHECKED), else 0.

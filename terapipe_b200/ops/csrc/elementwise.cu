@@ -1,6 +1,7 @@
 // Memory-bound kernels of the training step: LayerNorm forward/backward, bias-gradient
 // column sums, the fused mixed-precision Adam update and small helpers.  All use 16-byte
 // vector accesses; statistics and reductions are fp32.
+#include "adam.cuh"
 #include "common.cuh"
 #include "ln_geometry.h"
 #include "ptx.cuh"
@@ -299,7 +300,7 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
 }
 
 // ------------------------------------------------------------------ bias and LayerNorm gradients
-// All column sums of a layer in one launch: db[n] += sum_rows dy[row][n] for up to kMaxColsums
+// All column sums of a layer, or of all layers, in one launch: db[n] += sum_rows dy[row][n] for up to kMaxColsums
 // matrices of the same number of rows, and the fold of up to kMaxFolds sets of LayerNorm partial
 // slots (as layernorm_bwd_reduce_kernel, clearing the slots).  Each is a handful of CTAs or a few
 // microseconds long, so separate launches cost more than the sums.  A CTA of 256 threads takes 8 V
@@ -320,6 +321,9 @@ struct SumJobs {
   float* dgamma[kMaxFolds];
   float* dbeta[kMaxFolds];
   int folds, parts, H;           // the CTAs behind the matrices' fold 32 columns each
+  // blockIdx.y = layer: elements from a layer's matrices, slots and sums to the next's
+  long long dy_stride[kMaxColsums], slot_stride, out_stride;
+  int overwrite;                 // the sums replace what the gradients hold
 };
 
 // Fold 32 columns, from column c0 on, of slots [parts][2][H]; thread (tx, ty) of (32, 8), 4 loads in
@@ -383,7 +387,7 @@ layer_sums_kernel(const SumJobs j) {
       const int r_end = min(j.rows, (chunk + 1) * j.rows_per_chunk);
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       if (col < j.N[i]) {
-        const T* src = static_cast<const T*>(j.dy[i]) + col;
+        const T* src = static_cast<const T*>(j.dy[i]) + blockIdx.y * j.dy_stride[i] + col;
         for (int r = chunk * j.rows_per_chunk + lane_row; r < r_end; r += 8 * kRows) {
           uint4 v[8];
 #pragma unroll
@@ -421,7 +425,10 @@ layer_sums_kernel(const SumJobs j) {
         cluster_sync_all();   // nobody leaves while its sums may be read
         if (chunk != 0) return;
       }
-      if (tid < kCols && col0 + tid < j.N[i]) j.db[i][col0 + tid] += s;
+      if (tid < kCols && col0 + tid < j.N[i]) {
+        float* db = j.db[i] + blockIdx.y * j.out_stride + col0 + tid;
+        *db = j.overwrite ? s : *db + s;
+      }
       return;
     }
     first = j.cta_end[i];
@@ -429,8 +436,9 @@ layer_sums_kernel(const SumJobs j) {
   const int per_fold = (2 * j.H + 31) / 32;
   const int f = (cta - first) / per_fold;
   if (f >= j.folds) return;        // (the grid is a whole number of clusters)
-  fold_slots(j.slots[f], j.parts, j.H, (cta - first) % per_fold * 32, j.dgamma[f], j.dbeta[f],
-             tid & 31, tid >> 5, 1, sm.fold);
+  fold_slots(j.slots[f] + blockIdx.y * j.slot_stride, j.parts, j.H, (cta - first) % per_fold * 32,
+             j.dgamma[f] + blockIdx.y * j.out_stride, j.dbeta[f] + blockIdx.y * j.out_stride,
+             tid & 31, tid >> 5, j.overwrite ? 3 : 1, sm.fold);
 }
 
 // ------------------------------------------------------------------ fused Adam
@@ -445,40 +453,49 @@ __global__ void adam_tick_kernel(float* state, float beta1, float beta2) {
 // One pass over flat buffers: g = grad * grad_scale; m, v, p (fp32 master) updated in place;
 // the 16-bit model copy is rewritten and the gradient accumulator is zeroed.
 template <typename T>
-__global__ void fused_adam_kernel(float* __restrict__ grad, float* __restrict__ p,
-                                  float* __restrict__ m, float* __restrict__ v,
-                                  T* __restrict__ model, long long n4, const float* __restrict__ state,
-                                  float lr, float beta1, float beta2, float eps, float weight_decay,
-                                  float grad_scale) {
-  const float bc1 = state[1], bc2 = state[2];
-  const float inv_bc2_sqrt = rsqrtf(bc2);
-  const float step = lr / bc1;
+__device__ __forceinline__ void adam_vec4(float4* grad, const AdamBuffers& a, const AdamCoef& co, long long i) {
+  float4 p4 = reinterpret_cast<float4*>(a.p)[i];
+  float4 m4 = reinterpret_cast<float4*>(a.m)[i];
+  float4 v4 = reinterpret_cast<float4*>(a.v)[i];
+  adam_update(grad[i], p4, m4, v4, co);
+  reinterpret_cast<float4*>(a.p)[i] = p4;
+  reinterpret_cast<float4*>(a.m)[i] = m4;
+  reinterpret_cast<float4*>(a.v)[i] = v4;
+  grad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  uint2 o;
+  o.x = Elem<T>::pack2(p4.x, p4.y);
+  o.y = Elem<T>::pack2(p4.z, p4.w);
+  reinterpret_cast<uint2*>(a.model)[i] = o;
+}
+
+template <typename T>
+__global__ void fused_adam_kernel(float* __restrict__ grad, const AdamBuffers a, long long n4) {
+  const AdamCoef co = adam_coef(a);
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    float4 g4 = reinterpret_cast<float4*>(grad)[i];
-    float4 p4 = reinterpret_cast<float4*>(p)[i];
-    float4 m4 = reinterpret_cast<float4*>(m)[i];
-    float4 v4 = reinterpret_cast<float4*>(v)[i];
-    float* g = reinterpret_cast<float*>(&g4);
-    float* pp = reinterpret_cast<float*>(&p4);
-    float* mm = reinterpret_cast<float*>(&m4);
-    float* vv = reinterpret_cast<float*>(&v4);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float gj = g[j] * grad_scale;
-      mm[j] = beta1 * mm[j] + (1.0f - beta1) * gj;
-      vv[j] = beta2 * vv[j] + (1.0f - beta2) * gj * gj;
-      const float denom = sqrtf(vv[j]) * inv_bc2_sqrt + eps;
-      pp[j] = pp[j] - step * (mm[j] / denom) - lr * weight_decay * pp[j];
+       i += static_cast<long long>(gridDim.x) * blockDim.x)
+    adam_vec4<T>(reinterpret_cast<float4*>(grad), a, co, i);
+}
+
+// The same for a few ranges of every layer (what the weight-gradient products have not updated
+// already: biases and LayerNorm parameters).  blockIdx.y = layer; offsets and lengths in float4.
+constexpr int kMaxAdamRanges = 8;
+struct AdamRanges {
+  long long begin[kMaxAdamRanges], layer_stride;
+  int len[kMaxAdamRanges];
+  int n;
+};
+template <typename T>
+__global__ void adam_ranges_kernel(float* __restrict__ grad, const AdamBuffers a, const AdamRanges r) {
+  pdl_wait();
+  const AdamCoef co = adam_coef(a);
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll 1
+  for (int k = 0; k < r.n; ++k) {
+    if (i < r.len[k]) {
+      adam_vec4<T>(reinterpret_cast<float4*>(grad), a, co, r.begin[k] + blockIdx.y * r.layer_stride + i);
+      return;
     }
-    reinterpret_cast<float4*>(p)[i] = p4;
-    reinterpret_cast<float4*>(m)[i] = m4;
-    reinterpret_cast<float4*>(v)[i] = v4;
-    reinterpret_cast<float4*>(grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    uint2 o;
-    o.x = Elem<T>::pack2(pp[0], pp[1]);
-    o.y = Elem<T>::pack2(pp[2], pp[3]);
-    reinterpret_cast<uint2*>(model)[i] = o;
+    i -= r.len[k];
   }
 }
 
@@ -677,9 +694,10 @@ extern "C" int tp_layernorm_bwd_finish_assign(float* slots, int parts, int H, fl
 }
 
 namespace tp {
-static int layer_sums_launch(int dtype, SumJobs& j, cudaStream_t s) {
+static int layer_sums_launch(int dtype, SumJobs& j, int layers, cudaStream_t s) {
   long long blocks = 0;           // of 256 columns
   for (int i = 0; i < j.n; ++i) blocks += (j.N[i] + 255) / 256;
+  blocks *= layers;
   // V = 32 once its CTAs fill the chip, us V = 8 / V = 32:
   //   one layer's four matrices of width  768 (27 blocks)   2048 (72)     4096 (144)
   //     rows    256                         3.8 / 5.0       5.3 / 6.3     7.8 / 10.2
@@ -707,7 +725,7 @@ static int layer_sums_launch(int dtype, SumJobs& j, cudaStream_t s) {
   if (ctas == 0) return kOk;
   ctas = (ctas + j.chunks - 1) / j.chunks * j.chunks;
   if (ctas > 0x7fffffffLL) return kErrTooLarge;
-  const dim3 grid(static_cast<unsigned>(ctas)), block(256);
+  const dim3 grid(static_cast<unsigned>(ctas), static_cast<unsigned>(layers)), block(256);
   cudaError_t e;
   if (dtype == 1)
     e = wide ? launch_pdl(layer_sums_kernel<__nv_bfloat16, 32>, grid, block, 0, s, j.chunks, j)
@@ -726,26 +744,39 @@ extern "C" int tp_colsum(int dtype, const void* dy, long long ld, int rows, int 
   SumJobs j = {};
   j.dy[0] = dy; j.ld[0] = ld; j.N[0] = N; j.db[0] = db;
   j.n = 1; j.rows = rows;
-  return layer_sums_launch(dtype, j, static_cast<cudaStream_t>(stream));
+  return layer_sums_launch(dtype, j, 1, static_cast<cudaStream_t>(stream));
 }
 
 // The bias gradients (`n` <= 4 matrices dy[i] [rows][N[i]], added to db[i]) and LayerNorm parameter
-// gradients (`folds` <= 2 sets of slots as for tp_layernorm_bwd_finish) of one layer in one launch.
-extern "C" int tp_layer_sums(int dtype, int n, const void* const* dy, const long long* ld, const int* N,
+// gradients (`folds` <= 2 sets of slots as for tp_layernorm_bwd_finish) of `layers` layers in one launch; the
+// layers' matrices lie dy_stride[i], slots slot_stride and sums out_stride elements apart.
+// overwrite: the sums replace what db, dgamma and dbeta hold.
+extern "C" int tp_stage_sums(int dtype, int n, const void* const* dy, const long long* ld, const int* N,
                              float* const* db, int rows, int folds, float* const* slots, int parts, int H,
-                             float* const* dgamma, float* const* dbeta, void* stream) {
+                             float* const* dgamma, float* const* dbeta, int layers, const long long* dy_stride,
+                             long long slot_stride, long long out_stride, int overwrite, void* stream) {
   if (n < 0 || n > kMaxColsums || folds < 0 || folds > kMaxFolds || rows < 0 ||
-      (folds > 0 && (H <= 0 || parts <= 0)))
+      (folds > 0 && (H <= 0 || parts <= 0)) || layers < 1 || layers > 65535)
     return kErrBadArgument;
   SumJobs j = {};
   j.n = n; j.rows = rows;
   for (int i = 0; i < n; ++i) {
-    if (N[i] <= 0 || N[i] % 8 || ld[i] % 8) return kErrBadArgument;
+    j.dy_stride[i] = layers > 1 ? dy_stride[i] : 0;
+    if (N[i] <= 0 || N[i] % 8 || ld[i] % 8 || j.dy_stride[i] % 8) return kErrBadArgument;
     j.dy[i] = dy[i]; j.ld[i] = ld[i]; j.N[i] = N[i]; j.db[i] = db[i];
   }
   j.folds = folds; j.parts = parts; j.H = H;
+  j.slot_stride = slot_stride; j.out_stride = out_stride; j.overwrite = overwrite;
   for (int f = 0; f < folds; ++f) { j.slots[f] = slots[f]; j.dgamma[f] = dgamma[f]; j.dbeta[f] = dbeta[f]; }
-  return layer_sums_launch(dtype, j, static_cast<cudaStream_t>(stream));
+  return layer_sums_launch(dtype, j, layers, static_cast<cudaStream_t>(stream));
+}
+
+// The same for one layer, added to the gradients.
+extern "C" int tp_layer_sums(int dtype, int n, const void* const* dy, const long long* ld, const int* N,
+                             float* const* db, int rows, int folds, float* const* slots, int parts, int H,
+                             float* const* dgamma, float* const* dbeta, void* stream) {
+  return tp_stage_sums(dtype, n, dy, ld, N, db, rows, folds, slots, parts, H, dgamma, dbeta, 1, nullptr, 0, 0, 0,
+                       stream);
 }
 
 extern "C" int tp_adam_tick(float* state, float beta1, float beta2, void* stream) {
@@ -763,15 +794,37 @@ extern "C" int tp_fused_adam(int dtype, float* grad, float* p, float* m, float* 
   long long blocks = (n4 + 255) / 256;
   const long long cap = 8ll * num_sms();
   if (blocks > cap) blocks = cap;
-  if (dtype == 1)
-    fused_adam_kernel<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, s>>>(
-        grad, p, m, v, static_cast<__nv_bfloat16*>(model), n4, state, lr, beta1, beta2, eps,
-        weight_decay, grad_scale);
-  else
-    fused_adam_kernel<__half><<<static_cast<int>(blocks), 256, 0, s>>>(
-        grad, p, m, v, static_cast<__half*>(model), n4, state, lr, beta1, beta2, eps, weight_decay,
-        grad_scale);
+  const AdamBuffers a{p, m, v, model, state, lr, beta1, beta2, eps, weight_decay, grad_scale};
+  if (dtype == 1) fused_adam_kernel<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, s>>>(grad, a, n4);
+  else fused_adam_kernel<__half><<<static_cast<int>(blocks), 256, 0, s>>>(grad, a, n4);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}
+
+// tp_fused_adam over `n` <= 8 ranges [begin[k], begin[k] + len[k]) of each of `layers` layers, whose flat
+// ranges lie `layer_stride` apart (elements; all multiples of 4).
+extern "C" int tp_fused_adam_ranges(int dtype, float* grad, float* p, float* m, float* v, void* model, int n,
+                                    const long long* begin, const long long* len, int layers,
+                                    long long layer_stride, const float* state, float lr, float beta1,
+                                    float beta2, float eps, float weight_decay, float grad_scale, void* stream) {
+  if (n < 0 || n > kMaxAdamRanges || layers < 0 || layers > 65535 || layer_stride % 4) return kErrBadArgument;
+  AdamRanges r = {};
+  long long total = 0;
+  for (int k = 0; k < n; ++k) {
+    if (begin[k] < 0 || len[k] < 0 || begin[k] % 4 || len[k] % 4) return kErrBadArgument;
+    r.begin[k] = begin[k] / 4;
+    r.len[k] = static_cast<int>(len[k] / 4);
+    total += len[k] / 4;
+    if (total > 0x3fffffffLL) return kErrTooLarge;
+  }
+  r.n = n;
+  r.layer_stride = layer_stride / 4;
+  if (total == 0 || layers == 0) return kOk;
+  const AdamBuffers a{p, m, v, model, state, lr, beta1, beta2, eps, weight_decay, grad_scale};
+  const dim3 grid(static_cast<unsigned>((total + 255) / 256), static_cast<unsigned>(layers));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = dtype == 1 ? launch_pdl(adam_ranges_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, 1, grad, a, r)
+                                   : launch_pdl(adam_ranges_kernel<__half>, grid, dim3(256), 0, s, 1, grad, a, r);
+  return e == cudaSuccess ? kOk : kErrLaunch;
 }
 
 extern "C" int tp_fill(int dtype, void* p, long long n, float value, void* stream) {

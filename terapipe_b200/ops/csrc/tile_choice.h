@@ -66,4 +66,23 @@ inline int choose_tile(int M, int N, int K, bool b_mn, bool second, bool allow_2
   return best;
 }
 
+// Columns of a CTA pair's tile for the weight gradients of `layers` layers in one launch (wgrad_sm100.cu).
+// A wave takes its main loop or, where that is shorter, what its epilogue moves at the copy bandwidth
+// (kilo-cycles of 1.8 GHz: 26 bytes an element with Adam, else the staged stores); the last wave's epilogue is
+// exposed.
+inline int choose_wgrad_tile(int M, int N, int K, int layers, bool adam, int sms) {
+  struct Cand { int bn; float loop, adam, store; };
+  constexpr Cand cands[3] = {{256, 16.7f, 35.0f, 8.5f}, {192, 13.7f, 26.2f, 7.0f}, {128, 10.0f, 17.5f, 5.5f}};
+  int best = 256;
+  float best_t = 1e30f;
+  for (const Cand& c : cands) {
+    const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + c.bn - 1) / c.bn) * layers;
+    const float waves = static_cast<float>((tiles + sms / 2 - 1) / (sms / 2));
+    const float loop = c.loop * static_cast<float>(K) / 2048.0f, epi = adam ? c.adam : c.store;
+    const float t = waves * (loop > epi ? loop : epi) + epi;
+    if (t < 0.97f * best_t) { best_t = t; best = c.bn; }
+  }
+  return best;
+}
+
 }  // namespace tp

@@ -7,6 +7,7 @@ status word: call :func:`check_device_status` after a synchronisation point.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -153,6 +154,50 @@ def fused_adam(grad, master, m, v, model, state, lr, beta1=0.9, beta2=0.999, eps
                                   v.data_ptr(), model.data_ptr(), n, state.data_ptr(), lr, beta1,
                                   beta2, eps, weight_decay, grad_scale, _stream())
     check(st, "tp_fused_adam")
+
+
+def _wgrad_args(dy, x, out):
+    """``[layers, rows, width]`` operands and ``[layers, M, N]`` output (or one layer without the dimension)."""
+    dy, x, out = (t if t.dim() == 3 else t.unsqueeze(0) for t in (dy, x, out))
+    n, K, M = dy.shape
+    N = x.shape[2]
+    assert x.shape[:2] == (n, K) and out.shape == (n, M, N)
+    assert dy.stride(2) == 1 and x.stride(2) == 1 and out.stride(2) == 1
+    return (_dt(dy), dy.data_ptr(), dy.stride(1), dy.stride(0), x.data_ptr(), x.stride(1), x.stride(0)), \
+           (out.stride(1), out.stride(0), n, M, N, K)
+
+
+def weight_grad(dy, x, out, accumulate=False):
+    """``out[l] (+)= dy[l]^T @ x[l]`` (fp32) for every layer: the weight gradients of one kind of a stage."""
+    operands, sizes = _wgrad_args(dy, x, out)
+    st = cuda_lib().tp_wgrad(*operands, out.data_ptr(), *sizes, int(accumulate), status_word(dy.device).data_ptr(),
+                             _stream())
+    check(st, "tp_wgrad")
+    return out
+
+
+def weight_grad_adam(dy, x, master, m, v, model, state, lr, beta1=0.9, beta2=0.999, eps=1e-8,
+                     weight_decay=0.0, grad_scale=1.0):
+    """:func:`weight_grad` and :func:`fused_adam` in one kernel: the gradients of the ``[layers, M, N]`` matrices
+    ``master``/``m``/``v``/``model`` are not stored."""
+    operands, sizes = _wgrad_args(dy, x, master)
+    for t in (m, v, model):
+        assert t.shape == master.shape and t.stride() == master.stride()
+    st = cuda_lib().tp_wgrad_adam(*operands, master.data_ptr(), m.data_ptr(), v.data_ptr(), model.data_ptr(), *sizes,
+                                  state.data_ptr(), lr, beta1, beta2, eps, weight_decay, grad_scale,
+                                  status_word(dy.device).data_ptr(), _stream())
+    check(st, "tp_wgrad_adam")
+
+
+def fused_adam_ranges(grad, master, m, v, model, state, ranges, layers: int, layer_stride: int, lr,
+                      beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0, grad_scale=1.0):
+    """:func:`fused_adam` on the ranges ``[(begin, length), ...]`` of every layer of the flat buffers."""
+    LL = ctypes.c_longlong * len(ranges)
+    st = cuda_lib().tp_fused_adam_ranges(_dt(model), grad.data_ptr(), master.data_ptr(), m.data_ptr(),
+                                         v.data_ptr(), model.data_ptr(), len(ranges), LL(*[r[0] for r in ranges]),
+                                         LL(*[r[1] for r in ranges]), layers, layer_stride, state.data_ptr(), lr,
+                                         beta1, beta2, eps, weight_decay, grad_scale, _stream())
+    check(st, "tp_fused_adam_ranges")
 
 
 def fill(t, value: float):

@@ -3,8 +3,9 @@
 What one rank owns
 ------------------
 * Flat parameter state for its layers: a 16-bit model copy, fp32 master weights, Adam
-  moments and an fp32 main-gradient buffer.  One fused Adam launch updates the whole
-  stage; weight-gradient GEMMs accumulate straight into the main-gradient buffer.
+  moments and an fp32 main-gradient buffer.  Without data parallelism the weight-gradient
+  products apply Adam to the weights themselves and one small launch updates the rest; with it
+  they accumulate into the main-gradient buffer and one launch updates the whole stage.
 * Full-length activation buffers ``[L*B, width]`` per layer.  A token slice is a contiguous
   row range, so the "KV cache" is simply the QKV projection buffer: slice *j* writes rows
   ``[c, c+t)`` and attends over rows ``[0, c+t)`` in place.
@@ -36,7 +37,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
-from typing import Dict, List, Optional, Sequence
+from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 import torch.distributed as dist
@@ -95,6 +96,18 @@ class _Layout:
                 off += _align(math.prod(self.shapes[name]))
             self.offsets.append(entry)
         self.total = _align(off, 8)
+        # elements from a layer to the next; (offset, length) of what lies between its weight matrices
+        self.layer_stride = off // n_layers if n_layers else 0
+        self.small_ranges: List[Tuple[int, int]] = []
+        if n_layers:
+            matrices = [n for n in PARAM_ORDER if len(self.shapes[n]) == 2]
+            pos = 0
+            for name in matrices:
+                if self.offsets[0][name] > pos:
+                    self.small_ranges.append((pos, self.offsets[0][name] - pos))
+                pos = self.offsets[0][name] + _align(math.prod(self.shapes[name]))
+            if self.layer_stride > pos:
+                self.small_ranges.append((pos, self.layer_stride - pos))
 
 
 class StageEngine:
@@ -194,6 +207,12 @@ class StageEngine:
         self.exp_avg = torch.zeros(n, dtype=torch.float32, device=dev)
         self.exp_avg_sq = torch.zeros(n, dtype=torch.float32, device=dev)
         self.adam_state = torch.zeros(3, dtype=torch.float32, device=dev)
+        # Where a weight's whole gradient is one product on this rank (no data-parallel sum), the product's
+        # epilogue applies Adam and the gradient is never stored; biases and LayerNorm parameters, whose
+        # gradients come from column sums, follow in one small launch.  (Sequence parallel: the
+        # LayerNorm gradients are summed over the ranks after the products.)
+        self._adam_in_products = self.dp == 1 and not self.sp
+        self._grad_seen = self.grad._version     # of the buffer when an update last left it zero
         self._init_weights(init)
         # A CUDA graph may hold this library's kernels only: captured NCCL point-to-point or
         # collective calls deadlocked on replay here, so a stage that calls NCCL runs eagerly.
@@ -247,10 +266,11 @@ class StageEngine:
         self._streams_ready = False
         # launches of this library's own kernels (NCCL and torch kernels are not counted):
         # per layer and slice 7 forward (2 LN, 4 GEMM, attention) and 9 backward (4 GEMM,
-        # 2 LN, 3 attention); per layer 5 after the last slice (4 weight-gradient GEMMs, the bias
-        # and LayerNorm gradients in one); plus 2 for the optimizer
+        # 2 LN, 3 attention); after the last slice 5 for each group of layers (4 weight-gradient
+        # GEMMs, the bias and LayerNorm gradients in one); plus 2 for the optimizer
         n_slices = len(self.batch_slices) * len(self.seq_slices)
-        self._launches = {merged: self.n_layers * (per_layer + 5 + (2 if self.sp else 0)) + 2
+        groups = self.n_layers if self.dp > 1 and self.dp_overlap else len(self._wgrad_groups)
+        self._launches = {merged: self.n_layers * (per_layer + (2 if self.sp else 0)) + 5 * groups + 2
                           for merged, per_layer in ((True, 12 + 4 * len(self.batch_slices)),
                                                     (False, 16 * n_slices))}
         self.launch_count = 0
@@ -421,6 +441,15 @@ class StageEngine:
             # per layer: folded LayerNorm gamma/beta gradient sums of this rank's token shard
             self._ln_pack, self._off_ln_pack = self.ar.alloc((max(self.n_layers, 1), 4 * H), torch.float32)
 
+        def bufs(width):
+            # the layers' matrices one after the other: one weight-gradient launch reaches all of them
+            return list(torch.empty(self.n_layers, rows, width, dtype=dt, device=dev).unbind(0))
+
+        def syms(name, pooled=True):
+            if self.ar is None or not pooled:
+                return bufs(H)
+            return [sym(f"{name}{l}", rows) for l in range(self.n_layers)]
+
         def sym(name, nrows, pooled=True):
             if self.ar is None or not pooled:
                 return torch.empty(nrows, H, dtype=dt, device=dev)
@@ -434,12 +463,12 @@ class StageEngine:
         self.X = [buf(H)] + [sym(f"X{l + 1}", rows, not sp) for l in range(self.n_layers)]
         if sp and self.n_layers:
             self.X[-1].zero_()   # rows of other ranks' shards are never written; the loss sums all
-        self.ln1 = [sym(f"ln1_{l}", rows, sp) for l in range(self.n_layers)]
-        self.ln2 = [sym(f"ln2_{l}", rows, sp) for l in range(self.n_layers)]
+        self.ln1 = syms("ln1_", sp)
+        self.ln2 = syms("ln2_", sp)
         self.xmid = [sym(f"xmid{l}", rows, not sp) for l in range(self.n_layers)]
         self.qkv = [buf(3 * Hl) for _ in range(self.n_layers)]
-        self.ao = [buf(Hl) for _ in range(self.n_layers)]
-        self.fa = [buf(Fl) for _ in range(self.n_layers)]
+        self.ao = bufs(Hl)
+        self.fa = bufs(Fl)
         self.fz = [buf(Fl) for _ in range(self.n_layers)] if self.act == "gelu" else None
         self.stats = [torch.empty(4, rows, dtype=torch.float32, device=dev) for _ in range(self.n_layers)]
         self.lse = [torch.empty(self.B * self.h, self.L, dtype=torch.float32, device=dev)
@@ -447,11 +476,11 @@ class StageEngine:
         self.delta = [torch.empty(self.B * self.h, self.L, dtype=torch.float32, device=dev)
                       for _ in range(self.n_layers)]
         # gradients, full length (see the module docstring)
-        self.dMid = [sym(f"dMid{l}", rows, sp) for l in range(self.n_layers)]
-        self.dFc = [buf(Fl) for _ in range(self.n_layers)]
-        self.dQKV = [buf(3 * Hl) for _ in range(self.n_layers)]
+        self.dMid = syms("dMid", sp)
+        self.dFc = bufs(Fl)
+        self.dQKV = bufs(3 * Hl)
         self.dAO = [buf(Hl) for _ in range(self.n_layers)]
-        self.dXo = [sym(f"dXo{l}", rows, sp) for l in range(self.n_layers)]   # d(layer output); the last one is
+        self.dXo = syms("dXo", sp)                           # d(layer output); the last one is
         self.dY = self.dXo[-1] if self.n_layers else None    # received from the next stage
         self.dX0 = buf(H) if not self.is_first else None    # gradients sent to the previous stage
         self.dA = torch.empty(tmax, H, dtype=dt, device=dev)
@@ -459,8 +488,11 @@ class StageEngine:
         # LayerNorm parameter gradients: every backward launch adds its per-CTA partial sums
         # into persistent slots; one reduction per layer folds them after the last slice
         self.ln_parts = self.lib.tp_layernorm_bwd_parts(int(tmax))
-        self.ln_slots = [torch.zeros(2, self.ln_parts, 2 * H, dtype=torch.float32, device=dev)
-                         for _ in range(self.n_layers)]
+        self.ln_slots = torch.zeros(self.n_layers, 2, self.ln_parts, 2 * H, dtype=torch.float32, device=dev).unbind(0)
+        # layers whose weight gradients share a launch: all of them, unless their operands are pooled matrices
+        # (whose distance is the pool's affair)
+        self._wgrad_groups = [(0, self.n_layers)] if self.n_layers and not sp else \
+            [(l, 1) for l in reversed(range(self.n_layers))]
         numel = self.L * self.B * H
         if self.is_last and self.n_layers:
             # loss = mean(output): the seed gradient is the same constant everywhere
@@ -488,6 +520,23 @@ class StageEngine:
                               0, self._status_ptr, self._stream)
         if st:
             F.check(st, "tp_gemm")
+
+    def _wgrad(self, dy, M, x, N, l, n, name, mode):
+        """``dW = dy^T x`` over all rows for layers ``[l, l + n)``: ``mode`` "add" to or "assign" the gradient, or
+        "update" the weight ``name`` with it."""
+        R = self.rows
+        operands = (self.dt, dy[l].data_ptr(), M, R * M, x[l].data_ptr(), N, R * N)
+        sizes = (N, self.layout.layer_stride, n, M, N, R)
+        if mode == "update":
+            st = self.lib.tp_wgrad_adam(*operands, self._p(l, name, self.master), self._p(l, name, self.exp_avg),
+                                        self._p(l, name, self.exp_avg_sq), self._p(l, name), *sizes,
+                                        self.adam_state.data_ptr(), self.lr, 0.9, 0.999, 1e-8, 0.0,
+                                        1.0 / (self.loss_scale * self.dp), self._status_ptr, self._stream)
+        else:
+            st = self.lib.tp_wgrad(*operands, self._p(l, name, self.grad), *sizes, int(mode == "add"),
+                                   self._status_ptr, self._stream)
+        if st:
+            F.check(st, "tp_wgrad")
 
     def _ln(self, fn_name, *args):
         """An entry point of the library whose status must be zero (LayerNorm, column sums, ...);
@@ -837,11 +886,13 @@ class StageEngine:
                                            H, s)
         self._ag_join()
 
-    def _weight_grads(self) -> None:
+    def _weight_grads(self, mode: str = "add") -> None:
         """Weight and bias gradients of every layer over all ``L*B`` rows at once:
-        ``dW += dY^T X`` with the token dimension as the (long) GEMM K dimension."""
-        R, H, Hl, Fl = self.rows, self.H, self.Hl, self.Fl
-        lib, dt, s, g = self.lib, self.dt, self._stream, self.grad
+        ``dW += dY^T X`` with the token dimension as the (long) GEMM K dimension, all layers of a kind of
+        weight in one launch.  ``mode``: "add" to the gradients, "assign" them, or "update" the weights
+        instead (:meth:`_reduce_and_update` then does the rest)."""
+        H, Hl, Fl = self.H, self.Hl, self.Fl
+        lib, s, g = self.lib, self._stream, self.grad
         # Data-parallel reduction overlapped with these products: as soon as the gradients of a
         # layer are complete (layers are visited last to first), its reduction - and with the fused
         # kernel its Adam update and parameter push - starts on a side stream (NCCL: on NCCL's own
@@ -850,25 +901,23 @@ class StageEngine:
         works = []
         if overlap and self.dp_sym is not None:
             self._dp_begin_update()
-        for l in reversed(range(self.n_layers)):
-            if l != self.n_layers - 1 and overlap:
+        if mode == "update" and self._plan is None:    # (a recorded plan only holds calls made through self.lib)
+            F.adam_tick(self.adam_state)
+        groups = [(l, 1) for l in reversed(range(self.n_layers))] if overlap else self._wgrad_groups
+        for l, n in groups:
+            if l + n < self.n_layers and overlap:
                 self._dp_layer_done(l + 1, works)
-            dxo, dmid = self.dXo[l].data_ptr(), self.dMid[l].data_ptr()
-            dfc, dqkv = self.dFc[l].data_ptr(), self.dQKV[l].data_ptr()
-            self._gemm(dxo, H, self.fa[l].data_ptr(), Fl, self._p(l, "fc2.weight", g), Fl, H, Fl, R,
-                       a_mn=1, b_mn=1, out_f32=1, accumulate=1)
-            self._gemm(dfc, Fl, self.ln2[l].data_ptr(), H, self._p(l, "fc1.weight", g), H, Fl, H, R,
-                       a_mn=1, b_mn=1, out_f32=1, accumulate=1)
-            self._gemm(dmid, H, self.ao[l].data_ptr(), Hl, self._p(l, "attn.out_proj.weight", g), Hl,
-                       H, Hl, R, a_mn=1, b_mn=1, out_f32=1, accumulate=1)
-            self._gemm(dqkv, 3 * Hl, self.ln1[l].data_ptr(), H, self._p(l, "attn.in_proj.weight", g),
-                       H, 3 * Hl, H, R, a_mn=1, b_mn=1, out_f32=1, accumulate=1)
+            for dy, M, x, N, name in ((self.dXo, H, self.fa, Fl, "fc2.weight"), (self.dFc, Fl, self.ln2, H, "fc1.weight"),
+                                      (self.dMid, H, self.ao, Hl, "attn.out_proj.weight"),
+                                      (self.dQKV, 3 * Hl, self.ln1, H, "attn.in_proj.weight")):
+                self._wgrad(dy, M, x, N, l, n, name, mode)
             slots = self.ln_slots[l].data_ptr()
             # all bias gradients (column sums of the same dY) and, unless the ranks' sums have to be
             # added up first, the LayerNorm gradients: one launch
-            self._layer_sums(l, ((dxo, H, "fc2.bias"), (dfc, Fl, "fc1.bias"), (dmid, H, "attn.out_proj.bias"),
-                                 (dqkv, 3 * Hl, "attn.in_proj.bias")),
-                             () if self.sp else ((slots, "attn_ln"), (slots + self.ln_parts * 2 * H * 4, "fc_ln")))
+            self._layer_sums(l, n, ((self.dXo, H, "fc2.bias"), (self.dFc, Fl, "fc1.bias"),
+                                    (self.dMid, H, "attn.out_proj.bias"), (self.dQKV, 3 * Hl, "attn.in_proj.bias")),
+                             () if self.sp else ((slots, "attn_ln"), (slots + self.ln_parts * 2 * H * 4, "fc_ln")),
+                             mode == "assign")
             if self.sp:
                 # this rank's slots hold the sums over its token shards only: fold them into a
                 # peer-visible pack; the sums of all ranks are added after the barrier below
@@ -891,16 +940,20 @@ class StageEngine:
                 self._ln("tp_peer_sum", self._p(l, "fc_ln.weight", g), 2 * H, self.ar.out_ptrs(off + 2 * H * 4),
                                 self.tp, self.tp_idx, s)
 
-    def _layer_sums(self, l, mats, folds) -> None:
-        """``mats``: (address of ``[rows, width]``, width, bias name) whose column sums are added to the
-        bias gradient; ``folds``: (address of the partial slots, LayerNorm name)."""
+    def _layer_sums(self, l, layers, mats, folds, assign) -> None:
+        """``mats``: (the layers' ``[rows, width]``, width, bias name) whose column sums are added to (or assigned
+        to) the bias gradients of ``layers`` layers from ``l`` on; ``folds``: (address of the partial slots,
+        LayerNorm name)."""
         n, m, g = len(mats), len(folds), self.grad
         P, LL, I = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
-        self._ln("tp_layer_sums", self.dt, n, (P * n)(*[a for a, _, _ in mats]), (LL * n)(*[w for _, w, _ in mats]),
-                 (I * n)(*[w for _, w, _ in mats]), (P * n)(*[self._p(l, name, g) for _, _, name in mats]), self.rows,
+        widths = [w for _, w, _ in mats]
+        self._ln("tp_stage_sums", self.dt, n, (P * n)(*[a[l].data_ptr() for a, _, _ in mats]), (LL * n)(*widths),
+                 (I * n)(*widths), (P * n)(*[self._p(l, name, g) for _, _, name in mats]), self.rows,
                  m, (P * m)(*[a for a, _ in folds]), self.ln_parts, self.H,
                  (P * m)(*[self._p(l, name + ".weight", g) for _, name in folds]),
-                 (P * m)(*[self._p(l, name + ".bias", g) for _, name in folds]), self._stream)
+                 (P * m)(*[self._p(l, name + ".bias", g) for _, name in folds]), layers,
+                 (LL * n)(*[self.rows * w for w in widths]), 4 * self.ln_parts * self.H, self.layout.layer_stride,
+                 int(assign), self._stream)
 
     def _group_barrier(self, index: int) -> None:
         """Device-side barrier of the tensor-parallel group (``index`` 1 or 2 within a step)."""
@@ -1001,7 +1054,7 @@ class StageEngine:
         rpr = T // self.tp
         return r0 + self.tp_idx * rpr, r0 + (self.tp_idx + 1) * rpr
 
-    def _forward_backward(self):
+    def _forward_backward(self, mode: str = "add"):
         pipelined = self.pp > 1
         if pipelined:
             self._setup_streams()
@@ -1049,7 +1102,9 @@ class StageEngine:
         if self.dp > 1 and self.dp_sym is None:
             self._weight_grads()           # starts NCCL all-reduces: not for a captured segment
         else:
-            self._segment(("weight_grads",), self._weight_grads)
+            if mode == "update" and self._plan is not None:
+                F.adam_tick(self.adam_state)
+            self._segment(("weight_grads", mode), self._weight_grads, mode)
         for w in sends:
             w.wait()
 
@@ -1093,7 +1148,13 @@ class StageEngine:
             works.append(dist.all_reduce(self.grad[lo:hi], group=mpu.get_data_parallel_group(),
                                          async_op=True))
 
-    def _reduce_and_update(self):
+    def _reduce_and_update(self, fused_update: bool = False):
+        if fused_update:
+            # the weights are done (_weight_grads): biases and LayerNorm parameters
+            F.fused_adam_ranges(self.grad, self.master, self.exp_avg, self.exp_avg_sq, self.model,
+                                self.adam_state, self.layout.small_ranges, self.n_layers, self.layout.layer_stride,
+                                lr=self.lr, grad_scale=1.0 / (self.loss_scale * self.dp))
+            return
         if self.dp_sym is not None:
             if self._dp_overlap and not self.sp:
                 return                     # done layer by layer underneath the weight gradients
@@ -1140,13 +1201,16 @@ class StageEngine:
             self._group_barrier(1)
         self._dp_overlap = bool(update and self.dp > 1 and self.dp_overlap)
         self._dp_works = None
-        self._forward_backward()
+        fused_update = update and self._updates_in_products
+        self._forward_backward("update" if fused_update else "add" if update or self.dp > 1 or self.sp else "assign")
         if update and not (self.dp_sym is not None and self._dp_overlap and not self.sp):
             if self._seg_graphs is not None and (self.dp == 1 or self.dp_sym is not None):
                 # (a recorded launch plan only sees calls made through self.lib: not this one)
-                self._segment(("update",), self._reduce_and_update)
+                self._segment(("update", fused_update), self._reduce_and_update, fused_update)
             else:
-                self._reduce_and_update()
+                self._reduce_and_update(fused_update)
+            if not torch.cuda.is_current_stream_capturing():
+                self._grad_seen = self.grad._version
 
     def set_input(self, x: torch.Tensor) -> None:
         """Copy this replica's ``[L, B, H]`` input into the stage-0 activation buffer.  Rows are
@@ -1191,21 +1255,32 @@ class StageEngine:
 
     def compute_grads(self) -> None:
         """Forward + backward without the optimizer; scaled grads stay in ``self.grad``."""
-        self.grad.zero_()
+        self._grad_seen = None
+        if self.dp > 1 or self.sp:
+            self.grad.zero_()      # (else the gradients are assigned, not added up)
         self._iteration(update=False)
         if self.dp > 1:
             dist.all_reduce(self.grad, group=mpu.get_data_parallel_group())
             self.grad.div_(self.dp)
 
+    @property
+    def _updates_in_products(self) -> bool:
+        """Whether the next update happens inside the weight-gradient products.  Not if ``grad`` has been
+        written since the last update (:meth:`compute_grads`, or by the caller): what it holds then
+        counts too, as it always has, so the gradients are added to it and one pass updates everything."""
+        return self._adam_in_products and self.grad._version == self._grad_seen
+
     def step(self) -> None:
         """One training iteration on the current stream.  With ``use_graph`` the first call
         runs eagerly (it also sets up kernel attributes) and records the iteration into a
-        CUDA graph; later calls replay the graph."""
-        if self.use_graph and self._graph is not None:
+        CUDA graph; later calls replay the graph.  (An iteration that has to add to gradients left by
+        :meth:`compute_grads` runs eagerly as well and is not recorded.)"""
+        usual = self._updates_in_products == self._adam_in_products
+        if self.use_graph and self._graph is not None and usual:
             self._graph.replay()
         else:
             self._iteration()
-            if self.use_graph:
+            if self.use_graph and self._graph is None and usual:
                 self._capture()
         self.step_count += 1
         self.launch_count += self._launches[self._walked_merged]   # of the iteration that ran, or was captured
