@@ -14,8 +14,8 @@
 // of an accumulating gradient and the 34 of a pass over flat buffers, and they move under the main loop of
 // the next tile.  us for the four weights of a layer, rows x width: product + pass / this kernel (of which the
 // bare product):
-//   256 x 256 68.7 / 5.5 (1.5), 8192 x 768 183 / 103 (87), 16384 x 2048 1543 / 1418 (1296), 6144 x 2560
-//   1306 / 901 (717), 16384 x 5120 9248 / 7618 (7210), 4096 x 12288 20970 / 15301 (9960).
+//   256 x 256 68.7 / 4.4 (1.5), 8192 x 768 183 / 103 (87), 16384 x 2048 1543 / 1418 (1296), 6144 x 2560
+//   1306 / 901 (717), 16384 x 5120 9248 / 7618 (7210), 4096 x 12288 20970 / 14500 (9960).
 //
 // The product is the CTA-pair GEMM (two CTAs of a cluster, one 256 x BN tile, see gemm_sm100.cu).
 #include "adam.cuh"
@@ -39,33 +39,34 @@ struct WgradParams {
 
 constexpr int kWgBM = 128, kWgBK = 64;
 constexpr int kWgThreads = 320, kWgEpiWarps = 8;
-constexpr int kWgEpiBytes = 4096;       // a 32 x 32 fp32 chunk per epilogue warp
+constexpr int kWgEpiBytes = 8192;       // a 32 x 64 fp32 chunk per epilogue warp
 
 template <int BN> struct WgradCfg {
   static constexpr int kABytes = kWgBM * kWgBK * 2;
   static constexpr int kBChunks = (BN / 2 + 63) / 64;   // a CTA's half of B comes in 64-column chunks
   static constexpr int kStageBytes = kABytes + kBChunks * 64 * kWgBK * 2;
-  static constexpr int kStages = BN > 128 ? 6 : 7;
+  static constexpr int kStages = BN > 128 ? 5 : 6;
   static constexpr int kAccCols = BN > 128 ? 256 : 128;
   static constexpr int kTmemCols = 2 * kAccCols;
   static constexpr int kSmemBytes = kStages * kStageBytes + kWgEpiWarps * kWgEpiBytes + 1024 + 256;
 };
 
-// What the epilogue needs from memory for half a 32 x 32 chunk: four rows a lane, 16 bytes of each.  A thread
-// holds a row of the accumulator, but the matrices in memory are wanted 128 contiguous bytes a row, so the
-// chunk turns round in the warp's shared memory.  One such set (48 registers with Adam) is fetched ahead of its
-// use; all epilogue warps of an SM have 48 KB in flight.  (An L2 prefetch of a tile's whole 390 KB at the start
-// of its main loop made the products 1 to 10 % slower.)
+// What the epilogue needs from memory for 8 rows of a 32 x 64 chunk: four rows a lane, 16 bytes of each.  A
+// thread holds a row of the accumulator, but the matrices in memory are wanted in long pieces of a row, so
+// the chunk turns round in the warp's shared memory.  256 bytes a row, 512 with the chunk of the quarter's
+// other warp beside it, keep DRAM rows open: with 128 and 256, 4096 x 12288 over 4096 rows took 443 us
+// instead of 422.  One set (48 registers with Adam) is fetched ahead of its use; the epilogue warps of an SM have
+// 48 KB in flight.
 template <bool ADAM> struct WgradRegs { float4 p[4], m[ADAM ? 4 : 1], v[ADAM ? 4 : 1]; };
 
 template <bool ADAM>
 __device__ __forceinline__ void wgrad_fetch(const WgradParams& p, WgradRegs<ADAM>& a, long long base, int row0, int n,
-                                            int hf, int lane) {
+                                            int q, int lane) {
   if (!ADAM && !p.accumulate) return;
-  const int col = n + (lane & 7) * 4;
+  const int col = n + (lane & 15) * 4;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int row = row0 + hf * 16 + k * 4 + (lane >> 3);
+    const int row = row0 + q * 8 + k * 2 + (lane >> 4);
     if (row < p.M && col < p.N) {
       const long long i = base + row * p.ldo + col;
       if (ADAM) {
@@ -81,13 +82,13 @@ __device__ __forceinline__ void wgrad_fetch(const WgradParams& p, WgradRegs<ADAM
 
 template <typename T, bool ADAM>
 __device__ __forceinline__ void wgrad_finish(const WgradParams& p, const AdamCoef& co, WgradRegs<ADAM>& a,
-                                             const uint8_t* sb, long long base, int row0, int n, int hf, int lane) {
-  const int col = n + (lane & 7) * 4;
+                                             const uint8_t* sb, long long base, int row0, int n, int q, int lane) {
+  const int col = n + (lane & 15) * 4;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int rr = hf * 16 + k * 4 + (lane >> 3), row = row0 + rr;
+    const int rr = q * 8 + k * 2 + (lane >> 4), row = row0 + rr;
     if (row < p.M && col < p.N) {
-      float4 g = *reinterpret_cast<const float4*>(sb + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
+      float4 g = *reinterpret_cast<const float4*>(sb + rr * 256 + (((lane & 15) ^ (rr & 7)) << 4));
       const long long i = base + row * p.ldo + col;
       if (ADAM) {
         adam_update(g, a.p[k], a.m[k], a.v[k], co);
@@ -102,6 +103,24 @@ __device__ __forceinline__ void wgrad_finish(const WgradParams& p, const AdamCoe
         if (p.accumulate) { g.x += a.p[k].x; g.y += a.p[k].y; g.z += a.p[k].z; g.w += a.p[k].w; }
         __stcs(reinterpret_cast<float4*>(p.grad + i), g);
       }
+    }
+  }
+}
+
+// The optimizer's values of a 32 x 64 chunk on their way to L2: two lines a row and matrix.  Where the main loop
+// is shorter than the epilogue, the epilogue's latency is what a tile waits for; under a longer one the lines
+// only get in the operands' way.  4096 x 12288, us without / with, over 512 rows 377 / 299, 1536 382 / 323, 2048
+// 386 / 341, 3072 408 / 403, 4096 415 / 436.
+constexpr int kWgPrefetchK = 3072;
+__device__ __forceinline__ void wgrad_prefetch(const WgradParams& p, long long base, int row0, int n, int lane) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int row = row0 + h * 16 + (lane >> 1), col = n + (lane & 1) * 32;
+    if (row < p.M && col < p.N) {
+      const long long i = base + row * p.ldo + col;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.adam.p + i));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.adam.m + i));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.adam.v + i));
     }
   }
 }
@@ -234,30 +253,39 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       // checked build: the tile lies inside the grid (rows and columns past the matrix are skipped below)
       const bool tile_ok = TP_CHECK(layer >= 0 && layer < p.layers && m_idx >= 0 && m_idx < p.num_m_tiles &&
                                         n_idx >= 0 && n_idx < p.num_n_tiles, p.err, kErrCheckTile);
-      const int nc = tile_ok && row0 < p.M ? (min(BN, p.N - n0) + 31) / 32 : 0;
+      const int nc = tile_ok && row0 < p.M ? (min(BN, p.N - n0) + 63) / 64 : 0;
       const long long base = layer * p.layer_stride;
       WgradRegs<ADAM> a, b;
-      if (half < nc) wgrad_fetch<ADAM>(p, a, base, row0, n0 + half * 32, 0, lane);   // under this tile's main loop
+      if (half < nc) wgrad_fetch<ADAM>(p, a, base, row0, n0 + half * 64, 0, lane);   // under this tile's main loop
+      if (ADAM && p.K <= kWgPrefetchK)
+        for (int c = half; c < nc; c += 2) wgrad_prefetch(p, base, row0, n0 + c * 64, lane);
       ok = mbar_wait(&tfull[acc], (it >> 1) & 1, wctx, kErrWaitEpilogue);
       if (!ok) break;
       tc_fence_after();
       const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kAccCols;
 #pragma unroll 1
       for (int c = half; c < nc; c += 2) {
-        const int n = n0 + c * 32;
+        const int n = n0 + c * 64;
         uint32_t r[32];
         __syncwarp();      // (and the last chunk has been read)
-        tmem_ld_32x32(t_acc + c * 32, r);
         wgrad_fetch<ADAM>(p, b, base, row0, n, 1, lane);
-        tmem_ld_wait();
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          tmem_ld_32x32(t_acc + c * 64 + h * 32, r);
+          tmem_ld_wait();
 #pragma unroll
-        for (int g = 0; g < 8; ++g)   // 128-byte rows, 16-byte pieces turned by the row: no bank conflicts either way
-          *reinterpret_cast<uint4*>(sb + lane * 128 + ((g ^ (lane & 7)) << 4)) =
-              make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+          for (int g = 0; g < 8; ++g)   // 16-byte pieces turned by the row: no bank conflicts either way
+            *reinterpret_cast<uint4*>(sb + lane * 256 + ((((h << 3) | g) ^ (lane & 7)) << 4)) =
+                make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+        }
         __syncwarp();
         wgrad_finish<T, ADAM>(p, co, a, sb, base, row0, n, 0, lane);
-        if (c + 2 < nc) wgrad_fetch<ADAM>(p, a, base, row0, n + 64, 0, lane);
+        wgrad_fetch<ADAM>(p, a, base, row0, n, 2, lane);
         wgrad_finish<T, ADAM>(p, co, b, sb, base, row0, n, 1, lane);
+        wgrad_fetch<ADAM>(p, b, base, row0, n, 3, lane);
+        wgrad_finish<T, ADAM>(p, co, a, sb, base, row0, n, 2, lane);
+        if (c + 2 < nc) wgrad_fetch<ADAM>(p, a, base, row0, n + 128, 0, lane);
+        wgrad_finish<T, ADAM>(p, co, b, sb, base, row0, n, 3, lane);
       }
       tc_fence_before();
       __syncwarp();
