@@ -770,6 +770,250 @@ static int dispatch_layout(int a_mn, int b_mn, int out_f32, const CUtensorMap& t
 }
 
 // ---------------------------------------------------------------------------------------------
+// Split along K.  A product of few rows has few tiles (77 x 768: 12 of 64 columns) and each walks all of K at
+// what one SM can fetch, 64 bytes a cycle, while most of the chip is idle.  Here a cluster of CTAs shares a 128 x
+// BN tile: each takes a part of K into its own TMEM and owns BN / parts columns of the result.  It stores its fp32
+// partial sums of the other columns into the shared memory of their owners, and after one cluster barrier every
+// owner adds up its columns in the order of the parts (the result does not depend on timing) and finishes them
+// (bias, activation, residual, ...).  No workspace, no flags, and no round trip through distributed shared
+// memory (owners that fetched the partial tiles instead needed two barriers and 0.5 us more).
+constexpr int kSplitThreads = 256;
+constexpr int kMaxSplit = 8;        // a portable cluster
+constexpr int kSplitBK = 128;       // K of a stage
+constexpr int kSplitMaxStages = 8;
+constexpr int kSplitSmemBytes = 226 * 1024;
+// The ring takes what the partial sums leave.  A stage holds only the rows of A that exist (a_rows, a multiple of
+// 8): with few rows more stages fit, and the loads' latency is what a stage waits for.  (The MMA reads 128 rows all
+// the same; what it finds past a_rows gives rows of the product that nobody looks at.)
+struct SplitRing {
+  int a_bytes, stage_bytes, stages;
+  __host__ __device__ __forceinline__ SplitRing(int bn, int parts, int a_rows) {
+    a_bytes = a_rows * kSplitBK * 2;
+    stage_bytes = a_bytes + bn * kSplitBK * 2;
+    stages = (kSplitSmemBytes - 1024 /*align*/ - 512 /*barriers*/ - sums_bytes(bn, parts)) / stage_bytes;
+    if (stages > kSplitMaxStages) stages = kSplitMaxStages;
+  }
+  // partial sums [part][row][bn / parts columns + 4 floats, which keep the rows' stores off each other's banks]
+  static __host__ __device__ __forceinline__ int sums_bytes(int bn, int parts) { return (bn + 4 * parts) * kBM * 4; }
+};
+
+// Eight columns from n on of row `row`: the epilogue of epilogue_chunk, for a thread that has them in fp32.
+template <typename T>
+__device__ __forceinline__ void split_finish(const GemmParams& p, float (&v)[8], long long row, int n) {
+  auto add = [&](const void* src, long long at) {
+    const uint4 u = __ldcg(reinterpret_cast<const uint4*>(static_cast<const T*>(src) + at));
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = Elem<T>::unpack2(w[j]);
+      v[2 * j] += f.x;
+      v[2 * j + 1] += f.y;
+    }
+  };
+  auto pack = [&]() {
+    return make_uint4(Elem<T>::pack2(v[0], v[1]), Elem<T>::pack2(v[2], v[3]), Elem<T>::pack2(v[4], v[5]),
+                      Elem<T>::pack2(v[6], v[7]));
+  };
+  if (p.alpha != 1.0f) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] *= p.alpha;
+  }
+  if (p.bias) add(p.bias, n);
+  if (p.act == 2) {
+    if (p.aux_out) __stcg(reinterpret_cast<uint4*>(static_cast<T*>(p.aux_out) + row * p.ld_aux + n), pack());
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const float2 g = gelu2(make_float2(v[j], v[j + 1]));
+      v[j] = g.x;
+      v[j + 1] = g.y;
+    }
+  } else if (p.act == 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j], 0.0f);
+  }
+  if (p.residual) add(p.residual, row * p.ldr + n);
+  if (p.dact) {
+    const uint4 u = __ldcg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.aux_in) + row * p.ld_aux + n));
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = Elem<T>::unpack2(w[j]);
+      if (p.dact == 1) {
+        v[2 * j] = f.x > 0.0f ? v[2 * j] : 0.0f;
+        v[2 * j + 1] = f.y > 0.0f ? v[2 * j + 1] : 0.0f;
+      } else {
+        const float2 d = gelu_grad2(f);
+        v[2 * j] *= d.x;
+        v[2 * j + 1] *= d.y;
+      }
+    }
+  }
+  __stcg(reinterpret_cast<uint4*>(static_cast<T*>(p.out) + row * p.ldo + n), pack());
+}
+
+template <typename T, int BN, bool B_MN>
+__global__ void __launch_bounds__(kSplitThreads, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                  const GemmParams p, const int parts, const int a_rows) {
+  const SplitRing ring(BN, parts, a_rows);
+  const int S = ring.stages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  float* sums = reinterpret_cast<float*>(smem + S * ring.stage_bytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * ring.stage_bytes + SplitRing::sums_bytes(BN, parts));
+  uint64_t *full = bars, *empty = bars + kSplitMaxStages, *tfull = bars + 2 * kSplitMaxStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int part = static_cast<int>(cluster_ctarank()), tile = blockIdx.x / parts;
+  const int m0 = (tile % p.num_m_tiles) * kBM, n0 = (tile / p.num_m_tiles) * BN;
+  const int num_kb = (p.K + kSplitBK - 1) / kSplitBK;
+  const int kb0 = num_kb * part / parts, kb1 = num_kb * (part + 1) / parts;
+  const int own = BN / parts, pitch = own + 4;       // columns of an owner, floats of a row of them
+  const WaitCtx wctx{abort_flag, p.err};
+
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this CTA runs
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(tfull, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, BN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // set-up done; from here on the predecessor's results are read
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");             // so do the others
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&empty[stage], phase ^ 1, wctx, kErrWaitProducer)) break;
+        uint8_t* sA = smem + stage * ring.stage_bytes;
+        uint8_t* sB = sA + ring.a_bytes;
+        mbar_expect_tx(&full[stage], ring.stage_bytes);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          tma_load_2d(sA + h * (ring.a_bytes / 2), &tmA, &full[stage], kb * kSplitBK + h * 64, m0);
+        if (!B_MN) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            tma_load_2d(sB + h * (BN * kBK * 2), &tmB, &full[stage], kb * kSplitBK + h * 64, n0);
+        } else {
+#pragma unroll
+          for (int c = 0; c < BN / 64; ++c)
+            tma_load_2d(sB + c * (kSplitBK * 128), &tmB, &full[stage], n0 + c * 64, kb * kSplitBK);
+        }
+        if (++stage == S) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_f16(Elem<T>::fmt, 0, B_MN ? 1 : 0, kBM, BN);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait(&full[stage], phase, wctx, kErrWaitMma);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t a_base = smem_u32(smem + stage * ring.stage_bytes), b_base = a_base + ring.a_bytes;
+#pragma unroll
+        for (int k = 0; k < kSplitBK / 16; ++k)
+          umma_f16(tmem, umma_desc_sw128(a_base + (k >> 2) * (ring.a_bytes / 2) + (k & 3) * 32, 16, 1024),
+                   B_MN ? umma_desc_sw128(b_base + k * 2048, kSplitBK * 128, 1024)
+                        : umma_desc_sw128(b_base + (k >> 2) * (BN * kBK * 2) + (k & 3) * 32, 16, 1024),
+                   idesc, (kb > kb0 || k != 0) ? 1u : 0u);
+        umma_commit(&empty[stage]);
+        if (++stage == S) { stage = 0; phase ^= 1; }
+      }
+      if (ok) umma_commit(tfull);
+    }
+  } else if (warp < 6) {
+    // this part's sums to the columns' owners, a row a thread
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(tfull, 0, wctx, kErrWaitEpilogue));
+    tc_fence_after();
+    if (ok && m0 + quarter * 32 < p.M) {
+      const uint32_t mine = smem_u32(sums + (part * kBM + row) * pitch);
+#pragma unroll 1
+      for (int c = 0; c < BN; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + c, r);
+        tmem_ld_wait();
+        if (m0 + row < p.M) {
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const int col = c + 4 * g, owner = col / own;
+            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                             mapa_u32(mine + (col - owner * own) * 4, owner)),
+                         "r"(r[4 * g]), "r"(r[4 * g + 1]), "r"(r[4 * g + 2]), "r"(r[4 * g + 3])
+                         : "memory");
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();
+  if (!*abort_flag) {
+    const int per_row = own / 8, units = min(kBM, p.M - m0) * per_row;     // of eight columns
+    for (int u = threadIdx.x; u < units; u += kSplitThreads) {
+      const int rr = u / per_row, cc = (u - rr * per_row) * 8, n = n0 + part * own + cc;
+      if (n >= p.N) continue;
+      const float* src = sums + rr * pitch + cc;
+      float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+      for (int q = 0; q < parts; ++q) {
+        const float4 x = *reinterpret_cast<const float4*>(src + q * kBM * pitch);
+        const float4 y = *reinterpret_cast<const float4*>(src + q * kBM * pitch + 4);
+        v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+        v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+      }
+      split_finish<T>(p, v, m0 + rr, n);
+    }
+  } else {             // let copies in flight land before the shared memory is released
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem, BN);
+}
+
+template <typename T, int BN, bool B_MN>
+static int launch_gemm_split(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int parts,
+                             int a_rows, cudaStream_t stream) {
+  static_assert(kSplitSmemBytes >= kTmemKernelMinSmem, "allocates TMEM before pdl_wait");
+  auto kern = gemm_split_kernel<T, BN, B_MN>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes) != cudaSuccess)
+      return kErrLaunch;
+    configured = true;
+  }
+  return launch_pdl(kern, dim3(p.num_tiles * parts), dim3(kSplitThreads), kSplitSmemBytes, stream, parts, tmA, tmB, p,
+                    parts, a_rows) == cudaSuccess
+             ? kOk
+             : kErrLaunch;
+}
+
+// ---------------------------------------------------------------------------------------------
 // CTA-pair variant (tcgen05 cta_group::2).  A cluster of two CTAs, one per SM of a TPC, owns a
 // 256 x BN output tile: CTA r of the pair loads rows [128 r, 128 r + 128) of the A tile and
 // rows [BN/2 r, BN/2 r + BN/2) of the B tile into its own shared memory and keeps 128 lanes x
@@ -1524,12 +1768,16 @@ static bool g_ar_exchange = false;     // one-hop exchange instead of reduce-sca
 
 // `forced` is a tile code (tile_choice.h), 0: by the model.
 static int pick_tile(int M, int N, int K, bool b_mn, bool second, int forced, bool allow_256x256,
-                     bool allow_pair, bool allow_cut) {
-  if (forced == 64 || forced == 128 || forced == 256) return forced;
+                     bool allow_pair, bool allow_cut, bool allow_split) {
+  if (forced == 64 || forced == 128 || forced == 256 || forced >= kSplitCode) return forced;
   if (forced == 512) return allow_256x256 ? 512 : 256;
   if (forced == 1128 || forced == 1256) return allow_pair ? forced : forced - 1000;
   if (forced == 1192 || forced == 1224) return allow_pair ? forced : 256;
-  return choose_tile(M, N, K, b_mn, second, allow_256x256, allow_pair && g_pair_default, allow_cut, num_sms());
+  float time;
+  const int code = choose_tile(M, N, K, b_mn, second, allow_256x256, allow_pair && g_pair_default, allow_cut, num_sms(),
+                               &time);
+  const int split = allow_split ? choose_split(M, N, K, time, num_sms()) : 0;
+  return split ? split : code;
 }
 
 }  // namespace tp
@@ -1562,16 +1810,22 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   // only the three layouts of a Linear layer's forward / dgrad / wgrad products have the
   // 256-row tiles instantiated
   int tile_code = pick_tile(M, N, K, b_mn != 0, residual || aux_in || aux_out, force_bn, common_layout,
-                            common_layout, ag == nullptr);
+                            common_layout, ag == nullptr, ag == nullptr && !a_mn && !out_f32);
   if (ag) {
     // the wait lives in the CTA-pair kernel's producer
     if (a_mn || !common_layout || ag->rows_per_rank <= 0) return kErrBadArgument;
     if (tile_code < 1000) tile_code = (N % 256 == 0 && N >= 2048) ? 1256 : 1128;
   }
+  const int parts = tile_code / kSplitCode;   // of K, 0: a kernel of another kind
+  tile_code %= kSplitCode;
+  if (parts && (a_mn || out_f32 || (tile_code != 64 && tile_code != 128) || parts > kMaxSplit ||
+                (parts & (parts - 1)) || (K + kSplitBK - 1) / kSplitBK < parts))
+    return kErrBadArgument;
   const bool pair = tile_code > 1000;
   const int BN = pair ? tile_code - 1000 : (tile_code == 512 ? 256 : tile_code);
   const int BM = (pair || tile_code == 512) ? 256 : kBM;   // rows of one output tile
-  const int box_m = pair ? kBM : BM;                       // rows of A one CTA loads
+  // rows of A one CTA loads
+  const int box_m = parts ? (M < kBM ? (M + 7) / 8 * 8 : kBM) : pair ? kBM : BM;
   const int box_n = pair ? BN / 2 : BN;                    // rows of B one CTA loads
   CUtensorMap tmA, tmB;
   bool ok;
@@ -1579,7 +1833,7 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   else ok = make_tmap_2d(&tmA, A, M, K, lda, 64, kBK, bf16);
   if (!ok) return kErrDriver;
   if (!b_mn) ok = make_tmap_2d(&tmB, B, K, N, ldb, kBK, box_n, bf16);
-  else ok = make_tmap_2d(&tmB, B, N, K, ldb, 64, kBK, bf16);
+  else ok = make_tmap_2d(&tmB, B, N, K, ldb, 64, parts ? kSplitBK : kBK, bf16);
   if (!ok) return kErrDriver;
   CUtensorMap tmO;
   if (!make_tmap_out(&tmO, out, N, M, ldo, out_f32 != 0, bf16)) return kErrDriver;
@@ -1608,6 +1862,15 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   p.trace = nullptr;
   p.prefetch = g_prefetch;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (parts) {
+#define TP_SPLIT(T)                                                                        \
+  (BN == 64 ? (b_mn ? launch_gemm_split<T, 64, true>(tmA, tmB, p, parts, box_m, s)         \
+                    : launch_gemm_split<T, 64, false>(tmA, tmB, p, parts, box_m, s))       \
+            : (b_mn ? launch_gemm_split<T, 128, true>(tmA, tmB, p, parts, box_m, s)        \
+                    : launch_gemm_split<T, 128, false>(tmA, tmB, p, parts, box_m, s)))
+    return bf16 ? TP_SPLIT(__nv_bfloat16) : TP_SPLIT(__half);
+#undef TP_SPLIT
+  }
 #define TP_DISPATCH(T)                                                                   \
   (pair ? (BN == 256 ? dispatch_layout_pair<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)  \
            : BN == 224 ? dispatch_layout_pair<T, 224>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s) \

@@ -48,3 +48,10 @@ int tp_choose_tile(int M, int N, int K, int b_mn, int second, int cut, int sms) 
 }
 
 }  // extern "C"
+
+// The code of a product that ordinary calls split along K, or 0.
+extern "C" int tp_choose_split(int M, int N, int K, int b_mn, int second, int sms) {
+  float time;
+  tp::choose_tile(M, N, K, b_mn != 0, second != 0, true, true, true, sms, &time);
+  return tp::choose_split(M, N, K, time, sms);
+}

@@ -10,6 +10,8 @@ namespace tp {
 // epilogue of the last tile.  Wave quantisation matters because M is only ~1024 rows per token slice.
 // `loop` is per 2048 of K: the CTA-pair tiles run at 80-98 % of the MMA rate, the one-CTA tiles
 // at 50-67 % (L2 -> shared-memory feed of one SM).
+// kSplitCode * parts + BN = one CTA, 128 x BN tile (BN = 64, 128), K shared by `parts` CTAs of a cluster.
+constexpr int kSplitCode = 10000;
 struct TileCand {
   int code, bm, bn;
   bool pair;
@@ -35,8 +37,9 @@ inline float tile_waves(const TileCand& c, int M, int N, int sms) {
 // second: the epilogue reads or writes a second matrix of the output's size (residual, pre-activation).
 // allow_cut: an all-gather -> GEMM product keeps the full widths, with which its order of tiles (this
 // rank's row blocks first) was built and measured on several GPUs.
+// time: the model's estimate.
 inline int choose_tile(int M, int N, int K, bool b_mn, bool second, bool allow_256x256, bool allow_pair,
-                       bool allow_cut, int sms) {
+                       bool allow_cut, int sms, float* time = nullptr) {
   int best = 128;
   float best_t = 1e30f;
   for (const TileCand& c : kTileCands) {
@@ -44,6 +47,7 @@ inline int choose_tile(int M, int N, int K, bool b_mn, bool second, bool allow_2
     const float t = tile_waves(c, M, N, sms) * (c.loop * static_cast<float>(K) / 2048.0f + c.epi_each) + c.tail;
     if (t < best_t) { best_t = t; best = c.code; }
   }
+  if (time) *time = best_t;
   // A one-CTA tile of 128 or 256 columns wins where the rows are an odd number of 128-row blocks, few
   // of them: the second CTA of the last pair row has no rows.  The model puts such a tile too slow by
   // up to a third, so a cut pair tile may not take its place: 77 x 12288 x 4096 takes 21.8 us on
@@ -62,6 +66,37 @@ inline int choose_tile(int M, int N, int K, bool b_mn, bool second, bool allow_2
     const float loop = c.loop * (chunks ? 1.04f : 1.0f) * static_cast<float>(K) / 2048.0f;
     const float t = waves * (loop + c.epi_each + (chunks ? 0.3f : 0.0f)) + c.tail;
     if (t < 0.97f * best_t) { best_t = t; best = c.code; }   // near ties go to the full widths
+  }
+  if (time) *time = best_t;
+  return best;
+}
+
+// Whether a product is better off with K shared by a cluster (gemm_split_kernel): the code, or 0.  `time` is the
+// estimate of choose_tile; the same units here.  A step of 64 of K takes what the MMA needs to read its operands
+// from shared memory, all of them together at least their bytes at 13 TB/s out of L2; what a split pays for is the
+// exchange of the partial sums, which grows with the rows and, where they are many, with the CTAs.  All clusters
+// have to run at once, and an SM group holds few large ones: 36 clusters of 4 take two rounds (16 x 2304 x 768 7.9 us
+// instead of 4.3 in 36 pairs), 16 of 8 as well (32 x 1024 x 4096 10.0, 16 of 4 6.3).  us without / with:
+//   77 x 768 x 768 5.5 / 4.5 (4 parts of 64 columns), 77 x 768 x 3072 12.3 / 5.9 (8), 256 x 256 x 1024 6.2 / 5.5 (4),
+//   128 x 1024 x 4096 15.4 / 7.7 (4), 128 x 2048 x 8192 27.6 / 11.4 (4), 16 x 8192 x 2048 16.5 / 7.5 (2 of 128
+//   columns), 64 x 4096 x 16384 52.6 / 27.9 (4 of 128), 256 x 2048 x 8192 27.9 / 16.3 (2 of 64).
+inline int choose_split(int M, int N, int K, float time, int sms) {
+  struct Cand { int bn, parts; float ctas, step, base, rows; };   // share of the SMs; per 64 of K; per 128 rows
+  constexpr Cand cands[5] = {{64, 2, 1.0f, 0.254f, 4.0f, 1.5f}, {64, 4, 0.87f, 0.254f, 3.3f, 2.5f},
+                             {64, 8, 0.65f, 0.254f, 3.4f, 3.8f}, {128, 2, 1.0f, 0.287f, 3.2f, 6.2f},
+                             {128, 4, 0.87f, 0.287f, 3.4f, 5.8f}};
+  const int rows = M < 128 ? M : 128;
+  const float r = static_cast<float>(rows) / 128.0f;
+  int best = 0;
+  float best_t = 0.9f * time;
+  for (const Cand& c : cands) {
+    const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + c.bn - 1) / c.bn), ctas = tiles * c.parts;
+    if (static_cast<float>(ctas) > c.ctas * static_cast<float>(sms) || (K + 127) / 128 < c.parts) continue;
+    const float crowd = ctas > 64 ? 0.025f * static_cast<float>(ctas - 64) : 0.0f;
+    const float mma = (c.bn == 128 && M > 96 ? 0.4f : c.step) * static_cast<float>(K) / (64.0f * c.parts);
+    const float feed = 2.4e-7f * static_cast<float>(tiles) * static_cast<float>(rows + c.bn) * static_cast<float>(K);
+    const float t = (mma > feed ? mma : feed) + c.base + r * (c.rows + crowd);
+    if (t < best_t) { best_t = t; best = kSplitCode * c.parts + c.bn; }
   }
   return best;
 }
