@@ -18,20 +18,30 @@ _ACT = {None: 0, "none": 0, "relu": 1, "gelu": 2}
 _status = {}
 
 
+_DT = {torch.float16: 0, torch.bfloat16: 1}
+
+
 def _dt(t: torch.Tensor) -> int:
-    if t.dtype == torch.float16:
-        return 0
-    if t.dtype == torch.bfloat16:
-        return 1
-    raise KernelError(f"unsupported dtype {t.dtype}; kernels take float16 or bfloat16")
+    code = _DT.get(t.dtype)
+    if code is None:
+        raise KernelError(f"unsupported dtype {t.dtype}; kernels take float16 or bfloat16")
+    return code
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+# A short slice's layer is 14 calls of a few microseconds of device work each, so what a call costs here counts:
+# 16 us for gemm() with torch.cuda.current_stream() (3.2, the object it makes) and a method call for every size and
+# stride, 9 with the raw handle and one tuple each.
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _status_ptr(t: torch.Tensor) -> int:
+    word = _status.get(t.get_device())
+    return (status_word(t.device) if word is None else word).data_ptr()
 
 
 def status_word(device=None) -> torch.Tensor:
@@ -69,19 +79,22 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn=False, b_m
     activation derivative evaluated on ``aux_in`` (post-activation for relu,
     pre-activation for gelu); ``out`` may be fp32 and may ``accumulate``."""
     M, N = out.shape
-    K = a.shape[0] if a_mn else a.shape[1]
-    assert a.stride(-1) == 1 and b.stride(-1) == 1 and out.stride(-1) == 1
-    assert (a.shape[1] if a_mn else a.shape[0]) == M, "A does not match out rows"
-    assert (b.shape[1] if b_mn else b.shape[0]) == N and (b.shape[0] if b_mn else b.shape[1]) == K
-    out_f32 = out.dtype == torch.float32
+    rows, cols = a.shape, b.shape
+    lda, ldb, ldo = a.stride(), b.stride(), out.stride()
+    K = rows[0] if a_mn else rows[1]
+    assert lda[-1] == 1 and ldb[-1] == 1 and ldo[-1] == 1
+    assert (rows[1] if a_mn else rows[0]) == M, "A does not match out rows"
+    assert (cols[1] if b_mn else cols[0]) == N and (cols[0] if b_mn else cols[1]) == K
     aux = aux_out if aux_out is not None else aux_in
     st = cuda_lib().tp_gemm(
-        _dt(a), int(a_mn), int(b_mn), a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
-        out.data_ptr(), out.stride(0), int(out_f32), int(accumulate), M, N, K, float(alpha),
-        _ptr(bias), _ptr(residual), residual.stride(0) if residual is not None else 0,
-        _ACT[act], _ptr(aux_out), _ACT[dact], _ptr(aux_in), aux.stride(0) if aux is not None else 0,
-        int(force_bn), status_word(a.device).data_ptr(), _stream())
-    check(st, "tp_gemm")
+        _dt(a), int(a_mn), int(b_mn), a.data_ptr(), lda[0], b.data_ptr(), ldb[0],
+        out.data_ptr(), ldo[0], int(out.dtype == torch.float32), int(accumulate), M, N, K, float(alpha),
+        None if bias is None else bias.data_ptr(), None if residual is None else residual.data_ptr(),
+        0 if residual is None else residual.stride(0), _ACT[act], None if aux_out is None else aux_out.data_ptr(),
+        _ACT[dact], None if aux_in is None else aux_in.data_ptr(), 0 if aux is None else aux.stride(0),
+        int(force_bn), _status_ptr(a), _stream())
+    if st:
+        check(st, "tp_gemm")
     return out
 
 
@@ -101,7 +114,7 @@ def gemm_pair_trace(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bn: int
     trace = torch.zeros(n_ctas, GEMM_TRACE_SLOTS, dtype=torch.int64, device=a.device)
     st = cuda_lib().tp_gemm_trace(int(bn), a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
                                   out.data_ptr(), out.stride(0), M, N, K, trace.data_ptr(),
-                                  status_word(a.device).data_ptr(), _stream())
+                                  _status_ptr(a), _stream())
     check(st, "tp_gemm_trace")
     return trace
 
@@ -170,7 +183,7 @@ def _wgrad_args(dy, x, out):
 def weight_grad(dy, x, out, accumulate=False):
     """``out[l] (+)= dy[l]^T @ x[l]`` (fp32) for every layer: the weight gradients of one kind of a stage."""
     operands, sizes = _wgrad_args(dy, x, out)
-    st = cuda_lib().tp_wgrad(*operands, out.data_ptr(), *sizes, int(accumulate), status_word(dy.device).data_ptr(),
+    st = cuda_lib().tp_wgrad(*operands, out.data_ptr(), *sizes, int(accumulate), _status_ptr(dy),
                              _stream())
     check(st, "tp_wgrad")
     return out
@@ -185,7 +198,7 @@ def weight_grad_adam(dy, x, master, m, v, model, state, lr, beta1=0.9, beta2=0.9
         assert t.shape == master.shape and t.stride() == master.stride()
     st = cuda_lib().tp_wgrad_adam(*operands, master.data_ptr(), m.data_ptr(), v.data_ptr(), model.data_ptr(), *sizes,
                                   state.data_ptr(), lr, beta1, beta2, eps, weight_decay, grad_scale,
-                                  status_word(dy.device).data_ptr(), _stream())
+                                  _status_ptr(dy), _stream())
     check(st, "tp_wgrad_adam")
 
 
@@ -216,7 +229,7 @@ def attn_fwd(qkv, b: int, h: int, D: int, t: int, c: int, o, lse2, scale: float 
     columns are zero pass the scale of their real width."""
     st = cuda_lib().tp_attn_fwd_scaled(_dt(qkv), D, float(scale), qkv.data_ptr(), b, h, t, c,
                                        o.data_ptr(), o.stride(0), lse2.data_ptr(), lse2.stride(0),
-                                       status_word(qkv.device).data_ptr(), _stream())
+                                       _status_ptr(qkv), _stream())
     check(st, "tp_attn_fwd_scaled")
     return o
 
@@ -235,6 +248,6 @@ def attn_bwd(qkv, b: int, h: int, D: int, t: int, c: int, q_end: int, o, do_full
                                        o.data_ptr(), o.stride(0), do_full.data_ptr(),
                                        do_full.stride(0), lse2.data_ptr(), lse2.stride(0),
                                        delta.data_ptr(), dqkv.data_ptr(), dqkv.stride(0),
-                                       status_word(qkv.device).data_ptr(), _stream())
+                                       _status_ptr(qkv), _stream())
     check(st, "tp_attn_bwd_scaled")
     return dqkv
