@@ -69,6 +69,7 @@ struct GemmParams {
   long long* trace;  // optional per-CTA phase stamps (trace builds of the kernel only)
   int prefetch;      // CTA-pair kernel: operand tiles are prefetched into L2 this many k-steps
                      // ahead of the loads that fill the ring (0 = off)
+  int mat_tma;       // the residual, or else aux_in, comes as tiles (EpiMaps::mat)
 };
 
 constexpr int kMaxTp = 8;
@@ -143,7 +144,7 @@ template <int BN, int MT = 1, bool AR = false> struct GemmCfg {
   static constexpr int kAccBuffers = MT == 2 ? 1 : 2;
   static constexpr int kEpiStageBytes = AR ? 0 : kEpiBytes;  // staged output path (not used with AR)
   static constexpr int kSmemBytes =
-      kStages * kStageBytes + kArStageBytes + kEpiStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+      kStages * kStageBytes + kArStageBytes + kEpiStageBytes + 1024 /*align*/ + 512 /*barriers*/;
 };
 
 // GeLU and its derivative for two values at a time.  Both come from the upper tail of the normal
@@ -205,10 +206,41 @@ __device__ __forceinline__ long long clock_ordered() {
   return t;
 }
 
+// A second matrix of the output's size, the residual or the argument of the activation's derivative, comes the same
+// way (16-bit output): as a tile load into the very buffer that the chunk's result then leaves from, two chunks
+// ahead, a tile's first two under its main loop.  With 16-byte loads of 32 rows an instruction it bound products with
+// a short K; us before / now, 8192 rows: 3072 x 768 with ReLU's derivative 80 / 49, with GeLU's 82 / 60, 768 x 3072
+// with a residual 41 / 36; 2048 x 6400 x 1600 with ReLU's derivative 47 / 36, 4096 x 2048 x 2048 with a residual
+// 33 / 29.  (The pre-activation that GeLU stores gained nothing from leaving as a tile.)
 struct EpiStage {
-  uint8_t* buf;  // this warp's two buffers (1024-byte aligned)
-  int issued;    // chunks stored so far by this warp
+  uint8_t* buf;  // this warp's buffers (1024-byte aligned)
+  int issued;    // buffers used so far by this warp
+  uint64_t* bars;   // a barrier for each of the four buffers: the tile load into it
 };
+struct EpiMaps {
+  CUtensorMap out, mat;
+};
+constexpr int kEpiBufs16 = 4, kEpiBuf16Bytes = 2048;
+
+// The bias of columns [n, n + 32), fetched a chunk ahead: a short product's epilogue waited 400 to 800 cycles for it.
+template <typename T>
+__device__ __forceinline__ void epi_bias(const GemmParams& p, uint4 (&bv)[4], int n) {
+  if (!p.bias) return;
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+    bv[g] = n + g * 8 + 8 <= p.N ? __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.bias) + n + g * 8))
+                                 : make_uint4(0, 0, 0, 0);
+}
+
+// Buffer number q receives columns [n, n + 32) of the matrix (every chunk before has committed one store).
+__device__ __forceinline__ void epi_request(const CUtensorMap* mat, const EpiStage& es, int q, int n, int row0, int lane) {
+  if (lane == 0) {
+    bulk_wait_read<kEpiBufs16 - 2>();      // the store of four buffers ago has read its source
+    uint64_t* bar = &es.bars[q % kEpiBufs16];
+    mbar_expect_tx(bar, kEpiBuf16Bytes);
+    tma_load_2d(es.buf + (q % kEpiBufs16) * kEpiBuf16Bytes, mat, bar, n, row0);
+  }
+}
 
 __device__ __forceinline__ void epi_drain(int lane) {
   if (lane == 0) bulk_wait<0>();
@@ -218,39 +250,34 @@ __device__ __forceinline__ void epi_drain(int lane) {
 // Fused epilogue of one 32-column chunk: r holds the fp32 accumulators of columns [n, n + 32)
 // of row `row` (thread = row).  row0 is the first row of the warp's 32-row group (row0 < M);
 // the caller has checked n < N.  t_next: TMEM address of the next chunk to load into r, or 0.  Rows >= M and columns >= N are clipped by the tile store.
-template <typename T, bool OUT_F32, bool TRACE = false>
-__device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const CUtensorMap* tmO,
-                                               EpiStage& es, uint32_t (&r)[32], long long row,
+// bv: the bias of these columns, and at the end of those from n_next on (-1: none).  TILES: the other matrix may come
+// as tiles (p.mat_tma); n_ahead: the chunk two further on, or -1.
+template <typename T, bool OUT_F32, bool TRACE = false, bool TILES = false>
+__device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMaps& tm,
+                                               EpiStage& es, const WaitCtx& wctx, uint32_t (&r)[32], uint4 (&bv)[4], long long row,
                                                bool row_ok, int n, int row0, int lane,
-                                               uint32_t t_next, long long* cyc = nullptr,
+                                               uint32_t t_next, int n_next, int n_ahead, long long* cyc = nullptr,
                                                const T* part = nullptr, long long part_stride = 0,
                                                int n_src = 0, int self = 0) {
   const long long t_0 = TRACE ? clock_ordered() : 0;
-  // Issue every global load of this 32-column chunk before any dependent math or store,
+  // Without tiles every global load of this 32-column chunk is issued before any dependent math or store,
   // so the chunk pays one memory latency instead of one per 8-column group.
   bool gok[4];
-  uint4 bv[4], rv[4], av[4];
 #pragma unroll
   for (int g = 0; g < 4; ++g) gok[g] = n + g * 8 + 8 <= p.N;
-  const uint4 zero4 = make_uint4(0, 0, 0, 0);
-  if (p.bias) {
+  const bool tiles = TILES && p.mat_tma;
+  auto direct = [&](const void* x, long long ld, int g) {
+    return gok[g] && row_ok ? __ldcg(reinterpret_cast<const uint4*>(static_cast<const T*>(x) + row * ld + n + g * 8))
+                            : make_uint4(0, 0, 0, 0);
+  };
+  uint4 rv[4], av[4];
+  if (!TILES && p.residual) {
 #pragma unroll
-    for (int g = 0; g < 4; ++g)
-      bv[g] = gok[g] ? __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.bias) + n + g * 8)) : zero4;
+    for (int g = 0; g < 4; ++g) rv[g] = direct(p.residual, p.ldr, g);
   }
-  if (p.residual) {
+  if (!TILES && p.dact) {
 #pragma unroll
-    for (int g = 0; g < 4; ++g)
-      rv[g] = (gok[g] && row_ok)
-                  ? __ldcg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.residual) + row * p.ldr + n + g * 8))
-                  : zero4;
-  }
-  if (p.dact) {
-#pragma unroll
-    for (int g = 0; g < 4; ++g)
-      av[g] = (gok[g] && row_ok)
-                  ? __ldcg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.aux_in) + row * p.ld_aux + n + g * 8))
-                  : zero4;
+    for (int g = 0; g < 4; ++g) av[g] = direct(p.aux_in, p.ld_aux, g);
   }
   // Reduce-scatter: the other ranks' 16-bit partials of this chunk (thread = row, 64 contiguous
   // bytes per source in this rank's staging buffer); the first source is fetched here with the
@@ -266,9 +293,15 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const CUtens
   // A tile store reads its source a good thousand cycles after it was issued, so the buffers
   // rotate: four 2 KB buffers for 16-bit output, two 4 KB buffers for fp32.  The buffer about
   // to be overwritten was the source of the store issued kBufs chunks ago.
-  constexpr int kBufs = OUT_F32 ? 2 : 4;
+  constexpr int kBufs = OUT_F32 ? 2 : kEpiBufs16;
+  static_assert(OUT_F32 || kEpiBytesPerWarp == kEpiBufs16 * kEpiBuf16Bytes, "four buffers a warp");
   uint8_t* sb = es.buf + (es.issued % kBufs) * (kEpiBytesPerWarp / kBufs);
-  if (es.issued >= kBufs) {
+  const int sw = (lane >> 1) & 3;      // 64-byte rows, 64-byte swizzle: 16-byte chunk index ^= (row >> 1) & 3
+  if (tiles) {
+    // (the request waited for the buffer's last store)
+    mbar_wait(&es.bars[es.issued % kBufs], (es.issued / kBufs) & 1, wctx, kErrWaitEpilogue);
+    __syncwarp();
+  } else if (es.issued >= kBufs) {
     if (lane == 0) bulk_wait_read<kBufs - 1>();
     __syncwarp();
   }
@@ -350,10 +383,12 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const CUtens
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
   }
+  auto tile = [&](int g) { return *reinterpret_cast<const uint4*>(sb + lane * 64 + ((g ^ sw) << 4)); };
   if (p.residual) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      const uint32_t rw[4] = {rv[g].x, rv[g].y, rv[g].z, rv[g].w};
+      const uint4 r4 = !TILES ? rv[g] : tiles ? tile(g) : direct(p.residual, p.ldr, g);
+      const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 f = Elem<T>::unpack2(rw[j]);
@@ -365,7 +400,8 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const CUtens
   if (p.dact) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      const uint32_t aw[4] = {av[g].x, av[g].y, av[g].z, av[g].w};
+      const uint4 a4 = !TILES ? av[g] : tiles && !p.residual ? tile(g) : direct(p.aux_in, p.ld_aux, g);
+      const uint32_t aw[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 f = Elem<T>::unpack2(aw[j]);
@@ -380,6 +416,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const CUtens
       }
     }
   }
+  if (n_next >= 0) epi_bias<T>(p, bv, n_next);
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     if (OUT_F32) {
@@ -390,23 +427,23 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const CUtens
       *reinterpret_cast<float4*>(rowp + (((2 * g + 1) ^ (lane & 7)) << 4)) =
           make_float4(v[g * 8 + 4], v[g * 8 + 5], v[g * 8 + 6], v[g * 8 + 7]);
     } else {
-      // 64-byte rows, 64-byte swizzle: 16-byte chunk index ^= (row >> 1) & 3
       uint4 ov;
       ov.x = Elem<T>::pack2(v[g * 8 + 0], v[g * 8 + 1]);
       ov.y = Elem<T>::pack2(v[g * 8 + 2], v[g * 8 + 3]);
       ov.z = Elem<T>::pack2(v[g * 8 + 4], v[g * 8 + 5]);
       ov.w = Elem<T>::pack2(v[g * 8 + 6], v[g * 8 + 7]);
-      *reinterpret_cast<uint4*>(sb + lane * 64 + ((g ^ ((lane >> 1) & 3)) << 4)) = ov;
+      *reinterpret_cast<uint4*>(sb + lane * 64 + ((g ^ sw) << 4)) = ov;
     }
   }
   const long long t_2 = TRACE ? clock_ordered() : 0;
   fence_proxy_async();
   __syncwarp();
   if (lane == 0) {
-    if (OUT_F32 && p.accumulate) tma_reduce_add_2d(tmO, sb, n, row0);
-    else tma_store_2d(tmO, sb, n, row0);
+    if (OUT_F32 && p.accumulate) tma_reduce_add_2d(&tm.out, sb, n, row0);
+    else tma_store_2d(&tm.out, sb, n, row0);
     bulk_commit();
   }
+  if (tiles && n_ahead >= 0) epi_request(&tm.mat, es, es.issued + 2, n_ahead, row0, lane);
   ++es.issued;
   if (TRACE) {
     cyc[0] += t_1 - t_0;        // loads issued, staging buffer free
@@ -422,10 +459,10 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const CUtens
 // The chunk code exists once (it is large); the TMEM
 // load of chunk c + 1 is issued from inside it as soon as chunk c's values have been copied out
 // of the load registers.
-template <typename T, bool OUT_F32, bool TRACE = false>
-__device__ __forceinline__ void epilogue_rows(const GemmParams& p, const CUtensorMap* tmO,
-                                              EpiStage& es, uint32_t t_acc, int nc, int row0, int n0,
-                                              int lane, int c_first = 0, int c_step = 1,
+template <typename T, bool OUT_F32, bool TRACE = false, bool TILES = false>
+__device__ __forceinline__ void epilogue_rows(const GemmParams& p, const EpiMaps& tm,
+                                              EpiStage& es, const WaitCtx& wctx, uint4 (&bv)[4], uint32_t t_acc,
+                                              int nc, int row0, int n0, int lane, int c_first = 0, int c_step = 1,
                                               long long* cyc = nullptr, const T* part = nullptr,
                                               long long part_stride = 0, int n_src = 0, int self = 0) {
   const long long row = row0 + lane;
@@ -437,20 +474,34 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, const CUtenso
 #pragma unroll 1
   for (int c = c_first; c < nc; c += c_step) {
     tmem_ld_wait();
-    epilogue_chunk<T, OUT_F32, TRACE>(p, tmO, es, r, row, row_ok, n0 + c * 32, row0, lane,
-                                      c + c_step < nc ? t_acc + (c + c_step) * 32 : 0u, cyc,
-                                      part ? part + c * 4096 : nullptr, part_stride, n_src, self);
+    epilogue_chunk<T, OUT_F32, TRACE, TILES>(p, tm, es, wctx, r, bv, row, row_ok, n0 + c * 32, row0, lane,
+                                             c + c_step < nc ? t_acc + (c + c_step) * 32 : 0u,
+                                             c + c_step < nc ? n0 + (c + c_step) * 32 : -1,
+                                             c + 2 * c_step < nc ? n0 + (c + 2 * c_step) * 32 : -1, cyc,
+                                             part ? part + c * 4096 : nullptr, part_stride, n_src, self);
   }
+}
+// What the first of these chunks need (any time after the last chunk before them): the bias, two tiles.
+template <typename T, bool TILES>
+__device__ __forceinline__ void epilogue_ahead(const GemmParams& p, const EpiMaps& tm, const EpiStage& es,
+                                               uint4 (&bv)[4], int nc, int row0, int n0, int lane, int c_first = 0,
+                                               int c_step = 1) {
+  if (row0 >= p.M) return;
+  epi_bias<T>(p, bv, n0 + c_first * 32);
+  if (!TILES || !p.mat_tma) return;
+  for (int i = 0; i < 2 && c_first + i * c_step < nc; ++i)
+    epi_request(&tm.mat, es, es.issued + i, n0 + (c_first + i * c_step) * 32, row0, lane);
 }
 
 template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool AR = false, int MT = 1>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-            const __grid_constant__ CUtensorMap tmO, const GemmParams p, const ArParams ar) {
+            const __grid_constant__ EpiMaps tmE, const GemmParams p, const ArParams ar) {
   using Cfg = GemmCfg<BN, MT, AR>;
   constexpr int S = Cfg::kStages;
   constexpr int BM = MT * kBM;
   constexpr int NACC = Cfg::kAccBuffers;
+  constexpr bool TILES = !OUT_F32 && !AR;     // of the epilogue's other matrices
   static_assert(!(AR && MT != 1), "the fused all-reduce path uses 128-row tiles");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -464,6 +515,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint64_t* tempty = bars + 2 * S + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* epi_bars = bars + 2 * S + 6;     // TILES: four for each epilogue warp
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -482,7 +534,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     fence_barrier_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
-    if (!AR) prefetch_tmap(&tmO);
+    if (!AR) prefetch_tmap(&tmE.out);
+  }
+  if (TILES && warp >= 2 && lane < kEpiBufs16) {
+    mbar_init(&epi_bars[(warp & 3) * kEpiBufs16 + lane], 1);
+    fence_barrier_init();
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -574,7 +630,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else {
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access
     const int row_in_tile = quarter * 32 + lane;
-    EpiStage es{epi_smem + quarter * kEpiBytesPerWarp, 0};
+    EpiStage es{epi_smem + quarter * kEpiBytesPerWarp, 0, epi_bars + quarter * kEpiBufs16};
     int it = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++it) {
@@ -582,6 +638,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const uint32_t acc_phase = (it / NACC) & 1;
       const int m0 = (tile % p.num_m_tiles) * BM;
       const int n0 = (tile / p.num_m_tiles) * BN;
+      const int nc = (min(BN, p.N - n0) + 31) / 32;   // 32-column chunks of this tile inside the matrix (warp-uniform)
+      uint4 bv[4];
+      if (!AR) epilogue_ahead<T, TILES>(p, tmE, es, bv, nc, m0 + quarter * 32, n0, lane);
       ok = mbar_wait(&tfull[acc], acc_phase, wctx, kErrWaitEpilogue);
       if (!ok) break;
       tc_fence_after();
@@ -606,13 +665,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       } else {
-        // columns of this tile inside the matrix, in 32-column chunks (warp-uniform)
-        const int nc = (min(BN, p.N - n0) + 31) / 32;
 #pragma unroll 1
         for (int mt = 0; mt < MT; ++mt) {
           const int row0 = m0 + mt * kBM + quarter * 32;
           if (row0 >= p.M) continue;  // warp-uniform: nothing to store
-          epilogue_rows<T, OUT_F32>(p, &tmO, es, t_acc + mt * BN, nc, row0, n0, lane);
+          if (mt > 0) epilogue_ahead<T, TILES>(p, tmE, es, bv, nc, row0, n0, lane);
+          epilogue_rows<T, OUT_F32, false, TILES>(p, tmE, es, wctx, bv, t_acc + mt * BN, nc, row0, n0, lane);
         }
       }
       tc_fence_before();
@@ -733,7 +791,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 }
 
 template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool AR = false, int MT = 1>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmO,
+static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& tmE,
                        const GemmParams& p, cudaStream_t stream, const ArParams* arp = nullptr) {
   using Cfg = GemmCfg<BN, MT, AR>;
   static_assert(Cfg::kSmemBytes >= kTmemKernelMinSmem, "allocates TMEM before pdl_wait");
@@ -749,7 +807,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
     configured = true;
   }
   int grid = p.num_tiles < num_sms() ? p.num_tiles : num_sms();
-  return launch_pdl(kern, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream, 1, tmA, tmB, tmO, p, ar) ==
+  return launch_pdl(kern, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream, 1, tmA, tmB, tmE, p, ar) ==
                  cudaSuccess
              ? kOk
              : kErrLaunch;
@@ -757,14 +815,14 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
 
 template <typename T, int BN, int MT = 1>
 static int dispatch_layout(int a_mn, int b_mn, int out_f32, const CUtensorMap& tmA,
-                           const CUtensorMap& tmB, const CUtensorMap& tmO, const GemmParams& p,
+                           const CUtensorMap& tmB, const EpiMaps& tmE, const GemmParams& p,
                            cudaStream_t s) {
-  if (!a_mn && !b_mn && !out_f32) return launch_gemm<T, BN, false, false, false, false, MT>(tmA, tmB, tmO, p, s);
-  if (!a_mn && b_mn && !out_f32) return launch_gemm<T, BN, false, true, false, false, MT>(tmA, tmB, tmO, p, s);
-  if (a_mn && b_mn && out_f32) return launch_gemm<T, BN, true, true, true, false, MT>(tmA, tmB, tmO, p, s);
+  if (!a_mn && !b_mn && !out_f32) return launch_gemm<T, BN, false, false, false, false, MT>(tmA, tmB, tmE, p, s);
+  if (!a_mn && b_mn && !out_f32) return launch_gemm<T, BN, false, true, false, false, MT>(tmA, tmB, tmE, p, s);
+  if (a_mn && b_mn && out_f32) return launch_gemm<T, BN, true, true, true, false, MT>(tmA, tmB, tmE, p, s);
   if (MT == 1) {  // rarely used layouts: only the 128-row tile is instantiated
-    if (!a_mn && !b_mn && out_f32) return launch_gemm<T, BN, false, false, true>(tmA, tmB, tmO, p, s);
-    if (a_mn && b_mn && !out_f32) return launch_gemm<T, BN, true, true, false>(tmA, tmB, tmO, p, s);
+    if (!a_mn && !b_mn && out_f32) return launch_gemm<T, BN, false, false, true>(tmA, tmB, tmE, p, s);
+    if (a_mn && b_mn && !out_f32) return launch_gemm<T, BN, true, true, false>(tmA, tmB, tmE, p, s);
   }
   return kErrBadArgument;
 }
@@ -1046,7 +1104,7 @@ template <int BN> struct PairCfg {
   static constexpr int kAccCols = BN > 128 ? 256 : 128;   // TMEM columns of one accumulator
   static constexpr int kTmemCols = 2 * kAccCols;
   static constexpr int kEpiStageBytes = kPairEpiWarps * kEpiBytesPerWarp;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kEpiStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kEpiStageBytes + 1024 /*align*/ + 512 /*barriers*/;
 };
 
 // TRACE = true additionally records, per CTA, SM-clock stamps of the pipeline phases into
@@ -1169,12 +1227,13 @@ template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool TRACE = f
           bool RS = false>
 __global__ void __launch_bounds__(kPairThreads + (RS ? 32 : 0), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmO, const GemmParams p, const ArParams ar) {
+                 const __grid_constant__ EpiMaps tmE, const GemmParams p, const ArParams ar) {
   static_assert(!AR || (BN == 128 && !OUT_F32 && !TRACE), "fused all-reduce: 256 x 128 pair tiles, 16-bit output");
   static_assert(!RS || (BN == 128 && !OUT_F32 && !TRACE && !AR && !A_MN), "fused reduce-scatter: 256 x 128 pair tiles, 16-bit output");
   using Cfg = PairCfg<BN>;
   constexpr int S = Cfg::kStages;
   constexpr int HB = BN / 2;  // B rows held by one CTA
+  constexpr bool TILES = !OUT_F32 && !AR && !RS;   // of the epilogue's other matrices
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -1190,6 +1249,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* s_next = reinterpret_cast<volatile int*>(tmem_slot + 3);   // AR: next owned tile
   uint64_t* pub_full = bars + 2 * S + 6;                                    // RS: block stored by all warps
   volatile int* pub_done = reinterpret_cast<volatile int*>(bars + 2 * S + 8);  // RS: blocks published
+
+  uint64_t* epi_bars = bars + 2 * S + 9;     // TILES: four for each epilogue warp
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1220,7 +1281,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     fence_barrier_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
-    prefetch_tmap(&tmO);
+    prefetch_tmap(&tmE.out);
+  }
+  if (TILES && warp >= 2 && lane < kEpiBufs16) {
+    mbar_init(&epi_bars[(warp - 2) * kEpiBufs16 + lane], 1);
+    fence_barrier_init();
   }
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote arrival
@@ -1369,7 +1434,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp < 10) {
     const int quarter = warp & 3;      // TMEM lane quarter this warp may access
     const int half = (warp - 2) >> 2;  // which of the two warps of that quarter
-    EpiStage es{epi_smem + (warp - 2) * kEpiBytesPerWarp, 0};
+    EpiStage es{epi_smem + (warp - 2) * kEpiBytesPerWarp, 0, epi_bars + (warp - 2) * kEpiBufs16};
     int it = 0;
     bool ok = true;
     // AR: index (into this rank's owned tiles) of the next one this CTA reduces
@@ -1390,6 +1455,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                      kErrCheckTile);
       const int m0 = m_idx * (2 * kBM) + static_cast<int>(cta) * kBM;
       const int n0 = n_idx * BN;
+      const int nc = (min(BN, p.N - n0) + 31) / 32;
+      uint4 bv[4];
+      if (!AR) epilogue_ahead<T, TILES>(p, tmE, es, bv, nc, m0 + quarter * 32, n0, lane, half, 2);
       const long long t_e = TRACE ? clock64() : 0;
       ok = mbar_wait(&tfull[acc], acc_phase, wctx, kErrWaitEpilogue);
       if (!ok) break;
@@ -1444,8 +1512,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           got = __shfl_sync(0xffffffffu, got, 0);
           const T* part = static_cast<const T*>(ar.stage[ar.rank]) + stage_half + unit * tile_elems +
                           quarter * 1024 + lane * 32;
-          const int nc = (min(BN, p.N - n0) + 31) / 32;
-          epilogue_rows<T, OUT_F32, false>(p, &tmO, es, t_acc, nc, row0, n0, lane, half, 2, nullptr,
+          epilogue_rows<T, OUT_F32, false>(p, tmE, es, wctx, bv, t_acc, nc, row0, n0, lane, half, 2, nullptr,
                                            got ? part : nullptr, ar.max_tiles * tile_elems, ar.tp, ar.rank);
         } else if (row0 < p.M) {
           // rows of another rank: 16-bit partial chunks into its staging buffer
@@ -1597,10 +1664,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         continue;
       }
       if (row0 < p.M) {
-        const int nc = (min(BN, p.N - n0) + 31) / 32;
         const long long t_l = TRACE ? clock64() : 0;
-        epilogue_rows<T, OUT_F32, TRACE>(
-            p, &tmO, es, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kAccCols, nc, row0,
+        epilogue_rows<T, OUT_F32, TRACE, TILES>(
+            p, tmE, es, wctx, bv, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kAccCols, nc, row0,
             n0, lane, half, 2, cyc3);
         if (TRACE) cyc_rest += clock64() - t_l;
       }
@@ -1730,7 +1796,7 @@ static int max_pairs() {
 
 template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool TRACE = false, bool AR = false,
           bool RS = false>
-static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmO,
+static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& tmE,
                             const GemmParams& p, cudaStream_t stream, const ArParams* arp = nullptr) {
   using Cfg = PairCfg<BN>;
   static_assert(Cfg::kSmemBytes + kTmemKernelMinSmem > kSmemPerSm, "allocates TMEM after pdl_wait");
@@ -1747,18 +1813,18 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   else { ar.tp = 0; ar.exchange = 0; ar.rows_per_rank = 0; }
   const int pairs = p.num_tiles < max_pairs() ? p.num_tiles : max_pairs();
   return launch_pdl(kern, dim3(2 * pairs), dim3(kPairThreads + (RS ? 32 : 0)), Cfg::kSmemBytes, stream, 2,
-                    tmA, tmB, tmO, p, ar) == cudaSuccess
+                    tmA, tmB, tmE, p, ar) == cudaSuccess
              ? kOk
              : kErrLaunch;
 }
 
 template <typename T, int BN>
 static int dispatch_layout_pair(int a_mn, int b_mn, int out_f32, const CUtensorMap& tmA,
-                                const CUtensorMap& tmB, const CUtensorMap& tmO, const GemmParams& p,
+                                const CUtensorMap& tmB, const EpiMaps& tmE, const GemmParams& p,
                                 cudaStream_t s) {
-  if (!a_mn && !b_mn && !out_f32) return launch_gemm_pair<T, BN, false, false, false>(tmA, tmB, tmO, p, s);
-  if (!a_mn && b_mn && !out_f32) return launch_gemm_pair<T, BN, false, true, false>(tmA, tmB, tmO, p, s);
-  if (a_mn && b_mn && out_f32) return launch_gemm_pair<T, BN, true, true, true>(tmA, tmB, tmO, p, s);
+  if (!a_mn && !b_mn && !out_f32) return launch_gemm_pair<T, BN, false, false, false>(tmA, tmB, tmE, p, s);
+  if (!a_mn && b_mn && !out_f32) return launch_gemm_pair<T, BN, false, true, false>(tmA, tmB, tmE, p, s);
+  if (a_mn && b_mn && out_f32) return launch_gemm_pair<T, BN, true, true, true>(tmA, tmB, tmE, p, s);
   return kErrBadArgument;
 }
 
@@ -1835,9 +1901,9 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   if (!b_mn) ok = make_tmap_2d(&tmB, B, K, N, ldb, kBK, box_n, bf16);
   else ok = make_tmap_2d(&tmB, B, N, K, ldb, 64, parts ? kSplitBK : kBK, bf16);
   if (!ok) return kErrDriver;
-  CUtensorMap tmO;
-  if (!make_tmap_out(&tmO, out, N, M, ldo, out_f32 != 0, bf16)) return kErrDriver;
-  GemmParams p;
+  EpiMaps tmE = {};
+  if (!make_tmap_out(&tmE.out, out, N, M, ldo, out_f32 != 0, bf16)) return kErrDriver;
+  GemmParams p = {};
   p.M = M; p.N = N; p.K = K;
   p.num_m_tiles = (M + BM - 1) / BM;
   p.num_n_tiles = (N + BN - 1) / BN;
@@ -1861,6 +1927,14 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   p.err = err_flag;
   p.trace = nullptr;
   p.prefetch = g_prefetch;
+  if (!parts && !out_f32) {
+    // as tiles, where a tensor map can describe them (16-byte addresses and strides)
+    auto tile_map = [&](CUtensorMap* m, const void* x, long long ld) {
+      return x && ld % 8 == 0 && ld >= N && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+             make_tmap_out(m, x, N, M, ld, false, bf16);
+    };
+    p.mat_tma = residual ? tile_map(&tmE.mat, residual, ldr) : dact ? tile_map(&tmE.mat, aux_in, ld_aux) : 0;
+  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (parts) {
 #define TP_SPLIT(T)                                                                        \
@@ -1872,14 +1946,14 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
 #undef TP_SPLIT
   }
 #define TP_DISPATCH(T)                                                                   \
-  (pair ? (BN == 256 ? dispatch_layout_pair<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)  \
-           : BN == 224 ? dispatch_layout_pair<T, 224>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s) \
-           : BN == 192 ? dispatch_layout_pair<T, 192>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s) \
-                     : dispatch_layout_pair<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)) \
-   : tile_code == 512 ? dispatch_layout<T, 256, 2>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)  \
-   : BN == 256 ? dispatch_layout<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)            \
-   : BN == 128 ? dispatch_layout<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s)            \
-               : dispatch_layout<T, 64>(a_mn, b_mn, out_f32, tmA, tmB, tmO, p, s))
+  (pair ? (BN == 256 ? dispatch_layout_pair<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)  \
+           : BN == 224 ? dispatch_layout_pair<T, 224>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s) \
+           : BN == 192 ? dispatch_layout_pair<T, 192>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s) \
+                     : dispatch_layout_pair<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)) \
+   : tile_code == 512 ? dispatch_layout<T, 256, 2>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)  \
+   : BN == 256 ? dispatch_layout<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)            \
+   : BN == 128 ? dispatch_layout<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)            \
+               : dispatch_layout<T, 64>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s))
   return bf16 ? TP_DISPATCH(__nv_bfloat16) : TP_DISPATCH(__half);
 #undef TP_DISPATCH
 }
@@ -1929,7 +2003,7 @@ extern "C" int tp_gemm_ar(int dtype, int b_mn, const void* A, long long lda, con
   const bool bf16 = dtype == 1;
   const bool pair = g_pair_default;  // 256 x 128 CTA-pair tiles; all-reduce tiles stay 128 x 128
   const int BM = pair ? 2 * kBM : kBM;
-  GemmParams p;
+  GemmParams p = {};
   p.M = M; p.N = N; p.K = K;
   p.num_m_tiles = (M + BM - 1) / BM;
   p.num_n_tiles = (N + BN - 1) / BN;
@@ -1960,19 +2034,19 @@ extern "C" int tp_gemm_ar(int dtype, int b_mn, const void* A, long long lda, con
     ar.out[i] = i < tp ? out_ptrs[i] : nullptr;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const CUtensorMap& tmO = tmA;  // the fused all-reduce epilogue stores through peer pointers
+  const EpiMaps tmE = {};        // the fused all-reduce epilogue stores through peer pointers
   if (pair) {
     if (bf16)
-      return b_mn ? launch_gemm_pair<__nv_bfloat16, BN, false, true, false, false, true>(tmA, tmB, tmO, p, s, &ar)
-                  : launch_gemm_pair<__nv_bfloat16, BN, false, false, false, false, true>(tmA, tmB, tmO, p, s, &ar);
-    return b_mn ? launch_gemm_pair<__half, BN, false, true, false, false, true>(tmA, tmB, tmO, p, s, &ar)
-                : launch_gemm_pair<__half, BN, false, false, false, false, true>(tmA, tmB, tmO, p, s, &ar);
+      return b_mn ? launch_gemm_pair<__nv_bfloat16, BN, false, true, false, false, true>(tmA, tmB, tmE, p, s, &ar)
+                  : launch_gemm_pair<__nv_bfloat16, BN, false, false, false, false, true>(tmA, tmB, tmE, p, s, &ar);
+    return b_mn ? launch_gemm_pair<__half, BN, false, true, false, false, true>(tmA, tmB, tmE, p, s, &ar)
+                : launch_gemm_pair<__half, BN, false, false, false, false, true>(tmA, tmB, tmE, p, s, &ar);
   }
   if (bf16)
-    return b_mn ? launch_gemm<__nv_bfloat16, BN, false, true, false, true>(tmA, tmB, tmO, p, s, &ar)
-                : launch_gemm<__nv_bfloat16, BN, false, false, false, true>(tmA, tmB, tmO, p, s, &ar);
-  return b_mn ? launch_gemm<__half, BN, false, true, false, true>(tmA, tmB, tmO, p, s, &ar)
-              : launch_gemm<__half, BN, false, false, false, true>(tmA, tmB, tmO, p, s, &ar);
+    return b_mn ? launch_gemm<__nv_bfloat16, BN, false, true, false, true>(tmA, tmB, tmE, p, s, &ar)
+                : launch_gemm<__nv_bfloat16, BN, false, false, false, true>(tmA, tmB, tmE, p, s, &ar);
+  return b_mn ? launch_gemm<__half, BN, false, true, false, true>(tmA, tmB, tmE, p, s, &ar)
+              : launch_gemm<__half, BN, false, false, false, true>(tmA, tmB, tmE, p, s, &ar);
 }
 
 // Fused GEMM + tensor-parallel reduce-scatter over the rows (CTA-pair kernel, 256 x 128 tiles):
@@ -1995,7 +2069,7 @@ extern "C" int tp_gemm_rs(int dtype, int b_mn, const void* A, long long lda, con
   if (static_cast<long long>(rows_per_rank) * tp < M) return kErrBadArgument;
   constexpr int BN = 128;
   const bool bf16 = dtype == 1;
-  GemmParams p;
+  GemmParams p = {};
   p.M = M; p.N = N; p.K = K;
   p.num_m_tiles = (M + 2 * kBM - 1) / (2 * kBM);
   p.num_n_tiles = (N + BN - 1) / BN;
@@ -2006,12 +2080,13 @@ extern "C" int tp_gemm_rs(int dtype, int b_mn, const void* A, long long lda, con
   apply_tile_order(p, rs_tile_order(M, N, K, p.num_m_tiles, p.num_n_tiles, 2 * kBM, rank, rows_per_rank,
                                     max_pairs()));
   p.ag_flags = nullptr; p.ag_epoch_base = nullptr; p.ag_epoch = 0; p.ag_rows = 1; p.ag_rank = 0;
-  CUtensorMap tmA, tmB, tmO;
+  CUtensorMap tmA, tmB;
+  EpiMaps tmE = {};
   if (!make_tmap_2d(&tmA, A, K, M, lda, kBK, kBM, bf16)) return kErrDriver;
   if (!(b_mn ? make_tmap_2d(&tmB, B, N, K, ldb, 64, kBK, bf16)
              : make_tmap_2d(&tmB, B, K, N, ldb, kBK, BN / 2, bf16)))
     return kErrDriver;
-  if (!make_tmap_out(&tmO, out, N, M, ldo, false, bf16)) return kErrDriver;
+  if (!make_tmap_out(&tmE.out, out, N, M, ldo, false, bf16)) return kErrDriver;
   p.out = out; p.ldo = ldo;
   p.bias = bias; p.residual = residual; p.ldr = ldr;
   p.aux_out = nullptr; p.aux_in = nullptr; p.ld_aux = 0;
@@ -2030,10 +2105,10 @@ extern "C" int tp_gemm_rs(int dtype, int b_mn, const void* A, long long lda, con
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (bf16)
-    return b_mn ? launch_gemm_pair<__nv_bfloat16, BN, false, true, false, false, false, true>(tmA, tmB, tmO, p, s, &ar)
-                : launch_gemm_pair<__nv_bfloat16, BN, false, false, false, false, false, true>(tmA, tmB, tmO, p, s, &ar);
-  return b_mn ? launch_gemm_pair<__half, BN, false, true, false, false, false, true>(tmA, tmB, tmO, p, s, &ar)
-              : launch_gemm_pair<__half, BN, false, false, false, false, false, true>(tmA, tmB, tmO, p, s, &ar);
+    return b_mn ? launch_gemm_pair<__nv_bfloat16, BN, false, true, false, false, false, true>(tmA, tmB, tmE, p, s, &ar)
+                : launch_gemm_pair<__nv_bfloat16, BN, false, false, false, false, false, true>(tmA, tmB, tmE, p, s, &ar);
+  return b_mn ? launch_gemm_pair<__half, BN, false, true, false, false, false, true>(tmA, tmB, tmE, p, s, &ar)
+              : launch_gemm_pair<__half, BN, false, false, false, false, false, true>(tmA, tmB, tmE, p, s, &ar);
 }
 
 TP_DEFINE_WAIT_LIMIT_SETTER(tp_set_wait_limit_ns_gemm)
@@ -2063,9 +2138,9 @@ extern "C" int tp_gemm_trace(int bn, const void* A, long long lda, const void* B
   CUtensorMap tmA, tmB;
   if (!make_tmap_2d(&tmA, A, K, M, lda, kBK, kBM, false)) return kErrDriver;
   if (!make_tmap_2d(&tmB, B, K, N, ldb, kBK, bn / 2, false)) return kErrDriver;
-  CUtensorMap tmO;
-  if (!make_tmap_out(&tmO, out, N, M, ldo, false, false)) return kErrDriver;
-  GemmParams p;
+  EpiMaps tmE = {};
+  if (!make_tmap_out(&tmE.out, out, N, M, ldo, false, false)) return kErrDriver;
+  GemmParams p = {};
   p.M = M; p.N = N; p.K = K;
   p.num_m_tiles = (M + 2 * kBM - 1) / (2 * kBM);
   p.num_n_tiles = (N + bn - 1) / bn;
@@ -2080,8 +2155,8 @@ extern "C" int tp_gemm_trace(int bn, const void* A, long long lda, const void* B
   p.trace = trace;
   p.prefetch = g_prefetch;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return bn == 256 ? launch_gemm_pair<__half, 256, false, false, false, true>(tmA, tmB, tmO, p, s)
-                   : launch_gemm_pair<__half, 128, false, false, false, true>(tmA, tmB, tmO, p, s);
+  return bn == 256 ? launch_gemm_pair<__half, 256, false, false, false, true>(tmA, tmB, tmE, p, s)
+                   : launch_gemm_pair<__half, 128, false, false, false, true>(tmA, tmB, tmE, p, s);
 }
 
 // Fused all-reduce, CTA-pair kernel.  exchange = 1: every rank sends each partial tile to every
