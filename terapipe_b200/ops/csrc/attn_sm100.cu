@@ -583,7 +583,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();  // set-up done; from here on the predecessor's results are read
+  // Set-up done; from here on the predecessor's results are read.  dQ follows dK/dV, of which it reads nothing: it
+  // starts once all CTAs of dK/dV run, which they do when everything before them is done, and waits for them
+  // at its own end, so that whoever waits for dQ waits for both.
+  if (MODE == 0) pdl_wait();
+  else pdl_trigger();
   const uint32_t tmem = sh->tmem_slot;
   // columns: S / P of buffer 0 at 0, of 1 at 64, dP / dS at 128 and 192, Acc1 256, Acc2 256 + D
   const uint32_t tA1 = tmem + 256, tA2 = tmem + 256 + D;
@@ -844,6 +848,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV128,
   }
   tc_fence_after();
   if (warp == 9) tmem_dealloc(tmem, kTmemCols);
+  if (MODE == 1) pdl_wait(false);
 }
 
 // ---------------------------------------------------------------------------- host side
