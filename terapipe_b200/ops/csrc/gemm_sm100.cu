@@ -69,6 +69,7 @@ struct GemmParams {
   long long* trace;  // optional per-CTA phase stamps (trace builds of the kernel only)
   int prefetch;      // CTA-pair kernel: operand tiles are prefetched into L2 this many k-steps
                      // ahead of the loads that fill the ring (0 = off)
+  int a_bytes;       // one-CTA kernel: of A in a stage (fewer where M < 128)
   int mat_tma;       // the residual, or else aux_in, comes as tiles (EpiMaps::mat)
 };
 
@@ -138,9 +139,10 @@ template <int BN, int MT = 1, bool AR = false> struct GemmCfg {
   static constexpr int kStages = (MT == 2 ? 3 : (BN == 256 ? 4 : (BN == 128 ? 6 : 8))) - (AR ? 1 : 0);
   static constexpr int kArStageBytes = AR ? kBM * BN * 2 : 0;
   static constexpr int kABytes = MT * kBM * kBK * 2;
-  static constexpr int kBBytes = BN * kBK * 2;
+  // (32 columns: half a chunk of 64 where N is contiguous)
+  static constexpr int kBBytes = (BN < 64 ? 64 : BN) * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kTmemCols = BN == 64 ? 128 : 2 * BN;  // two accumulators, power of two
+  static constexpr int kTmemCols = 2 * BN;  // two accumulators, power of two
   static constexpr int kAccBuffers = MT == 2 ? 1 : 2;
   static constexpr int kEpiStageBytes = AR ? 0 : kEpiBytes;  // staged output path (not used with AR)
   static constexpr int kSmemBytes =
@@ -566,7 +568,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           if (!ok) break;
           uint8_t* sA = smem + stage * Cfg::kStageBytes;
           uint8_t* sB = sA + Cfg::kABytes;
-          mbar_expect_tx(&full[stage], Cfg::kStageBytes);
+          mbar_expect_tx(&full[stage], p.a_bytes + (B_MN ? Cfg::kBBytes : BN * kBK * 2));
           if (!A_MN) {
             tma_load_2d(sA, &tmA, &full[stage], kb * kBK, m0);
           } else {
@@ -578,7 +580,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             tma_load_2d(sB, &tmB, &full[stage], kb * kBK, n0);
           } else {
 #pragma unroll
-            for (int c = 0; c < BN / 64; ++c)
+            for (int c = 0; c < (BN + 63) / 64; ++c)
               tma_load_2d(sB + c * (kBK * 128), &tmB, &full[stage], n0 + c * 64, kb * kBK);
           }
           if (++stage == S) { stage = 0; phase ^= 1; }
@@ -1834,16 +1836,18 @@ static bool g_ar_exchange = false;     // one-hop exchange instead of reduce-sca
 
 // `forced` is a tile code (tile_choice.h), 0: by the model.
 static int pick_tile(int M, int N, int K, bool b_mn, bool second, int forced, bool allow_256x256,
-                     bool allow_pair, bool allow_cut, bool allow_split) {
-  if (forced == 64 || forced == 128 || forced == 256 || forced >= kSplitCode) return forced;
+                     bool allow_pair, bool allow_cut, bool allow_small) {
+  if (forced == 32 || forced == 64 || forced == 128 || forced == 256 || forced >= kSplitCode) return forced;
   if (forced == 512) return allow_256x256 ? 512 : 256;
   if (forced == 1128 || forced == 1256) return allow_pair ? forced : forced - 1000;
   if (forced == 1192 || forced == 1224) return allow_pair ? forced : 256;
   float time;
   const int code = choose_tile(M, N, K, b_mn, second, allow_256x256, allow_pair && g_pair_default, allow_cut, num_sms(),
                                &time);
-  const int split = allow_split ? choose_split(M, N, K, time, num_sms()) : 0;
-  return split ? split : code;
+  if (!allow_small) return code;
+  const bool narrow = choose_narrow(M, N, K, code, num_sms(), &time);
+  const int split = choose_split(M, N, K, time, num_sms());
+  return split ? split : narrow ? 32 : code;
 }
 
 }  // namespace tp
@@ -1887,11 +1891,14 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   if (parts && (a_mn || out_f32 || (tile_code != 64 && tile_code != 128) || parts > kMaxSplit ||
                 (parts & (parts - 1)) || (K + kSplitBK - 1) / kSplitBK < parts))
     return kErrBadArgument;
+  if (tile_code == 32 && (a_mn || out_f32)) return kErrBadArgument;
   const bool pair = tile_code > 1000;
   const int BN = pair ? tile_code - 1000 : (tile_code == 512 ? 256 : tile_code);
   const int BM = (pair || tile_code == 512) ? 256 : kBM;   // rows of one output tile
-  // rows of A one CTA loads
-  const int box_m = parts ? (M < kBM ? (M + 7) / 8 * 8 : kBM) : pair ? kBM : BM;
+  // Rows of A one CTA loads; of a lone tile only those that exist, in eights: the others would be filled with zeros,
+  // which takes the tile load longer than reading them (rows of the product do not mix, and what the MMA
+  // finds in the other rows gives rows that are not stored).
+  const int box_m = M < kBM && !pair && !a_mn ? (M + 7) / 8 * 8 : pair || parts ? kBM : BM;
   const int box_n = pair ? BN / 2 : BN;                    // rows of B one CTA loads
   CUtensorMap tmA, tmB;
   bool ok;
@@ -1927,6 +1934,7 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   p.err = err_flag;
   p.trace = nullptr;
   p.prefetch = g_prefetch;
+  p.a_bytes = (a_mn ? BM : box_m) * kBK * 2;
   if (!parts && !out_f32) {
     // as tiles, where a tensor map can describe them (16-byte addresses and strides)
     auto tile_map = [&](CUtensorMap* m, const void* x, long long ld) {
@@ -1953,7 +1961,9 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
    : tile_code == 512 ? dispatch_layout<T, 256, 2>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)  \
    : BN == 256 ? dispatch_layout<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)            \
    : BN == 128 ? dispatch_layout<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)            \
-               : dispatch_layout<T, 64>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s))
+   : BN == 64 ? dispatch_layout<T, 64>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)              \
+   : b_mn ? launch_gemm<T, 32, false, true, false>(tmA, tmB, tmE, p, s)                       \
+          : launch_gemm<T, 32, false, false, false>(tmA, tmB, tmE, p, s))
   return bf16 ? TP_DISPATCH(__nv_bfloat16) : TP_DISPATCH(__half);
 #undef TP_DISPATCH
 }
@@ -2023,6 +2033,7 @@ extern "C" int tp_gemm_ar(int dtype, int b_mn, const void* A, long long lda, con
   p.err = err_flag;
   p.trace = nullptr;
   p.prefetch = g_prefetch;
+  p.a_bytes = kBM * kBK * 2;
   ArParams ar;
   ar.tp = tp; ar.rank = rank; ar.epoch = epoch; ar.epoch_base = epoch_base; ar.max_tiles = max_tiles;
   ar.exchange = (g_pair_default && g_ar_exchange) ? 1 : 0;

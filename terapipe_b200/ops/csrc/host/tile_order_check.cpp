@@ -49,9 +49,11 @@ int tp_choose_tile(int M, int N, int K, int b_mn, int second, int cut, int sms) 
 
 }  // extern "C"
 
-// The code of a product that ordinary calls split along K, or 0.
-extern "C" int tp_choose_split(int M, int N, int K, int b_mn, int second, int sms) {
+// The tile code of an ordinary forward or data-gradient product: 32 columns and splits along K included.
+extern "C" int tp_choose_small(int M, int N, int K, int b_mn, int second, int sms) {
   float time;
-  tp::choose_tile(M, N, K, b_mn != 0, second != 0, true, true, true, sms, &time);
-  return tp::choose_split(M, N, K, time, sms);
+  const int code = tp::choose_tile(M, N, K, b_mn != 0, second != 0, true, true, true, sms, &time);
+  const bool narrow = tp::choose_narrow(M, N, K, code, sms, &time);
+  const int split = tp::choose_split(M, N, K, time, sms);
+  return split ? split : narrow ? 32 : code;
 }

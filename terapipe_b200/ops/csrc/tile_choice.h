@@ -71,13 +71,26 @@ inline int choose_tile(int M, int N, int K, bool b_mn, bool second, bool allow_2
   return best;
 }
 
+// 32 columns a tile where the tiles of 64 or more leave SMs idle and those of 32 still run at once: a warp's
+// epilogue then is one chunk, and it is most of such a product's time.  us with 64 / 32: 256 x 768 x 256 4.0 / 3.2,
+// 256 x 1024 x 256 with GeLU 5.3 / 3.9, 77 x 3072 x 768 5.5 / 4.8, 128 x 4096 x 1024 6.5 / 5.6; in two rounds
+// 154 x 3072 x 768 takes 7.2 instead of 5.8.  A long K is better shared where it can be (640 x 768 x 3072 9.5, 11.8
+// on 32 columns), so `time` stays what it was there.
+inline bool choose_narrow(int M, int N, int K, int code, int sms, float* time) {
+  if (code != 64 && code != 128) return false;
+  if (static_cast<long long>((M + 127) / 128) * ((N + 31) / 32) > sms) return false;
+  const float t = 8.96f * static_cast<float>(K) / 2048.0f + 1.9f;
+  if (K <= 1024 && t < *time) *time = t;
+  return true;
+}
+
 // Whether a product is better off with K shared by a cluster (gemm_split_kernel): the code, or 0.  `time` is the
 // estimate of choose_tile; the same units here.  A step of 64 of K takes what the MMA needs to read its operands
 // from shared memory, all of them together at least their bytes at 13 TB/s out of L2; what a split pays for is the
 // exchange of the partial sums, which grows with the rows and, where they are many, with the CTAs.  All clusters
 // have to run at once, and an SM group holds few large ones: 36 clusters of 4 take two rounds (16 x 2304 x 768 7.9 us
 // instead of 4.3 in 36 pairs), 16 of 8 as well (32 x 1024 x 4096 10.0, 16 of 4 6.3).  us without / with:
-//   77 x 768 x 768 5.5 / 4.5 (4 parts of 64 columns), 77 x 768 x 3072 12.3 / 5.9 (8), 256 x 256 x 1024 6.2 / 5.5 (4),
+//   77 x 768 x 3072 12.3 / 5.9 (8 parts of 64 columns), 16 x 768 x 768 4.7 / 4.1 (4),
 //   128 x 1024 x 4096 15.4 / 7.7 (4), 128 x 2048 x 8192 27.6 / 11.4 (4), 16 x 8192 x 2048 16.5 / 7.5 (2 of 128
 //   columns), 64 x 4096 x 16384 52.6 / 27.9 (4 of 128), 256 x 2048 x 8192 27.9 / 16.3 (2 of 64).
 inline int choose_split(int M, int N, int K, float time, int sms) {

@@ -75,8 +75,8 @@ def host_lib() -> ctypes.CDLL:
                       c_void_p]
         _host.tp_choose_tile.restype = c_int
         _host.tp_choose_tile.argtypes = [c_int] * 7
-        _host.tp_choose_split.restype = c_int
-        _host.tp_choose_split.argtypes = [c_int] * 6
+        _host.tp_choose_small.restype = c_int
+        _host.tp_choose_small.argtypes = [c_int] * 6
         _host.tp_ln_bwd_geometry.restype = c_int
         _host.tp_ln_bwd_geometry.argtypes = [c_int, c_int, c_int, c_void_p]
     return _host

@@ -4,7 +4,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-TILES = (64, 128, 256, 512, 1128, 1192, 1224, 1256)
+TILES = (32, 64, 128, 256, 512, 1128, 1192, 1224, 1256)
 
 
 def _check(M, N, K, code, dtype, ld=None, shift=0):

@@ -1,10 +1,10 @@
-"""Products whose K is shared by the CTAs of a cluster."""
+"""Products of few tiles: tiles of 32 columns, and K shared by the CTAs of a cluster."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-CODES = [parts * 10000 + bn for bn in (64, 128) for parts in (1, 2, 4, 8)]
+CODES = [32] + [parts * 10000 + bn for bn in (64, 128) for parts in (1, 2, 4, 8)]
 
 
 def _gelu_grad(z):
@@ -71,7 +71,7 @@ def test_ordinary_calls_split(M, N, K, b_mn):
     """The choice's own codes, against the same product on a one-CTA tile."""
     from terapipe_b200.ops import functional as F
     from terapipe_b200.ops.lib import host_lib
-    assert host_lib().tp_choose_split(M, N, K, int(b_mn), 0, 148) >= 20000
+    assert host_lib().tp_choose_small(M, N, K, int(b_mn), 0, 148) >= 20000
     torch.manual_seed(1)
     a = torch.randn(M, K, device="cuda").half()
     w = (torch.randn(*((K, N) if b_mn else (N, K)), device="cuda") * K ** -0.5).half()

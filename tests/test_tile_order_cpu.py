@@ -70,15 +70,17 @@ def test_all_gather_products_keep_full_widths(M, N, K, b_mn):
 
 @pytest.mark.parametrize("M,N,K,code", [
     # few tiles and a long K: two to eight parts
-    (77, 768, 3072, 80064), (77, 768, 768, 40064), (128, 2048, 8192, 40064), (16, 2048, 8192, 40064),
-    (64, 4096, 16384, 40128), (16, 8192, 2048, 20128), (256, 256, 1024, 40064),
+    (77, 768, 3072, 80064), (16, 768, 768, 40064), (128, 2048, 8192, 40064), (16, 2048, 8192, 40064),
+    (64, 4096, 16384, 40128), (16, 8192, 2048, 20128), (256, 256, 4096, 80064),
     # clusters that would not all run at once: fewer parts
-    (16, 2304, 768, 40128), (32, 1024, 4096, 40064), (300, 768, 3072, 20064),
-    # short K, enough tiles, or operands that take longer to fetch twice
-    (256, 256, 256, 0), (128, 15360, 5120, 0), (1024, 2048, 8192, 0), (256, 4096, 16384, 0), (16384, 2048, 8192, 0)])
-def test_split_choice(M, N, K, code):
+    (32, 1024, 4096, 40064), (300, 768, 3072, 20064),
+    # 32 columns where these tiles run at once
+    (256, 256, 256, 32), (77, 768, 768, 32), (77, 3072, 768, 32), (128, 4096, 1024, 32), (154, 3072, 768, 64),
+    # enough tiles, or operands that take longer to fetch twice
+    (128, 15360, 5120, 128), (1024, 2048, 8192, 1128), (640, 768, 3072, 20064), (16384, 2048, 8192, 1256)])
+def test_small_products(M, N, K, code):
     from terapipe_b200.ops.lib import host_lib
-    assert host_lib().tp_choose_split(M, N, K, 0, 0, 148) == code
+    assert host_lib().tp_choose_small(M, N, K, 0, 0, 148) == code
 
 
 def test_a_split_runs_at_once():
@@ -87,8 +89,10 @@ def test_a_split_runs_at_once():
     for M in (1, 16, 77, 128, 129, 300, 1000):
         for N in (8, 64, 256, 768, 2048, 5120, 12288):
             for K in (8, 128, 256, 1000, 4096, 49152):
-                code = host_lib().tp_choose_split(M, N, K, 0, 0, 148)
-                if code:
-                    parts, bn = divmod(code, 10000)
+                code = host_lib().tp_choose_small(M, N, K, 0, 0, 148)
+                parts, bn = divmod(code, 10000)
+                if code == 32:
+                    assert -(-M // 128) * -(-N // 32) <= 148
+                if parts:
                     assert parts in (2, 4, 8) and bn in (64, 128) and parts <= -(-K // 128)
                     assert -(-M // 128) * -(-N // bn) * parts <= {2: 148, 4: 128, 8: 96}[parts]
