@@ -45,6 +45,10 @@ __device__ __forceinline__ void pdl_wait(bool trigger = true) {
   if (trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Instead of pdl_wait(), in a kernel that reads nothing its predecessor writes and writes nothing that it touches,
+// where the predecessor's CTAs run only after everything before them is done: the kernel starts
+// once they all run, and pdl_wait(false) in one of its threads at its end makes whoever waits for it
+// wait for both.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ bool elect_one() {

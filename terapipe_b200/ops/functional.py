@@ -183,7 +183,7 @@ def _wgrad_args(dy, x, out):
 def weight_grad(dy, x, out, accumulate=False):
     """``out[l] (+)= dy[l]^T @ x[l]`` (fp32) for every layer: the weight gradients of one kind of a stage."""
     operands, sizes = _wgrad_args(dy, x, out)
-    st = cuda_lib().tp_wgrad(*operands, out.data_ptr(), *sizes, int(accumulate), _status_ptr(dy),
+    st = cuda_lib().tp_wgrad(*operands, out.data_ptr(), *sizes, int(accumulate), 0, _status_ptr(dy),
                              _stream())
     check(st, "tp_wgrad")
     return out
@@ -198,7 +198,7 @@ def weight_grad_adam(dy, x, master, m, v, model, state, lr, beta1=0.9, beta2=0.9
         assert t.shape == master.shape and t.stride() == master.stride()
     st = cuda_lib().tp_wgrad_adam(*operands, master.data_ptr(), m.data_ptr(), v.data_ptr(), model.data_ptr(), *sizes,
                                   state.data_ptr(), lr, beta1, beta2, eps, weight_decay, grad_scale,
-                                  _status_ptr(dy), _stream())
+                                  0, _status_ptr(dy), _stream())
     check(st, "tp_wgrad_adam")
 
 

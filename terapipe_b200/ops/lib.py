@@ -98,8 +98,8 @@ SIGNATURES = {
     "tp_adam_tick": [P, F, F, P],
     "tp_fused_adam": [I, P, P, P, P, P, L, P, F, F, F, F, F, F, P],
     "tp_fused_adam_ranges": [I, P, P, P, P, P, I, P, P, I, L, P, F, F, F, F, F, F, P],
-    "tp_wgrad": [I, P, L, L, P, L, L, P, L, L, I, I, I, I, I, P, P],
-    "tp_wgrad_adam": [I, P, L, L, P, L, L, P, P, P, P, L, L, I, I, I, I, P, F, F, F, F, F, F, P, P],
+    "tp_wgrad": [I, P, L, L, P, L, L, P, L, L, I, I, I, I, I, I, P, P],
+    "tp_wgrad_adam": [I, P, L, L, P, L, L, P, P, P, P, L, L, I, I, I, I, P, F, F, F, F, F, F, I, P, P],
     "tp_stage_sums": [I, I, P, P, P, P, I, I, P, I, I, P, P, I, P, L, L, I, P],
     "tp_fill": [I, P, L, F, P],
     "tp_gemm_ar": [I, I, P, L, P, L, L, I, I, I, P, P, L, I, I, I, P, I, P, P, P, P, P, P],

@@ -521,9 +521,9 @@ class StageEngine:
         if st:
             F.check(st, "tp_gemm")
 
-    def _wgrad(self, dy, M, x, N, l, n, name, mode):
+    def _wgrad(self, dy, M, x, N, l, n, name, mode, follows):
         """``dW = dy^T x`` over all rows for layers ``[l, l + n)``: ``mode`` "add" to or "assign" the gradient, or
-        "update" the weight ``name`` with it."""
+        "update" the weight ``name`` with it.  ``follows``: the call before this one was another product's."""
         R = self.rows
         operands = (self.dt, dy[l].data_ptr(), M, R * M, x[l].data_ptr(), N, R * N)
         sizes = (N, self.layout.layer_stride, n, M, N, R)
@@ -531,10 +531,10 @@ class StageEngine:
             st = self.lib.tp_wgrad_adam(*operands, self._p(l, name, self.master), self._p(l, name, self.exp_avg),
                                         self._p(l, name, self.exp_avg_sq), self._p(l, name), *sizes,
                                         self.adam_state.data_ptr(), self.lr, 0.9, 0.999, 1e-8, 0.0,
-                                        1.0 / (self.loss_scale * self.dp), self._status_ptr, self._stream)
+                                        1.0 / (self.loss_scale * self.dp), int(follows), self._status_ptr, self._stream)
         else:
             st = self.lib.tp_wgrad(*operands, self._p(l, name, self.grad), *sizes, int(mode == "add"),
-                                   self._status_ptr, self._stream)
+                                   int(follows), self._status_ptr, self._stream)
         if st:
             F.check(st, "tp_wgrad")
 
@@ -910,7 +910,7 @@ class StageEngine:
             for dy, M, x, N, name in ((self.dXo, H, self.fa, Fl, "fc2.weight"), (self.dFc, Fl, self.ln2, H, "fc1.weight"),
                                       (self.dMid, H, self.ao, Hl, "attn.out_proj.weight"),
                                       (self.dQKV, 3 * Hl, self.ln1, H, "attn.in_proj.weight")):
-                self._wgrad(dy, M, x, N, l, n, name, mode)
+                self._wgrad(dy, M, x, N, l, n, name, mode, dy is not self.dXo)
             slots = self.ln_slots[l].data_ptr()
             # all bias gradients (column sums of the same dY) and, unless the ranks' sums have to be
             # added up first, the LayerNorm gradients: one launch

@@ -47,3 +47,35 @@ def test_attention_backward_in_a_row(b, h, D, L, t, c, set_pdl):
         F.check_device_status()
         out.append(torch.cat([x.view(-1) for x in outs + [dqkv]]))
     assert not out[0].isnan().any() and torch.equal(out[0], out[1])
+
+
+# all four products on the chip at once, one wave each, several; gradients added and assigned, weights updated
+@pytest.mark.parametrize("layers,H,heads,L", [(1, 128, 2, 40), (3, 256, 4, 512), (2, 1024, 16, 136), (5, 1600, 25, 64)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_weight_gradients_in_a_row(layers, H, heads, L, dtype, set_pdl):
+    from terapipe_b200.models import TransformerConfig
+    from terapipe_b200.runtime.engine import StageEngine
+    cfg = TransformerConfig(batch_size=2, seq_len=L, n_layers=layers, embedding_dim=H, num_attention_heads=heads,
+                            n_devices=1)
+    gen = torch.Generator(device="cuda").manual_seed(H + L)
+    xs = [torch.randn(L, 2, H, device="cuda", generator=gen).to(dtype) for _ in range(4)]
+    out = []
+    for pdl in (0, 1):
+        set_pdl(pdl)
+        eng = StageEngine(cfg, [2], [L], dtype=dtype, use_graph=False, lr=1e-3, loss_scale=1024.0)
+        got = []
+        eng.set_input(xs[0])
+        eng.step()
+        torch.cuda.synchronize()
+        torch.cuda._sleep(3_000_000)       # the launches below queue up behind it
+        for x in xs:
+            eng.set_input(x)
+            eng.compute_grads()            # assigned
+            got.append(eng.grad.clone())
+            eng.step()                     # added to those, which the next product's weights come from
+            eng.step()                     # weights updated in the products
+            got += [eng.master.clone(), eng.exp_avg_sq.clone(), eng.model.clone().float(), eng.grad.clone()]
+        eng.check_status()
+        out.append(got)
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+    assert out[0][0].abs().max() > 0 and not any(t.isnan().any() for t in out[0])
