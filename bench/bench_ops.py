@@ -52,7 +52,7 @@ def _rel(a, b):
 
 def case_gemm(a):
     """Layer GEMMs of one token slice.  ``--tile`` takes a comma list of tile codes to force
-    (0 = automatic choice, 64/128/256 = one CTA with a 128 x BN tile, 512 = one CTA 256 x 256,
+    (0 = automatic choice, 32/64/128/256 = one CTA with a 128 x BN tile, 512 = one CTA 256 x 256,
     1128/1256 = CTA pair with a 256 x 128 / 256 x 256 tile); every forced run is also checked
     against torch."""
     dt, dev, H, T = a.dtype, "cuda", a.hidden, a.tokens

@@ -4,7 +4,7 @@
 
 namespace tp {
 
-// Codes: 64 / 128 / 256 = one CTA, 128 x BN tile; 512 = one CTA, 256 x 256; 1000 + BN = CTA pair,
+// Codes: 32 / 64 / 128 / 256 = one CTA, 128 x BN tile; 512 = one CTA, 256 x 256; 1000 + BN = CTA pair,
 // 256 x BN (BN = 128, 192, 224, 256).  Measured model of one launch, in kilo-cycles: waves x (main
 // loop of one tile, proportional to K, + epilogue where it does not overlap the next tile) + exposed
 // epilogue of the last tile.  Wave quantisation matters because M is only ~1024 rows per token slice.
