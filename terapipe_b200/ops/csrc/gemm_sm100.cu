@@ -1283,7 +1283,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     fence_barrier_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
-    prefetch_tmap(&tmE.out);
+    if (!AR) prefetch_tmap(&tmE.out);   // (all-reduce: stores through peer pointers, the maps stay empty)
   }
   if (TILES && warp >= 2 && lane < kEpiBufs16) {
     mbar_init(&epi_bars[(warp - 2) * kEpiBufs16 + lane], 1);
