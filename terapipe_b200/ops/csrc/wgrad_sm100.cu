@@ -344,6 +344,11 @@ static int wgrad(int dtype, const void* A, long long lda, long long a_stride, co
       (p.layer_stride % 8) || lda < p.M || ldb < p.N || p.ldo < p.N)
     return kErrBadArgument;
   if (p.layers > 1 && (a_stride < p.M || b_stride < p.N)) return kErrBadArgument;
+  // no two layers write the same element: whole matrices apart, or side by side in the rows of a wider one
+  const long long ends = (p.M - 1) * p.ldo + p.N;
+  if (p.layers > 1 && p.layer_stride < ends &&
+      (p.layer_stride < p.N || (p.layers - 1) * p.layer_stride + p.N > p.ldo))
+    return kErrBadArgument;
   const uintptr_t out = ADAM ? reinterpret_cast<uintptr_t>(p.adam.p) | reinterpret_cast<uintptr_t>(p.adam.m) |
                                    reinterpret_cast<uintptr_t>(p.adam.v) | reinterpret_cast<uintptr_t>(p.adam.model)
                              : reinterpret_cast<uintptr_t>(p.grad);

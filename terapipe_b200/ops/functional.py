@@ -170,13 +170,19 @@ def fused_adam(grad, master, m, v, model, state, lr, beta1=0.9, beta2=0.999, eps
 
 
 def _wgrad_args(dy, x, out):
-    """``[layers, rows, width]`` operands and ``[layers, M, N]`` output (or one layer without the dimension)."""
+    """``[layers, rows, width]`` operands and ``[layers, M, N]`` fp32 output (or one layer without the dimension).
+    The kernel reads ``x`` as ``dy``'s type and stores fp32, whatever the tensors are: other types end here."""
+    dtype = _dt(dy)
+    if x.dtype != dy.dtype:
+        raise KernelError(f"operands of one type: {dy.dtype} and {x.dtype}")
+    if out.dtype != torch.float32:
+        raise KernelError(f"weight gradients and their optimizer state are float32, not {out.dtype}")
     dy, x, out = (t if t.dim() == 3 else t.unsqueeze(0) for t in (dy, x, out))
     n, K, M = dy.shape
     N = x.shape[2]
     assert x.shape[:2] == (n, K) and out.shape == (n, M, N)
     assert dy.stride(2) == 1 and x.stride(2) == 1 and out.stride(2) == 1
-    return (_dt(dy), dy.data_ptr(), dy.stride(1), dy.stride(0), x.data_ptr(), x.stride(1), x.stride(0)), \
+    return (dtype, dy.data_ptr(), dy.stride(1), dy.stride(0), x.data_ptr(), x.stride(1), x.stride(0)), \
            (out.stride(1), out.stride(0), n, M, N, K)
 
 
@@ -194,7 +200,9 @@ def weight_grad_adam(dy, x, master, m, v, model, state, lr, beta1=0.9, beta2=0.9
     """:func:`weight_grad` and :func:`fused_adam` in one kernel: the gradients of the ``[layers, M, N]`` matrices
     ``master``/``m``/``v``/``model`` are not stored."""
     operands, sizes = _wgrad_args(dy, x, master)
-    for t in (m, v, model):
+    for t, dtype in ((m, torch.float32), (v, torch.float32), (model, dy.dtype)):
+        if t.dtype != dtype:
+            raise KernelError(f"moments are float32 and the model copy is the operands' type, not {t.dtype}")
         assert t.shape == master.shape and t.stride() == master.stride()
     st = cuda_lib().tp_wgrad_adam(*operands, master.data_ptr(), m.data_ptr(), v.data_ptr(), model.data_ptr(), *sizes,
                                   state.data_ptr(), lr, beta1, beta2, eps, weight_decay, grad_scale,
@@ -204,7 +212,15 @@ def weight_grad_adam(dy, x, master, m, v, model, state, lr, beta1=0.9, beta2=0.9
 
 def fused_adam_ranges(grad, master, m, v, model, state, ranges, layers: int, layer_stride: int, lr,
                       beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0, grad_scale=1.0):
-    """:func:`fused_adam` on the ranges ``[(begin, length), ...]`` of every layer of the flat buffers."""
+    """:func:`fused_adam` on the ranges ``[(begin, length), ...]`` of every layer of the flat buffers.  The ranges
+    lie inside the buffers, and one layer's before the next one's."""
+    if any(t.dtype != torch.float32 for t in (grad, master, m, v, state)):
+        raise KernelError("gradients, optimizer state and step state are float32")
+    if ranges and layers > 0:
+        lo, hi = min(r[0] for r in ranges), max(r[0] + r[1] for r in ranges)
+        end = hi + (layers - 1) * layer_stride
+        if lo < 0 or end > min(t.numel() for t in (grad, master, m, v, model)) or (layers > 1 and layer_stride < hi - lo):
+            raise KernelError(f"ranges [{lo}, {hi}) of {layers} layers, {layer_stride} apart, do not fit the buffers")
     LL = ctypes.c_longlong * len(ranges)
     st = cuda_lib().tp_fused_adam_ranges(_dt(model), grad.data_ptr(), master.data_ptr(), m.data_ptr(),
                                          v.data_ptr(), model.data_ptr(), len(ranges), LL(*[r[0] for r in ranges]),
