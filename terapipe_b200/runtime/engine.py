@@ -1104,6 +1104,8 @@ class StageEngine:
         else:
             if mode == "update" and self._plan is not None:
                 F.adam_tick(self.adam_state)
+                # the products' calls hold the optimizer's numbers, which may change from step to step
+                self._plan.expect(("weight_grads", mode), (self.lr, self.loss_scale))
             self._segment(("weight_grads", mode), self._weight_grads, mode)
         for w in sends:
             w.wait()

@@ -57,19 +57,27 @@ class RecordingLibrary:
 class SegmentCache:
     """``run(key, fn, *args)``: the first time, call ``fn(*args)`` while recording the library
     calls it makes; later, replay them.  ``token`` guards the recordings: when it changes (for
-    example the launch stream), everything is recorded afresh."""
+    example the launch stream), everything is recorded afresh.  :meth:`expect` does that for one
+    segment, whose calls hold values that the others' do not."""
 
     def __init__(self, lib: RecordingLibrary, on_error: Optional[Callable[[int, str], None]] = None):
         self.lib = lib
         self.on_error = on_error
         self.segments: Dict[Hashable, Segment] = {}
         self.token: Any = None
+        self.values: Dict[Hashable, Any] = {}
         self.replayed = 0
 
     def validate(self, token) -> None:
         if token != self.token:
             self.segments.clear()
             self.token = token
+
+    def expect(self, key: Hashable, values: Any) -> None:
+        """Before :meth:`run`: forget segment ``key`` if it was recorded with other ``values``."""
+        if self.values.setdefault(key, values) != values:
+            self.segments.pop(key, None)
+            self.values[key] = values
 
     def run(self, key: Hashable, fn: Callable[..., Any], *args) -> None:
         seg = self.segments.get(key)
