@@ -309,6 +309,12 @@ layernorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
 // memory, so the sums do not depend on timing.  V = 32 reads longer pieces of a row and V = 8 makes four
 // times as many CTAs of them; layer_sums_launch has the line between them.  (One launch per matrix with
 // one load in flight per thread ran on 64 of 148 SMs: 16384 x 2048 alone took 63 us.)
+//
+// LAYERS: several layers, blockIdx.y; a single one does without their strides, which cost it 0.1 us.  The chunk's
+// address is hidden from the compiler: left to fold it into the loads' own it took 72 registers for bf16 layers, three
+// CTAs an SM where the launch counts on four, and slower loops for the others.  us folded / hidden: one matrix of
+// 16384 x 8192 51.7 / 48.6 (bf16 58.3 / 48.4), 8192 x 768 5.8 / 5.3; all four of 5 layers of 2048 columns, 16384 rows,
+// 515 / 438 (bf16 500 / 439), 4 of 1600, 5120 rows, 110 / 102 (bf16 145 / 103).
 constexpr int kMaxColsums = 4, kMaxFolds = 2;
 struct SumJobs {
   const void* dy[kMaxColsums];
@@ -321,7 +327,7 @@ struct SumJobs {
   float* dgamma[kMaxFolds];
   float* dbeta[kMaxFolds];
   int folds, parts, H;           // the CTAs behind the matrices' fold 32 columns each
-  // blockIdx.y = layer: elements from a layer's matrices, slots and sums to the next's
+  // LAYERS: elements from a layer's matrices, slots and sums to the next's
   long long dy_stride[kMaxColsums], slot_stride, out_stride;
   int overwrite;                 // the sums replace what the gradients hold
 };
@@ -368,7 +374,7 @@ __global__ void layernorm_bwd_reduce_kernel(float* __restrict__ scratch, int par
   fold_slots(scratch, parts, H, blockIdx.x * 32, dgamma, dbeta, threadIdx.x, threadIdx.y, clear, sm);
 }
 
-template <typename T, int V>
+template <typename T, int V, bool LAYERS>
 __global__ void __launch_bounds__(256)
 layer_sums_kernel(const SumJobs j) {
   constexpr int kCols = 8 * V, kRows = 256 / V;   // columns of a CTA, rows of one load
@@ -376,6 +382,7 @@ layer_sums_kernel(const SumJobs j) {
   __shared__ float chunk_sum[kCols];
   const int tid = threadIdx.x, vec = tid % V, lane_row = tid / V;
   const int cta = blockIdx.x;
+  const long long layer = LAYERS ? blockIdx.y : 0;
   pdl_wait();
   int first = 0;
 #pragma unroll
@@ -387,7 +394,8 @@ layer_sums_kernel(const SumJobs j) {
       const int r_end = min(j.rows, (chunk + 1) * j.rows_per_chunk);
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       if (col < j.N[i]) {
-        const T* src = static_cast<const T*>(j.dy[i]) + blockIdx.y * j.dy_stride[i] + col;
+        const T* src = static_cast<const T*>(j.dy[i]) + layer * j.dy_stride[i] + col;
+        asm("" : "+l"(src));
         for (int r = chunk * j.rows_per_chunk + lane_row; r < r_end; r += 8 * kRows) {
           uint4 v[8];
 #pragma unroll
@@ -426,7 +434,7 @@ layer_sums_kernel(const SumJobs j) {
         if (chunk != 0) return;
       }
       if (tid < kCols && col0 + tid < j.N[i]) {
-        float* db = j.db[i] + blockIdx.y * j.out_stride + col0 + tid;
+        float* db = j.db[i] + layer * j.out_stride + col0 + tid;
         *db = j.overwrite ? s : *db + s;
       }
       return;
@@ -436,8 +444,8 @@ layer_sums_kernel(const SumJobs j) {
   const int per_fold = (2 * j.H + 31) / 32;
   const int f = (cta - first) / per_fold;
   if (f >= j.folds) return;        // (the grid is a whole number of clusters)
-  fold_slots(j.slots[f] + blockIdx.y * j.slot_stride, j.parts, j.H, (cta - first) % per_fold * 32,
-             j.dgamma[f] + blockIdx.y * j.out_stride, j.dbeta[f] + blockIdx.y * j.out_stride,
+  fold_slots(j.slots[f] + layer * j.slot_stride, j.parts, j.H, (cta - first) % per_fold * 32,
+             j.dgamma[f] + layer * j.out_stride, j.dbeta[f] + layer * j.out_stride,
              tid & 31, tid >> 5, j.overwrite ? 3 : 1, sm.fold);
 }
 
@@ -707,11 +715,12 @@ static int layer_sums_launch(int dtype, SumJobs& j, int layers, cudaStream_t s) 
   const int cols = wide ? 256 : 64, round = 8 * 256 / (cols / 8);   // rows of one round of loads
   // Chunks of at least one round, a portable cluster of them at most; with V = 32 no more than 4 CTAs per
   // SM, which run at once (2560-wide layer, 16384 rows: 156 us with 8 chunks a block, 131 with 4;
-  // 5120-wide, 1024 rows: 28.6 with 8, 21.8 with 2), unless even two chunks take several rounds.
+  // 5120-wide, 1024 rows: 28.6 with 8, 21.8 with 2), unless even two chunks are too many for five per SM, which
+  // still run at once (360 blocks of 16384 rows: 435 us with 2, 477 with 4).
   int most = 8;
   if (wide) {
     while (most > 2 && blocks * most > 4 * num_sms()) most /= 2;
-    if (blocks * most > 4 * num_sms()) most = 4;
+    if (blocks * most > 5 * num_sms()) most = 4;
   }
   j.chunks = 1;
   while (j.n > 0 && j.chunks < most && j.rows >= 2 * round * j.chunks) j.chunks *= 2;
@@ -726,13 +735,12 @@ static int layer_sums_launch(int dtype, SumJobs& j, int layers, cudaStream_t s) 
   ctas = (ctas + j.chunks - 1) / j.chunks * j.chunks;
   if (ctas > 0x7fffffffLL) return kErrTooLarge;
   const dim3 grid(static_cast<unsigned>(ctas), static_cast<unsigned>(layers)), block(256);
-  cudaError_t e;
-  if (dtype == 1)
-    e = wide ? launch_pdl(layer_sums_kernel<__nv_bfloat16, 32>, grid, block, 0, s, j.chunks, j)
-             : launch_pdl(layer_sums_kernel<__nv_bfloat16, 8>, grid, block, 0, s, j.chunks, j);
-  else
-    e = wide ? launch_pdl(layer_sums_kernel<__half, 32>, grid, block, 0, s, j.chunks, j)
-             : launch_pdl(layer_sums_kernel<__half, 8>, grid, block, 0, s, j.chunks, j);
+#define TP_SUMS(T, LAYERS)                                                                  \
+  (wide ? launch_pdl(layer_sums_kernel<T, 32, LAYERS>, grid, block, 0, s, j.chunks, j)      \
+        : launch_pdl(layer_sums_kernel<T, 8, LAYERS>, grid, block, 0, s, j.chunks, j))
+  const cudaError_t e = dtype == 1 ? (layers > 1 ? TP_SUMS(__nv_bfloat16, true) : TP_SUMS(__nv_bfloat16, false))
+                                   : (layers > 1 ? TP_SUMS(__half, true) : TP_SUMS(__half, false));
+#undef TP_SUMS
   return e == cudaSuccess ? kOk : kErrLaunch;
 }
 }  // namespace tp
@@ -771,7 +779,7 @@ extern "C" int tp_stage_sums(int dtype, int n, const void* const* dy, const long
   return layer_sums_launch(dtype, j, layers, static_cast<cudaStream_t>(stream));
 }
 
-// The same for one layer, added to the gradients.
+// The same for one layer, added to the gradients (for callers that have the layers' matrices in buffers of their own).
 extern "C" int tp_layer_sums(int dtype, int n, const void* const* dy, const long long* ld, const int* N,
                              float* const* db, int rows, int folds, float* const* slots, int parts, int H,
                              float* const* dgamma, float* const* dbeta, void* stream) {
