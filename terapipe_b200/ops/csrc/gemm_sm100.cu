@@ -70,7 +70,7 @@ struct GemmParams {
   int prefetch;      // CTA-pair kernel: operand tiles are prefetched into L2 this many k-steps
                      // ahead of the loads that fill the ring (0 = off)
   int a_bytes;       // one-CTA kernel: of A in a stage (fewer where M < 128)
-  int mat_tma;       // the residual, or else aux_in, comes as tiles (EpiMaps::mat)
+  int mat_tma;       // AHEAD kernels: the residual, or else aux_in, comes as tiles (EpiMaps::mat)
 };
 
 constexpr int kMaxTp = 8;
@@ -208,8 +208,8 @@ __device__ __forceinline__ long long clock_ordered() {
   return t;
 }
 
-// A second matrix of the output's size, the residual or the argument of the activation's derivative, comes the same
-// way (16-bit output): as a tile load into the very buffer that the chunk's result then leaves from, two chunks
+// In AHEAD kernels a second matrix of the output's size, the residual or the argument of the activation's derivative,
+// comes the same way (16-bit output): as a tile load into the very buffer that the chunk's result then leaves from, two chunks
 // ahead, a tile's first two under its main loop.  With 16-byte loads of 32 rows an instruction it bound products with
 // a short K; us before / now, 8192 rows: 3072 x 768 with ReLU's derivative 80 / 49, with GeLU's 82 / 60, 768 x 3072
 // with a residual 41 / 36; 2048 x 6400 x 1600 with ReLU's derivative 47 / 36, 4096 x 2048 x 2048 with a residual
@@ -224,7 +224,8 @@ struct EpiMaps {
 };
 constexpr int kEpiBufs16 = 4, kEpiBuf16Bytes = 2048;
 
-// The bias of columns [n, n + 32), fetched a chunk ahead: a short product's epilogue waited 400 to 800 cycles for it.
+// The bias of columns [n, n + 32); AHEAD kernels fetch it a chunk early: a short product's epilogue waited 400 to 800
+// cycles for it.
 template <typename T>
 __device__ __forceinline__ void epi_bias(const GemmParams& p, uint4 (&bv)[4], int n) {
   if (!p.bias) return;
@@ -252,9 +253,9 @@ __device__ __forceinline__ void epi_drain(int lane) {
 // Fused epilogue of one 32-column chunk: r holds the fp32 accumulators of columns [n, n + 32)
 // of row `row` (thread = row).  row0 is the first row of the warp's 32-row group (row0 < M);
 // the caller has checked n < N.  t_next: TMEM address of the next chunk to load into r, or 0.  Rows >= M and columns >= N are clipped by the tile store.
-// bv: the bias of these columns, and at the end of those from n_next on (-1: none).  TILES: the other matrix may come
-// as tiles (p.mat_tma); n_ahead: the chunk two further on, or -1.
-template <typename T, bool OUT_F32, bool TRACE = false, bool TILES = false>
+// AHEAD: bv holds the bias of these columns, and at the end of those from n_next on (-1: none); the residual, or else
+// aux_in, comes as tiles (p.mat_tma); n_ahead: the chunk two further on, or -1.
+template <typename T, bool OUT_F32, bool TRACE = false, bool AHEAD = false>
 __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMaps& tm,
                                                EpiStage& es, const WaitCtx& wctx, uint32_t (&r)[32], uint4 (&bv)[4], long long row,
                                                bool row_ok, int n, int row0, int lane,
@@ -262,22 +263,22 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMap
                                                const T* part = nullptr, long long part_stride = 0,
                                                int n_src = 0, int self = 0) {
   const long long t_0 = TRACE ? clock_ordered() : 0;
-  // Without tiles every global load of this 32-column chunk is issued before any dependent math or store,
+  // Otherwise every global load of this 32-column chunk is issued before any dependent math or store,
   // so the chunk pays one memory latency instead of one per 8-column group.
   bool gok[4];
 #pragma unroll
   for (int g = 0; g < 4; ++g) gok[g] = n + g * 8 + 8 <= p.N;
-  const bool tiles = TILES && p.mat_tma;
   auto direct = [&](const void* x, long long ld, int g) {
     return gok[g] && row_ok ? __ldcg(reinterpret_cast<const uint4*>(static_cast<const T*>(x) + row * ld + n + g * 8))
                             : make_uint4(0, 0, 0, 0);
   };
   uint4 rv[4], av[4];
-  if (!TILES && p.residual) {
+  if (!AHEAD) epi_bias<T>(p, bv, n);
+  if (!AHEAD && p.residual) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) rv[g] = direct(p.residual, p.ldr, g);
   }
-  if (!TILES && p.dact) {
+  if (!AHEAD && p.dact) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) av[g] = direct(p.aux_in, p.ld_aux, g);
   }
@@ -299,7 +300,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMap
   static_assert(OUT_F32 || kEpiBytesPerWarp == kEpiBufs16 * kEpiBuf16Bytes, "four buffers a warp");
   uint8_t* sb = es.buf + (es.issued % kBufs) * (kEpiBytesPerWarp / kBufs);
   const int sw = (lane >> 1) & 3;      // 64-byte rows, 64-byte swizzle: 16-byte chunk index ^= (row >> 1) & 3
-  if (tiles) {
+  if (AHEAD && p.mat_tma) {
     // (the request waited for the buffer's last store)
     mbar_wait(&es.bars[es.issued % kBufs], (es.issued / kBufs) & 1, wctx, kErrWaitEpilogue);
     __syncwarp();
@@ -389,7 +390,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMap
   if (p.residual) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      const uint4 r4 = !TILES ? rv[g] : tiles ? tile(g) : direct(p.residual, p.ldr, g);
+      const uint4 r4 = AHEAD ? tile(g) : rv[g];
       const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -402,7 +403,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMap
   if (p.dact) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      const uint4 a4 = !TILES ? av[g] : tiles && !p.residual ? tile(g) : direct(p.aux_in, p.ld_aux, g);
+      const uint4 a4 = !AHEAD ? av[g] : p.residual ? direct(p.aux_in, p.ld_aux, g) : tile(g);
       const uint32_t aw[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -418,7 +419,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMap
       }
     }
   }
-  if (n_next >= 0) epi_bias<T>(p, bv, n_next);
+  if (AHEAD && n_next >= 0) epi_bias<T>(p, bv, n_next);
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     if (OUT_F32) {
@@ -445,7 +446,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMap
     else tma_store_2d(&tm.out, sb, n, row0);
     bulk_commit();
   }
-  if (tiles && n_ahead >= 0) epi_request(&tm.mat, es, es.issued + 2, n_ahead, row0, lane);
+  if (AHEAD && p.mat_tma && n_ahead >= 0) epi_request(&tm.mat, es, es.issued + 2, n_ahead, row0, lane);
   ++es.issued;
   if (TRACE) {
     cyc[0] += t_1 - t_0;        // loads issued, staging buffer free
@@ -461,7 +462,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const EpiMap
 // The chunk code exists once (it is large); the TMEM
 // load of chunk c + 1 is issued from inside it as soon as chunk c's values have been copied out
 // of the load registers.
-template <typename T, bool OUT_F32, bool TRACE = false, bool TILES = false>
+template <typename T, bool OUT_F32, bool TRACE = false, bool AHEAD = false>
 __device__ __forceinline__ void epilogue_rows(const GemmParams& p, const EpiMaps& tm,
                                               EpiStage& es, const WaitCtx& wctx, uint4 (&bv)[4], uint32_t t_acc,
                                               int nc, int row0, int n0, int lane, int c_first = 0, int c_step = 1,
@@ -476,7 +477,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, const EpiMaps
 #pragma unroll 1
   for (int c = c_first; c < nc; c += c_step) {
     tmem_ld_wait();
-    epilogue_chunk<T, OUT_F32, TRACE, TILES>(p, tm, es, wctx, r, bv, row, row_ok, n0 + c * 32, row0, lane,
+    epilogue_chunk<T, OUT_F32, TRACE, AHEAD>(p, tm, es, wctx, r, bv, row, row_ok, n0 + c * 32, row0, lane,
                                              c + c_step < nc ? t_acc + (c + c_step) * 32 : 0u,
                                              c + c_step < nc ? n0 + (c + c_step) * 32 : -1,
                                              c + 2 * c_step < nc ? n0 + (c + 2 * c_step) * 32 : -1, cyc,
@@ -484,18 +485,18 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, const EpiMaps
   }
 }
 // What the first of these chunks need (any time after the last chunk before them): the bias, two tiles.
-template <typename T, bool TILES>
+template <typename T, bool AHEAD>
 __device__ __forceinline__ void epilogue_ahead(const GemmParams& p, const EpiMaps& tm, const EpiStage& es,
                                                uint4 (&bv)[4], int nc, int row0, int n0, int lane, int c_first = 0,
                                                int c_step = 1) {
-  if (row0 >= p.M) return;
+  if (!AHEAD || row0 >= p.M) return;
   epi_bias<T>(p, bv, n0 + c_first * 32);
-  if (!TILES || !p.mat_tma) return;
+  if (!p.mat_tma) return;
   for (int i = 0; i < 2 && c_first + i * c_step < nc; ++i)
     epi_request(&tm.mat, es, es.issued + i, n0 + (c_first + i * c_step) * 32, row0, lane);
 }
 
-template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool AR = false, int MT = 1>
+template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool AR = false, int MT = 1, bool AHEAD = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ EpiMaps tmE, const GemmParams p, const ArParams ar) {
@@ -503,7 +504,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   constexpr int S = Cfg::kStages;
   constexpr int BM = MT * kBM;
   constexpr int NACC = Cfg::kAccBuffers;
-  constexpr bool TILES = !OUT_F32 && !AR;     // of the epilogue's other matrices
+  static_assert(!AHEAD || (!OUT_F32 && !AR && MT == 1), "for a staged 16-bit output");
   static_assert(!(AR && MT != 1), "the fused all-reduce path uses 128-row tiles");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -517,7 +518,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint64_t* tempty = bars + 2 * S + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint64_t* epi_bars = bars + 2 * S + 6;     // TILES: four for each epilogue warp
+  uint64_t* epi_bars = bars + 2 * S + 6;     // AHEAD: four for each epilogue warp
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -538,7 +539,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     prefetch_tmap(&tmB);
     if (!AR) prefetch_tmap(&tmE.out);
   }
-  if (TILES && warp >= 2 && lane < kEpiBufs16) {
+  if (AHEAD && warp >= 2 && lane < kEpiBufs16) {
     mbar_init(&epi_bars[(warp & 3) * kEpiBufs16 + lane], 1);
     fence_barrier_init();
   }
@@ -642,7 +643,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const int n0 = (tile / p.num_m_tiles) * BN;
       const int nc = (min(BN, p.N - n0) + 31) / 32;   // 32-column chunks of this tile inside the matrix (warp-uniform)
       uint4 bv[4];
-      if (!AR) epilogue_ahead<T, TILES>(p, tmE, es, bv, nc, m0 + quarter * 32, n0, lane);
+      epilogue_ahead<T, AHEAD>(p, tmE, es, bv, nc, m0 + quarter * 32, n0, lane);
       ok = mbar_wait(&tfull[acc], acc_phase, wctx, kErrWaitEpilogue);
       if (!ok) break;
       tc_fence_after();
@@ -671,8 +672,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         for (int mt = 0; mt < MT; ++mt) {
           const int row0 = m0 + mt * kBM + quarter * 32;
           if (row0 >= p.M) continue;  // warp-uniform: nothing to store
-          if (mt > 0) epilogue_ahead<T, TILES>(p, tmE, es, bv, nc, row0, n0, lane);
-          epilogue_rows<T, OUT_F32, false, TILES>(p, tmE, es, wctx, bv, t_acc + mt * BN, nc, row0, n0, lane);
+          epilogue_rows<T, OUT_F32, false, AHEAD>(p, tmE, es, wctx, bv, t_acc + mt * BN, nc, row0, n0, lane);
         }
       }
       tc_fence_before();
@@ -792,12 +792,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::kTmemCols);
 }
 
-template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool AR = false, int MT = 1>
+template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool AR = false, int MT = 1, bool AHEAD = false>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& tmE,
                        const GemmParams& p, cudaStream_t stream, const ArParams* arp = nullptr) {
   using Cfg = GemmCfg<BN, MT, AR>;
   static_assert(Cfg::kSmemBytes >= kTmemKernelMinSmem, "allocates TMEM before pdl_wait");
-  auto kern = gemm_kernel<T, BN, A_MN, B_MN, OUT_F32, AR, MT>;
+  auto kern = gemm_kernel<T, BN, A_MN, B_MN, OUT_F32, AR, MT, AHEAD>;
   ArParams ar;
   if (arp) ar = *arp;
   else { ar.tp = 0; ar.exchange = 0; ar.rows_per_rank = 0; }
@@ -817,12 +817,19 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Epi
 
 template <typename T, int BN, int MT = 1>
 static int dispatch_layout(int a_mn, int b_mn, int out_f32, const CUtensorMap& tmA,
-                           const CUtensorMap& tmB, const EpiMaps& tmE, const GemmParams& p,
+                           const CUtensorMap& tmB, const EpiMaps& tmE, const GemmParams& p, bool ahead,
                            cudaStream_t s) {
+  if constexpr (MT == 1) {
+    if (ahead)
+      return b_mn ? launch_gemm<T, BN, false, true, false, false, 1, true>(tmA, tmB, tmE, p, s)
+                  : launch_gemm<T, BN, false, false, false, false, 1, true>(tmA, tmB, tmE, p, s);
+  }
   if (!a_mn && !b_mn && !out_f32) return launch_gemm<T, BN, false, false, false, false, MT>(tmA, tmB, tmE, p, s);
   if (!a_mn && b_mn && !out_f32) return launch_gemm<T, BN, false, true, false, false, MT>(tmA, tmB, tmE, p, s);
-  if (a_mn && b_mn && out_f32) return launch_gemm<T, BN, true, true, true, false, MT>(tmA, tmB, tmE, p, s);
-  if (MT == 1) {  // rarely used layouts: only the 128-row tile is instantiated
+  if constexpr (BN >= 64) {
+    if (a_mn && b_mn && out_f32) return launch_gemm<T, BN, true, true, true, false, MT>(tmA, tmB, tmE, p, s);
+  }
+  if constexpr (MT == 1 && BN >= 64) {  // rarely used layouts: only the 128-row tile is instantiated
     if (!a_mn && !b_mn && out_f32) return launch_gemm<T, BN, false, false, true>(tmA, tmB, tmE, p, s);
     if (a_mn && b_mn && !out_f32) return launch_gemm<T, BN, true, true, false>(tmA, tmB, tmE, p, s);
   }
@@ -1226,16 +1233,16 @@ __device__ __forceinline__ void ar_reduce_tile(const GemmParams& p, const ArPara
 // blocks of this rank visited last, the partials have arrived long before they are needed and
 // nothing follows the last tile: no second hop, no result flags.
 template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool TRACE = false, bool AR = false,
-          bool RS = false>
+          bool RS = false, bool AHEAD = false>
 __global__ void __launch_bounds__(kPairThreads + (RS ? 32 : 0), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ EpiMaps tmE, const GemmParams p, const ArParams ar) {
   static_assert(!AR || (BN == 128 && !OUT_F32 && !TRACE), "fused all-reduce: 256 x 128 pair tiles, 16-bit output");
+  static_assert(!AHEAD || (!OUT_F32 && !AR && !RS), "for a staged 16-bit output");
   static_assert(!RS || (BN == 128 && !OUT_F32 && !TRACE && !AR && !A_MN), "fused reduce-scatter: 256 x 128 pair tiles, 16-bit output");
   using Cfg = PairCfg<BN>;
   constexpr int S = Cfg::kStages;
   constexpr int HB = BN / 2;  // B rows held by one CTA
-  constexpr bool TILES = !OUT_F32 && !AR && !RS;   // of the epilogue's other matrices
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -1252,7 +1259,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* pub_full = bars + 2 * S + 6;                                    // RS: block stored by all warps
   volatile int* pub_done = reinterpret_cast<volatile int*>(bars + 2 * S + 8);  // RS: blocks published
 
-  uint64_t* epi_bars = bars + 2 * S + 9;     // TILES: four for each epilogue warp
+  uint64_t* epi_bars = bars + 2 * S + 9;     // AHEAD: four for each epilogue warp
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1285,7 +1292,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     prefetch_tmap(&tmB);
     if (!AR) prefetch_tmap(&tmE.out);   // (all-reduce: stores through peer pointers, the maps stay empty)
   }
-  if (TILES && warp >= 2 && lane < kEpiBufs16) {
+  if (AHEAD && warp >= 2 && lane < kEpiBufs16) {
     mbar_init(&epi_bars[(warp - 2) * kEpiBufs16 + lane], 1);
     fence_barrier_init();
   }
@@ -1459,7 +1466,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int n0 = n_idx * BN;
       const int nc = (min(BN, p.N - n0) + 31) / 32;
       uint4 bv[4];
-      if (!AR) epilogue_ahead<T, TILES>(p, tmE, es, bv, nc, m0 + quarter * 32, n0, lane, half, 2);
+      epilogue_ahead<T, AHEAD>(p, tmE, es, bv, nc, m0 + quarter * 32, n0, lane, half, 2);
       const long long t_e = TRACE ? clock64() : 0;
       ok = mbar_wait(&tfull[acc], acc_phase, wctx, kErrWaitEpilogue);
       if (!ok) break;
@@ -1667,7 +1674,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       if (row0 < p.M) {
         const long long t_l = TRACE ? clock64() : 0;
-        epilogue_rows<T, OUT_F32, TRACE, TILES>(
+        epilogue_rows<T, OUT_F32, TRACE, AHEAD>(
             p, tmE, es, wctx, bv, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kAccCols, nc, row0,
             n0, lane, half, 2, cyc3);
         if (TRACE) cyc_rest += clock64() - t_l;
@@ -1797,12 +1804,12 @@ static int max_pairs() {
 }
 
 template <typename T, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool TRACE = false, bool AR = false,
-          bool RS = false>
+          bool RS = false, bool AHEAD = false>
 static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& tmE,
                             const GemmParams& p, cudaStream_t stream, const ArParams* arp = nullptr) {
   using Cfg = PairCfg<BN>;
   static_assert(Cfg::kSmemBytes + kTmemKernelMinSmem > kSmemPerSm, "allocates TMEM after pdl_wait");
-  auto kern = gemm_pair_kernel<T, BN, A_MN, B_MN, OUT_F32, TRACE, AR, RS>;
+  auto kern = gemm_pair_kernel<T, BN, A_MN, B_MN, OUT_F32, TRACE, AR, RS, AHEAD>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) !=
@@ -1822,8 +1829,11 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
 
 template <typename T, int BN>
 static int dispatch_layout_pair(int a_mn, int b_mn, int out_f32, const CUtensorMap& tmA,
-                                const CUtensorMap& tmB, const EpiMaps& tmE, const GemmParams& p,
+                                const CUtensorMap& tmB, const EpiMaps& tmE, const GemmParams& p, bool ahead,
                                 cudaStream_t s) {
+  if (ahead)
+    return b_mn ? launch_gemm_pair<T, BN, false, true, false, false, false, false, true>(tmA, tmB, tmE, p, s)
+                : launch_gemm_pair<T, BN, false, false, false, false, false, false, true>(tmA, tmB, tmE, p, s);
   if (!a_mn && !b_mn && !out_f32) return launch_gemm_pair<T, BN, false, false, false>(tmA, tmB, tmE, p, s);
   if (!a_mn && b_mn && !out_f32) return launch_gemm_pair<T, BN, false, true, false>(tmA, tmB, tmE, p, s);
   if (a_mn && b_mn && out_f32) return launch_gemm_pair<T, BN, true, true, true>(tmA, tmB, tmE, p, s);
@@ -1935,13 +1945,22 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
   p.trace = nullptr;
   p.prefetch = g_prefetch;
   p.a_bytes = (a_mn ? BM : box_m) * kBK * 2;
-  if (!parts && !out_f32) {
-    // as tiles, where a tensor map can describe them (16-byte addresses and strides)
-    auto tile_map = [&](CUtensorMap* m, const void* x, long long ld) {
+  // Kernels that ask for the epilogue's other operands ahead of their chunk (AHEAD).  A tensor map has to describe the
+  // matrix (16-byte addresses and strides, rows that do not overlap), and the loads need something to run under: the
+  // seven other epilogue warps of a CTA, the main loop of its only tile, or long main loops.  Several short tiles a CTA
+  // are faster with all loads at a chunk's start, and so is the derivative in wide tiles.  us at the start / ahead:
+  // one-CTA tiles of 64 columns, 8192 x 1024 x 64 with a residual 15.7 / 17.9, 4356 x 1024 x 256 with GeLU's derivative
+  // 14.2 / 15.6, 1024 x 1024 x 256 (one tile each) with a residual 5.1 / 4.6; of 128, 1024 x 2048 x 512 (one each) with a
+  // residual 7.7 / 7.3, with the derivative 9.2 / 9.4; of 256, 333 x 24576 x 4096 with the derivative 85 / 81; CTA pairs, 8192 x
+  // 1024 x 64 with a residual 15.8 / 14.1, 4356 x 3072 x 64 24.6 / 20.0, with the derivative 29.7 / 30.4 (8192 x 3072 x 768 83 / 60).
+  const bool wide_dact = dact && BN > 64, lone = p.num_tiles <= num_sms();
+  bool ahead = !parts && !a_mn && !out_f32 && (pair || (tile_code != 512 && (K >= 4096 || (lone && !wide_dact))));
+  if (ahead && (residual || dact)) {
+    auto tile_map = [&](const void* x, long long ld) {
       return x && ld % 8 == 0 && ld >= N && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
-             make_tmap_out(m, x, N, M, ld, false, bf16);
+             make_tmap_out(&tmE.mat, x, N, M, ld, false, bf16);
     };
-    p.mat_tma = residual ? tile_map(&tmE.mat, residual, ldr) : dact ? tile_map(&tmE.mat, aux_in, ld_aux) : 0;
+    p.mat_tma = ahead = residual ? tile_map(residual, ldr) : tile_map(aux_in, ld_aux);
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (parts) {
@@ -1953,17 +1972,16 @@ static int gemm_impl(int dtype, int a_mn, int b_mn, const void* A, long long lda
     return bf16 ? TP_SPLIT(__nv_bfloat16) : TP_SPLIT(__half);
 #undef TP_SPLIT
   }
-#define TP_DISPATCH(T)                                                                   \
-  (pair ? (BN == 256 ? dispatch_layout_pair<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)  \
-           : BN == 224 ? dispatch_layout_pair<T, 224>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s) \
-           : BN == 192 ? dispatch_layout_pair<T, 192>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s) \
-                     : dispatch_layout_pair<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)) \
-   : tile_code == 512 ? dispatch_layout<T, 256, 2>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)  \
-   : BN == 256 ? dispatch_layout<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)            \
-   : BN == 128 ? dispatch_layout<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)            \
-   : BN == 64 ? dispatch_layout<T, 64>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, s)              \
-   : b_mn ? launch_gemm<T, 32, false, true, false>(tmA, tmB, tmE, p, s)                       \
-          : launch_gemm<T, 32, false, false, false>(tmA, tmB, tmE, p, s))
+#define TP_DISPATCH(T)                                                                                \
+  (pair ? (BN == 256 ? dispatch_layout_pair<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s)  \
+           : BN == 224 ? dispatch_layout_pair<T, 224>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s) \
+           : BN == 192 ? dispatch_layout_pair<T, 192>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s) \
+                     : dispatch_layout_pair<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s)) \
+   : tile_code == 512 ? dispatch_layout<T, 256, 2>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s)   \
+   : BN == 256 ? dispatch_layout<T, 256>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s)             \
+   : BN == 128 ? dispatch_layout<T, 128>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s)             \
+   : BN == 64 ? dispatch_layout<T, 64>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s)               \
+              : dispatch_layout<T, 32>(a_mn, b_mn, out_f32, tmA, tmB, tmE, p, ahead, s))
   return bf16 ? TP_DISPATCH(__nv_bfloat16) : TP_DISPATCH(__half);
 #undef TP_DISPATCH
 }
@@ -2166,8 +2184,8 @@ extern "C" int tp_gemm_trace(int bn, const void* A, long long lda, const void* B
   p.trace = trace;
   p.prefetch = g_prefetch;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return bn == 256 ? launch_gemm_pair<__half, 256, false, false, false, true>(tmA, tmB, tmE, p, s)
-                   : launch_gemm_pair<__half, 128, false, false, false, true>(tmA, tmB, tmE, p, s);
+  return bn == 256 ? launch_gemm_pair<__half, 256, false, false, false, true, false, false, true>(tmA, tmB, tmE, p, s)
+                   : launch_gemm_pair<__half, 128, false, false, false, true, false, false, true>(tmA, tmB, tmE, p, s);
 }
 
 // Fused all-reduce, CTA-pair kernel.  exchange = 1: every rank sends each partial tile to every
