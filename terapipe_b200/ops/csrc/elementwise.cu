@@ -374,12 +374,13 @@ __global__ void layernorm_bwd_reduce_kernel(float* __restrict__ scratch, int par
   fold_slots(scratch, parts, H, blockIdx.x * 32, dgamma, dbeta, threadIdx.x, threadIdx.y, clear, sm);
 }
 
-template <typename T, int V, bool LAYERS>
+// PER: chunks of a CTA, one after the other (their sums are folded in the same order).
+template <typename T, int V, bool LAYERS, int PER>
 __global__ void __launch_bounds__(256)
 layer_sums_kernel(const SumJobs j) {
   constexpr int kCols = 8 * V, kRows = 256 / V;   // columns of a CTA, rows of one load
   __shared__ union { float col[kRows][kCols + 1]; float fold[8][33]; } sm;
-  __shared__ float chunk_sum[kCols];
+  __shared__ float chunk_sum[PER][kCols];
   const int tid = threadIdx.x, vec = tid % V, lane_row = tid / V;
   const int cta = blockIdx.x;
   const long long layer = LAYERS ? blockIdx.y : 0;
@@ -389,49 +390,59 @@ layer_sums_kernel(const SumJobs j) {
   for (int i = 0; i < kMaxColsums; ++i) {
     if (i >= j.n) break;
     if (cta < j.cta_end[i]) {
-      const int chunk = (cta - first) % j.chunks;
-      const int col0 = (cta - first) / j.chunks * kCols, col = col0 + vec * 8;
-      const int r_end = min(j.rows, (chunk + 1) * j.rows_per_chunk);
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (col < j.N[i]) {
-        const T* src = static_cast<const T*>(j.dy[i]) + layer * j.dy_stride[i] + col;
-        asm("" : "+l"(src));
-        for (int r = chunk * j.rows_per_chunk + lane_row; r < r_end; r += 8 * kRows) {
-          uint4 v[8];
+      const int ctas = j.chunks / PER, rank = (cta - first) % ctas;   // of a column block: a cluster
+      const int col0 = (cta - first) / ctas * kCols, col = col0 + vec * 8;
+      float s = 0.0f;
+#pragma unroll 1
+      for (int u = 0; u < PER; ++u) {
+        const int chunk = rank * PER + u;
+        const int r_end = min(j.rows, (chunk + 1) * j.rows_per_chunk);
+        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (col < j.N[i]) {
+          const T* src = static_cast<const T*>(j.dy[i]) + layer * j.dy_stride[i] + col;
+          asm("" : "+l"(src));
+          for (int r = chunk * j.rows_per_chunk + lane_row; r < r_end; r += 8 * kRows) {
+            uint4 v[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            v[k] = r + kRows * k < r_end ? *reinterpret_cast<const uint4*>(src + (r + kRows * k) * j.ld[i])
-                                         : make_uint4(0, 0, 0, 0);
+            for (int k = 0; k < 8; ++k)
+              v[k] = r + kRows * k < r_end ? *reinterpret_cast<const uint4*>(src + (r + kRows * k) * j.ld[i])
+                                           : make_uint4(0, 0, 0, 0);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            float f[8];
-            unpack8<T>(v[k], f);
+            for (int k = 0; k < 8; ++k) {
+              float f[8];
+              unpack8<T>(v[k], f);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) acc[q] += f[q];
+              for (int q = 0; q < 8; ++q) acc[q] += f[q];
+            }
           }
         }
-      }
+        if (u > 0) __syncthreads();      // the last chunk's values have been added up
 #pragma unroll
-      for (int q = 0; q < 8; ++q) sm.col[lane_row][vec * 8 + q] = acc[q];
-      __syncthreads();
-      float s = 0.0f;
-      if (tid < kCols) {
+        for (int q = 0; q < 8; ++q) sm.col[lane_row][vec * 8 + q] = acc[q];
+        __syncthreads();
+        if (tid < kCols) {
+          float t = 0.0f;
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) s += sm.col[r][tid];
+          for (int r = 0; r < kRows; ++r) t += sm.col[r][tid];
+          if (PER > 1 || ctas > 1) chunk_sum[u][tid] = t;
+          s = u == 0 ? t : s + t;
+        }
       }
-      if (j.chunks > 1) {   // (the CTAs of a cluster are the chunks of one column block)
-        if (tid < kCols) chunk_sum[tid] = s;
+      if (ctas > 1) {
         cluster_sync_all();
-        if (chunk == 0 && tid < kCols) {
-          for (int q = 1; q < j.chunks; ++q) {
-            float v;
-            asm volatile("ld.shared::cluster.f32 %0, [%1];"
-                         : "=f"(v) : "r"(mapa_u32(smem_u32(&chunk_sum[tid]), q)) : "memory");
-            s += v;
+        if (rank == 0 && tid < kCols) {
+          for (int q = 1; q < ctas; ++q) {
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+              float v;
+              asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                           : "=f"(v) : "r"(mapa_u32(smem_u32(&chunk_sum[u][tid]), q)) : "memory");
+              s += v;
+            }
           }
         }
         cluster_sync_all();   // nobody leaves while its sums may be read
-        if (chunk != 0) return;
+        if (rank != 0) return;
       }
       if (tid < kCols && col0 + tid < j.N[i]) {
         float* db = j.db[i] + layer * j.out_stride + col0 + tid;
@@ -715,29 +726,33 @@ static int layer_sums_launch(int dtype, SumJobs& j, int layers, cudaStream_t s) 
   const int cols = wide ? 256 : 64, round = 8 * 256 / (cols / 8);   // rows of one round of loads
   // Chunks of at least one round, a portable cluster of them at most; with V = 32 no more than 4 CTAs per
   // SM, which run at once (2560-wide layer, 16384 rows: 156 us with 8 chunks a block, 131 with 4;
-  // 5120-wide, 1024 rows: 28.6 with 8, 21.8 with 2), unless even two chunks are too many for five per SM, which
-  // still run at once (360 blocks of 16384 rows: 435 us with 2, 477 with 4).
+  // 5120-wide, 1024 rows: 28.6 with 8, 21.8 with 2), unless even two chunks take several rounds: four then, of which
+  // a CTA takes two where pairs of CTAs are few enough for five per SM, which still run at once (360 blocks of 16384
+  // rows: 435 us instead of 477).
   int most = 8;
   if (wide) {
     while (most > 2 && blocks * most > 4 * num_sms()) most /= 2;
-    if (blocks * most > 5 * num_sms()) most = 4;
+    if (blocks * most > 4 * num_sms()) most = 4;
   }
   j.chunks = 1;
   while (j.n > 0 && j.chunks < most && j.rows >= 2 * round * j.chunks) j.chunks *= 2;
+  const bool twice = wide && j.chunks == 4 && blocks * 4 > 5 * num_sms() && blocks * 2 <= 5 * num_sms();
+  const int cluster = twice ? 2 : j.chunks;      // CTAs of a block
   j.rows_per_chunk = (j.rows + j.chunks - 1) / j.chunks;
   long long ctas = 0;
   for (int i = 0; i < j.n; ++i) {
-    ctas += (j.N[i] + cols - 1) / cols * static_cast<long long>(j.chunks);
+    ctas += (j.N[i] + cols - 1) / cols * static_cast<long long>(cluster);
     j.cta_end[i] = static_cast<int>(ctas);
   }
   ctas += static_cast<long long>(j.folds) * ((2 * j.H + 31) / 32);
   if (ctas == 0) return kOk;
-  ctas = (ctas + j.chunks - 1) / j.chunks * j.chunks;
+  ctas = (ctas + cluster - 1) / cluster * cluster;
   if (ctas > 0x7fffffffLL) return kErrTooLarge;
   const dim3 grid(static_cast<unsigned>(ctas), static_cast<unsigned>(layers)), block(256);
-#define TP_SUMS(T, LAYERS)                                                                  \
-  (wide ? launch_pdl(layer_sums_kernel<T, 32, LAYERS>, grid, block, 0, s, j.chunks, j)      \
-        : launch_pdl(layer_sums_kernel<T, 8, LAYERS>, grid, block, 0, s, j.chunks, j))
+#define TP_SUMS(T, LAYERS)                                                                     \
+  (twice  ? launch_pdl(layer_sums_kernel<T, 32, LAYERS, 2>, grid, block, 0, s, cluster, j)     \
+   : wide ? launch_pdl(layer_sums_kernel<T, 32, LAYERS, 1>, grid, block, 0, s, cluster, j)     \
+          : launch_pdl(layer_sums_kernel<T, 8, LAYERS, 1>, grid, block, 0, s, cluster, j))
   const cudaError_t e = dtype == 1 ? (layers > 1 ? TP_SUMS(__nv_bfloat16, true) : TP_SUMS(__nv_bfloat16, false))
                                    : (layers > 1 ? TP_SUMS(__half, true) : TP_SUMS(__half, false));
 #undef TP_SUMS
