@@ -258,7 +258,8 @@ class StageEngine:
         self._alloc_activations()
         self.status = F.status_word(dev)
         self.loss_buf = torch.zeros(1, dtype=torch.float32, device=dev)
-        self._graph = None
+        self._graph = self._add_graph = None    # of the usual step, of one that adds to gradients left in the buffer
+        self._add_eager = False
         self._cap_stream = None
         self.timeline = None   # set to a utils.trace.SliceTimeline to record per-slice device times
         self.step_count = 0
@@ -1175,7 +1176,9 @@ class StageEngine:
         F.fused_adam(self.grad, self.master, self.exp_avg, self.exp_avg_sq, self.model,
                      self.adam_state, lr=self.lr, grad_scale=1.0 / (self.loss_scale * self.dp))
 
-    def _iteration(self, update=True):
+    def _iteration(self, update=True, fused=None):
+        """``fused``: whether the update happens inside the weight-gradient products (``None``: as the gradient
+        buffer has it)."""
         if not self._first_step_synced:
             # Kernels that wait for a peer on the device are bounded by the wait limit; the first
             # step follows minutes of set-up whose length differs between ranks (weight
@@ -1203,7 +1206,7 @@ class StageEngine:
             self._group_barrier(1)
         self._dp_overlap = bool(update and self.dp > 1 and self.dp_overlap)
         self._dp_works = None
-        fused_update = update and self._updates_in_products
+        fused_update = update and (self._updates_in_products if fused is None else fused)
         self._forward_backward("update" if fused_update else "add" if update or self.dp > 1 or self.sp else "assign")
         if update and not (self.dp_sym is not None and self._dp_overlap and not self.sp):
             if self._seg_graphs is not None and (self.dp == 1 or self.dp_sym is not None):
@@ -1275,19 +1278,23 @@ class StageEngine:
     def step(self) -> None:
         """One training iteration on the current stream.  With ``use_graph`` the first call
         runs eagerly (it also sets up kernel attributes) and records the iteration into a
-        CUDA graph; later calls replay the graph.  (An iteration that has to add to gradients left by
-        :meth:`compute_grads` runs eagerly as well and is not recorded.)"""
-        usual = self._updates_in_products == self._adam_in_products
-        if self.use_graph and self._graph is not None and usual:
-            self._graph.replay()
+        CUDA graph; later calls replay the graph.  An iteration that has to add to gradients left by
+        :meth:`compute_grads` has a graph of its own: 24 layers of 256 columns, 256 rows, 2.1 ms
+        issued from Python, 1.8 replayed."""
+        fused = self._updates_in_products
+        usual = fused == self._adam_in_products
+        graph = self._graph if usual else self._add_graph
+        if self.use_graph and graph is not None:
+            graph.replay()
+            self._grad_seen = self.grad._version
         else:
             self._iteration()
-            if self.use_graph and self._graph is None and usual:
-                self._capture()
+            if self.use_graph and (usual or not self._add_eager):
+                self._capture(fused, usual)
         self.step_count += 1
         self.launch_count += self._launches[self._walked_merged]   # of the iteration that ran, or was captured
 
-    def _capture(self):
+    def _capture(self, fused, usual):
         torch.cuda.synchronize()
         # (torch.cuda.graph() would also collect garbage and give torch's cached memory back to
         # the driver first, which takes far longer than the capture: tens of milliseconds, and
@@ -1295,36 +1302,44 @@ class StageEngine:
         # the capture runs, though: the destructor of an old graph is not a legal call then.
         try:
             try:
-                self._graph = self._captured_iteration()
+                graph = self._captured_iteration(fused)
             except (RuntimeError, KernelError):
                 # Torch does not give memory back during a capture, so one that finds a few MB free
                 # beside a large cache has no room for its stream, the loss sum or the graph.
                 torch.cuda.synchronize()
                 torch.cuda.empty_cache()
                 self._ag_pending = False
-                self._graph = self._captured_iteration()
+                graph = self._captured_iteration(fused)
+            if usual:
+                self._graph = graph
+            else:
+                self._add_graph = graph
         except (RuntimeError, KernelError) as e:
             # The whole step could not be captured (seen with a 48-layer stage of GPT3-44B width:
             # a launch inside the capture failed although the same step had just run eagerly).
             # Fall back to one graph per launch-only segment, which captures far smaller pieces.
+            # (Steps that add to what the buffer holds are rare: they go on without a graph.)
             import warnings
             warnings.warn(f"whole-step CUDA graph capture failed ({type(e).__name__}: {str(e)[:120]}); "
-                          "using per-segment graphs instead")
+                          + ("using per-segment graphs instead" if usual else "steps that add to gradients run eagerly"))
             torch.cuda.synchronize()
+            self._ag_pending = False
+            if not usual:
+                self._add_eager = True
+                return
             self.use_graph = False
             self._graph = None
-            self._ag_pending = False
             if self._plan is None and self._seg_graphs is None:
                 self._seg_graphs = {}
 
-    def _captured_iteration(self):
+    def _captured_iteration(self, fused):
         graph = torch.cuda.CUDAGraph()
         if self._cap_stream is None:
             self._cap_stream = torch.cuda.Stream()
         with collection_paused(), torch.cuda.stream(self._cap_stream):
             graph.capture_begin(capture_error_mode="thread_local")
             try:
-                self._iteration()
+                self._iteration(fused=fused)
             finally:
                 graph.capture_end()
         return graph
@@ -1335,7 +1350,7 @@ class StageEngine:
     def close(self) -> None:
         """Release the peer-mapped buffers (collective over the tensor- and data-parallel groups;
         call it between steps).  The engine must not be used afterwards."""
-        self._graph = None
+        self._graph = self._add_graph = None
         if self._seg_graphs is not None:
             self._seg_graphs.clear()
         torch.cuda.synchronize()
