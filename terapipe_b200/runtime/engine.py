@@ -47,6 +47,7 @@ from ..models import TransformerConfig
 from ..ops import functional as F
 from ..ops.lib import KernelError, cuda_lib
 from ..utils.misc import collection_paused
+from .grad_buffer import GradBuffer
 
 LOSS_SCALE_FACTOR = 128.0
 _ACT = {"none": 0, "relu": 1, "gelu": 2}
@@ -185,7 +186,7 @@ class StageEngine:
             self.dp_sym = SymmetricBuffer(1024 + model_bytes + n * 4, mpu.get_data_parallel_group())
             self._dp_off_model, self._dp_off_grad = 1024, 1024 + model_bytes
             self.model = self.dp_sym.view(self._dp_off_model, (n,), dtype)
-            self.grad = self.dp_sym.view(self._dp_off_grad, (n,), torch.float32)
+            grad = self.dp_sym.view(self._dp_off_grad, (n,), torch.float32)
             self.dp_epoch_base = torch.zeros(1, dtype=torch.int32, device=dev)
             # Ownership of the fused reduction + sharded Adam: within the flat range of every
             # layer, replica r owns the r-th chunk.  (lo, hi, begin, end) per layer.
@@ -202,7 +203,8 @@ class StageEngine:
             self._dp_stream = None
         else:
             self.model = torch.zeros(n, dtype=dtype, device=dev)
-            self.grad = torch.zeros(n, dtype=torch.float32, device=dev)
+            grad = torch.zeros(n, dtype=torch.float32, device=dev)
+        self._grads = GradBuffer(grad)
         self.master = torch.zeros(n, dtype=torch.float32, device=dev)
         self.exp_avg = torch.zeros(n, dtype=torch.float32, device=dev)
         self.exp_avg_sq = torch.zeros(n, dtype=torch.float32, device=dev)
@@ -212,7 +214,6 @@ class StageEngine:
         # gradients come from column sums, follow in one small launch.  (Sequence parallel: the
         # LayerNorm gradients are summed over the ranks after the products.)
         self._adam_in_products = self.dp == 1 and not self.sp
-        self._grad_seen = self.grad._version     # of the buffer when an update last left it zero
         self._init_weights(init)
         # A CUDA graph may hold this library's kernels only: captured NCCL point-to-point or
         # collective calls deadlocked on replay here, so a stage that calls NCCL runs eagerly.
@@ -300,6 +301,12 @@ class StageEngine:
     def launches_per_step(self) -> int:
         """Launches of this library's kernels that the next iteration makes."""
         return self._launches[self.merges_slices]
+
+    @property
+    def grad(self) -> torch.Tensor:
+        """The flat fp32 gradients, for reading and writing; what is in it when a step is taken is added to that step's
+        gradients.  (The step after that, and all while a view of it is held, takes the path that can add.)"""
+        return self._grads.share()
 
     # ------------------------------------------------------------------ parameters
     def param(self, layer: int, name: str, buf: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -401,7 +408,7 @@ class StageEngine:
 
     def named_grads(self, unscale=True) -> Dict[str, torch.Tensor]:
         s = 1.0 / self.loss_scale if unscale else 1.0
-        return {f"layers.layers.{l}.{name}": self.get_param(l, name, self.grad).clone() * s
+        return {f"layers.layers.{l}.{name}": self.get_param(l, name, self._grads.tensor).clone() * s
                 for l in range(self.n_layers) for name in PARAM_ORDER}
 
     # ------------------------------------------------------------------ buffers
@@ -534,7 +541,7 @@ class StageEngine:
                                         self.adam_state.data_ptr(), self.lr, 0.9, 0.999, 1e-8, 0.0,
                                         1.0 / (self.loss_scale * self.dp), int(follows), self._status_ptr, self._stream)
         else:
-            st = self.lib.tp_wgrad(*operands, self._p(l, name, self.grad), *sizes, int(mode == "add"),
+            st = self.lib.tp_wgrad(*operands, self._p(l, name, self._grads.tensor), *sizes, int(mode == "add"),
                                    int(follows), self._status_ptr, self._stream)
         if st:
             F.check(st, "tp_wgrad")
@@ -893,7 +900,9 @@ class StageEngine:
         weight in one launch.  ``mode``: "add" to the gradients, "assign" them, or "update" the weights
         instead (:meth:`_reduce_and_update` then does the rest)."""
         H, Hl, Fl = self.H, self.Hl, self.Fl
-        lib, s, g = self.lib, self._stream, self.grad
+        lib, s, g = self.lib, self._stream, self._grads.tensor
+        if mode != "update" and not torch.cuda.is_current_stream_capturing():
+            self._grads.left = True
         # Data-parallel reduction overlapped with these products: as soon as the gradients of a
         # layer are complete (layers are visited last to first), its reduction - and with the fused
         # kernel its Adam update and parameter push - starts on a side stream (NCCL: on NCCL's own
@@ -945,7 +954,7 @@ class StageEngine:
         """``mats``: (the layers' ``[rows, width]``, width, bias name) whose column sums are added to (or assigned
         to) the bias gradients of ``layers`` layers from ``l`` on; ``folds``: (address of the partial slots,
         LayerNorm name)."""
-        n, m, g = len(mats), len(folds), self.grad
+        n, m, g = len(mats), len(folds), self._grads.tensor
         P, LL, I = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
         widths = [w for _, w, _ in mats]
         self._ln("tp_stage_sums", self.dt, n, (P * n)(*[a[l].data_ptr() for a, _, _ in mats]), (LL * n)(*widths),
@@ -1136,7 +1145,7 @@ class StageEngine:
             1.0 / (self.loss_scale * self.dp), self._status_ptr, stream_handle)
         if st:
             F.check(st, "tp_dp_reduce_adam")
-        self.grad[lo:hi].zero_()
+        self._grads.tensor[lo:hi].zero_()
 
     def _dp_layer_done(self, l, works):
         """The gradients of layer ``l`` are complete on the current stream: start reducing them."""
@@ -1148,13 +1157,13 @@ class StageEngine:
         else:
             lo = self.layout.offsets[l][PARAM_ORDER[0]]
             hi = self.layout.offsets[l + 1][PARAM_ORDER[0]] if l + 1 < self.n_layers else self.layout.total
-            works.append(dist.all_reduce(self.grad[lo:hi], group=mpu.get_data_parallel_group(),
+            works.append(dist.all_reduce(self._grads.tensor[lo:hi], group=mpu.get_data_parallel_group(),
                                          async_op=True))
 
     def _reduce_and_update(self, fused_update: bool = False):
         if fused_update:
             # the weights are done (_weight_grads): biases and LayerNorm parameters
-            F.fused_adam_ranges(self.grad, self.master, self.exp_avg, self.exp_avg_sq, self.model,
+            F.fused_adam_ranges(self._grads.tensor, self.master, self.exp_avg, self.exp_avg_sq, self.model,
                                 self.adam_state, self.layout.small_ranges, self.n_layers, self.layout.layer_stride,
                                 lr=self.lr, grad_scale=1.0 / (self.loss_scale * self.dp))
             return
@@ -1171,9 +1180,9 @@ class StageEngine:
                     w.wait()
                 self._dp_works = None
             else:
-                dist.all_reduce(self.grad, group=mpu.get_data_parallel_group())
+                dist.all_reduce(self._grads.tensor, group=mpu.get_data_parallel_group())
         F.adam_tick(self.adam_state)
-        F.fused_adam(self.grad, self.master, self.exp_avg, self.exp_avg_sq, self.model,
+        F.fused_adam(self._grads.tensor, self.master, self.exp_avg, self.exp_avg_sq, self.model,
                      self.adam_state, lr=self.lr, grad_scale=1.0 / (self.loss_scale * self.dp))
 
     def _iteration(self, update=True, fused=None):
@@ -1215,7 +1224,7 @@ class StageEngine:
             else:
                 self._reduce_and_update(fused_update)
             if not torch.cuda.is_current_stream_capturing():
-                self._grad_seen = self.grad._version
+                self._grads.cleared()
 
     def set_input(self, x: torch.Tensor) -> None:
         """Copy this replica's ``[L, B, H]`` input into the stage-0 activation buffer.  Rows are
@@ -1260,20 +1269,20 @@ class StageEngine:
 
     def compute_grads(self) -> None:
         """Forward + backward without the optimizer; scaled grads stay in ``self.grad``."""
-        self._grad_seen = None
+        self._grads.left = True
         if self.dp > 1 or self.sp:
-            self.grad.zero_()      # (else the gradients are assigned, not added up)
+            self._grads.tensor.zero_()      # (else the gradients are assigned, not added up)
         self._iteration(update=False)
         if self.dp > 1:
-            dist.all_reduce(self.grad, group=mpu.get_data_parallel_group())
-            self.grad.div_(self.dp)
+            dist.all_reduce(self._grads.tensor, group=mpu.get_data_parallel_group())
+            self._grads.tensor.div_(self.dp)
 
     @property
     def _updates_in_products(self) -> bool:
-        """Whether the next update happens inside the weight-gradient products.  Not if ``grad`` has been
-        written since the last update (:meth:`compute_grads`, or by the caller): what it holds then
+        """Whether the next update happens inside the weight-gradient products.  Not if ``grad`` may hold something
+        (:meth:`compute_grads`, or a caller's writes): what it holds then
         counts too, as it always has, so the gradients are added to it and one pass updates everything."""
-        return self._adam_in_products and self.grad._version == self._grad_seen
+        return self._adam_in_products and not self._grads.may_hold
 
     def step(self) -> None:
         """One training iteration on the current stream.  With ``use_graph`` the first call
@@ -1286,7 +1295,7 @@ class StageEngine:
         graph = self._graph if usual else self._add_graph
         if self.use_graph and graph is not None:
             graph.replay()
-            self._grad_seen = self.grad._version
+            self._grads.cleared()
         else:
             self._iteration()
             if self.use_graph and (usual or not self._add_eager):
