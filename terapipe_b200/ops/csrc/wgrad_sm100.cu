@@ -32,7 +32,7 @@ struct WgradParams {
   int num_n_tiles, m_major, m_first, order_split, order_group, order_first_only, order_pipelined;  // TileOrder
   long long ldo, layer_stride;          // of the output matrices, in elements
   float* grad;                          // gradient kernels
-  int accumulate;
+  int accumulate;                       // 1: fetched ahead and added here, 2: added in L2
   AdamBuffers adam;                     // ADAM kernels: the optimizer's matrices
   int follows;                          // the launch before this one is another of these products
   int* err;
@@ -58,34 +58,38 @@ template <int BN> struct WgradCfg {
 // other warp beside it, keep DRAM rows open: with 128 and 256, 4096 x 12288 over 4096 rows took 443 us
 // instead of 422.  One set (48 registers with Adam) is fetched ahead of its use; the epilogue warps of an SM have
 // 48 KB in flight.
-struct WgradRegs { float4 p[4], m[4], v[4]; };
+template <bool ADAM> struct WgradRegs { float4 p[4], m[ADAM ? 4 : 1], v[ADAM ? 4 : 1]; };
 
 template <bool ADAM>
-__device__ __forceinline__ void wgrad_fetch(const WgradParams& p, WgradRegs& a, long long base, int row0, int n,
+__device__ __forceinline__ void wgrad_fetch(const WgradParams& p, WgradRegs<ADAM>& a, long long base, int row0, int n,
                                             int q, int lane) {
-  if (!ADAM) return;
+  if (!ADAM && p.accumulate != 1) return;
   const int col = n + (lane & 15) * 4;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int row = row0 + q * 8 + k * 2 + (lane >> 4);
     if (row < p.M && col < p.N) {
       const long long i = base + row * p.ldo + col;
-      a.p[k] = __ldcs(reinterpret_cast<const float4*>(p.adam.p + i));
-      a.m[k] = __ldcs(reinterpret_cast<const float4*>(p.adam.m + i));
-      a.v[k] = __ldcs(reinterpret_cast<const float4*>(p.adam.v + i));
+      if (ADAM) {
+        a.p[k] = __ldcs(reinterpret_cast<const float4*>(p.adam.p + i));
+        a.m[k] = __ldcs(reinterpret_cast<const float4*>(p.adam.m + i));
+        a.v[k] = __ldcs(reinterpret_cast<const float4*>(p.adam.v + i));
+      } else {
+        a.p[k] = __ldcs(reinterpret_cast<const float4*>(p.grad + i));
+      }
     }
   }
 }
 
 template <typename T, bool ADAM>
-__device__ __forceinline__ void wgrad_finish(const WgradParams& p, const AdamCoef& co, WgradRegs& a,
+__device__ __forceinline__ void wgrad_finish(const WgradParams& p, const AdamCoef& co, WgradRegs<ADAM>& a,
                                              const uint8_t* sb, long long base, int row0, int n, int q, int lane) {
   const int col = n + (lane & 15) * 4;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int rr = q * 8 + k * 2 + (lane >> 4), row = row0 + rr;
     if (row < p.M && col < p.N) {
-      const float4 g = *reinterpret_cast<const float4*>(sb + rr * 256 + (((lane & 15) ^ (rr & 7)) << 4));
+      float4 g = *reinterpret_cast<const float4*>(sb + rr * 256 + (((lane & 15) ^ (rr & 7)) << 4));
       const long long i = base + row * p.ldo + col;
       if (ADAM) {
         adam_update(g, a.p[k], a.m[k], a.v[k], co);
@@ -97,12 +101,10 @@ __device__ __forceinline__ void wgrad_finish(const WgradParams& p, const AdamCoe
         w.y = Elem<T>::pack2(a.p[k].z, a.p[k].w);
         __stcs(reinterpret_cast<uint2*>(static_cast<T*>(p.adam.model) + i), w);
       } else {
-        float4* out = reinterpret_cast<float4*>(p.grad + i);
-        // Adding to the gradient happens in L2: nobody waits for what it holds.  (One addition an element a launch,
-        // so the order is the launches'.)  us fetched / added there, the four weights of one layer: 1600 wide over
-        // 32 rows 73.7 / 50.8, 2048 over 256 114 / 92, 4096 over 256 413 / 332, over 4096 1123 / 1169.
-        if (p.accumulate) atomicAdd(out, g);
-        else __stcs(out, g);
+        if (p.accumulate == 1) { g.x += a.p[k].x; g.y += a.p[k].y; g.z += a.p[k].z; g.w += a.p[k].w; }
+        // (in L2: one addition an element a launch, so the order is the launches')
+        if (p.accumulate == 2) atomicAdd(reinterpret_cast<float4*>(p.grad + i), g);
+        else __stcs(reinterpret_cast<float4*>(p.grad + i), g);
       }
     }
   }
@@ -113,6 +115,11 @@ __device__ __forceinline__ void wgrad_finish(const WgradParams& p, const AdamCoe
 // only get in the operands' way.  4096 x 12288, us without / with, over 512 rows 377 / 299, 1536 382 / 323, 2048
 // 386 / 341, 3072 408 / 403, 4096 415 / 436.
 constexpr int kWgPrefetchK = 3072;
+// Gradients that are added to, the other way round: under a longer main loop the values fetched ahead come for nothing,
+// under a short one that chain is what a tile waits for, and nobody waits for what L2 adds up.  us fetched / added in L2,
+// the four weights of one layer: 1600 wide over 32 rows 73.7 / 50.8, 2048 over 256 114 / 92, 4096 over 256 413 / 332; one
+// weight, four times as high: 2048 wide over 1024 41.5 / 32.5, 4096 over 1024 155 / 144, over 2048 216 / 222, over 4096 467 / 482.
+constexpr int kWgAddInL2K = 1024;
 __device__ __forceinline__ void wgrad_prefetch(const WgradParams& p, long long base, int row0, int n, int lane) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -257,7 +264,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                                         n_idx >= 0 && n_idx < p.num_n_tiles, p.err, kErrCheckTile);
       const int nc = tile_ok && row0 < p.M ? (min(BN, p.N - n0) + 63) / 64 : 0;
       const long long base = layer * p.layer_stride;
-      WgradRegs a, b;
+      WgradRegs<ADAM> a, b;
       if (half < nc) wgrad_fetch<ADAM>(p, a, base, row0, n0 + half * 64, 0, lane);   // under this tile's main loop
       if (ADAM && p.K <= kWgPrefetchK)
         for (int c = half; c < nc; c += 2) wgrad_prefetch(p, base, row0, n0 + c * 64, lane);
@@ -359,6 +366,7 @@ static int wgrad(int dtype, const void* A, long long lda, long long a_stride, co
       !wgrad_tmap(&tmB, B, ldb, b_stride, p.layers, p.N, p.K, bf16))
     return kErrDriver;
   const int BN = choose_wgrad_tile(p.M, p.N, p.K, p.layers, ADAM, num_sms());
+  if (p.accumulate) p.accumulate = p.K <= kWgAddInL2K ? 2 : 1;
   p.num_m_tiles = (p.M + 255) / 256;
   p.num_n_tiles = (p.N + BN - 1) / BN;
   const long long tiles = static_cast<long long>(p.num_m_tiles) * p.num_n_tiles;
