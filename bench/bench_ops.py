@@ -96,6 +96,10 @@ def case_gemm(a):
             err = _rel(dw, dy.float().t() @ x.float())
             print(f"wgrad fc1 over {R} rows tile {tile:4d}: {us:7.1f} us "
                   f"{2 * R * 4 * H * H / us / 1e6:7.1f} TFLOP/s  rel.err {err:.1e}")
+        us = _timeit(lambda: F.weight_grad(dy, x, dw), n=5)      # (what a training step runs)
+        err = _rel(dw, dy.float().t() @ x.float())
+        print(f"weight_grad fc1 over {R} rows: {us:7.1f} us "
+              f"{2 * R * 4 * H * H / us / 1e6:7.1f} TFLOP/s  rel.err {err:.1e}")
         F.check_device_status()
 
 

@@ -139,10 +139,13 @@ inline int num_sms() {
 // successor that allocated all of it first and then waited for that kernel would never end, so the two
 // must not fit on one SM together: every kernel that allocates TMEM before pdl_wait() takes at least
 // kTmemKernelMinSmem of shared memory, and one that allocates it afterwards leaves less than that.
+// In a chain of several (pdl_trigger in ptx.cuh) the argument holds for each pair: dQ and dK/dV have their TMEM before they
+// trigger, so that a later CTA beside one of them waits for TMEM that is given back by a kernel that waits for nothing later;
+// the weight gradients allocate after they trigger, but fill their SM, so that nothing that allocates lies beside them.
 constexpr int kSmemPerSm = 228 * 1024, kTmemKernelMinSmem = 96 * 1024;
 
 // Launch with programmatic stream serialization (see pdl_wait in ptx.cuh).  The kernel must call
-// pdl_wait() in every thread before its first access to global data.  On unless tp_set_pdl(0) was
+// pdl_wait() in every thread before its first access to global data, or keep to what pdl_trigger asks for.  On unless tp_set_pdl(0) was
 // called or the environment variable TERAPIPE_PDL=0 is set at first use: the set-up of a kernel
 // (barriers, TMEM, tensor maps) under the end of its predecessor saves 1 to 2 us a launch, 9 % of a
 // step of the 24-layer test model, 6 % of a 1024-row slice of a 2048-wide layer.  Launches of more

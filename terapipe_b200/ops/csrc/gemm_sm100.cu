@@ -1854,10 +1854,7 @@ static int pick_tile(int M, int N, int K, bool b_mn, bool second, int forced, bo
   float time;
   const int code = choose_tile(M, N, K, b_mn, second, allow_256x256, allow_pair && g_pair_default, allow_cut, num_sms(),
                                &time);
-  if (!allow_small) return code;
-  const bool narrow = choose_narrow(M, N, K, code, num_sms(), &time);
-  const int split = choose_split(M, N, K, time, num_sms());
-  return split ? split : narrow ? 32 : code;
+  return allow_small ? choose_small(M, N, K, code, time, num_sms()) : code;
 }
 
 }  // namespace tp

@@ -53,7 +53,5 @@ int tp_choose_tile(int M, int N, int K, int b_mn, int second, int cut, int sms) 
 extern "C" int tp_choose_small(int M, int N, int K, int b_mn, int second, int sms) {
   float time;
   const int code = tp::choose_tile(M, N, K, b_mn != 0, second != 0, true, true, true, sms, &time);
-  const bool narrow = tp::choose_narrow(M, N, K, code, sms, &time);
-  const int split = tp::choose_split(M, N, K, time, sms);
-  return split ? split : narrow ? 32 : code;
+  return tp::choose_small(M, N, K, code, time, sms);
 }

@@ -35,9 +35,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // attribute (see launch_pdl in common.cuh) may begin while its predecessor in the stream still
 // runs: its CTAs are placed as SMs free up and execute their set-up (barrier initialisation,
 // TMEM allocation, tensor-map prefetch).  pdl_wait() blocks until the predecessor has completed
-// and its memory operations are visible; every thread calls it before it touches global data.
-// The trigger directly after it lets the successor do the same with this kernel, and no
-// earlier, so at most two kernels overlap.  Without the attribute both are no-ops.
+// and its memory operations are visible; every thread calls it before it touches global data (but see
+// pdl_trigger below).  The trigger directly after it lets the successor do the same with this kernel, and no
+// earlier, so that only pdl_trigger's kernels run beside more than one other.  Without the attribute both are no-ops.
 // trigger = false: a kernel that waits for other ranks keeps the SMs to itself and to the small
 // kernels of other streams that its peers wait for; its successor starts when it has ended.
 __device__ __forceinline__ void pdl_wait(bool trigger = true) {
@@ -48,7 +48,9 @@ __device__ __forceinline__ void pdl_wait(bool trigger = true) {
 // Instead of pdl_wait(), in a kernel that reads nothing its predecessor writes and writes nothing that it touches,
 // where the predecessor's CTAs run only after everything before them is done: the kernel starts
 // once they all run, and pdl_wait(false) in one of its threads at its end makes whoever waits for it
-// wait for both.
+// wait for both.  Such kernels form chains (dQ behind dK/dV, the weight gradients of a stage, and the set-up of whatever
+// comes next).  A kernel of a chain starts when all CTAs of the one before it are placed, so that nothing earlier waits for an
+// SM, and it depends on later ones in nothing.  For TMEM see kTmemKernelMinSmem in common.cuh.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ bool elect_one() {

@@ -114,6 +114,13 @@ inline int choose_split(int M, int N, int K, float time, int sms) {
   return best;
 }
 
+// What an ordinary forward or data-gradient product takes instead of choose_tile's `code`, whose estimate is `time`.
+inline int choose_small(int M, int N, int K, int code, float time, int sms) {
+  const bool narrow = choose_narrow(M, N, K, code, sms, &time);
+  const int split = choose_split(M, N, K, time, sms);
+  return split ? split : narrow ? 32 : code;
+}
+
 // Columns of a CTA pair's tile for the weight gradients of `layers` layers in one launch (wgrad_sm100.cu).
 // A wave takes its main loop or, where that is shorter, what its epilogue moves at the copy bandwidth
 // (kilo-cycles of 1.8 GHz: 26 bytes an element with Adam, else the staged stores); the last wave's epilogue is

@@ -7,15 +7,15 @@
 // epilogue of its own; the tiles of all layers fill whole waves but for one.  The layers' buffers lie a
 // constant distance apart, so one 3-D tensor map reaches all of them.
 //
-// 256 rows of 256 columns, 24 layers: 65 us for the products of a layer one by one, 1.5 in these launches;
-// 8192 x 768, 10 layers: 141 and 87.
+// 256 rows of 256 columns, 24 layers: 18 us for the products of a layer one by one, 1.6 in these launches;
+// 8192 x 768, 10 layers: 131 and 87.
 //
 // Adam in the epilogue: 26 bytes a parameter move (12 read, 12 written, the 16-bit copy) instead of the 8
 // of an accumulating gradient and the 34 of a pass over flat buffers, and they move under the main loop of
 // the next tile.  us for the four weights of a layer, rows x width: product + pass / this kernel (of which the
 // bare product):
-//   256 x 256 68.7 / 4.4 (1.5), 8192 x 768 183 / 103 (87), 16384 x 2048 1543 / 1418 (1296), 6144 x 2560
-//   1306 / 901 (717), 16384 x 5120 9248 / 7618 (7210), 4096 x 12288 20970 / 14500 (9960).
+//   256 x 256 22.6 / 4.5 (1.6), 8192 x 768 170 / 105 (87), 16384 x 2048 1804 / 1433 (1254), 6144 x 2560
+//   1232 / 844 (658), 16384 x 5120 10653 / 9057 (8271), 4096 x 12288 26125 / 16440 (12678).
 //
 // The product is the CTA-pair GEMM (two CTAs of a cluster, one 256 x BN tile, see gemm_sm100.cu).
 #include "adam.cuh"
