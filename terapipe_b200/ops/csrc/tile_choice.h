@@ -93,6 +93,8 @@ inline bool choose_narrow(int M, int N, int K, int code, int sms, float* time) {
 //   77 x 768 x 3072 12.3 / 5.9 (8 parts of 64 columns), 16 x 768 x 768 4.7 / 4.1 (4),
 //   128 x 1024 x 4096 15.4 / 7.7 (4), 128 x 2048 x 8192 27.6 / 11.4 (4), 16 x 8192 x 2048 16.5 / 7.5 (2 of 128
 //   columns), 64 x 4096 x 16384 52.6 / 27.9 (4 of 128), 256 x 2048 x 8192 27.9 / 16.3 (2 of 64).
+// (Above 80 rows the ring of a 128-column split is shallow; with weights out of DRAM it is 2 to 10 % slower there than whole K
+// on 64 columns: 80 x 6144 x 8192 30.6 / 27.0, but 104 x 6144 x 8192 31.0 / 34.0.)
 inline int choose_split(int M, int N, int K, float time, int sms) {
   struct Cand { int bn, parts; float ctas, step, base, rows; };   // share of the SMs; per 64 of K; per 128 rows
   constexpr Cand cands[5] = {{64, 2, 1.0f, 0.254f, 4.0f, 1.5f}, {64, 4, 0.87f, 0.254f, 3.3f, 2.5f},
