@@ -69,3 +69,23 @@ def test_engine_made_in_inference_mode(use_graph):
         for name in ("master", "exp_avg", "exp_avg_sq", "model"):
             assert torch.equal(getattr(want, name), getattr(got, name)), name
         got.check_status()
+
+
+@pytest.mark.parametrize("kind", [dict(launch_plan=True, segment_graphs=False), dict(launch_plan=False, segment_graphs=True)])
+def test_writes_count_in_replayed_segments(kind):
+    """Plans and segment graphs keep the adding products apart from those that update."""
+    x, eng = _input(), [_engine(use_graph=False, merge_slices=False, **k) for k in (kind, dict(segment_graphs=False))]
+    assert (eng[0]._plan is not None) == kind["launch_plan"] and (eng[0]._seg_graphs is not None) == kind["segment_graphs"]
+    for i in range(12):
+        for e in eng:
+            e.set_input(x)
+            if i % 3 == 1:
+                _write(e, "kernels", None)
+            if i % 3 == 2:
+                e.compute_grads()
+            e.step()
+    for name in ("master", "exp_avg", "exp_avg_sq", "model"):
+        assert torch.equal(getattr(eng[0], name), getattr(eng[1], name)), name
+    for e in eng:
+        e.check_status()
+        assert e.grad.abs().max().item() == 0
